@@ -721,7 +721,7 @@ __device__ __forceinline__ unsigned long long window_key(const unsigned long lon
 // threads: the body of reproj_kernel, also run as a work unit of batch_kernel.  `maps`: the
 // views' key-tile tensor maps; `bar`: the block's TMA completion barrier, initialised once per
 // thread block; `round`: TMA rounds that barrier has completed so far (its phase carries over
-// from unit to unit); `aborted`: a shared word, 0 when the block starts, that a thread whose
+// from unit to unit, also across units whose tiles came by plain loads); `aborted`: a shared word, 0 when the block starts, that a thread whose
 // wait for the key tiles gave up sets to 1; `block_id`: the index the test hook
 // `withhold_block` refers to, compiled in only where HOOK is set.  Every thread returns
 // together (early exits are block-uniform or come after the last barrier).
@@ -741,7 +741,6 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
     const uint32_t x0 = bx * 32, x = x0 + lane, yb = by * (ROWS * np);
     const bool xok = x < p.out_w;
     const bool leader = lane == 0 && vw == 0;
-    const int round0 = round;
     {
         const DevView &v = p.v[vw];
         const uint32_t ix = v.sx == 1 ? x : x / v.sx, tx0 = v.sx == 1 ? x0 : x0 / v.sx;
@@ -765,10 +764,10 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
             const float qy[ROWS] = {__ldg(v0.lut + v0.w + y0c), __ldg(v0.lut + v0.w + y1c)};
             const float pcy[ROWS] = {__ldg(v.lut + v.w + min(iy0, vhei - 1)), __ldg(v.lut + v.w + min(iy1, vhei - 1))};
 #pragma unroll 1
-        for (int k = 0; k < nf; k++, round++)
+        for (int k = 0; k < nf; k++, round += p.use_tma) // plain loads leave the barrier's phase where it is
         {
             const int u = k * np + rp;
-            if (round > round0)
+            if (rp + k > 0)
                 __syncthreads(); // every warp is done with the previous unit's tiles
             bool arrived = true;
             if (p.use_tma)

@@ -89,6 +89,33 @@ def test_mixed_pairs_chained_equal_render_batch(cuda, mode, units):
     ref.close()
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+def test_pairs_with_tma_and_plain_key_tiles_equal_render_batch(cuda, mode):
+    """Pairs whose key tiles come by TMA (even widths) and by plain loads (odd widths) in one
+    call, an odd number of tile rounds per reprojection block: the units of the former must
+    not lose step with their barrier over the units of the latter."""
+    import torch
+    jobs, wants = [], []
+    ref = Renderer()
+    for i, (w, h) in enumerate([(400, 240), (333, 197), (320, 180), (397, 211), (402, 239)] * 2):
+        seq = scene.Sequence(w, h, 2, seed=4500 + i, max_speed=2.0)
+        clients = [seq.client(0, b, mode=mode) for b in (1, 2, 3)]
+        frame = DeviceFrame.from_host(seq.frame(0))
+        want = [torch.full((h, w, 4), 7, dtype=torch.uint8, device="cuda") for _ in clients]
+        jobs.append(([o.clone() for o in want], clients, frame))
+        ref.render_batch(want, clients, frame, chain=False)
+        wants.append(want)
+    r = Renderer()
+    r.render_pairs(jobs)
+    torch.cuda.synchronize()
+    assert r.device_status() == native.ISTI_OK
+    for i, ((outs, _, _), want) in enumerate(zip(jobs, wants)):
+        for k, (a, b) in enumerate(zip(outs, want)):
+            assert torch.equal(a, b), f"pair {i} frame {k}: {int((a != b).any(-1).sum())} pixels differ"
+    r.close()
+    ref.close()
+
+
 def test_graph_capture_and_uncaptured_calls_alternate(cuda):
     """A captured isti_render_pairs call replays with its own parameters after uncaptured calls
     of the same renderer with other parameters (separate staging buffers)."""
