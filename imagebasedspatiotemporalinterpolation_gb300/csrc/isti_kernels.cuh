@@ -82,6 +82,14 @@ struct DevView
     float vp_self[16];         // this view's viewproj (timewarp)
 };
 
+// Timewarp: the sum of one row of depths and what decides whether sums of it are exact.
+struct TwRow
+{
+    double sum;
+    uint32_t zmax;  // largest |z| of the row (bits)
+    uint32_t e_min; // smallest exponent field of a non-zero z (1 for denormals); 0: the sum is rounded
+};
+
 // Per-frame settings (RenderInfo / AdditionalRenderInfo, include/renderer.h:18-35)
 struct FrameCfg
 {
@@ -96,8 +104,8 @@ struct alignas(16) FrameParams
 {
     float cam_vp[MAX_FRAMES][16];
     float cam_ivp[MAX_FRAMES][16]; // client inverse viewproj (timewarp rays)
-    double *tw_rows;               // timewarp: per-row sums of the forward keyframe's z
-    float *tw_mean;                // timewarp: mean z (the reference's ImageBuffer::average)
+    TwRow *tw_rows;                // timewarp: per-row sums of the forward keyframe's z
+    float4 *tw_plane;              // timewarp: the plane's normal and the mean z (the reference's ImageBuffer::average)
     uint32_t *out[MAX_FRAMES];
     FrameCfg f[MAX_FRAMES];
     size_t key_stride; // elements between frames in the key block
@@ -986,33 +994,100 @@ __global__ void __maxnreg__(REGS) reproj_kernel(const __grid_constant__ FramePar
 // ---- timewarp (mode 4), src/renderer.cu:467-522, 615-629 ----
 //
 // Mean NDC z of the forward keyframe (ImageBuffer::average, src/util/image_buffer.cu:80-100).
-// The reference accumulates with a float atomicAdd in an unspecified order; here every row is
-// summed left to right in double (one thread per row), the rows top to bottom in double, and
-// the total is rounded to float and divided by the pixel count in float like the reference's
-// final division.  The C oracle uses the same order.
-
-__global__ void __launch_bounds__(128) timewarp_rowsum_kernel(const __grid_constant__ FrameParams p)
+// The reference accumulates with a float atomicAdd in an unspecified order; the value defined
+// here (and in the C oracle) is every row summed left to right in double, the rows top to
+// bottom in double, the total rounded to float and divided by the pixel count in float.
+//
+// Where no addition of that order rounds, any order gives the same sum, so the rows are summed
+// in parallel and the order only matters to the sums that do round.  All values are multiples
+// of u, the smallest unit in the last place among the non-zero ones, and no partial sum exceeds
+// n * max|z|; with n * max|z| <= 2^53 u every partial sum is a multiple of u that a double
+// holds exactly.  NDC depths of a 1080p frame meet that for |z| >= 2^-18 (rows) and 2^-9
+// (total); a row or total that does not (and NaN or infinity) is summed in order by one warp.
+// Whether sums of n values of at most |zmax| that are multiples of 2^(e_min - 150) are exact.
+__device__ __forceinline__ bool sums_exact(double n, uint32_t zmax, uint32_t e_min)
 {
-    const DevView &v = p.v[0];
-    const uint32_t y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= v.h)
-        return;
-    double acc = 0.0;
-    for (uint32_t x = 0; x < v.w; x++)
-        acc = __dadd_rn(acc, (double)__ldg(v.z + (y * v.w + x)));
-    p.tw_rows[y] = acc;
+    if (zmax >= 0x7f800000u || e_min == 0u)
+        return false;
+    const double unit53 = __hiloint2double((int)((min(e_min, 255u) - 150u + 53u + 1023u) << 20), 0); // 2^53 units
+    return n * (double)__uint_as_float(zmax) <= unit53;
 }
 
-__global__ void timewarp_mean_kernel(const __grid_constant__ FrameParams p)
+// Adds `count` doubles to acc one after the other; called by a whole warp, element i from
+// get(i).  A warp loads 32 at a time, so only the additions are serial.
+template <class Get>
+__device__ double warp_sum_in_order(double acc, uint32_t count, Get get)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0)
-        return;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t i0 = 0; i0 < count; i0 += 32)
+    {
+        const double v = i0 + lane < count ? get(i0 + lane) : 0.0;
+        const uint32_t n = min(32u, count - i0);
+        for (uint32_t j = 0; j < n; j++)
+            acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, v, (int)j));
+    }
+    return acc;
+}
+
+// Sum, largest |z| and smallest exponent over the block (TW_THREADS threads); valid in thread 0.
+constexpr int TW_THREADS = 128;
+__device__ __forceinline__ void tw_block_reduce(double &sum, uint32_t &zmax, uint32_t &e_min)
+{
+    __shared__ double s_sum[TW_THREADS / 32];
+    __shared__ uint32_t s_max[TW_THREADS / 32], s_min[TW_THREADS / 32];
+    for (int o = 16; o > 0; o >>= 1)
+        sum = __dadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, o));
+    zmax = __reduce_max_sync(0xffffffffu, zmax);
+    e_min = __reduce_min_sync(0xffffffffu, e_min);
+    if ((threadIdx.x & 31u) == 0u)
+    {
+        s_sum[threadIdx.x >> 5] = sum;
+        s_max[threadIdx.x >> 5] = zmax;
+        s_min[threadIdx.x >> 5] = e_min;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = 1; k < TW_THREADS / 32; k++)
+        {
+            sum = __dadd_rn(sum, s_sum[k]);
+            zmax = max(zmax, s_max[k]);
+            e_min = min(e_min, s_min[k]);
+        }
+}
+
+// One block per row, so that a row's loads are coalesced and in flight together (4 bytes a
+// pixel, each read once).  With one thread per row summing in order the two sums took 235 and
+// 65 us of a 1080p call; the whole call went from 289 to 43 us.
+__global__ void __launch_bounds__(TW_THREADS) timewarp_rowsum_kernel(const __grid_constant__ FrameParams p)
+{
     const DevView &v = p.v[0];
+    const float *row = v.z + (size_t)blockIdx.x * v.w;
     double acc = 0.0;
-    for (uint32_t y = 0; y < v.h; y++)
-        acc = __dadd_rn(acc, p.tw_rows[y]);
-    *p.tw_mean = xdiv(__double2float_rn(acc), (float)(v.w * v.h));
-    *p.status = 0;
+    uint32_t zmax = 0u, e_min = 255u;
+#pragma unroll 4
+    for (uint32_t x = threadIdx.x; x < v.w; x += TW_THREADS)
+    {
+        const float z = __ldg(row + x);
+        const uint32_t a = __float_as_uint(z) & 0x7fffffffu;
+        acc = __dadd_rn(acc, (double)z);
+        zmax = max(zmax, a);
+        if (a != 0u)
+            e_min = min(e_min, max(1u, a >> 23));
+    }
+    tw_block_reduce(acc, zmax, e_min);
+    __shared__ bool exact;
+    if (threadIdx.x == 0)
+    {
+        exact = sums_exact((double)v.w, zmax, e_min);
+        if (exact)
+            p.tw_rows[blockIdx.x] = TwRow{acc, zmax, e_min};
+    }
+    __syncthreads();
+    if (exact || threadIdx.x >= 32)
+        return;
+    acc = warp_sum_in_order(0.0, v.w, [&](uint32_t x) { return (double)__ldg(row + x); });
+    if (threadIdx.x == 0)
+        p.tw_rows[blockIdx.x] = TwRow{acc, 0u, 0u};
 }
 
 __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz)
@@ -1020,11 +1095,47 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
     return xadd(xadd(xmul(ax, bx), xmul(ay, by)), xmul(az, bz));
 }
 
-// timewarp_kernel body for one pixel and client camera; false: the ray is parallel to the plane (no write)
-__device__ __forceinline__ bool timewarp_pixel(const float *cam_ivp, const DevView &to, const DevView &aux, bool has_aux, float depth_to,
-                                               uint32_t x, uint32_t y, uint32_t out_w, uint32_t out_h, uint32_t &color)
+// One block: the mean, and the plane it defines -- through inv_viewproj_mat_to[3], facing the
+// centre of the keyframe at the mean depth -- whose normal is the same for every pixel.
+__global__ void __launch_bounds__(TW_THREADS) timewarp_mean_kernel(const __grid_constant__ FrameParams p)
 {
-    const float2 pcs = pixel2cs(x, y, out_w, out_h);
+    const DevView &to = p.v[0];
+    double acc = 0.0;
+    uint32_t zmax = 0u, e_min = 255u;
+#pragma unroll 4
+    for (uint32_t y = threadIdx.x; y < to.h; y += TW_THREADS)
+    {
+        const TwRow r = p.tw_rows[y];
+        acc = __dadd_rn(acc, r.sum);
+        zmax = max(zmax, r.zmax);
+        e_min = min(e_min, r.e_min);
+    }
+    tw_block_reduce(acc, zmax, e_min);
+    __shared__ bool exact;
+    if (threadIdx.x == 0)
+        exact = sums_exact((double)to.w * (double)to.h, zmax, e_min);
+    __syncthreads();
+    if (threadIdx.x >= 32)
+        return;
+    if (!exact)
+        acc = warp_sum_in_order(0.0, to.h, [&](uint32_t y) { return p.tw_rows[y].sum; });
+    if (threadIdx.x != 0)
+        return;
+    const float depth_to = xdiv(__double2float_rn(acc), (float)(to.w * to.h));
+    const float4 cws = project(to.inv_vp, make_float4(0.0f, 0.0f, depth_to, 1.0f));
+    const float cpx = to.inv_vp[12], cpy = to.inv_vp[13], cpz = to.inv_vp[14], cpw = to.inv_vp[15];
+    const float nx = xsub(cws.x, cpx), ny = xsub(cws.y, cpy), nz = xsub(cws.z, cpz);
+    const float nw = xsub(cws.w, cpw);
+    const float sn = xdiv(1.0f, xsqrt(xadd(dot3(nx, ny, nz, nx, ny, nz), xmul(nw, nw)))); // 4-component normalize
+    *p.tw_plane = make_float4(xmul(nx, sn), xmul(ny, sn), xmul(nz, sn), depth_to);
+    *p.status = 0;
+}
+
+// timewarp_kernel body for one pixel (pixel2CS pcs) and client camera on the plane with normal n;
+// false: the ray is parallel to the plane (no write)
+__device__ __forceinline__ bool timewarp_pixel(const float *cam_ivp, const DevView &to, const DevView &aux, bool has_aux, float4 n, float2 pcs,
+                                               uint32_t &color)
+{
     const float4 nws = project(cam_ivp, make_float4(pcs.x, pcs.y, 0.0f, 1.0f));
     const float4 fws = project(cam_ivp, make_float4(pcs.x, pcs.y, 1.0f, 1.0f));
     // ray_dir = normalize(vec3(farWS - nearWS)), glm-subset normalize: v * (1 / sqrt(dot(v, v)))
@@ -1033,19 +1144,11 @@ __device__ __forceinline__ bool timewarp_pixel(const float *cam_ivp, const DevVi
     dx = xmul(dx, sd);
     dy = xmul(dy, sd);
     dz = xmul(dz, sd);
-    // plane through inv_viewproj_mat_to[3] facing the centre of the keyframe at depth_to
-    const float4 cws = project(to.inv_vp, make_float4(0.0f, 0.0f, depth_to, 1.0f));
-    const float cpx = to.inv_vp[12], cpy = to.inv_vp[13], cpz = to.inv_vp[14], cpw = to.inv_vp[15];
-    float nx = xsub(cws.x, cpx), ny = xsub(cws.y, cpy), nz = xsub(cws.z, cpz);
-    const float nw = xsub(cws.w, cpw);
-    const float sn = xdiv(1.0f, xsqrt(xadd(dot3(nx, ny, nz, nx, ny, nz), xmul(nw, nw)))); // 4-component normalize
-    nx = xmul(nx, sn);
-    ny = xmul(ny, sn);
-    nz = xmul(nz, sn);
-    const float denom = dot3(dx, dy, dz, nx, ny, nz);
+    const float cpx = to.inv_vp[12], cpy = to.inv_vp[13], cpz = to.inv_vp[14];
+    const float denom = dot3(dx, dy, dz, n.x, n.y, n.z);
     if (fabsf(denom) < 1e-6f)
         return false;
-    const float t = xdiv(dot3(xsub(cpx, nws.x), xsub(cpy, nws.y), xsub(cpz, nws.z), nx, ny, nz), denom);
+    const float t = xdiv(dot3(xsub(cpx, nws.x), xsub(cpy, nws.y), xsub(cpz, nws.z), n.x, n.y, n.z), denom);
     const float4 hit = make_float4(xadd(nws.x, xmul(t, dx)), xadd(nws.y, xmul(t, dy)), xadd(nws.z, xmul(t, dz)), 1.0f);
     const float4 pc = project(to.vp_self, hit); // WS2CS(intersection, viewproj_mat_to)
     int2 pix = cs2pixel(pc.x, pc.y, to.w, to.h);
@@ -1065,17 +1168,23 @@ __device__ __forceinline__ bool timewarp_pixel(const float *cam_ivp, const DevVi
 // One thread per output pixel, looping over the frames of the batch (chained like the reprojection).
 __global__ void __launch_bounds__(256) timewarp_kernel(const __grid_constant__ FrameParams p)
 {
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
+    // pixel2CS of the block's columns and rows: one division each instead of two per pixel
+    __shared__ float2 pcs[32];
+    const uint32_t x = blockIdx.x * 32 + threadIdx.x;
+    const uint32_t y = blockIdx.y * 8 + threadIdx.y;
+    if (threadIdx.y == 0)
+        pcs[threadIdx.x] = pixel2cs(x, blockIdx.y * 8 + (threadIdx.x & 7u), p.out_w, p.out_h); // .x: column; .y: row (first 8)
+    __syncthreads();
     if (x >= p.out_w || y >= p.out_h)
         return;
     const bool has_aux = p.n_aux > 0;
-    const float depth_to = *p.tw_mean;
+    const float4 plane = *p.tw_plane;
+    const float2 pixel = make_float2(pcs[threadIdx.x].x, pcs[threadIdx.y].y);
     uint32_t run = 0;
     for (int k = 0; k < p.n_frames; k++)
     {
         uint32_t color = 0;
-        const bool ok = timewarp_pixel(p.cam_ivp[k], p.v[0], p.v[has_aux ? 2 : 0], has_aux, depth_to, x, y, p.out_w, p.out_h, color);
+        const bool ok = timewarp_pixel(p.cam_ivp[k], p.v[0], p.v[has_aux ? 2 : 0], has_aux, plane, pixel, color);
         uint32_t *o = p.out[k] + (y * p.out_w + x);
         if (!p.chain)
         {

@@ -20,10 +20,10 @@ namespace isti
 // keyframe (two kernels), then one kernel over the output pixels.
 cudaError_t launch_timewarp(isti::FrameParams &p, char *base, cudaStream_t stream, cudaEvent_t after_mean, cudaEvent_t after_nothing)
 {
-    p.tw_rows = reinterpret_cast<double *>(base);
-    p.tw_mean = reinterpret_cast<float *>(base + ((size_t)p.v[0].h * sizeof(double) + 255) / 256 * 256);
-    isti::timewarp_rowsum_kernel<<<(p.v[0].h + 127) / 128, 128, 0, stream>>>(p);
-    isti::timewarp_mean_kernel<<<1, 32, 0, stream>>>(p);
+    p.tw_rows = reinterpret_cast<isti::TwRow *>(base);
+    p.tw_plane = reinterpret_cast<float4 *>(base + ((size_t)p.v[0].h * sizeof(isti::TwRow) + 255) / 256 * 256);
+    isti::timewarp_rowsum_kernel<<<p.v[0].h, isti::TW_THREADS, 0, stream>>>(p);
+    isti::timewarp_mean_kernel<<<1, isti::TW_THREADS, 0, stream>>>(p);
     if (after_mean)
         cudaEventRecord(after_mean, stream);
     if (after_nothing)

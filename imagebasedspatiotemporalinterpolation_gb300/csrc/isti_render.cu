@@ -195,12 +195,12 @@ Layout layout_of(const isti_view *const *views, int n_views, int n_frames)
     return l;
 }
 
-// Timewarp (mode 4) needs no splat intermediates: [row sums, double per row of the
-// forward keyframe][mean z][status word].
+// Timewarp (mode 4) needs no splat intermediates: [row sums, one TwRow per row of the
+// forward keyframe][plane and mean z][status word].
 Layout timewarp_layout(const isti_view *const *views)
 {
     Layout l{};
-    l.total = align_up((size_t)views[0]->height * sizeof(double), 256) + 256 + STATUS_BYTES;
+    l.total = align_up((size_t)views[0]->height * sizeof(isti::TwRow), 256) + 256 + STATUS_BYTES;
     return l;
 }
 
@@ -682,7 +682,7 @@ isti_status isti_renderer_view_buffers(const isti_renderer *r, int32_t view, con
         return fail(ISTI_ERR_INVALID_ARG, "view index out of range");
     const int k = view / nv;
     const isti::DevView &d = r->last.v[view % nv];
-    const bool materialised = r->last.tw_mean == nullptr; // timewarp keeps no splat intermediates
+    const bool materialised = r->last.tw_plane == nullptr; // timewarp keeps no splat intermediates
     if (splat)
         *splat = materialised ? reinterpret_cast<const uint64_t *>(d.splat + k * r->last.key_stride) : nullptr;
     if (cam_xy)
@@ -705,7 +705,7 @@ isti_status isti_renderer_view_depth(const isti_renderer *r, int32_t view, const
         return fail(ISTI_ERR_INVALID_ARG, "view index out of range");
     const int k = view / nv;
     const isti::DevView &d = r->last.v[view % nv];
-    const bool materialised = r->last.tw_mean == nullptr;
+    const bool materialised = r->last.tw_plane == nullptr;
     if (cam_depth)
         *cam_depth = materialised && d.cam_depth ? d.cam_depth + k * r->last.depth_stride : nullptr;
     if (visible)
@@ -1073,7 +1073,7 @@ extern "C" isti_status isti_learned_labels(isti_renderer *r, int32_t frame_index
 {
     if (!r || !labels || ((uintptr_t)labels & 15u))
         return fail(ISTI_ERR_INVALID_ARG, "NULL or unaligned argument");
-    if (!r->has_frame || r->last.tw_mean != nullptr || r->last.n_aux != 0 || r->last.linear)
+    if (!r->has_frame || r->last.tw_plane != nullptr || r->last.n_aux != 0 || r->last.linear)
         return fail(ISTI_ERR_INVALID_ARG, "labels need a preceding plain render (main camera only, modes 0/2/3)");
     if (frame_index < 0 || frame_index >= r->last.n_frames)
         return fail(ISTI_ERR_INVALID_ARG, "frame index out of range");

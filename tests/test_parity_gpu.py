@@ -97,6 +97,34 @@ def test_timewarp_matches_oracle_1080p(cuda, aux):
     r.close()
 
 
+@pytest.mark.parametrize("size", [(333, 197), (96, 64), (31, 5), (640, 1)], ids=lambda s: f"{s[0]}x{s[1]}")
+@pytest.mark.parametrize("kind", ["exact", "row", "total", "zeros"])
+def test_timewarp_mean_is_summed_in_order_where_order_matters(cuda, size, kind):
+    """The mean depth is the in-order double sum: rows and totals whose additions round (values
+    that absorb others and cancel later) give what the oracle's order gives, not another order's."""
+    import torch
+    w, h = size
+    seq = Sequence(w, h, 2, seed=708)
+    frame = seq.frame(0)
+    z = np.random.default_rng(5).uniform(0.2, 0.95, (h, w)).astype(np.float32)
+    big = np.float32(2.0 ** 60)
+    if kind == "row":      # every row: what lies between +2^60 and -2^60 is absorbed
+        z[:, w // 5], z[:, w - w // 4] = big, -big
+    elif kind == "total":  # rows of equal values sum exactly, the rows between +2^60 and -2^60 are absorbed
+        z[0], z[-1 - h // 8] = big, -big
+    elif kind == "zeros":
+        z[:] = np.where(z > 0.5, np.float32(0.0), np.float32(-0.0))
+    frame.fwd.z = z
+    client = seq.client(0, 2, mode=native.MODE_TIMEWARP)
+    prev = np.full((h, w, 4), 11, np.uint8)
+    out = torch.from_numpy(prev.copy()).cuda()
+    r = Renderer()
+    r.render(out, client, DeviceFrame.from_host(frame))
+    exp = oracle.run_oracle(frame, client, prev, with_intermediates=False)[0]
+    assert np.array_equal(out.cpu().numpy(), exp)
+    r.close()
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2, 3])
 @pytest.mark.parametrize("b", [1, 2, 3])
 def test_oracle_parity_640x360_main_only(cuda, mode, b):
