@@ -2,7 +2,7 @@
 // the reference's evaluation script (scripts/eval.py:66-132,
 // scripts/loss_utils.py:17-57), as two kernels.
 //
-// quality_tile_kernel: one block per 32x16 output tile.  For each colour
+// quality_tile_kernel: one block per 32x32 output tile.  For each colour
 // channel the tile plus a 5-pixel halo of both images is staged in shared
 // memory as floats in [0, 1] (zero outside the image: the reference's zero
 // padding), the five moments x, y, x^2, y^2, xy are filtered horizontally
@@ -24,122 +24,183 @@
 
 namespace
 {
-constexpr int TW = 32, TH = 16, R = 5, WIN = 2 * R + 1;
+constexpr int TW = 32, TH = 32, R = 5, WIN = 2 * R + 1;
 constexpr int SW = TW + 2 * R, SH = TH + 2 * R;
-constexpr int THREADS = 256; // 32 x 8: each thread owns one column and two rows of the tile
+constexpr int THREADS = 256;   // final kernels, FLIP tiles
+constexpr int Q_THREADS = 128; // SSIM tiles
 
 struct Gauss
 {
-    float g[WIN];
+    float2 g[WIN]; // each tap twice: the packed operations take a pair
 };
 
-__global__ void __launch_bounds__(THREADS) quality_tile_kernel(const uint32_t *__restrict__ a, const uint32_t *__restrict__ b,
-                                                               int w, int h, double *__restrict__ partials, const Gauss gw)
+// Running sum of floats as an unevaluated pair: the rounding error of every addition is kept
+// (Knuth's two-sum), so the pair is as exact as a double sum without the few FP64 units.
+struct PairSum
 {
-    __shared__ float xs[SH][SW], ys[SH][SW];
-    __shared__ float hm[5][SH][TW]; // horizontally filtered x, y, x^2, y^2, xy
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
-    double ssim_sum = 0.0;
-    unsigned long long sq_sum = 0;
+    float hi = 0.0f, lo = 0.0f;
+    __device__ __forceinline__ void add(float v)
+    {
+        const float s = __fadd_rn(hi, v), t = __fsub_rn(s, hi);
+        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(v, t)));
+        hi = s;
+    }
+    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+};
 
+// v / 255 for an integer v in 0..255, correctly rounded: the product with RN(1 / 255) corrected
+// by its exact remainder (Markstein's division step; equal to the division for all 256 values).
+__device__ __forceinline__ float byte_to_unit(uint32_t v)
+{
+    const float f = (float)v, q = __fmul_rn(f, 1.0f / 255.0f);
+    return fmaf(fmaf(-q, 255.0f, f), 1.0f / 255.0f, q);
+}
+
+// Both passes are bound by FMA issue and shared-memory reads, so a thread filters several
+// neighbouring outputs from one set of reads (4 along a row, then 8 down a column), and the
+// images' moments travel as pairs (x, y), (x^2, y^2) through the packed fma.rn.f32x2.  Rows
+// are spread over the lanes in the horizontal pass: the pitches (21 and 17 sixteen-byte words,
+// 9 for the single plane) are odd, so their 16-byte accesses meet no bank conflict.
+// 1080p: 112 -> 66 us (one output per thread and pass, 32x16 tiles, scalar operations before).
+constexpr int Q_PITCH = TW + 2, Q_PITCH1 = TW + 4;
+__global__ void __launch_bounds__(Q_THREADS) quality_tile_kernel(const uint32_t *__restrict__ a, const uint32_t *__restrict__ b, int w,
+                                                                 int h, double *__restrict__ partials, const __grid_constant__ Gauss gw)
+{
+    __shared__ __align__(16) float2 xy[SH * SW];
+    __shared__ __align__(16) float2 hm[SH * Q_PITCH], hq[SH * Q_PITCH]; // horizontally filtered (x, y) and (x^2, y^2)
+    __shared__ __align__(16) float hc[SH * Q_PITCH1];                   // and xy
+    constexpr int PER = (SH * SW + Q_THREADS - 1) / Q_THREADS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
+
+    uint32_t pa[PER], pb[PER]; // this thread's staged pixels, read once for the three channels
+    uint32_t sq = 0;
+#pragma unroll
+    for (int i = 0; i < PER; i++)
+    {
+        const int e = tid + i * Q_THREADS, yy = e / SW, xx = e % SW;
+        const int gx = x0 + xx - R, gy = y0 + yy - R;
+        pa[i] = pb[i] = 0u;
+        if (e < SH * SW && gx >= 0 && gx < w && gy >= 0 && gy < h)
+        {
+            const size_t idx = (size_t)gy * w + gx;
+            pa[i] = __ldg(a + idx);
+            pb[i] = __ldg(b + idx);
+            if (xx >= R && xx < R + TW && yy >= R && yy < R + TH)
+            {
+                const uint32_t d = __vabsdiffu4(pa[i], pb[i]) & 0xffffffu;
+                sq = __dp4a(d, d, sq);
+            }
+        }
+    }
+    PairSum ssim;
+#pragma unroll 1
     for (int c = 0; c < 3; c++)
     {
         const int shift = 8 * c;
-        for (int i = tid; i < SH * SW; i += THREADS)
+#pragma unroll
+        for (int i = 0; i < PER; i++)
+            if (tid + i * Q_THREADS < SH * SW)
+                xy[tid + i * Q_THREADS] = make_float2(byte_to_unit((pa[i] >> shift) & 255u), byte_to_unit((pb[i] >> shift) & 255u));
+        __syncthreads();
+#pragma unroll 1
+        for (int i = tid; i < SH * (TW / 4); i += Q_THREADS)
         {
-            const int yy = i / SW, xx = i % SW;
-            const int gx = x0 + xx - R, gy = y0 + yy - R;
-            float va = 0.0f, vb = 0.0f;
-            if (gx >= 0 && gx < w && gy >= 0 && gy < h)
+            const int col = i / SH * 4, row = i % SH;
+            const float4 *src = reinterpret_cast<const float4 *>(xy + row * SW + col);
+            float2 m[4] = {}, q[4] = {};
+            float x12[4] = {};
+#pragma unroll
+            for (int t = 0; t < WIN + 3; t += 2)
             {
-                const size_t idx = (size_t)gy * w + gx;
-                va = __fdiv_rn((float)((__ldg(a + idx) >> shift) & 255u), 255.0f);
-                vb = __fdiv_rn((float)((__ldg(b + idx) >> shift) & 255u), 255.0f);
+                const float4 two = src[t / 2];
+                const float2 v[2] = {make_float2(two.x, two.y), make_float2(two.z, two.w)};
+#pragma unroll
+                for (int s = 0; s < 2; s++)
+                {
+                    const float2 v2 = __fmul2_rn(v[s], v[s]);
+                    const float vc = v[s].x * v[s].y;
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                    {
+                        const int k = t + s - j;
+                        if (k < 0 || k >= WIN)
+                            continue;
+                        m[j] = __ffma2_rn(gw.g[k], v[s], m[j]);
+                        q[j] = __ffma2_rn(gw.g[k], v2, q[j]);
+                        x12[j] = fmaf(gw.g[k].x, vc, x12[j]);
+                    }
+                }
             }
-            xs[yy][xx] = va;
-            ys[yy][xx] = vb;
+            float4 *om = reinterpret_cast<float4 *>(hm + row * Q_PITCH + col), *oq = reinterpret_cast<float4 *>(hq + row * Q_PITCH + col);
+            om[0] = make_float4(m[0].x, m[0].y, m[1].x, m[1].y);
+            om[1] = make_float4(m[2].x, m[2].y, m[3].x, m[3].y);
+            oq[0] = make_float4(q[0].x, q[0].y, q[1].x, q[1].y);
+            oq[1] = make_float4(q[2].x, q[2].y, q[3].x, q[3].y);
+            *reinterpret_cast<float4 *>(hc + row * Q_PITCH1 + col) = make_float4(x12[0], x12[1], x12[2], x12[3]);
         }
         __syncthreads();
-        for (int i = tid; i < SH * TW; i += THREADS)
-        {
-            const int row = i / TW, col = i % TW;
-            float s1 = 0.f, s2 = 0.f, s11 = 0.f, s22 = 0.f, s12 = 0.f;
+        constexpr int ROWS_EACH = TH / (Q_THREADS / 32);
+        float2 m[ROWS_EACH] = {}, q[ROWS_EACH] = {};
+        float x12[ROWS_EACH] = {};
 #pragma unroll
-            for (int k = 0; k < WIN; k++)
+        for (int t = 0; t < ROWS_EACH + WIN - 1; t++)
+        {
+            const int row = warp * ROWS_EACH + t;
+            const float2 vm = hm[row * Q_PITCH + lane], vq = hq[row * Q_PITCH + lane];
+            const float vc = hc[row * Q_PITCH1 + lane];
+#pragma unroll
+            for (int j = 0; j < ROWS_EACH; j++)
             {
-                const float g = gw.g[k], x = xs[row][col + k], y = ys[row][col + k];
-                s1 = fmaf(g, x, s1);
-                s2 = fmaf(g, y, s2);
-                s11 = fmaf(g, x * x, s11);
-                s22 = fmaf(g, y * y, s22);
-                s12 = fmaf(g, x * y, s12);
+                const int k = t - j;
+                if (k < 0 || k >= WIN)
+                    continue;
+                m[j] = __ffma2_rn(gw.g[k], vm, m[j]);
+                q[j] = __ffma2_rn(gw.g[k], vq, q[j]);
+                x12[j] = fmaf(gw.g[k].x, vc, x12[j]);
             }
-            hm[0][row][col] = s1;
-            hm[1][row][col] = s2;
-            hm[2][row][col] = s11;
-            hm[3][row][col] = s22;
-            hm[4][row][col] = s12;
         }
-        __syncthreads();
-        const int tx = threadIdx.x;
 #pragma unroll
-        for (int r = 0; r < 2; r++)
+        for (int j = 0; j < ROWS_EACH; j++)
         {
-            const int oy = threadIdx.y * 2 + r;
-            const int gx = x0 + tx, gy = y0 + oy;
-            if (gx >= w || gy >= h)
+            if (x0 + lane >= w || y0 + warp * ROWS_EACH + j >= h)
                 continue;
-            float m1 = 0.f, m2 = 0.f, e11 = 0.f, e22 = 0.f, e12 = 0.f;
-#pragma unroll
-            for (int k = 0; k < WIN; k++)
-            {
-                const float g = gw.g[k];
-                m1 = fmaf(g, hm[0][oy + k][tx], m1);
-                m2 = fmaf(g, hm[1][oy + k][tx], m2);
-                e11 = fmaf(g, hm[2][oy + k][tx], e11);
-                e22 = fmaf(g, hm[3][oy + k][tx], e22);
-                e12 = fmaf(g, hm[4][oy + k][tx], e12);
-            }
             constexpr float C1 = 0.01f * 0.01f, C2 = 0.03f * 0.03f;
-            const float m1s = m1 * m1, m2s = m2 * m2, m12 = m1 * m2;
-            const float v1 = e11 - m1s, v2 = e22 - m2s, v12 = e12 - m12;
+            const float m1s = m[j].x * m[j].x, m2s = m[j].y * m[j].y, m12 = m[j].x * m[j].y;
+            const float v1 = q[j].x - m1s, v2 = q[j].y - m2s, v12 = x12[j] - m12;
             const float num = (2.0f * m12 + C1) * (2.0f * v12 + C2);
             const float den = (m1s + m2s + C1) * (v1 + v2 + C2);
-            ssim_sum += (double)__fdiv_rn(num, den);
-            const size_t idx = (size_t)gy * w + gx;
-            const int d = (int)((__ldg(a + idx) >> shift) & 255u) - (int)((__ldg(b + idx) >> shift) & 255u);
-            sq_sum += (unsigned long long)(d * d);
+            ssim.add(__fdiv_rn(num, den));
         }
-        __syncthreads();
+        // the next channel's staging writes xy, which every thread has read before the last
+        // barrier; its horizontal pass writes hm, hq and hc after the next one
     }
 
     // block reduction (warp shuffles, then one value per warp)
+    double ssim_sum = ssim.value();
     for (int o = 16; o > 0; o >>= 1)
-    {
         ssim_sum += __shfl_down_sync(0xffffffffu, ssim_sum, o);
-        sq_sum += __shfl_down_sync(0xffffffffu, sq_sum, o);
-    }
-    __shared__ double ws[THREADS / 32];
-    __shared__ unsigned long long wq[THREADS / 32];
-    if ((tid & 31) == 0)
+    sq = __reduce_add_sync(0xffffffffu, sq); // a tile has 1024 pixels: 1024 * 3 * 65025 < 2^32
+    __shared__ double ws[Q_THREADS / 32];
+    __shared__ uint32_t wq[Q_THREADS / 32];
+    if (lane == 0)
     {
-        ws[tid >> 5] = ssim_sum;
-        wq[tid >> 5] = sq_sum;
+        ws[warp] = ssim_sum;
+        wq[warp] = sq;
     }
     __syncthreads();
     if (tid == 0)
     {
         double s = 0.0;
         unsigned long long q = 0;
-        for (int k = 0; k < THREADS / 32; k++)
+        for (int k = 0; k < Q_THREADS / 32; k++)
         {
             s += ws[k];
             q += wq[k];
         }
         const size_t blk = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
         partials[2 * blk] = s;
-        partials[2 * blk + 1] = (double)q; // exact: at most 3 * 512 * 65025 per block
+        partials[2 * blk + 1] = (double)q; // exact: at most 3 * 1024 * 65025 per block
     }
 }
 
@@ -186,19 +247,39 @@ __global__ void __launch_bounds__(THREADS) quality_final_kernel(const double *__
 
 constexpr int FR_MAX = ISTI_FLIP_MAX_RADIUS;
 constexpr int FTAPS = 2 * FR_MAX + 1;
-constexpr int FTW = 32, FTH = 16;
+constexpr int FGROUPS_MAX = (FTAPS + 3) / 4; // taps are applied in groups of 4, the last one padded with zeros
+constexpr int FTW = 32, FTH = 32;
+
+enum FlipFilter
+{
+    CSF_A,   // achromatic CSF, 1-D factor
+    CSF_RG,  // red-green CSF
+    CSF_BY1, // blue-yellow CSF = by1(x) by1(y) + by2(x) by2(y)
+    CSF_BY2,
+    GAUSS,   // feature detectors: normalised Gaussian factor
+    EDGE,    // d/dx factor of the edge detector
+    POINT,   // d2/dx2 factor of the point detector
+    N_FLIP_FILTERS
+};
 
 struct FlipFilters
 {
-    int r;                     // common radius of every 1-D filter
-    float csf_a[FTAPS];        // achromatic CSF, 1-D factor
-    float csf_rg[FTAPS];       // red-green CSF
-    float csf_by1[FTAPS];      // blue-yellow CSF = by1(x) by1(y) + by2(x) by2(y)
-    float csf_by2[FTAPS];
-    float gauss[FTAPS];        // feature detectors: normalised Gaussian factor
-    float edge[FTAPS];         // d/dx factor of the edge detector
-    float point[FTAPS];        // d2/dx2 factor of the point detector
-    float cmax;                // maximum HyAB^qc (green vs blue), redistribute_errors
+    int r;      // common radius of every 1-D filter
+    int groups; // groups of 4 taps: (2 r + 1) rounded up
+    float cmax; // maximum HyAB^qc (green vs blue), redistribute_errors
+    float2 tap[N_FLIP_FILTERS][4 * FGROUPS_MAX]; // tap k (offset k - r) twice, for the packed operations; zeros past 2 r
+};
+
+// Shared memory of a FLIP tile: three input planes (Y or the normalised Y, Cx, Cz) of (reference,
+// test) pairs, two buffers of horizontally filtered rows, the sRGB table.
+struct FlipTile
+{
+    int sh, pitch, hrows; // input rows; input pitch; rows of a filtered buffer (padded taps read past sh)
+    __host__ __device__ explicit FlipTile(int r, int groups) : sh(FTH + 2 * r), pitch(FTW + 4 * groups + 2), hrows(FTH + 4 * groups) {}
+    __host__ __device__ int plane() const { return sh * pitch; }
+    __host__ __device__ int hplane() const { return hrows * FH_PITCH; }
+    __host__ __device__ size_t bytes() const { return (size_t)(3 * plane() + 2 * hplane()) * sizeof(float2) + 256 * sizeof(float); }
+    static constexpr int FH_PITCH = FTW + 2;
 };
 
 constexpr float FLIP_QC = 0.7f, FLIP_QF = 0.5f, FLIP_PC = 0.4f, FLIP_PT = 0.95f, FLIP_EPS = 1e-15f;
@@ -215,17 +296,17 @@ __device__ __forceinline__ float3 lin_to_xyz_scaled(float r, float g, float b)
                        (L2X[2][0] * r + L2X[2][1] * g + L2X[2][2] * b) * 0.918357670f);
 }
 
-// sRGB byte -> YCxCz (color_space_transform 'srgb2ycxcz'): Y, Cx, Cz
-__device__ __forceinline__ float3 srgb8_to_ycxcz(uint32_t p)
+// sRGB byte -> linear
+__device__ __forceinline__ float srgb8_to_linear(uint32_t byte)
 {
-    float c[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-    {
-        const float v = (float)((p >> (8 * k)) & 255u) / 255.0f;
-        c[k] = v > 0.04045f ? powf((fmaxf(v, 0.04045f) + 0.055f) / 1.055f, 2.4f) : v / 12.92f;
-    }
-    const float3 xyz = lin_to_xyz_scaled(c[0], c[1], c[2]);
+    const float v = (float)byte / 255.0f;
+    return v > 0.04045f ? powf((fmaxf(v, 0.04045f) + 0.055f) / 1.055f, 2.4f) : v / 12.92f;
+}
+
+// sRGB pixel -> YCxCz (color_space_transform 'srgb2ycxcz'): Y, Cx, Cz; lin: srgb8_to_linear of every byte
+__device__ __forceinline__ float3 srgb8_to_ycxcz(uint32_t p, const float *lin)
+{
+    const float3 xyz = lin_to_xyz_scaled(lin[p & 255u], lin[(p >> 8) & 255u], lin[(p >> 16) & 255u]);
     return make_float3(116.0f * xyz.y - 16.0f, 500.0f * (xyz.x - xyz.y), 200.0f * (xyz.y - xyz.z));
 }
 
@@ -251,115 +332,195 @@ __device__ __forceinline__ float3 ycxcz_to_hunt_lab(float Y, float Cx, float Cz)
     return make_float3(L, 0.01f * L * a, 0.01f * L * b);
 }
 
-// One block per 32x16 output tile; both images in turn: stage Y, Cx, Cz and the
-// normalised Y of the tile plus an R-pixel replicate-padded halo, filter rows
-// (7 outputs), then columns per output pixel; then combine per pixel.
-__global__ void __launch_bounds__(THREADS) flip_tile_kernel(const uint32_t *__restrict__ test, const uint32_t *__restrict__ ref, int w,
-                                                            int h, const __grid_constant__ FlipFilters f, double *__restrict__ partials,
-                                                            float *__restrict__ map)
+// The horizontal pass of NF filters over one plane: a thread filters 4 neighbouring outputs of a
+// row from one window of the row, 4 taps at a time.
+template <int NF>
+__device__ __forceinline__ void flip_rows(const FlipFilters &f, const FlipTile &t, const float2 *plane, const FlipFilter (&which)[NF],
+                                          float2 *const (&out)[NF])
 {
-    extern __shared__ float fsm[];
-    const int R = f.r, SW = FTW + 2 * R, SH = FTH + 2 * R;
-    float *pin = fsm;                     // [4][SH][SW]: Y, Cx, Cz, (Y + 16) / 116
-    float *hor = fsm + 4 * SH * SW;       // [7][SH][FTW]
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    const int x0 = blockIdx.x * FTW, y0 = blockIdx.y * FTH;
-    const int tx = threadIdx.x;
-    float Lab[2][2][3], en[2][2], pn[2][2]; // [image][row]
-
-#pragma unroll
-    for (int im = 0; im < 2; im++)
+#pragma unroll 1
+    for (int i = threadIdx.x; i < t.sh * (FTW / 4); i += THREADS)
     {
-        const uint32_t *src = im == 0 ? ref : test;
-        for (int i = tid; i < SH * SW; i += THREADS)
+        // lanes take different rows: pitches of an odd number of 16-byte words, no bank conflicts
+        const int g = i / t.sh, row = i - g * t.sh;
+        const float4 *src = reinterpret_cast<const float4 *>(plane + row * t.pitch + 4 * g);
+        float2 acc[NF][4] = {}, v[8];
+        auto load = [&](int at, int n) {
+            const float4 a = src[2 * n], b = src[2 * n + 1];
+            v[at] = make_float2(a.x, a.y);
+            v[at + 1] = make_float2(a.z, a.w);
+            v[at + 2] = make_float2(b.x, b.y);
+            v[at + 3] = make_float2(b.z, b.w);
+        };
+        load(0, 0);
+#pragma unroll 2
+        for (int n = 0; n < f.groups; n++)
         {
-            const int yy = i / SW, xx = i % SW;
-            const int gx = min(max(x0 + xx - R, 0), w - 1), gy = min(max(y0 + yy - R, 0), h - 1);
-            const float3 c = srgb8_to_ycxcz(__ldg(src + (size_t)gy * w + gx));
-            pin[i] = c.x;
-            pin[SH * SW + i] = c.y;
-            pin[2 * SH * SW + i] = c.z;
-            pin[3 * SH * SW + i] = (c.x + 16.0f) / 116.0f;
-        }
-        __syncthreads();
-        for (int i = tid; i < SH * FTW; i += THREADS)
-        {
-            const int row = i / FTW, col = i % FTW;
-            const float *rY = pin + row * SW + col, *rX = rY + SH * SW, *rZ = rY + 2 * SH * SW, *rN = rY + 3 * SH * SW;
-            float a = 0.f, rg = 0.f, by1 = 0.f, by2 = 0.f, g = 0.f, e = 0.f, p = 0.f;
-            for (int k = 0; k <= 2 * R; k++)
-            {
-                const int t = FR_MAX - R + k;
-                a = fmaf(f.csf_a[t], rY[k], a);
-                rg = fmaf(f.csf_rg[t], rX[k], rg);
-                by1 = fmaf(f.csf_by1[t], rZ[k], by1);
-                by2 = fmaf(f.csf_by2[t], rZ[k], by2);
-                g = fmaf(f.gauss[t], rN[k], g);
-                e = fmaf(f.edge[t], rN[k], e);
-                p = fmaf(f.point[t], rN[k], p);
-            }
-            float *o = hor + row * FTW + col;
-            o[0] = a;
-            o[SH * FTW] = rg;
-            o[2 * SH * FTW] = by1;
-            o[3 * SH * FTW] = by2;
-            o[4 * SH * FTW] = g;
-            o[5 * SH * FTW] = e;
-            o[6 * SH * FTW] = p;
-        }
-        __syncthreads();
+            load(4, n + 1);
 #pragma unroll
-        for (int r = 0; r < 2; r++)
-        {
-            const int oy = threadIdx.y * 2 + r;
-            const float *c = hor + oy * FTW + tx;
-            float a = 0.f, rg = 0.f, by = 0.f, ex = 0.f, ey = 0.f, px = 0.f, py = 0.f;
-            for (int k = 0; k <= 2 * R; k++)
-            {
-                const int t = FR_MAX - R + k;
-                const float *ck = c + k * FTW;
-                a = fmaf(f.csf_a[t], ck[0], a);
-                rg = fmaf(f.csf_rg[t], ck[SH * FTW], rg);
-                by = fmaf(f.csf_by1[t], ck[2 * SH * FTW], by);
-                by = fmaf(f.csf_by2[t], ck[3 * SH * FTW], by);
-                ex = fmaf(f.gauss[t], ck[5 * SH * FTW], ex);
-                ey = fmaf(f.edge[t], ck[4 * SH * FTW], ey);
-                px = fmaf(f.gauss[t], ck[6 * SH * FTW], px);
-                py = fmaf(f.point[t], ck[4 * SH * FTW], py);
-            }
-            const float3 lab = ycxcz_to_hunt_lab(a, rg, by);
-            Lab[im][r][0] = lab.x;
-            Lab[im][r][1] = lab.y;
-            Lab[im][r][2] = lab.z;
-            en[im][r] = sqrtf(ex * ex + ey * ey);
-            pn[im][r] = sqrtf(px * px + py * py);
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int q = 0; q < NF; q++)
+                {
+                    const float2 c = f.tap[which[q]][4 * n + k];
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        acc[q][j] = __ffma2_rn(c, v[k + j], acc[q][j]);
+                }
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                v[k] = v[4 + k];
         }
-        __syncthreads(); // the staging buffers are reused by the next image
+#pragma unroll
+        for (int q = 0; q < NF; q++)
+        {
+            float4 *o = reinterpret_cast<float4 *>(out[q] + row * FlipTile::FH_PITCH + 4 * g);
+            o[0] = make_float4(acc[q][0].x, acc[q][0].y, acc[q][1].x, acc[q][1].y);
+            o[1] = make_float4(acc[q][2].x, acc[q][2].y, acc[q][3].x, acc[q][3].y);
+        }
     }
+}
 
-    double sum = 0.0;
-    const float pccmax = FLIP_PC * f.cmax;
+constexpr int F_ROWS_EACH = FTH / (THREADS / 32);
+
+// The vertical pass: a thread filters F_ROWS_EACH outputs of its column.  Term q is filter
+// which[q] over buffer rows[from[q]], added to acc[to[q]]; terms of one sum alternate tap by tap.
+template <int NB, int NF, int NA>
+__device__ __forceinline__ void flip_columns(const FlipFilters &f, const float2 *const (&rows)[NB], const int (&from)[NF],
+                                             const FlipFilter (&which)[NF], const int (&to)[NF], float2 (&acc)[NA][F_ROWS_EACH])
+{
+    static_assert(F_ROWS_EACH == 4, "the window holds 4 outputs and 4 taps");
+    const int at = (threadIdx.x >> 5) * F_ROWS_EACH * FlipTile::FH_PITCH + (threadIdx.x & 31);
+    float2 v[NB][8];
 #pragma unroll
-    for (int r = 0; r < 2; r++)
+    for (int b = 0; b < NB; b++)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            v[b][k] = rows[b][at + k * FlipTile::FH_PITCH];
+#pragma unroll 2
+    for (int n = 0; n < f.groups; n++)
     {
-        const int gx = x0 + tx, gy = y0 + threadIdx.y * 2 + r;
-        if (gx >= w || gy >= h)
+#pragma unroll
+        for (int b = 0; b < NB; b++)
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                v[b][4 + k] = rows[b][at + (4 * (n + 1) + k) * FlipTile::FH_PITCH];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int q = 0; q < NF; q++)
+            {
+                const float2 c = f.tap[which[q]][4 * n + k];
+#pragma unroll
+                for (int j = 0; j < F_ROWS_EACH; j++)
+                    acc[to[q]][j] = __ffma2_rn(c, v[from[q]][k + j], acc[to[q]][j]);
+            }
+#pragma unroll
+        for (int b = 0; b < NB; b++)
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                v[b][k] = v[b][4 + k];
+    }
+}
+
+// One block per 32x32 output tile.  Both images travel together as (reference, test) pairs:
+// every filter step is one packed fma.rn.f32x2 for both.  The tile and an R-pixel
+// replicate-padded halo are staged as Y, Cx, Cz; plane by plane, rows are filtered into shared
+// memory, then columns per output pixel.  Cz and Cx go first: the feature detectors (three
+// filters over the normalised Y, computed in place) reuse the space of Cz as a third buffer, so
+// two blocks of a 21-tap tile share an SM.
+// Bound by FMA issue and shared-memory reads (not by HBM: 2 x 4 bytes a pixel): the register
+// windows read each staged value once per 4 outputs.  1080p: 510 -> 238 us (the images in turn,
+// one output per thread and pass, a power per staged colour value before).
+__global__ void __launch_bounds__(THREADS, 2) flip_tile_kernel(const uint32_t *__restrict__ test, const uint32_t *__restrict__ ref, int w,
+                                                               int h, const __grid_constant__ FlipFilters f,
+                                                               double *__restrict__ partials, float *__restrict__ map)
+{
+    extern __shared__ __align__(16) float2 fsm[];
+    const FlipTile t(f.r, f.groups);
+    float2 *pz = fsm, *px = pz + t.plane(), *py = px + t.plane(); // Cz, Cx, Y
+    float2 *h0 = py + t.plane(), *h1 = h0 + t.hplane(), *h2 = pz;
+    float *lin = reinterpret_cast<float *>(h1 + t.hplane());
+    const int tid = threadIdx.x;
+    const int x0 = blockIdx.x * FTW, y0 = blockIdx.y * FTH;
+    const float2 zero = make_float2(0.0f, 0.0f);
+    auto clear_tail = [&](float2 *rows) { // rows past the input's, read by padded (zero) taps
+        for (int i = t.sh * FlipTile::FH_PITCH + tid; i < t.hplane(); i += THREADS)
+            rows[i] = zero;
+    };
+
+    static_assert(THREADS == 256, "one table entry per thread");
+    lin[tid] = srgb8_to_linear((uint32_t)tid);
+    clear_tail(h0);
+    clear_tail(h1);
+    __syncthreads();
+    const int sw = FTW + 2 * f.r;
+    for (int i = tid; i < t.plane(); i += THREADS)
+    {
+        const int yy = i / t.pitch, xx = i - yy * t.pitch;
+        float3 cr = make_float3(0.f, 0.f, 0.f), ct = cr;
+        if (xx < sw)
+        {
+            const int gx = min(max(x0 + xx - f.r, 0), w - 1), gy = min(max(y0 + yy - f.r, 0), h - 1);
+            const size_t idx = (size_t)gy * w + gx;
+            cr = srgb8_to_ycxcz(__ldg(ref + idx), lin);
+            ct = srgb8_to_ycxcz(__ldg(test + idx), lin);
+        }
+        py[i] = make_float2(cr.x, ct.x);
+        px[i] = make_float2(cr.y, ct.y);
+        pz[i] = make_float2(cr.z, ct.z);
+    }
+    __syncthreads();
+
+    float2 by[1][F_ROWS_EACH] = {}, rg[1][F_ROWS_EACH] = {}, la[1][F_ROWS_EACH] = {};
+    flip_rows<2>(f, t, pz, {CSF_BY1, CSF_BY2}, {h0, h1});
+    __syncthreads();
+    flip_columns<2, 2>(f, {h0, h1}, {0, 1}, {CSF_BY1, CSF_BY2}, {0, 0}, by);
+    __syncthreads();
+    flip_rows<1>(f, t, px, {CSF_RG}, {h0});
+    flip_rows<1>(f, t, py, {CSF_A}, {h1});
+    clear_tail(h2);
+    __syncthreads();
+    flip_columns<1, 1>(f, {h0}, {0}, {CSF_RG}, {0}, rg);
+    flip_columns<1, 1>(f, {h1}, {0}, {CSF_A}, {0}, la);
+    for (int i = tid; i < t.plane(); i += THREADS)
+        py[i] = make_float2((py[i].x + 16.0f) / 116.0f, (py[i].y + 16.0f) / 116.0f);
+    __syncthreads();
+    flip_rows<3>(f, t, py, {GAUSS, EDGE, POINT}, {h0, h1, h2});
+    __syncthreads();
+    float2 gy[2][F_ROWS_EACH] = {}, ex[1][F_ROWS_EACH] = {}, fx[1][F_ROWS_EACH] = {}; // gy: edge and point along y
+    flip_columns<1, 2>(f, {h0}, {0, 0}, {EDGE, POINT}, {0, 1}, gy);
+    flip_columns<1, 1>(f, {h1}, {0}, {GAUSS}, {0}, ex);
+    flip_columns<1, 1>(f, {h2}, {0}, {GAUSS}, {0}, fx);
+
+    PairSum sum_v;
+    const float pccmax = FLIP_PC * f.cmax;
+    const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+    for (int r = 0; r < F_ROWS_EACH; r++)
+    {
+        const int gx = x0 + lane, gyy = y0 + warp * F_ROWS_EACH + r;
+        if (gx >= w || gyy >= h)
             continue;
+        const float3 lr = ycxcz_to_hunt_lab(la[0][r].x, rg[0][r].x, by[0][r].x), lt = ycxcz_to_hunt_lab(la[0][r].y, rg[0][r].y, by[0][r].y);
         // color pipeline: HyAB(reference, test) of the Hunt-adjusted colours
-        const float dL = Lab[0][r][0] - Lab[1][r][0], da = Lab[0][r][1] - Lab[1][r][1], db = Lab[0][r][2] - Lab[1][r][2];
+        const float dL = lr.x - lt.x, da = lr.y - lt.y, db = lr.z - lt.z;
         const float hy = sqrtf(fmaxf(dL * dL, FLIP_EPS)) + sqrtf(da * da + db * db);
         const float power = powf(hy, FLIP_QC);
         const float dec = power < pccmax ? (FLIP_PT / pccmax) * power
                                          : FLIP_PT + ((power - pccmax) / (f.cmax - pccmax)) * (1.0f - FLIP_PT);
         // feature pipeline
-        float def = fmaxf(fabsf(en[0][r] - en[1][r]), fabsf(pn[1][r] - pn[0][r]));
+        const float er = sqrtf(ex[0][r].x * ex[0][r].x + gy[0][r].x * gy[0][r].x), et = sqrtf(ex[0][r].y * ex[0][r].y + gy[0][r].y * gy[0][r].y);
+        const float pr = sqrtf(fx[0][r].x * fx[0][r].x + gy[1][r].x * gy[1][r].x), pt = sqrtf(fx[0][r].y * fx[0][r].y + gy[1][r].y * gy[1][r].y);
+        float def = fmaxf(fabsf(er - et), fabsf(pt - pr));
         def = fmaxf(def, FLIP_EPS);
         def = powf(0.70710678f * def, FLIP_QF);
         const float v = powf(dec, 1.0f - def);
-        sum += (double)v;
+        sum_v.add(v);
         if (map)
-            map[(size_t)gy * w + gx] = v;
+            map[(size_t)gyy * w + gx] = v;
     }
+    double sum = sum_v.value();
     for (int o = 16; o > 0; o >>= 1)
         sum += __shfl_down_sync(0xffffffffu, sum, o);
     __shared__ double ws[THREADS / 32];
@@ -407,6 +568,9 @@ bool make_flip_filters(double ppd, FlipFilters &f)
     if (rc > FR_MAX || rf > FR_MAX || rc < 0 || rf < 0)
         return false;
     f.r = std::max(rc, rf);
+    f.groups = (2 * f.r + 1 + 3) / 4;
+    auto tap = [&](FlipFilter which, int t) -> float2 & { return f.tap[which][t - FR_MAX + f.r]; }; // t - FR_MAX: the offset, -r..r
+    auto set = [&](FlipFilter which, int t, double v) { tap(which, t) = make_float2((float)v, (float)v); };
     const double dx = 1.0 / ppd;
     auto gauss_1d = [&](double b, std::vector<double> &e) {
         e.assign(FTAPS, 0.0);
@@ -420,12 +584,12 @@ bool make_flip_filters(double ppd, FlipFilters &f)
     // BY: 34.1 sqrt(pi / 0.04) e1(x) e1(y) + 13.5 sqrt(pi / 0.025) e2(x) e2(y), normalised to sum 1
     const double w1 = 34.1 * std::sqrt(pi / 0.04), w2 = 13.5 * std::sqrt(pi / 0.025);
     const double norm = w1 * s1 * s1 + w2 * s2 * s2;
-    for (int t = 0; t < FTAPS; t++)
+    for (int t = FR_MAX - f.r; t <= FR_MAX + f.r; t++)
     {
-        f.csf_a[t] = (float)(ea[t] / sa);
-        f.csf_rg[t] = (float)(erg[t] / srg);
-        f.csf_by1[t] = (float)(e1[t] * std::sqrt(w1 / norm));
-        f.csf_by2[t] = (float)(e2[t] * std::sqrt(w2 / norm));
+        set(CSF_A, t, ea[t] / sa);
+        set(CSF_RG, t, erg[t] / srg);
+        set(CSF_BY1, t, e1[t] * std::sqrt(w1 / norm));
+        set(CSF_BY2, t, e2[t] * std::sqrt(w2 / norm));
     }
     std::vector<double> g(FTAPS, 0.0), de(FTAPS, 0.0), dp(FTAPS, 0.0);
     double gs = 0.0, pos_e = 0.0, neg_e = 0.0, pos_p = 0.0, neg_p = 0.0;
@@ -439,11 +603,11 @@ bool make_flip_filters(double ppd, FlipFilters &f)
         (de[FR_MAX + x] < 0 ? neg_e : pos_e) += std::fabs(de[FR_MAX + x]);
         (dp[FR_MAX + x] < 0 ? neg_p : pos_p) += std::fabs(dp[FR_MAX + x]);
     }
-    for (int t = 0; t < FTAPS; t++)
+    for (int t = FR_MAX - f.r; t <= FR_MAX + f.r; t++)
     {
-        f.gauss[t] = (float)(g[t] / gs);
-        f.edge[t] = (float)(de[t] / (de[t] < 0 ? neg_e : pos_e));
-        f.point[t] = (float)(dp[t] / (dp[t] < 0 ? neg_p : pos_p));
+        set(GAUSS, t, g[t] / gs);
+        set(EDGE, t, de[t] / (de[t] < 0 ? neg_e : pos_e));
+        set(POINT, t, dp[t] / (dp[t] < 0 ? neg_p : pos_p));
     }
     // cmax = HyAB(hunt(lab(green)), hunt(lab(blue)))^qc
     auto hunt_lab = [&](double r, double gg, double b, double out[3]) {
@@ -481,11 +645,11 @@ Gauss make_gauss()
     float sum = 0.0f;
     for (int k = 0; k < WIN; k++)
     {
-        g.g[k] = (float)std::exp(-double((k - R) * (k - R)) / (2.0 * 1.5 * 1.5));
-        sum += g.g[k];
+        g.g[k].x = (float)std::exp(-double((k - R) * (k - R)) / (2.0 * 1.5 * 1.5));
+        sum += g.g[k].x;
     }
-    for (float &v : g.g)
-        v = v / sum;
+    for (float2 &v : g.g)
+        v.y = v.x = v.x / sum;
     return g;
 }
 
@@ -513,7 +677,7 @@ isti_status isti_quality_rgba8(const void *a, const void *b, int32_t width, int3
     static const Gauss gw = make_gauss();
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid((width + TW - 1) / TW, (height + TH - 1) / TH);
-    quality_tile_kernel<<<grid, dim3(32, 8), 0, s>>>(static_cast<const uint32_t *>(a), static_cast<const uint32_t *>(b),
+    quality_tile_kernel<<<grid, Q_THREADS, 0, s>>>(static_cast<const uint32_t *>(a), static_cast<const uint32_t *>(b),
                                                     width, height, static_cast<double *>(scratch), gw);
     quality_final_kernel<<<1, THREADS, 0, s>>>(static_cast<const double *>(scratch), n_tiles(width, height),
                                                3.0 * (double)width * (double)height, out);
@@ -541,19 +705,18 @@ isti_status isti_flip_rgba8(const void *test, const void *reference, int32_t wid
     FlipFilters f;
     if (!make_flip_filters((double)pixels_per_degree, f))
         return isti::set_error(ISTI_ERR_INVALID_ARG, "isti_flip_rgba8: pixels_per_degree too large for the filter radius limit");
-    const int R = f.r;
-    const size_t smem = (size_t)(4 * (FTH + 2 * R) * (FTW + 2 * R) + 7 * (FTH + 2 * R) * FTW) * sizeof(float);
+    const size_t smem = FlipTile(f.r, f.groups).bytes();
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(attr_once, [] {
-        const size_t max_smem = (size_t)(4 * (FTH + 2 * FR_MAX) * (FTW + 2 * FR_MAX) + 7 * (FTH + 2 * FR_MAX) * FTW) * sizeof(float);
+        const size_t max_smem = FlipTile(FR_MAX, FGROUPS_MAX).bytes();
         attr_err = cudaFuncSetAttribute(flip_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
     });
     if (attr_err != cudaSuccess)
         return isti::set_error(ISTI_ERR_CUDA, std::string("isti_flip_rgba8: ") + cudaGetErrorString(attr_err));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid((width + FTW - 1) / FTW, (height + FTH - 1) / FTH);
-    flip_tile_kernel<<<grid, dim3(32, 8), smem, s>>>(static_cast<const uint32_t *>(test), static_cast<const uint32_t *>(reference), width,
+    flip_tile_kernel<<<grid, THREADS, smem, s>>>(static_cast<const uint32_t *>(test), static_cast<const uint32_t *>(reference), width,
                                                      height, f, static_cast<double *>(scratch), out_map);
     flip_final_kernel<<<1, THREADS, 0, s>>>(static_cast<const double *>(scratch), flip_tiles(width, height),
                                             (double)width * (double)height, out_mean);
