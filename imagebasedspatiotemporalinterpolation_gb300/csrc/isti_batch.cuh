@@ -59,9 +59,10 @@ struct BatchParams
 };
 
 // Shared memory of a batch_kernel block: [the current pair's FrameParams prefix, padded to
-// batch_param_space][reprojection region][TMA barrier][control words][the current BatchPair].
+// batch_param_space][reprojection region][a TMA barrier per warp][control words][the current BatchPair].
 // The parameters sit at offset 0, so their fields are read at constant shared addresses.
-constexpr size_t BATCH_CTRL_BYTES = 8 + 32 + 48; // barrier, 8 control words, the current BatchPair
+constexpr size_t BATCH_BAR_BYTES = 8 * MAX_VIEWS;
+constexpr size_t BATCH_CTRL_BYTES = BATCH_BAR_BYTES + 32 + 48; // barriers, 8 control words, the current BatchPair
 __host__ __device__ constexpr size_t batch_param_space(size_t param_bytes) { return (param_bytes + 1023) & ~(size_t)1023; }
 static_assert(sizeof(FrameParams) % 16 == 0, "FrameParams is staged in 16-byte words");
 static_assert(sizeof(BatchPair) <= 48, "BatchPair is staged in 48 bytes");
@@ -82,23 +83,24 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
     uint4 *staged = reinterpret_cast<uint4 *>(smem);
     const FrameParams &p = *reinterpret_cast<const FrameParams *>(smem);
     unsigned char *region = smem + batch_param_space(bp.param_bytes);
-    unsigned long long &bar = *reinterpret_cast<unsigned long long *>(region + bp.region_bytes);
+    unsigned long long *bars = reinterpret_cast<unsigned long long *>(region + bp.region_bytes);
     // [0, 1] ticket of the current / next unit and [2, 3] the status word seen for it (both
     // alternating: the entry for the next unit is written before the barrier that ends this
     // one, while some threads may not have read this unit's entry yet), [4] dependency met,
     // [5] a reprojection unit's wait for its key tiles gave up (reproj_block's `aborted`)
-    uint32_t *ctrl = reinterpret_cast<uint32_t *>(region + bp.region_bytes + 8);
-    BatchPair &bpair = *reinterpret_cast<BatchPair *>(region + bp.region_bytes + 8 + 32);
+    uint32_t *ctrl = reinterpret_cast<uint32_t *>(region + bp.region_bytes + BATCH_BAR_BYTES);
+    BatchPair &bpair = *reinterpret_cast<BatchPair *>(region + bp.region_bytes + BATCH_BAR_BYTES + 32);
     const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x, nthreads = blockDim.x * blockDim.y;
     if (tid == 0)
     {
-        mbar_init(&bar, 1);
+        for (uint32_t i = 0; i < blockDim.y; i++)
+            mbar_init(bars + i, 1);
         ctrl[0] = atomicAdd(bp.ticket, 1u);
         ctrl[2] = 0u;
         ctrl[5] = 0u;
     }
     __syncthreads();
-    int round = 0;        // TMA rounds of this block's barrier (its phase carries across units)
+    int round = 0;        // TMA rounds of this warp's barrier (its phase carries across units)
     uint32_t slot = 0;    // ctrl word holding the current ticket
     // the segment of the current ticket; a block's tickets only grow, so the search resumes
     // where the previous unit's ended
@@ -192,7 +194,7 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
             else
             {
                 const uint32_t bx = u % bpair.reproj_gx, by = u / bpair.reproj_gx;
-                reproj_block<SW, SI, MAV, REGS>(p, bpair.maps, bx, by, u, region, bar, round, *reinterpret_cast<volatile uint32_t *>(ctrl + 5));
+                reproj_block<SW, SI, MAV, REGS>(p, bpair.maps, bx, by, u, region, bars, round, *reinterpret_cast<volatile uint32_t *>(ctrl + 5));
             }
         }
         if (helper)

@@ -689,24 +689,24 @@ __device__ __forceinline__ bool resolve_pixel(const DirRes *res, int lane, const
 //   l = +-inf, NaN, or negative non-zero  -> always true  -> bound 0xffffffff;
 //   l = -0.0                              -> always false -> bound 0;
 //   l in [+0, +max finite]                -> c < l, monotonic in the bits -> bound l_bits.
-__device__ __forceinline__ uint32_t key_bound(uint32_t l)
+__host__ __device__ __forceinline__ uint32_t key_bound(uint32_t l)
 {
     return l == 0x80000000u ? 0u : (l >= 0x7f800000u ? 0xffffffffu : l);
 }
 
-// initializeSearchFromSplatting<SW> on a shared-memory tile, src/renderer.cu:148-175, same
-// scan order.  Tile row `row` holds the view row of this pixel; keys outside the view read
-// as 0 (depth +0.0), which the window never selects, exactly like the reference's skipped
-// out-of-range neighbours.  Returns the selected raw key.
+// initializeSearchFromSplatting<SW> on a shared-memory tile, src/renderer.cu:148-175, in the
+// reference's scan order.  Tile row `row` holds the view row of this pixel; keys outside the
+// view read as 0 (depth +0.0), which the window never selects, exactly like the reference's
+// skipped out-of-range neighbours.  Returns the selected raw key.
 template <int SW>
-__device__ __forceinline__ unsigned long long window_key(const unsigned long long *tile, int row, int col)
+__host__ __device__ __noinline__ unsigned long long window_key_in_order(const unsigned long long *tile, int row, int col)
 {
     using T = Tile<SW>;
     unsigned long long best = tile[row * T::W + col];
     uint32_t bound = key_bound((uint32_t)(best >> 32));
-#pragma unroll
+#pragma unroll 1
     for (int yo = -SW; yo <= SW; yo++)
-#pragma unroll
+#pragma unroll 1
         for (int xo = -SW; xo <= SW; xo++)
         {
             const unsigned long long c = tile[(row + yo) * T::W + col + xo];
@@ -720,122 +720,222 @@ __device__ __forceinline__ unsigned long long window_key(const unsigned long lon
     return best;
 }
 
+// Depth bits and source pixel of a key.
+struct KeyWords
+{
+    uint32_t hi, lo;
+};
+
+// The first of N keys with the smallest depth bits (as unsigned numbers: negative depths, NaN and
+// empty keys compare above every positive depth).
+template <int N>
+__host__ __device__ __forceinline__ KeyWords first_min(const KeyWords (&k)[N])
+{
+    uint32_t m = k[0].hi;
+#pragma unroll
+    for (int i = 1; i + 1 < N; i += 2)
+        m = __vimin3_u32(m, k[i].hi, k[i + 1].hi);
+    if (N % 2 == 0)
+        m = min(m, k[N - 1].hi);
+    uint32_t lo = k[N - 1].lo;
+#pragma unroll
+    for (int i = N - 2; i >= 0; i--)
+        lo = k[i].hi == m ? k[i].lo : lo;
+    return {m, lo};
+}
+
+__host__ __device__ __forceinline__ KeyWords first_min(KeyWords a, KeyWords b)
+{
+    return a.hi <= b.hi ? a : b;
+}
+
+// The window keys of the two output rows of a thread: row 0 has its centre in tile row SW, row 1
+// in tile row SW + below (0 or 1).
+//
+// The reference's scan keeps a running best; among positive finite depths that is the centre if
+// none is smaller than it, else the first smallest one in scan order.  So the windows are taken
+// as minima: each tile row once for both output rows, then the rows, with the source pixel of the
+// first key that equals the minimum -- 3 instead of about 9 ALU instructions per key and output
+// row.  The ALU pipe, which issues at half rate, was the busiest (0.57 of its peak at 1080p with 6
+// views, 196 M instructions of 501 M; 153 M of 462 M now).  The scan order itself is only walked where the minimum does not tell what it finds: a
+// smallest depth of +0.0 (a border key) or +inf, a centre of -0.0.
+// Reprojection, 3 frames: 1080p 6 views 0.549 -> 0.513 ms, 1366x768 4 views 7x7 window 0.474 -> 0.378 ms.
+template <int SW>
+__host__ __device__ __forceinline__ void window_keys(const unsigned long long *tile, int col, int below, const bool (&wanted)[ROWS],
+                                            KeyWords (&key)[ROWS])
+{
+    using T = Tile<SW>;
+    static_assert(ROWS == 2 && T::H == 2 * SW + 2);
+    KeyWords rows[T::H], centre[ROWS];
+#pragma unroll
+    for (int r = 0; r < T::H; r++)
+    {
+        KeyWords k[2 * SW + 1];
+#pragma unroll
+        for (int x = 0; x < 2 * SW + 1; x++)
+        {
+            const unsigned long long c = tile[r * T::W + col - SW + x];
+            k[x] = {(uint32_t)(c >> 32), (uint32_t)c};
+        }
+        rows[r] = first_min(k);
+        if (r == SW || r == SW + 1)
+            centre[r - SW] = k[SW];
+    }
+    KeyWords shared[2 * SW];
+#pragma unroll
+    for (int r = 0; r < 2 * SW; r++)
+        shared[r] = rows[1 + r];
+    const KeyWords mid = first_min(shared);
+    key[0] = first_min(rows[0], mid);
+    key[1] = first_min(mid, rows[T::H - 1]);
+    if (below == 0) // both output rows lie in the same view row (warp-uniform)
+    {
+        key[1] = key[0];
+        centre[1] = centre[0];
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; r++)
+    {
+        const KeyWords m = key[r];
+        // the centre stays if nothing positive was found or nothing is smaller
+        if (m.hi >= 0x7f800000u || centre[r].hi == m.hi)
+            key[r] = centre[r];
+        if (wanted[r] && (m.hi == 0u || m.hi == 0x7f800000u || centre[r].hi == 0x80000000u))
+        {
+            const unsigned long long k = window_key_in_order<SW>(tile, SW + (r == 0 ? 0 : below), col);
+            key[r] = {(uint32_t)(k >> 32), (uint32_t)k};
+        }
+    }
+}
+
 // bidirectionalReprojection_kernel<SW, SI, MAIN_ALWAYS_VALID>, src/renderer.cu:400-465
 // block = (32, n_views): 32 output columns x (2 * row_pairs) output rows, one warp per source
-// view.  The block works through units (frame k, row pair): phase 1 runs one unit at a time
-// on every warp; phases 2-3 spread the units' rows over the warps.  More row pairs per block
-// (for single frames) keep every warp busy in phase 2.
+// view.  The block works through units (frame k, row pair).  Phase 1: every warp runs all units
+// of its own view, at its own pace: it fetches the unit's key tile itself (one elected lane, one
+// TMA copy, one barrier per warp) and issues the next unit's copy as soon as it has read the
+// window keys, so the copy lands during the search.  The warps meet only after phase 1; phases
+// 2-3 spread the units' rows over them.  (With one elected thread fetching every view's tile and
+// a block barrier per unit, each unit waited for its slowest view and for the copy:
+// calls of 3 frames at 1080p with 6 views 0.762 -> 0.709 ms, of 6 frames at 2064x2208 with 2 views
+// 1.375 -> 1.227 ms.)
+// More row pairs per block (for single frames) keep every warp busy in phase 2.
 // One reprojection block (bx, by) of frame batch p, executed by a block of (32, n_views)
 // threads: the body of reproj_kernel, also run as a work unit of batch_kernel.  `maps`: the
-// views' key-tile tensor maps; `bar`: the block's TMA completion barrier, initialised once per
-// thread block; `round`: TMA rounds that barrier has completed so far (its phase carries over
-// from unit to unit, also across units whose tiles came by plain loads); `aborted`: a shared word, 0 when the block starts, that a thread whose
-// wait for the key tiles gave up sets to 1; `block_id`: the index the test hook
-// `withhold_block` refers to, compiled in only where HOOK is set.  Every thread returns
-// together (early exits are block-uniform or come after the last barrier).
+// views' key-tile tensor maps; `bars`: the warps' TMA completion barriers, initialised once per
+// thread block; `round`: TMA rounds this warp's barrier has completed so far (its phase carries
+// over from unit to unit, also across units whose tiles came by plain loads); `aborted`: a
+// shared word, 0 when the block starts, that a warp whose wait for a key tile gave up sets to 1;
+// `block_id`: the index the test hook `withhold_block` refers to, compiled in only where HOOK is
+// set.  Every thread returns together (early exits are block-uniform or come after the last
+// barrier).
 template <int SW, int SI, bool MAV, int REGS, bool HOOK = false>
 __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtensorMap *maps, uint32_t bx, uint32_t by, uint32_t block_id,
-                                             unsigned char *smem, unsigned long long &bar, int &round, volatile uint32_t &aborted)
+                                             unsigned char *smem, unsigned long long *bars, int &round, volatile uint32_t &aborted)
 {
     using T = Tile<SW>;
     const int nv = p.n_views, nf = p.n_frames, np = p.row_pairs, nu = nf * np;
-    // [key tiles, phase 1 | chained colours and flags, phases 2-3 (same bytes)][results][barrier]
+    // [key tiles, phase 1 | chained colours and flags, phases 2-3 (same bytes)][results][barriers]
     unsigned long long *tiles = reinterpret_cast<unsigned long long *>(smem);                 // [nv][H][W]
     uint32_t *cols = reinterpret_cast<uint32_t *>(smem);                                      // [nu][ROWS][32]
     uint32_t *valid = cols + nu * ROWS * 32;                                                 // [nu][ROWS][32]
     DirRes *res = reinterpret_cast<DirRes *>(smem + reproj_tile_region<SW>(nv, nu));         // [nu][ROWS][nv][32]
 
-    const int lane = threadIdx.x, vw = threadIdx.y;
+    // the warp's view; the shuffle tells the compiler that it is the same for the whole warp, so
+    // that the view's fields are read and indexed on the uniform datapath
+    const int lane = threadIdx.x, vw = __shfl_sync(0xffffffffu, (int)threadIdx.y, 0);
     const uint32_t x0 = bx * 32, x = x0 + lane, yb = by * (ROWS * np);
     const bool xok = x < p.out_w;
-    const bool leader = lane == 0 && vw == 0;
     {
         const DevView &v = p.v[vw];
         const uint32_t ix = v.sx == 1 ? x : x / v.sx, tx0 = v.sx == 1 ? x0 : x0 / v.sx;
         const bool fwd = (vw & 1) == 0;
         const int xs = tile_x0(tx0, SW);
         const int col = (int)ix - xs;
+        unsigned long long *tg = tiles + (size_t)vw * T::ELEMS;
+        unsigned long long *bar = bars + vw;
+        // lane 0: announces a unit's tile and starts its copy (the fence orders this warp's reads
+        // of the tile before, and earlier uses of these bytes, against the copy's writes)
+        auto fetch = [&](int rp, int k) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_expect_tx(bar, (uint32_t)T::BYTES);
+            if (HOOK && p.withhold_block == (int32_t)block_id)
+                return;
+            const uint32_t y0 = yb + (uint32_t)rp * ROWS;
+            tma_load_3d(tg, &maps[vw], xs, (int)(v.sy == 1 ? y0 : y0 / v.sy) - SW, k, bar);
+        };
+        if (p.use_tma && lane == 0)
+            fetch(0, 0);
         // pixel2CS of the output pixels in the main view (the search target) and in this view (the error)
         const DevView &v0 = p.v[0];
         const uint32_t xc = min(x, p.out_w - 1);
         const float qx = __ldg(v0.lut + xc);
         const float pcx = __ldg(v.lut + min(ix, v.w - 1));
         const uint32_t vwid = v.w, vhei = v.h;
+        bool arrived = true;
 #pragma unroll 1
-        for (int rp = 0; rp < np; rp++)
+        for (int rp = 0; rp < np && arrived; rp++)
         {
             const uint32_t y0 = yb + (uint32_t)rp * ROWS; // the row pair's first output row
             const uint32_t iy0 = v.sy == 1 ? y0 : y0 / v.sy, iy1 = v.sy == 1 ? y0 + 1 : (y0 + 1) / v.sy;
             const bool rok[ROWS] = {xok && y0 < p.out_h, xok && y0 + 1 < p.out_h};
-            const int wrow[ROWS] = {SW, (int)(iy1 - iy0) + SW}; // tile row of each output row's window centre
             const uint32_t y0c = min(y0, p.out_h - 1), y1c = min(y0 + 1, p.out_h - 1);
             const float qy[ROWS] = {__ldg(v0.lut + v0.w + y0c), __ldg(v0.lut + v0.w + y1c)};
             const float pcy[ROWS] = {__ldg(v.lut + v.w + min(iy0, vhei - 1)), __ldg(v.lut + v.w + min(iy1, vhei - 1))};
 #pragma unroll 1
-        for (int k = 0; k < nf; k++, round += p.use_tma) // plain loads leave the barrier's phase where it is
-        {
-            const int u = k * np + rp;
-            if (rp + k > 0)
-                __syncthreads(); // every warp is done with the previous unit's tiles
-            bool arrived = true;
-            if (p.use_tma)
+            for (int k = 0; k < nf; k++)
             {
-                // Once a wait of this block has given up (marked before the barrier above), the
-                // leader issues no more rounds: its arrival on a barrier whose phase did not
-                // complete would overrun the barrier's count.  The other waits then run out too
-                // (bounded), and the block writes nothing.
-                if (leader && aborted == 0u)
+                const int u = k * np + rp;
+                if (p.use_tma)
                 {
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    mbar_expect_tx(&bar, (uint32_t)(nv * T::BYTES));
-                    if (!HOOK || p.withhold_block != (int32_t)block_id)
-                        for (int w = 0; w < nv; w++)
-                        {
-                            const DevView &vv = p.v[w];
-                            const uint32_t wx0 = vv.sx == 1 ? x0 : x0 / vv.sx, wy0 = vv.sy == 1 ? y0 : y0 / vv.sy;
-                            tma_load_3d(tiles + (size_t)w * T::ELEMS, &maps[w], tile_x0(wx0, SW), (int)wy0 - SW, k, &bar);
-                        }
-                }
-                // a thread whose copies did not arrive reads none of the tiles and marks the block,
-                // which then leaves after the barrier that ends phase 1, writing nothing (the
-                // mark is written before that barrier and read after it, by every thread)
-                arrived = mbar_wait_bounded(&bar, (uint32_t)(round & 1), p.status, p.wait_limit);
-                if (!arrived)
-                    aborted = 1u;
-            }
-            else
-            {
-                const unsigned long long *keys = v.splat + k * p.key_stride;
-                unsigned long long *tg = tiles + (size_t)vw * T::ELEMS;
-#pragma unroll
-                for (int r = 0; r < T::H; r++)
-                {
-                    const uint32_t gy = iy0 - SW + r;
-                    const bool row_ok = gy < vhei;
-                    for (int c = lane; c < T::W; c += 32)
+                    // A warp whose copy did not arrive reads nothing more, starts no further copy (an
+                    // arrival on a barrier whose phase did not complete would overrun its count) and
+                    // marks the block, which then leaves after the barrier that ends phase 1, writing
+                    // nothing (the mark is written before that barrier and read after it, by every thread).
+                    arrived = __all_sync(0xffffffffu, mbar_wait_bounded(bar, (uint32_t)(round & 1), p.status, p.wait_limit));
+                    if (!arrived)
                     {
-                        const uint32_t gx = (uint32_t)(xs + c);
-                        tg[r * T::W + c] = (row_ok && gx < vwid) ? __ldg(keys + (gy * vwid + gx)) : 0ull;
+                        aborted = 1u;
+                        break;
                     }
+                    round++;
                 }
-                __syncwarp();
-            }
-            if (arrived)
-            {
-                const unsigned long long *tg = tiles + (size_t)vw * T::ELEMS;
+                else
+                {
+                    const unsigned long long *keys = v.splat + k * p.key_stride;
+                    __syncwarp(); // the warp is done with the previous unit's tile
+#pragma unroll
+                    for (int r = 0; r < T::H; r++)
+                    {
+                        const uint32_t gy = iy0 - SW + r;
+                        const bool row_ok = gy < vhei;
+                        for (int c = lane; c < T::W; c += 32)
+                        {
+                            const uint32_t gx = (uint32_t)(xs + c);
+                            tg[r * T::W + c] = (row_ok && gx < vwid) ? __ldg(keys + (gy * vwid + gx)) : 0ull;
+                        }
+                    }
+                    __syncwarp();
+                }
                 const float2 *cam = v.cam_xy + k * p.cam_stride;
                 const float *cdep = v.cam_depth + k * p.depth_stride;
                 const bool search_ok = !fwd || p.f[k].alpha < 1.0f;
                 bool s[ROWS];
                 uint32_t ax[ROWS], ay[ROWS];
                 float d_init[ROWS];
+                KeyWords key[ROWS];
+                window_keys<SW>(tg, col, (int)(iy1 - iy0), rok, key);
+                if (p.use_tma && (k + 1 < nf || rp + 1 < np))
+                {
+                    __syncwarp(); // every lane has read the tile
+                    if (lane == 0)
+                        fetch(k + 1 < nf ? rp : rp + 1, k + 1 < nf ? k + 1 : 0);
+                }
 #pragma unroll
                 for (int r = 0; r < ROWS; r++)
                 {
-                    const unsigned long long lo = window_key<SW>(tg, wrow[r], col);
-                    d_init[r] = __uint_as_float((uint32_t)(lo >> 32));
-                    ax[r] = ((uint32_t)lo) >> 16;
-                    ay[r] = (uint32_t)lo & 0xFFFFu;
+                    d_init[r] = __uint_as_float(key[r].hi);
+                    ax[r] = key[r].lo >> 16;
+                    ay[r] = key[r].lo & 0xFFFFu;
                     s[r] = rok[r] && search_ok && d_init[r] > 0.0f;
                     // a selected key with positive depth is a splat of an in-range source pixel;
                     // the clamp keeps every gather inside the view even if a tile were stale
@@ -912,7 +1012,6 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                 }
             }
         }
-        }
     }
     __syncthreads();
     if (aborted)
@@ -976,19 +1075,20 @@ __global__ void __maxnreg__(REGS) reproj_kernel(const __grid_constant__ FramePar
     // dynamic shared memory only (no static __shared__ in front of it): the key tiles start at
     // the 1 KiB-aligned window base, so every TMA destination is 128-byte aligned
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned long long &bar = *reinterpret_cast<unsigned long long *>(
+    unsigned long long *bars = reinterpret_cast<unsigned long long *>(
         smem + reproj_tile_region<SW>(p.n_views, p.n_frames * p.row_pairs) +
-        (size_t)p.n_frames * p.row_pairs * ROWS * p.n_views * 32 * sizeof(DirRes)); // TMA completion barrier
-    volatile uint32_t &aborted = *reinterpret_cast<volatile uint32_t *>(&bar + 1);
-    if (threadIdx.x == 0 && threadIdx.y == 0)
+        (size_t)p.n_frames * p.row_pairs * ROWS * p.n_views * 32 * sizeof(DirRes)); // TMA completion barriers, one per warp
+    volatile uint32_t &aborted = *reinterpret_cast<volatile uint32_t *>(bars + p.n_views);
+    if (threadIdx.x == 0)
     {
         if (p.use_tma)
-            mbar_init(&bar, 1);
-        aborted = 0u;
+            mbar_init(bars + threadIdx.y, 1);
+        if (threadIdx.y == 0)
+            aborted = 0u;
     }
     __syncthreads();
     int round = 0;
-    reproj_block<SW, SI, MAV, REGS, HOOK>(p, km.m, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x, smem, bar, round, aborted);
+    reproj_block<SW, SI, MAV, REGS, HOOK>(p, km.m, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x, smem, bars, round, aborted);
 }
 
 // ---- timewarp (mode 4), src/renderer.cu:467-522, 615-629 ----
@@ -1298,6 +1398,6 @@ __global__ void clear_shadows_kernel(uint32_t *__restrict__ info, uint32_t *__re
 template <int SW>
 constexpr size_t reproj_smem(int n_views, int n_units)
 {
-    return reproj_tile_region<SW>(n_views, n_units) + (size_t)n_units * ROWS * n_views * 32 * sizeof(DirRes) + 16; // + mbarrier, abort word
+    return reproj_tile_region<SW>(n_views, n_units) + (size_t)n_units * ROWS * n_views * 32 * sizeof(DirRes) + (size_t)n_views * 8 + 16; // + mbarriers, abort word
 }
 } // namespace isti
