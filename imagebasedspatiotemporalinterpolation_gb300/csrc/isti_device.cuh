@@ -106,15 +106,16 @@ __device__ __forceinline__ float2 pixel2cs(uint32_t px, uint32_t py, uint32_t w,
 }
 
 // CS2pixel, include/util/helper_common.h:71-75: floor((cs + 1) * res * 0.5)
-// (float -> int conversion truncates and saturates, NaN -> 0)
+// (float -> int conversion truncates and saturates, NaN -> 0).  half_w, half_h: res * 0.5, exact;
+// halving commutes with the product's rounding (cs + 1 is 0 or at least 2^-24, never close to
+// underflow), and one conversion rounding down equals the floor and its conversion.
+__device__ __forceinline__ int2 cs2pixel_half(float cx, float cy, float half_w, float half_h)
+{
+    return make_int2(__float2int_rd((cx + 1.0f) * half_w), __float2int_rd((cy + 1.0f) * half_h));
+}
 __device__ __forceinline__ int2 cs2pixel(float cx, float cy, uint32_t w, uint32_t h)
 {
-    float ax = cx + 1.0f, ay = cy + 1.0f;
-    ax = ax * (float)w;
-    ay = ay * (float)h;
-    ax = ax * 0.5f;
-    ay = ay * 0.5f;
-    return make_int2(__float2int_rz(floorf(ax)), __float2int_rz(floorf(ay)));
+    return cs2pixel_half(cx, cy, (float)w * 0.5f, (float)h * 0.5f);
 }
 
 // inRange, include/util/helper_common.h:8-11 (a negative coordinate wraps to >= 2^31 > w)
@@ -174,47 +175,61 @@ __device__ __forceinline__ float4 project(const float *m, float4 v)
 __device__ __forceinline__ float z_to_depth(float z) { return xmul(xadd(z, 1.0f), 0.5f); } // :89-91
 __device__ __forceinline__ float depth_to_z(float d) { return xsub(xmul(d, 2.0f), 1.0f); } // :93-95
 
-// lerp_color, include/util/helper_common.h:22-25: (a + t * (b - a)) / 255
-__device__ __forceinline__ float lerp_ch(uint32_t a, uint32_t b, float t)
+// Byte c of a packed colour as a float, exact: the byte becomes the low mantissa bits of 2^23
+// (a byte permute and an addition; the integer conversion runs on a slower unit).
+__device__ __forceinline__ float byte_to_float(uint32_t color, int c)
 {
-    const float fa = (float)a, fb = (float)b;
-    return xdiv(xadd(fa, xmul(t, xsub(fb, fa))), 255.f);
+    return __uint_as_float(__byte_perm(color, 0x4b000000u, 0x7540u + (uint32_t)c)) - 8388608.0f;
+}
+
+// min(255, max(0, int(f))) with int() truncating and NaN -> 0, as the low byte of the result:
+// clamped as a float, truncated by an addition of 2^23 that rounds towards zero.
+__device__ __forceinline__ uint32_t clamp_byte(float f)
+{
+    return __float_as_uint(__fadd_rz(fminf(fmaxf(f, 0.0f), 255.0f), 8388608.0f)) & 255u;
 }
 
 // to_8bit, include/util/helper_common.h:27-30: min(255, max(0, int(f * 255)))
-__device__ __forceinline__ uint32_t to_8bit(float f)
+__device__ __forceinline__ uint32_t to_8bit(float f) { return clamp_byte(xmul(f, 255.f)); }
+
+// Low bytes of four words, packed.
+__device__ __forceinline__ uint32_t pack_bytes(uint32_t r, uint32_t g, uint32_t b, uint32_t a)
 {
-    const int v = __float2int_rz(xmul(f, 255.f));
-    return (uint32_t)min(255, max(0, v));
+    return __byte_perm(__byte_perm(r, g, 0x0040u), __byte_perm(b, a, 0x0040u), 0x5410u);
 }
 
-// to_8bit(v / 255) for v = a + t * (b - a).  The round trip RN(RN(v / 255) * 255)
-// stays within 256 * 2^-23 = 2^-15 of v for 0 <= v < 256 and returns every integer
-// 0..255 unchanged, so its truncation is floor(v) unless v lies within 2^-12 of an
-// integer without being one; only that case (and v outside [0, 256), NaN) takes
-// the division.
-__device__ __forceinline__ uint32_t to_8bit_255ths(float v)
-{
-    if constexpr (FAST_MATH)
-        return to_8bit(v / 255.f);
-    const float fl = floorf(v);
-    const float fr = xsub(v, fl);
-    if (v >= 0.0f && v < 256.0f && (fr == 0.0f || (fr > 0x1p-12f && fr < 1.0f - 0x1p-12f)))
-        return (uint32_t)fl;
-    return to_8bit(xdiv(v, 255.f));
-}
-
-// color_to_uchar4(lerp_color(a, b, t)), packed RGBA8 in a uint32 (R in bits 0-7)
+// color_to_uchar4(lerp_color(a, b, t)), include/util/helper_common.h:22-30: per channel
+// to_8bit((a + t * (b - a)) / 255), packed RGBA8 in a uint32 (R in bits 0-7).
+//
+// IEEE: the round trip RN(RN(v / 255) * 255) stays within 256 * 2^-23 = 2^-15 of v for
+// 0 <= v < 256 and returns every integer 0..255 unchanged, so its truncation is floor(v) unless
+// v lies close to an integer without being one; only a colour with such a channel (or with v
+// outside [0, 256), NaN) takes the divisions.  |fr - 0.5| < 0.4995 keeps fr away from 0 and 1
+// by more than 2^-12.
 __device__ __forceinline__ uint32_t lerp_color_u8(uint32_t a, uint32_t b, float t)
 {
-    uint32_t r = 0;
+    float v[4];
 #pragma unroll
     for (int c = 0; c < 4; c++)
     {
-        const float fa = (float)((a >> (8 * c)) & 255u), fb = (float)((b >> (8 * c)) & 255u);
-        r |= to_8bit_255ths(xadd(fa, xmul(t, xsub(fb, fa)))) << (8 * c);
+        const float fa = byte_to_float(a, c), fb = byte_to_float(b, c);
+        v[c] = xadd(fa, xmul(t, xsub(fb, fa)));
     }
-    return r;
+    if constexpr (!FAST_MATH)
+    {
+        uint32_t q[4];
+        bool plain = true;
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+        {
+            const float up = __fadd_rz(v[c], 8388608.0f), fr = v[c] - (up - 8388608.0f);
+            q[c] = __float_as_uint(up);
+            plain = plain && __float_as_uint(v[c]) < 0x43800000u && (fr == 0.0f || fabsf(fr - 0.5f) < 0.4995f);
+        }
+        if (plain)
+            return pack_bytes(q[0], q[1], q[2], q[3]);
+    }
+    return pack_bytes(to_8bit(xdiv(v[0], 255.f)), to_8bit(xdiv(v[1], 255.f)), to_8bit(xdiv(v[2], 255.f)), to_8bit(xdiv(v[3], 255.f)));
 }
 
 // sqrtf(s) < e; IEEE-exact mode: the square root is only taken within 0.01 % of e^2
@@ -231,8 +246,5 @@ __device__ __forceinline__ bool sqrt_less(float s, float e)
 }
 
 // float -> unsigned char of make_uchar4(float, ...): truncation, saturation, NaN -> 0
-__device__ __forceinline__ uint32_t cvt_u8(float f)
-{
-    return (uint32_t)min(255u, __float2uint_rz(f));
-}
+__device__ __forceinline__ uint32_t cvt_u8(float f) { return clamp_byte(f); }
 } // namespace isti

@@ -397,14 +397,14 @@ __device__ __forceinline__ uint32_t color_from_shadow_idx(uint32_t sidx, int32_t
         // (float)(1.0 - (double)t): t is k / d with d in {1, 2, 3} (or NaN), for which the
         // double difference is exact, so one float subtraction rounds identically.
         const float omt = xsub(1.0f, t);
-        uint32_t r = 255u << 24;
+        uint32_t r[3];
 #pragma unroll
         for (int c = 0; c < 3; c++)
         {
-            const float a = (float)((cmin >> (8 * c)) & 255u), b = (float)((cmax >> (8 * c)) & 255u);
-            r |= cvt_u8(xadd(xmul(a, omt), xmul(b, t))) << (8 * c);
+            const float a = byte_to_float(cmin, c), b = byte_to_float(cmax, c);
+            r[c] = cvt_u8(xadd(xmul(a, omt), xmul(b, t)));
         }
-        return r;
+        return pack_bytes(r[0], r[1], r[2], 255u);
     }
     return s.color;
 }
@@ -871,6 +871,7 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
         const float qx = __ldg(v0.lut + xc);
         const float pcx = __ldg(v.lut + min(ix, v.w - 1));
         const uint32_t vwid = v.w, vhei = v.h;
+        const float half_w = (float)vwid * 0.5f, half_h = (float)vhei * 0.5f;
         bool arrived = true;
 #pragma unroll 1
         for (int rp = 0; rp < np && arrived; rp++)
@@ -937,13 +938,11 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                     ax[r] = key[r].lo >> 16;
                     ay[r] = key[r].lo & 0xFFFFu;
                     s[r] = rok[r] && search_ok && d_init[r] > 0.0f;
-                    // a selected key with positive depth is a splat of an in-range source pixel;
-                    // the clamp keeps every gather inside the view even if a tile were stale
-                    if (s[r])
-                    {
-                        ax[r] = min(ax[r], vwid - 1u);
-                        ay[r] = min(ay[r], vhei - 1u);
-                    }
+                    // a selected key with positive depth is a splat of an in-range source pixel; the
+                    // clamp keeps every gather inside the view for the lanes that search nothing
+                    // (empty windows) and even if a tile were stale
+                    ax[r] = min(ax[r], vwid - 1u);
+                    ay[r] = min(ay[r], vhei - 1u);
                     // the depth read after the search is mostly at or next to the start (a
                     // splatted source pixel, in range): fetch its line into L1 during the search
                     // (3x3 window, 6 views: 0.537 -> 0.533 ms; no gain for the 7x7 window)
@@ -958,12 +957,12 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                     float2 m[ROWS];
 #pragma unroll
                     for (int r = 0; r < ROWS; r++)
-                        m[r] = s[r] ? __ldg(cam + (ay[r] * vwid + ax[r])) : make_float2(0.f, 0.f);
+                        m[r] = __ldg(cam + (ay[r] * vwid + ax[r]));
 #pragma unroll
                     for (int r = 0; r < ROWS; r++)
                     {
-                        const int2 t = cs2pixel(xsub(qx, m[r].x), xsub(qy[r], m[r].y), vwid, vhei);
-                        if (s[r] && in_range(t, vwid, vhei))
+                        const int2 t = cs2pixel_half(xsub(qx, m[r].x), xsub(qy[r], m[r].y), half_w, half_h);
+                        if (in_range(t, vwid, vhei))
                         {
                             ax[r] = (uint32_t)t.x;
                             ay[r] = (uint32_t)t.y;
@@ -973,41 +972,33 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                 // final flow, depth and computeReprojError, src/renderer.cu:338-341, 204-215
                 float2 m[ROWS];
                 float dz[ROWS], fx[ROWS], fy[ROWS];
-                bool vs[ROWS];
+                uint8_t vs[ROWS];
 #pragma unroll
                 for (int r = 0; r < ROWS; r++)
                 {
-                    m[r] = make_float2(0.f, 0.f);
-                    dz[r] = fx[r] = fy[r] = 0.f;
-                    vs[r] = false;
-                    if (s[r])
-                    {
-                        const uint32_t si = ay[r] * vwid + ax[r];
-                        m[r] = __ldg(cam + si);
-                        dz[r] = __ldg(cdep + si);
-                        vs[r] = __ldg(v.vis + si) != 0;
-                        fx[r] = __ldg(v.lut + ax[r]);
-                        fy[r] = __ldg(v.lut + vwid + ay[r]);
-                    }
+                    const uint32_t si = ay[r] * vwid + ax[r];
+                    m[r] = __ldg(cam + si);
+                    dz[r] = __ldg(cdep + si);
+                    vs[r] = __ldg(v.vis + si);
+                    fx[r] = __ldg(v.lut + ax[r]);
+                    fy[r] = __ldg(v.lut + vwid + ay[r]);
                 }
 #pragma unroll
                 for (int r = 0; r < ROWS; r++)
                 {
+                    // the scale res / min(res) (src/renderer.cu:213): the host's IEEE quotient, or
+                    // under the reference's GPU semantics its device division
+                    const float esx = FAST_MATH ? xdiv((float)vwid, (float)min(vwid, vhei)) : v.err_sx;
+                    const float esy = FAST_MATH ? xdiv((float)vhei, (float)min(vwid, vhei)) : v.err_sy;
+                    const float ex = xmul(xsub(xadd(fx[r], m[r].x), pcx), esx);
+                    const float ey = xmul(xsub(xadd(fy[r], m[r].y), pcy[r]), esy);
                     DirRes d;
-                    d.error_vis = ERR_UNSEARCHED_OF<SQUARED_ERRORS<REGS>>;
-                    d.depth = d_init[r];
-                    if (s[r])
-                    {
-                        d.depth = dz[r];
-                        // the scale res / min(res) (src/renderer.cu:213): the host's IEEE quotient, or
-                        // under the reference's GPU semantics its device division
-                        const float esx = FAST_MATH ? xdiv((float)vwid, (float)min(vwid, vhei)) : v.err_sx;
-                        const float esy = FAST_MATH ? xdiv((float)vhei, (float)min(vwid, vhei)) : v.err_sy;
-                        const float ex = xmul(xsub(xadd(fx[r], m[r].x), pcx), esx);
-                        const float ey = xmul(xsub(xadd(fy[r], m[r].y), pcy[r]), esy);
-                        d.error_vis = pack_error_vis<SQUARED_ERRORS<REGS>>(xadd(xmul(ex, ex), xmul(ey, ey)), vs[r]);
-                    }
-                    d.src = (ax[r] << 16) | ay[r];
+                    d.error_vis = s[r] ? pack_error_vis<SQUARED_ERRORS<REGS>>(xadd(xmul(ex, ex), xmul(ey, ey)), vs[r] != 0)
+                                       : ERR_UNSEARCHED_OF<SQUARED_ERRORS<REGS>>;
+                    d.depth = s[r] ? dz[r] : d_init[r];
+                    // a direction that was not searched is only read by the always-valid blend, which
+                    // uses the window's source pixel
+                    d.src = !MAV || s[r] ? (ax[r] << 16) | ay[r] : key[r].lo;
                     res[((u * ROWS + r) * nv + vw) * 32 + lane] = d;
                 }
             }
