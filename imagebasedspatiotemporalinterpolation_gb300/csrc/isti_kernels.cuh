@@ -13,11 +13,11 @@
 //            view) once, then per frame the client-camera projection, flow store
 //            and 64-bit atomicMin;
 //  3. reprojection: a block covers 2 rows x 32 output pixels with one warp per
-//            source view (view = threadIdx.y).  The block's splat-key tiles (every
-//            view, a group of frames) are fetched into shared memory by TMA
-//            (cp.async.bulk.tensor, one elected thread, mbarrier completion).
-//            Phase 1: each thread runs window initialisation + iterative search +
-//            reprojection error for its view and both rows, frame by frame.
+//            source view (view = threadIdx.y).  Phase 1: each warp fetches its
+//            view's splat-key tile of a frame into shared memory by TMA
+//            (cp.async.bulk.tensor, one elected lane, one mbarrier per warp); each
+//            thread runs window initialisation + iterative search + reprojection
+//            error for its view and both rows, frame by frame.
 //            Phase 2: the (frame, row) tasks are spread over the warps; each
 //            chooses the direction per camera and the winning camera and computes
 //            the colour (second chance, soft shadows) only for the result that is
@@ -43,13 +43,10 @@ namespace isti
 constexpr int MAX_VIEWS = 2 + 2 * ISTI_MAX_AUX_CAMS;
 constexpr int MAX_FRAMES = ISTI_MAX_BATCH_FRAMES;
 constexpr int ROWS = 2; // output rows searched together by one reprojection thread
-// Registers per reprojection thread (the kernel's register cap, a template argument).
-// The kernel waits on dependent gathers, so resident warps matter more than registers:
-// at 48 (no spills) a 6-view block of 192 threads fits 7 times into the register file
-// (5 times at its natural 62), at 40 (a few spilled words) 8 times.  Measured at 1080p,
-// 3 frames: for the 3x3 window 40 is faster with 4 or more views (4 views 0.441 -> 0.425
-// ms, 6 views 0.590 -> 0.564 ms) and 48 with 2 (0.240 -> 0.239 ms, 56: 0.252); the 7x7
-// window (mode 1) spills more and runs best at 56 (6 views: 40 1.203, 48 1.164, 56 1.153 ms).
+// Register caps of the reprojection (a template argument of the kernel; reproj_regs below says
+// what a build takes).  Issue slots and the latency of dependent gathers bound it, so resident
+// warps matter more than registers: 1080p, 3 frames, 3x3 window, 48 against 40 registers: 4 views
+// 0.283 and 0.269 ms, 6 views 0.402 and 0.368.
 constexpr int REPROJ_REGS = 48;
 constexpr int REPROJ_REGS_MANY_VIEWS = 40;
 constexpr int REPROJ_MANY_VIEWS = 4;
@@ -118,6 +115,7 @@ struct alignas(16) FrameParams
     int32_t n_views, n_aux, n_frames, linear, chain;
     int32_t use_tma;          // key tiles fetched by TMA (every view's row pitch a multiple of 16 bytes)
     int32_t row_pairs;        // pairs of output rows per reprojection block
+    int32_t group_frames;     // frames whose results a reprojection block holds at a time
     // Failure-detection test hook: the reprojection block with this linear index
     // (blockIdx.y * gridDim.x + blockIdx.x) announces its tile bytes but issues no copy,
     // so its bounded wait runs out after `wait_limit` polls; -1 = none.  0 = default limit.
@@ -549,8 +547,8 @@ struct Tile
 
 __device__ __forceinline__ int tile_x0(uint32_t tx0, int sw) { return ((int)tx0 - sw) & ~1; }
 
-// A reprojection block works through units = (frame, pair of output rows): n_frames x
-// row_pairs of them.  Bytes at the start of its shared memory: the key tiles of one unit
+// A reprojection block works through units = (frame, pair of output rows), group_frames x
+// row_pairs of them at a time.  Bytes at the start of its shared memory: the key tiles of one unit
 // (every view) in phase 1, then (the tiles are dead by then) the chained colours and flags
 // of phases 2-3.  A multiple of 128, so the results that follow stay aligned.
 template <int SW>
@@ -614,7 +612,7 @@ __device__ __forceinline__ CamRes cam_result(const DirRes &f, const DirRes &b, c
 // write (false: keep the previous output), src/renderer.cu:400-465.
 // res points at the [n_views][32] results of this pixel's row and frame.
 template <bool MAV, bool SQ>
-__device__ __forceinline__ bool resolve_pixel(const DirRes *res, int lane, const FrameParams &p, const FrameCfg &c, uint32_t &color)
+__device__ __forceinline__ bool resolve_pixel(const DirRes *res, int lane, const FrameParams &p, int n_cams, const FrameCfg &c, uint32_t &color)
 {
     const CamRes m = cam_result<SQ>(res[lane], res[32 + lane], p.v[0], p.v[1], ERR_EPS_1_FULL_RES<SQ>, EPS_2_FULL_RES, MAV);
     CamRes best;
@@ -624,7 +622,6 @@ __device__ __forceinline__ bool resolve_pixel(const DirRes *res, int lane, const
     best.error = 0u;
     best.depth = 0.0f;
     int best_cam = 0;
-    const int n_cams = p.n_views / 2;
     for (int cam = 1; cam < n_cams; cam++)
     {
         const CamRes r = cam_result<SQ>(res[(2 * cam) * 32 + lane], res[(2 * cam + 1) * 32 + lane], p.v[2 * cam], p.v[2 * cam + 1],
@@ -818,7 +815,9 @@ __host__ __device__ __forceinline__ void window_keys(const unsigned long long *t
 // a block barrier per unit, each unit waited for its slowest view and for the copy:
 // calls of 3 frames at 1080p with 6 views 0.762 -> 0.709 ms, of 6 frames at 2064x2208 with 2 views
 // 1.375 -> 1.227 ms.)
-// More row pairs per block (for single frames) keep every warp busy in phase 2.
+// More row pairs per block (for single frames) keep every warp busy in phase 2.  The frames are
+// taken in groups: a block's results of all frames at once (12 bytes per view, row, frame and
+// lane) would leave the SM with fewer resident blocks than its registers allow.
 // One reprojection block (bx, by) of frame batch p, executed by a block of (32, n_views)
 // threads: the body of reproj_kernel, also run as a work unit of batch_kernel.  `maps`: the
 // views' key-tile tensor maps; `bars`: the warps' TMA completion barriers, initialised once per
@@ -828,23 +827,30 @@ __host__ __device__ __forceinline__ void window_keys(const unsigned long long *t
 // `block_id`: the index the test hook `withhold_block` refers to, compiled in only where HOOK is
 // set.  Every thread returns together (early exits are block-uniform or come after the last
 // barrier).
-template <int SW, int SI, bool MAV, int REGS, bool HOOK = false>
+template <int SW, int SI, bool MAV, int REGS, int NV = 0, bool HOOK = false>
 __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtensorMap *maps, uint32_t bx, uint32_t by, uint32_t block_id,
                                              unsigned char *smem, unsigned long long *bars, int &round, volatile uint32_t &aborted)
 {
     using T = Tile<SW>;
-    const int nv = p.n_views, nf = p.n_frames, np = p.row_pairs, nu = nf * np;
+    const int nv = NV ? NV : p.n_views, nf = p.n_frames, np = p.row_pairs, gu = p.group_frames * np;
     // [key tiles, phase 1 | chained colours and flags, phases 2-3 (same bytes)][results][barriers]
     unsigned long long *tiles = reinterpret_cast<unsigned long long *>(smem);                 // [nv][H][W]
-    uint32_t *cols = reinterpret_cast<uint32_t *>(smem);                                      // [nu][ROWS][32]
-    uint32_t *valid = cols + nu * ROWS * 32;                                                 // [nu][ROWS][32]
-    DirRes *res = reinterpret_cast<DirRes *>(smem + reproj_tile_region<SW>(nv, nu));         // [nu][ROWS][nv][32]
+    uint32_t *cols = reinterpret_cast<uint32_t *>(smem);                                      // [gu][ROWS][32]
+    uint32_t *valid = cols + gu * ROWS * 32;                                                 // [gu][ROWS][32]
+    DirRes *res = reinterpret_cast<DirRes *>(smem + reproj_tile_region<SW>(nv, gu));         // [gu][ROWS][nv][32]
 
     // the warp's view; the shuffle tells the compiler that it is the same for the whole warp, so
     // that the view's fields are read and indexed on the uniform datapath
     const int lane = threadIdx.x, vw = __shfl_sync(0xffffffffu, (int)threadIdx.y, 0);
     const uint32_t x0 = bx * 32, x = x0 + lane, yb = by * (ROWS * np);
     const bool xok = x < p.out_w;
+    uint32_t run = 0; // phase 3: the persistent buffer's pixel of this thread, carried from group to group
+#pragma unroll 1
+    for (int g0 = 0; g0 < nf; g0 += p.group_frames)
+    {
+    const int gn = min(p.group_frames, nf - g0), nu = gn * np;
+    if (g0 > 0)
+        __syncthreads(); // the previous group's phases are done with the shared memory
     {
         const DevView &v = p.v[vw];
         const uint32_t ix = v.sx == 1 ? x : x / v.sx, tx0 = v.sx == 1 ? x0 : x0 / v.sx;
@@ -864,7 +870,7 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
             tma_load_3d(tg, &maps[vw], xs, (int)(v.sy == 1 ? y0 : y0 / v.sy) - SW, k, bar);
         };
         if (p.use_tma && lane == 0)
-            fetch(0, 0);
+            fetch(0, g0);
         // pixel2CS of the output pixels in the main view (the search target) and in this view (the error)
         const DevView &v0 = p.v[0];
         const uint32_t xc = min(x, p.out_w - 1);
@@ -872,6 +878,10 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
         const float pcx = __ldg(v.lut + min(ix, v.w - 1));
         const uint32_t vwid = v.w, vhei = v.h;
         const float half_w = (float)vwid * 0.5f, half_h = (float)vhei * 0.5f;
+        // the scale res / min(res) (src/renderer.cu:213): the host's IEEE quotient, or under the
+        // reference's GPU semantics its device division
+        const float esx = FAST_MATH ? xdiv((float)vwid, (float)min(vwid, vhei)) : v.err_sx;
+        const float esy = FAST_MATH ? xdiv((float)vhei, (float)min(vwid, vhei)) : v.err_sy;
         bool arrived = true;
 #pragma unroll 1
         for (int rp = 0; rp < np && arrived; rp++)
@@ -883,9 +893,9 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
             const float qy[ROWS] = {__ldg(v0.lut + v0.w + y0c), __ldg(v0.lut + v0.w + y1c)};
             const float pcy[ROWS] = {__ldg(v.lut + v.w + min(iy0, vhei - 1)), __ldg(v.lut + v.w + min(iy1, vhei - 1))};
 #pragma unroll 1
-            for (int k = 0; k < nf; k++)
+            for (int j = 0; j < gn; j++)
             {
-                const int u = k * np + rp;
+                const int k = g0 + j, u = j * np + rp;
                 if (p.use_tma)
                 {
                     // A warp whose copy did not arrive reads nothing more, starts no further copy (an
@@ -925,11 +935,11 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                 float d_init[ROWS];
                 KeyWords key[ROWS];
                 window_keys<SW>(tg, col, (int)(iy1 - iy0), rok, key);
-                if (p.use_tma && (k + 1 < nf || rp + 1 < np))
+                if (p.use_tma && (j + 1 < gn || rp + 1 < np))
                 {
                     __syncwarp(); // every lane has read the tile
                     if (lane == 0)
-                        fetch(k + 1 < nf ? rp : rp + 1, k + 1 < nf ? k + 1 : 0);
+                        fetch(j + 1 < gn ? rp : rp + 1, j + 1 < gn ? k + 1 : g0);
                 }
 #pragma unroll
                 for (int r = 0; r < ROWS; r++)
@@ -943,11 +953,6 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                     // (empty windows) and even if a tile were stale
                     ax[r] = min(ax[r], vwid - 1u);
                     ay[r] = min(ay[r], vhei - 1u);
-                    // the depth read after the search is mostly at or next to the start (a
-                    // splatted source pixel, in range): fetch its line into L1 during the search
-                    // (3x3 window, 6 views: 0.537 -> 0.533 ms; no gain for the 7x7 window)
-                    if (SW == 1 && s[r])
-                        asm volatile("prefetch.global.L1 [%0];" ::"l"(cdep + (ay[r] * vwid + ax[r])));
                 }
                 // iterativeSearch<SI>, src/renderer.cu:177-202, both rows interleaved.  The start is a
                 // splatted source pixel and every accepted step is in range: no border handling needed.
@@ -986,10 +991,6 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
 #pragma unroll
                 for (int r = 0; r < ROWS; r++)
                 {
-                    // the scale res / min(res) (src/renderer.cu:213): the host's IEEE quotient, or
-                    // under the reference's GPU semantics its device division
-                    const float esx = FAST_MATH ? xdiv((float)vwid, (float)min(vwid, vhei)) : v.err_sx;
-                    const float esy = FAST_MATH ? xdiv((float)vhei, (float)min(vwid, vhei)) : v.err_sy;
                     const float ex = xmul(xsub(xadd(fx[r], m[r].x), pcx), esx);
                     const float ey = xmul(xsub(xadd(fy[r], m[r].y), pcy[r]), esy);
                     DirRes d;
@@ -1013,11 +1014,12 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
     for (int t = vw; t < nu * ROWS; t += nv)
     {
         const int u = t / ROWS, r = t % ROWS;
-        // u = k * np + rp; np is 1..3 (the host's choice), so no general division
-        const int k = np == 1 ? u : (np == 2 ? (u >> 1) : (np == 3 ? u / 3 : u / np));
-        const uint32_t y = yb + (uint32_t)(u - k * np) * ROWS + r;
+        // u = j * np + rp; np is 1..3 (the host's choice), so no general division
+        const int j = np == 1 ? u : (np == 2 ? (u >> 1) : (np == 3 ? u / 3 : u / np));
+        const int k = g0 + j;
+        const uint32_t y = yb + (uint32_t)(u - j * np) * ROWS + r;
         uint32_t color = 0;
-        const bool ok = xok && y < p.out_h && resolve_pixel<MAV, SQUARED_ERRORS<REGS>>(res + t * nv * 32, lane, p, p.f[k], color);
+        const bool ok = xok && y < p.out_h && resolve_pixel<MAV, SQUARED_ERRORS<REGS>>(res + t * nv * 32, lane, p, nv / 2, p.f[k], color);
         if (!p.chain)
         {
             if (ok)
@@ -1030,19 +1032,17 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
         }
     }
     if (!p.chain)
-        return;
+        continue;
     __syncthreads();
     // phase 3: one persistent buffer per row, starting as out[0], copied to out[k] after frame k
-    if (vw >= np * ROWS)
-        return;
     const uint32_t y = yb + vw; // row vw of the block: row vw % ROWS of row pair vw / ROWS
-    if (!xok || y >= p.out_h)
-        return;
-    uint32_t run = 0;
-    for (int k = 0; k < nf; k++)
+    if (vw >= np * ROWS || !xok || y >= p.out_h)
+        continue;
+    for (int j = 0; j < gn; j++)
     {
+        const int k = g0 + j;
         uint32_t *o = p.out[k] + (y * p.out_w + x);
-        const int t = (k * np + vw / ROWS) * ROWS + vw % ROWS;
+        const int t = (j * np + vw / ROWS) * ROWS + vw % ROWS;
         if (k == 0)
             run = *o;
         if (valid[t * 32 + lane])
@@ -1053,23 +1053,32 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
         else if (k > 0)
             *o = run;
     }
+    }
 }
+
+// Registers that reproj_kernel is built with under a cap, for a constant view count (nv; 0: known
+// at run time only).  With the view count a constant, the two-view kernel of the 3x3 window and
+// those of the 7x7 window fit into 40 registers without spills, and more resident warps make them
+// faster: 6 frames at 2064x2208, 2 views 0.728 -> 0.685 ms (32 registers: 0.728, spills); 3 frames
+// at 1366x768, 4 views, 7x7 0.367 (56) -> 0.357 (48) -> 0.354 ms.
+constexpr int reproj_regs(int sw, int cap, int nv) { return nv != 0 && (sw == 3 || nv == 2) ? REPROJ_REGS_MANY_VIEWS : cap; }
 
 // bidirectionalReprojection_kernel<SW, SI, MAIN_ALWAYS_VALID>, src/renderer.cu:400-465
 // block = (32, n_views): 32 output columns x (2 * row_pairs) output rows, one warp per source
 // view (reproj_block).
 // HOOK: built with the failure-detection test hook (FrameParams::withhold_block); the
 // launch uses that instance only when the hook is armed.
-template <int SW, int SI, bool MAV, int REGS, bool HOOK = false>
-__global__ void __maxnreg__(REGS) reproj_kernel(const __grid_constant__ FrameParams p, const __grid_constant__ KeyMaps km)
+// NV: the number of source views, or 0 where it is only known at run time.
+template <int SW, int SI, bool MAV, int REGS, int NV, bool HOOK = false>
+__global__ void __maxnreg__(reproj_regs(SW, REGS, NV)) reproj_kernel(const __grid_constant__ FrameParams p, const __grid_constant__ KeyMaps km)
 {
     // dynamic shared memory only (no static __shared__ in front of it): the key tiles start at
     // the 1 KiB-aligned window base, so every TMA destination is 128-byte aligned
     extern __shared__ __align__(1024) unsigned char smem[];
+    const int nv = NV ? NV : p.n_views, gu = p.group_frames * p.row_pairs;
     unsigned long long *bars = reinterpret_cast<unsigned long long *>(
-        smem + reproj_tile_region<SW>(p.n_views, p.n_frames * p.row_pairs) +
-        (size_t)p.n_frames * p.row_pairs * ROWS * p.n_views * 32 * sizeof(DirRes)); // TMA completion barriers, one per warp
-    volatile uint32_t &aborted = *reinterpret_cast<volatile uint32_t *>(bars + p.n_views);
+        smem + reproj_tile_region<SW>(nv, gu) + (size_t)gu * ROWS * nv * 32 * sizeof(DirRes)); // TMA completion barriers, one per warp
+    volatile uint32_t &aborted = *reinterpret_cast<volatile uint32_t *>(bars + nv);
     if (threadIdx.x == 0)
     {
         if (p.use_tma)
@@ -1079,7 +1088,7 @@ __global__ void __maxnreg__(REGS) reproj_kernel(const __grid_constant__ FramePar
     }
     __syncthreads();
     int round = 0;
-    reproj_block<SW, SI, MAV, REGS, HOOK>(p, km.m, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x, smem, bars, round, aborted);
+    reproj_block<SW, SI, MAV, REGS, NV, HOOK>(p, km.m, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x, smem, bars, round, aborted);
 }
 
 // ---- timewarp (mode 4), src/renderer.cu:467-522, 615-629 ----

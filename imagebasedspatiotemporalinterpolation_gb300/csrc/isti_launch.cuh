@@ -151,12 +151,32 @@ int rule_regs(int sw, int n_views, int n_frames, int row_pairs)
                : isti::REPROJ_REGS_MANY_VIEWS;
 }
 
-// The rule's launch for a frame batch (register cap and row pairs; TMA key tiles).
-ReprojChoice rule_choice(int sw, const isti::FrameParams &p)
+// Frames whose results a block holds at a time: as many as cost no resident block, in groups of
+// about equal size.  More frames per group share the block's start (its tables and barriers), but
+// 12 bytes per view, row, frame and lane soon leave fewer resident blocks than the registers do
+// (2064x2208, 2 views, 6 frames in one group 0.791 ms, in two 0.764; 1080p, 6 views 0.783 and 0.735).
+int rule_group_frames(int sw, int regs, int n_views, int n_frames, int row_pairs)
 {
-    const int rp = rule_row_pairs(p.n_views, p.n_frames);
-    return ReprojChoice{rule_regs(sw, p.n_views, p.n_frames, rp), rp, 0};
+    auto blocks = [&](int frames) {
+        const int units = frames * row_pairs;
+        return resident_blocks(regs, n_views, sw == 1 ? isti::reproj_smem<1>(n_views, units) : isti::reproj_smem<3>(n_views, units));
+    };
+    int most = 1;
+    while (most < n_frames && blocks(most + 1) == blocks(1))
+        most++;
+    const int groups = (n_frames + most - 1) / most;
+    return (n_frames + groups - 1) / groups;
 }
+
+// The rule's launch for a frame batch (register cap and row pairs; TMA key tiles).  The cap is
+// the rule's for the frames of one group.
+ReprojChoice rule_choice(int sw, int n_views, int n_frames)
+{
+    const int rp = rule_row_pairs(n_views, n_frames);
+    const int least = sw != 1 ? isti::REPROJ_REGS_WIDE_WINDOW : isti::REPROJ_REGS_MANY_VIEWS;
+    return ReprojChoice{rule_regs(sw, n_views, rule_group_frames(sw, least, n_views, n_frames, rp), rp), rp, 0};
+}
+ReprojChoice rule_choice(int sw, const isti::FrameParams &p) { return rule_choice(sw, p.n_views, p.n_frames); }
 
 template <int SW, int SI, bool MAV, int REGS>
 cudaError_t launch_reproj_regs(isti::FrameParams &p, cudaStream_t stream, int row_pairs, bool plain_tiles)
@@ -176,6 +196,9 @@ cudaError_t launch_reproj_regs(isti::FrameParams &p, cudaStream_t stream, int ro
     // its unchained output (the persistent buffer is out[0] itself), so that launch runs unchained.
     if (p.chain && p.n_frames > 1)
         p.row_pairs = std::min(p.row_pairs, std::max(1, p.n_views / isti::ROWS));
+    // the view count as a constant for one to three cameras (NV index 1..3), else at run time
+    const int nvi = p.n_views <= 6 ? p.n_views / 2 : 0;
+    p.group_frames = rule_group_frames(SW, isti::reproj_regs(SW, REGS, 2 * nvi), p.n_views, p.n_frames, p.row_pairs);
     static thread_local isti::KeyMaps km; // 2 KiB, passed by value as a kernel parameter
     // the maps depend only on the key buffers' addresses and shapes: encode them again only
     // when those changed (a renderer reuses its arena from call to call)
@@ -205,23 +228,26 @@ cudaError_t launch_reproj_regs(isti::FrameParams &p, cudaStream_t stream, int ro
         last = key;
     }
     p.use_tma = (!plain_tiles && last_tma == 1) ? 1 : 0;
-    const size_t smem = isti::reproj_smem<SW>(p.n_views, p.n_frames * p.row_pairs);
+    const size_t smem = isti::reproj_smem<SW>(p.n_views, p.group_frames * p.row_pairs);
     const uint32_t block_rows = (uint32_t)(isti::ROWS * p.row_pairs);
     const dim3 gr((p.out_w + 31) / 32, (p.out_h + block_rows - 1) / block_rows);
     p.withhold_block = -1;
     if (p.withhold_x >= 0 && p.withhold_y >= 0 && (uint32_t)p.withhold_x < p.out_w && (uint32_t)p.withhold_y < p.out_h)
         p.withhold_block = (int32_t)(((uint32_t)p.withhold_y / block_rows) * gr.x + (uint32_t)p.withhold_x / 32u);
     const bool hook = p.withhold_block >= 0 && p.use_tma;
-    auto kernel = hook ? isti::reproj_kernel<SW, SI, MAV, REGS, true> : isti::reproj_kernel<SW, SI, MAV, REGS, false>;
+    using Kernel = void (*)(isti::FrameParams, isti::KeyMaps);
+    constexpr Kernel kernels[4] = {isti::reproj_kernel<SW, SI, MAV, REGS, 0>, isti::reproj_kernel<SW, SI, MAV, REGS, 2>,
+                                   isti::reproj_kernel<SW, SI, MAV, REGS, 4>, isti::reproj_kernel<SW, SI, MAV, REGS, 6>};
+    const Kernel kernel = hook ? isti::reproj_kernel<SW, SI, MAV, REGS, 0, true> : kernels[nvi];
     // raise the kernel's dynamic shared-memory limit once to the largest size requested, so
     // that calls inside a CUDA graph capture make no attribute calls after a first uncaptured
     // call of the same shape
     static std::mutex attr_mutex;
-    static int attr_set[2][64] = {}; // per kernel instance and device
+    static int attr_set[5][64] = {}; // per kernel instance and device
     if (smem > 48 * 1024)
     {
         std::lock_guard<std::mutex> lock(attr_mutex);
-        int &cur = attr_set[hook ? 1 : 0][dev & 63];
+        int &cur = attr_set[hook ? 4 : nvi][dev & 63];
         if ((int)smem > cur)
         {
             e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -242,7 +268,7 @@ template <int SW, int SI, bool MAV>
 cudaError_t launch_reproj(isti::FrameParams &p, cudaStream_t stream, ReprojChoice c)
 {
     const int rp = c.row_pairs > 0 ? std::min(c.row_pairs, 3) : rule_row_pairs(p.n_views, p.n_frames);
-    const int regs = c.regs > 0 ? c.regs : rule_regs(SW, p.n_views, p.n_frames, rp);
+    const int regs = c.regs > 0 ? c.regs : rule_choice(SW, p).regs;
     if constexpr (SW == 1)
     {
         if (regs == isti::REPROJ_REGS_MANY_VIEWS)

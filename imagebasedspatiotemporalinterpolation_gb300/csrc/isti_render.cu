@@ -914,10 +914,11 @@ extern "C" isti_status isti_render_pairs(isti_renderer *r, int32_t n_pairs, cons
         off += align_up(layouts[i].total, 256);
         p.status = dstatus;
         p.row_pairs = isti::rule_row_pairs(nv, pf.n_frames);
+        p.group_frames = isti::rule_group_frames(sw, regs, nv, pf.n_frames, p.row_pairs);
         isti::KeyMaps km;
         p.use_tma = (sw == 1 ? pair_maps<1>(p, km) : pair_maps<3>(p, km)) ? 1 : 0;
         std::memcpy(hmaps + (size_t)i * isti::MAX_VIEWS, km.m, sizeof(CUtensorMap) * nv);
-        const int nu = pf.n_frames * p.row_pairs;
+        const int nu = p.group_frames * p.row_pairs;
         const size_t reg = (sw == 1 ? isti::reproj_tile_region<1>(nv, nu) : isti::reproj_tile_region<3>(nv, nu)) +
                            (size_t)nu * isti::ROWS * nv * 32 * sizeof(isti::DirRes);
         region = std::max(region, align_up(reg, 16));

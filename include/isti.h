@@ -274,7 +274,8 @@ isti_status isti_renderer_set_autotune(isti_renderer *r, int32_t on);
  * register cap (40 or 48 for the 3x3 window, 56 for the 7x7 window; 0: the rule's), output
  * row pairs per block (1..3; 0: the rule's) and key tiles by plain loads (1) or TMA copies
  * where the views allow them (0).  A cap the render mode is not built with takes the mode's
- * own (48 for the 3x3 window, 56 for the 7x7).  A pinned launch takes precedence over a
+ * own (48 for the 3x3 window, 56 for the 7x7).  A cap is an upper bound: kernels built for
+ * one to three cameras may take fewer.  A pinned launch takes precedence over a
  * tuned one.  The output does not depend on it.  ISTI_ERR_INVALID_ARG for other values. */
 isti_status isti_renderer_set_reproj_launch(isti_renderer *r, int32_t regs, int32_t row_pairs, int32_t plain_tiles);
 
