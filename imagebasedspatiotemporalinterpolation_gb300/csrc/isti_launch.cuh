@@ -16,6 +16,24 @@
 
 namespace isti
 {
+// Launches a kernel whose prerequisite is the kernel enqueued just before it; `early`: as a
+// programmatic dependent launch (the kernel waits by itself), otherwise in full order.
+template <class... P, class... A>
+cudaError_t launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A &...args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Enqueues the timewarp of one batch (src/renderer.cu:615-629): mean z of the forward
 // keyframe (two kernels), then one kernel over the output pixels.
 cudaError_t launch_timewarp(isti::FrameParams &p, char *base, cudaStream_t stream, cudaEvent_t after_mean, cudaEvent_t after_nothing)
@@ -23,13 +41,14 @@ cudaError_t launch_timewarp(isti::FrameParams &p, char *base, cudaStream_t strea
     p.tw_rows = reinterpret_cast<isti::TwRow *>(base);
     p.tw_plane = reinterpret_cast<float4 *>(base + ((size_t)p.v[0].h * sizeof(isti::TwRow) + 255) / 256 * 256);
     isti::timewarp_rowsum_kernel<<<p.v[0].h, isti::TW_THREADS, 0, stream>>>(p);
-    isti::timewarp_mean_kernel<<<1, isti::TW_THREADS, 0, stream>>>(p);
+    cudaError_t e = launch_after(true, isti::timewarp_mean_kernel, 1, isti::TW_THREADS, 0, stream, p);
+    if (e != cudaSuccess)
+        return e;
     if (after_mean)
         cudaEventRecord(after_mean, stream);
     if (after_nothing)
         cudaEventRecord(after_nothing, stream); // no splat stage in this mode
-    isti::timewarp_kernel<<<dim3((p.out_w + 31) / 32, (p.out_h + 7) / 8), dim3(32, 8), 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_after(!after_nothing, isti::timewarp_kernel, dim3((p.out_w + 31) / 32, (p.out_h + 7) / 8), dim3(32, 8), 0, stream, p);
 }
 
 // ---- tensor maps for the TMA-staged key tiles ----
@@ -179,7 +198,7 @@ ReprojChoice rule_choice(int sw, int n_views, int n_frames)
 ReprojChoice rule_choice(int sw, const isti::FrameParams &p) { return rule_choice(sw, p.n_views, p.n_frames); }
 
 template <int SW, int SI, bool MAV, int REGS>
-cudaError_t launch_reproj_regs(isti::FrameParams &p, cudaStream_t stream, int row_pairs, bool plain_tiles)
+cudaError_t launch_reproj_regs(isti::FrameParams &p, cudaStream_t stream, int row_pairs, bool plain_tiles, bool early)
 {
     // One unit's key tiles per TMA round: the least shared memory per block, so the most
     // resident blocks and the largest L1 (1080p, 6 views, 3 frames, 8 blocks per SM: one
@@ -259,24 +278,24 @@ cudaError_t launch_reproj_regs(isti::FrameParams &p, cudaStream_t stream, int ro
     const int32_t chain = p.chain;
     if (p.n_frames == 1)
         p.chain = 0;
-    kernel<<<gr, dim3(32, p.n_views), smem, stream>>>(p, km);
+    e = launch_after(early, kernel, gr, dim3(32, p.n_views), smem, stream, p, km);
     p.chain = chain;
-    return cudaGetLastError();
+    return e;
 }
 
 template <int SW, int SI, bool MAV>
-cudaError_t launch_reproj(isti::FrameParams &p, cudaStream_t stream, ReprojChoice c)
+cudaError_t launch_reproj(isti::FrameParams &p, cudaStream_t stream, ReprojChoice c, bool early)
 {
     const int rp = c.row_pairs > 0 ? std::min(c.row_pairs, 3) : rule_row_pairs(p.n_views, p.n_frames);
     const int regs = c.regs > 0 ? c.regs : rule_choice(SW, p).regs;
     if constexpr (SW == 1)
     {
         if (regs == isti::REPROJ_REGS_MANY_VIEWS)
-            return launch_reproj_regs<SW, SI, MAV, isti::REPROJ_REGS_MANY_VIEWS>(p, stream, rp, c.plain_tiles != 0);
-        return launch_reproj_regs<SW, SI, MAV, isti::REPROJ_REGS>(p, stream, rp, c.plain_tiles != 0);
+            return launch_reproj_regs<SW, SI, MAV, isti::REPROJ_REGS_MANY_VIEWS>(p, stream, rp, c.plain_tiles != 0, early);
+        return launch_reproj_regs<SW, SI, MAV, isti::REPROJ_REGS>(p, stream, rp, c.plain_tiles != 0, early);
     }
     else
-        return launch_reproj_regs<SW, SI, MAV, isti::REPROJ_REGS_WIDE_WINDOW>(p, stream, rp, c.plain_tiles != 0);
+        return launch_reproj_regs<SW, SI, MAV, isti::REPROJ_REGS_WIDE_WINDOW>(p, stream, rp, c.plain_tiles != 0, early);
 }
 
 // window size of the reprojection of a render mode (src/renderer.cu:676-693)
@@ -290,17 +309,18 @@ std::vector<int> mode_regs(int mode)
     return {isti::REPROJ_REGS_WIDE_WINDOW};
 }
 
-cudaError_t launch_reproj_mode(isti::FrameParams &p, int mode, cudaStream_t stream, ReprojChoice c)
+// early: the kernel enqueued just before is the batch's splat
+cudaError_t launch_reproj_mode(isti::FrameParams &p, int mode, cudaStream_t stream, ReprojChoice c, bool early = false)
 {
     switch (mode)
     {
     case ISTI_MODE_OURS:
     case ISTI_MODE_BACKWARD_UNIDIRECTIONAL:
-        return launch_reproj<1, 3, false>(p, stream, c);
+        return launch_reproj<1, 3, false>(p, stream, c, early);
     case ISTI_MODE_SPLATTING:
-        return launch_reproj<1, 0, false>(p, stream, c);
+        return launch_reproj<1, 0, false>(p, stream, c, early);
     case ISTI_MODE_BACKWARD_BIDIRECTIONAL:
-        return launch_reproj<3, 5, true>(p, stream, c);
+        return launch_reproj<3, 5, true>(p, stream, c, early);
     }
     return cudaGetLastError();
 }
@@ -325,10 +345,12 @@ cudaError_t launch_batch(isti::FrameParams &p, int mode, cudaStream_t stream, cu
     if (after_init)
         cudaEventRecord(after_init, stream);
     const dim3 gs((max_w + 31) / 32, (max_h + 7) / 8, p.n_views);
-    isti::splat_kernel<<<gs, dim3(32, 8), 0, stream>>>(p);
+    const cudaError_t e = launch_after(!after_init, isti::splat_kernel, gs, dim3(32, 8), 0, stream, p);
+    if (e != cudaSuccess)
+        return e;
     if (after_splat)
         cudaEventRecord(after_splat, stream);
-    return launch_reproj_mode(p, mode, stream, choice);
+    return launch_reproj_mode(p, mode, stream, choice, !after_splat);
 }
 
 } // namespace isti
