@@ -191,27 +191,6 @@ __global__ void poolback_kernel(const bf16 *gskip, const bf16 *gq, const bf16 *a
     }
 }
 
-// Per-block partial sums over pixels of every channel: partial[block][c].  blockDim = 256,
-// c <= 256: the first (256 / c) * c threads take a channel each.
-__global__ void colsum_partial_kernel(const bf16 *g, size_t npix, int c, float *partial)
-{
-    __shared__ float red[256];
-    const int ch = threadIdx.x % c, lane_pix = threadIdx.x / c, ppb = 256 / c;
-    float acc = 0.0f;
-    if (lane_pix < ppb)
-        for (size_t p = (size_t)blockIdx.x * ppb + lane_pix; p < npix; p += (size_t)gridDim.x * ppb)
-            acc += __bfloat162float(g[p * c + ch]);
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x < c)
-    {
-        float s = 0.0f;
-        for (int k = 0; k < ppb; k++)
-            s += red[k * c + threadIdx.x];
-        partial[(size_t)blockIdx.x * c + threadIdx.x] = s;
-    }
-}
-
 // out[i] = sum over blocks of partial[block][i] (fixed order)
 __global__ void sum_partials_kernel(const float *partial, int blocks, int n, float *out)
 {
@@ -513,16 +492,8 @@ isti_status dgrad(isti_flownet *net, int l, const bf16 *g_out, int n, int h, int
 isti_status wgrad(isti_flownet *net, int l, const bf16 *g_out, const bf16 *x, int n, int h, int w, Buffers &b, cudaStream_t s)
 {
     const LayerDef &d = LAYERS[l];
-    isti_status st = isti_unet::wgrad_launch(d.taps, g_out, x, n, h, w, d.cin, d.cout, net->grads + net->w_off[l], 0, b.wscratch,
-                                             b.wscratch_bytes, net->status, s);
-    if (st != ISTI_OK)
-        return st;
-    // bias gradient: column sums of g_out
-    const size_t npix = (size_t)n * h * w;
-    colsum_partial_kernel<<<REDUCE_BLOCKS, 256, 0, s>>>(g_out, npix, d.cout, b.partial);
-    sum_partials_kernel<<<(d.cout + 127) / 128, 128, 0, s>>>(b.partial, REDUCE_BLOCKS, d.cout, net->grads + net->b_off[l]);
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "bias gradient");
+    return isti_unet::wgrad_launch(d.taps, g_out, x, n, h, w, d.cin, d.cout, net->grads + net->w_off[l], net->grads + net->b_off[l], 0, b.wscratch,
+                                   b.wscratch_bytes, net->status, s);
 }
 
 #define ISTI_TRY(x)                                                                                                                             \

@@ -255,69 +255,125 @@ isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, c
     return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "isti_unet_conv launch");
 }
 
-int wgrad_splits(int taps, int n_tiles)
+// The weight gradient's work split (wgrad_kernel) and its scratch.
+struct WgradConfig
 {
-    // about four CTAs per SM over all taps, at least 8 pixel tiles each
-    const int want = std::max(1, (152 * 4) / taps);
-    return std::max(1, std::min(want, (n_tiles + 7) / 8));
+    int n, h, w;              // the image, 1x1 layers as one row of pixels
+    int kseg, segs, n_units;
+    int n_dy, n_mb;           // per CTA
+    int grid_y, grid_z, splits, units_per_split, stages;
+    size_t smem;
+};
+
+bool wgrad_config(int taps, int n, int h, int w, int cin, int cout, WgradConfig &c)
+{
+    c = WgradConfig{};
+    c.n = taps == 9 ? n : 1;
+    c.h = taps == 9 ? h : 1;
+    const long long row = taps == 9 ? w : (long long)n * h * w;
+    if (row > INT32_MAX - 256)
+        return false;
+    c.w = (int)row;
+    const int mblocks = ((taps == 9 ? 3 : 1) * cout + 127) / 128;
+    c.n_dy = taps == 9 ? 3 : 1;
+    c.n_mb = mblocks;
+    // all accumulators of a CTA in the 512 TMEM columns: else one row (dy) per CTA, then one M block
+    if (c.n_dy == 3 && c.n_mb * wgrad_mb_cols(cin, 3) > 512)
+        c.n_dy = 1;
+    if (c.n_mb * wgrad_mb_cols(cin, c.n_dy) > 512)
+        c.n_mb = 1;
+    c.grid_y = taps == 9 && c.n_dy == 1 ? 3 : 1;
+    c.grid_z = mblocks / c.n_mb;
+    // 128 pixels per unit where three stages of them fit and the rows are that long, else 64
+    for (c.kseg = 128;; c.kseg = 64)
+    {
+        const size_t sb = wgrad_stage_bytes(cin, c.n_dy, c.n_mb, c.kseg);
+        c.stages = (int)std::min<size_t>(6, (SMEM_BUDGET - 256) / sb);
+        if (c.kseg == 64 || (c.stages >= 3 && c.w > 64))
+        {
+            c.smem = c.stages * sb + (2 * c.stages + 1) * 8 + 16;
+            break;
+        }
+    }
+    c.segs = (c.w + c.kseg - 1) / c.kseg;
+    c.n_units = c.n * c.h * c.segs;
+    // one CTA per SM, at least 4 units each
+    c.splits = std::max(1, std::min(152 / (c.grid_y * c.grid_z), (c.n_units + 3) / 4));
+    c.units_per_split = (c.n_units + c.splits - 1) / c.splits;
+    return c.stages >= 2;
 }
 
 size_t wgrad_scratch(int taps, int n, int h, int w, int cin, int cout)
 {
-    const int n_tiles = n * ((w + TILE_W - 1) / TILE_W) * ((h + TILE_H - 1) / TILE_H);
-    return (size_t)wgrad_splits(taps, n_tiles) * cout * taps * cin * sizeof(float);
+    WgradConfig c;
+    if ((taps != 9 && taps != 1) || n < 1 || h < 1 || w < 1 || cin < 16 || cout < 16 || !wgrad_config(taps, n, h, w, cin, cout, c))
+        return 0;
+    return (size_t)c.splits * cout * ((size_t)taps * cin + 1) * sizeof(float);
 }
 
-isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, int w, int cin, int cout, float *dw, int accumulate, void *scratch,
-                         size_t scratch_bytes, int32_t *status, cudaStream_t stream)
+// 5-D map over an NHWC bf16 tensor, the channels split as (8, c / 8) and the chunk index
+// outermost: box {8, kseg x, rows, chunks, 1}.
+isti_status nhwc_segment_map(CUtensorMap &m, const void *base, int n, int h, int w, int c, int kseg, int rows, int chunks)
 {
-    if ((taps != 9 && taps != 1) || n < 1 || h < 1 || w < 1 || cin % 16 || cout % 16 || cin < 16 || cin > 256 || cout > 128 || !dy || !x ||
-        !dw || !scratch)
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc)
+        return isti::set_error(ISTI_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
+    if (((uintptr_t)base & 15u) || c % 8)
+        return isti::set_error(ISTI_ERR_INVALID_ARG, "NHWC tensor: base 16-byte aligned, channels a multiple of 8");
+    const cuuint64_t dims[5] = {8, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)(c / 8), (cuuint64_t)n};
+    const cuuint64_t strides[4] = {(cuuint64_t)c * 2u, (cuuint64_t)w * c * 2u, 16u, (cuuint64_t)h * w * c * 2u};
+    const cuuint32_t box[5] = {8, (cuuint32_t)kseg, (cuuint32_t)rows, (cuuint32_t)chunks, 1};
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    if (enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return isti::set_error(ISTI_ERR_INVALID_ARG, "cuTensorMapEncodeTiled rejected an NHWC tensor");
+    return ISTI_OK;
+}
+
+isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, int w, int cin, int cout, float *dw, float *db, int accumulate,
+                         void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream)
+{
+    if ((taps != 9 && taps != 1) || n < 1 || h < 1 || w < 1 || cin % 16 || cout % 16 || cin < 16 || cin > 256 || cout < 16 || cout > 128 || !dy ||
+        !x || !dw || !scratch || (db && cin > 240))
         return isti::set_error(ISTI_ERR_INVALID_ARG, "isti_unet_wgrad: bad shape or NULL buffer");
+    WgradConfig c;
+    if (!wgrad_config(taps, n, h, w, cin, cout, c))
+        return isti::set_error(ISTI_ERR_INVALID_ARG, "isti_unet_wgrad: image too large");
     if (scratch_bytes < wgrad_scratch(taps, n, h, w, cin, cout))
         return isti::set_error(ISTI_ERR_INVALID_ARG, "isti_unet_wgrad: scratch too small");
     isti_status st = status_word(status);
     if (st != ISTI_OK)
         return st;
-    CUtensorMap dymap, xmap;
-    if ((st = nhwc_map(dymap, dy, n, h, w, cout)) != ISTI_OK || (st = nhwc_map(xmap, x, n, h, w, cin)) != ISTI_OK)
-        return st;
     WgradParams p{};
     p.partial = static_cast<float *>(scratch);
+    p.bpartial = db ? p.partial + (size_t)c.splits * cout * taps * cin : nullptr;
     p.status = status;
-    p.w = w;
-    p.h = h;
-    p.b = n;
+    p.w = c.w;
+    p.h = c.h;
+    p.b = c.n;
     p.cin = cin;
     p.cout = cout;
-    p.tiles_x = (w + TILE_W - 1) / TILE_W;
-    p.tiles_y = (h + TILE_H - 1) / TILE_H;
-    p.n_tiles = n * p.tiles_x * p.tiles_y;
-    const int splits = wgrad_splits(taps, p.n_tiles);
-    p.tiles_per_split = (p.n_tiles + splits - 1) / splits;
-    const uint32_t sb = wgrad_stage_bytes(cin);
-    p.stages = (int)std::max<size_t>(2, std::min<size_t>(4, (160 * 1024) / sb));
-    const size_t smem = (size_t)p.stages * sb + (2 * p.stages + 1) * 8 + 16;
-    if (smem > SMEM_BUDGET)
-        return isti::set_error(ISTI_ERR_INVALID_ARG, "isti_unet_wgrad: stage does not fit in shared memory");
-    const dim3 grid((unsigned)splits, (unsigned)taps);
-    cudaError_t e;
-    if (taps == 9)
-    {
-        e = smem_limit(wgrad_kernel<9>, smem);
-        if (e == cudaSuccess)
-            wgrad_kernel<9><<<grid, CONV_THREADS, smem, stream>>>(p, dymap, xmap);
-    }
-    else
-    {
-        e = smem_limit(wgrad_kernel<1>, smem);
-        if (e == cudaSuccess)
-            wgrad_kernel<1><<<grid, CONV_THREADS, smem, stream>>>(p, dymap, xmap);
-    }
+    p.kseg = c.kseg;
+    p.segs = c.segs;
+    p.n_units = c.n_units;
+    p.units_per_split = c.units_per_split;
+    p.n_dy = c.n_dy;
+    p.n_mb = c.n_mb;
+    p.box_chunks = c.grid_z == 1 ? cout / 8 : 1;
+    p.stages = c.stages;
+    CUtensorMap dymap, xmap;
+    if ((st = nhwc_segment_map(dymap, dy, c.n, c.h, c.w, cout, c.kseg, 1, p.box_chunks)) != ISTI_OK ||
+        (st = nhwc_segment_map(xmap, x, c.n, c.h, c.w, cin, c.kseg, c.n_dy, cin / 8)) != ISTI_OK)
+        return st;
+    const dim3 grid((unsigned)c.splits, (unsigned)c.grid_y, (unsigned)c.grid_z);
+    auto kernel = taps == 9 ? wgrad_kernel<9> : wgrad_kernel<1>;
+    cudaError_t e = smem_limit(kernel, c.smem);
     if (e == cudaSuccess)
     {
-        const size_t nw = (size_t)cout * taps * cin;
-        wgrad_reduce_kernel<<<(unsigned)((nw + 255) / 256), 256, 0, stream>>>(p.partial, splits, nw, dw, accumulate);
+        kernel<<<grid, WGRAD_THREADS, c.smem, stream>>>(p, dymap, xmap);
+        const int nw = cout * taps * cin;
+        wgrad_reduce_kernel<<<(unsigned)((nw + (db ? cout : 0) + 31) / 32), dim3(32, WREDUCE_PARTS), 0, stream>>>(p.partial, p.bpartial, c.splits, nw,
+                                                                                                              cout, dw, db, accumulate);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "isti_unet_wgrad launch");
@@ -357,7 +413,7 @@ size_t isti_unet_wgrad_scratch_bytes(int32_t taps, int32_t n, int32_t h, int32_t
 isti_status isti_unet_wgrad(int32_t taps, const void *dy, const void *x, int32_t n, int32_t h, int32_t w, int32_t cin, int32_t cout,
                             float *dw, int32_t accumulate, void *scratch, size_t scratch_bytes, int32_t *status, void *stream)
 {
-    return isti_unet::wgrad_launch(taps, dy, x, n, h, w, cin, cout, dw, accumulate, scratch, scratch_bytes, status,
+    return isti_unet::wgrad_launch(taps, dy, x, n, h, w, cin, cout, dw, nullptr, accumulate, scratch, scratch_bytes, status,
                                    static_cast<cudaStream_t>(stream));
 }
 

@@ -20,12 +20,9 @@
 // Every mbarrier wait is bounded; on timeout the status word is set, the loops stop, the
 // producer waits (bounded) for the copies it issued, and TMEM is freed before returning.
 //
-// wgrad_kernel (weight gradient): D[co][ci] of one tap = sum over pixels of
-// dY[p][co] * X[p + offset(tap)][ci], with M = 128 (cout padded; the padding boxes are
-// never loaded and stay zero), N = cin, K = pixels: both operands are MN-major (the
-// channel runs along the 16-byte row), again as TMA boxes of 8 channels x 128 pixels; for
-// them the descriptor's LBO steps along K and its SBO along M/N (checked against torch).
-// A CTA covers one tap and a range of pixel tiles and writes its partial sums; a second
+// wgrad_kernel (weight gradient): K = pixels, both operands MN-major (the channel runs along the
+// 16-byte row; for them the descriptor's LBO steps along K and its SBO along M/N, checked
+// against torch).  A CTA covers a range of row segments and writes its partial sums; a second
 // kernel adds the partials in a fixed order (deterministic).
 #pragma once
 
@@ -39,7 +36,6 @@ namespace isti_unet
 {
 using namespace isti_tc;
 
-constexpr int CONV_THREADS = 128; // weight-gradient kernel: warp 0 producer, warp 1 MMA, all four epilogue
 constexpr int TILE_W = 16, TILE_H = 8, TILE_M = TILE_W * TILE_H;
 constexpr uint32_t BOX_BYTES = TILE_M * 16; // one TMA box: 8 channels x 128 pixels
 
@@ -523,40 +519,77 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     }
 }
 
+// ---- weight gradient ----
+//
+// dW[co][tap][ci] = sum over pixels p of dY[p + s][co] * X[p + dy rows][ci] with tap = (dy, dx = -s):
+// the horizontal offset is taken on dY's side.  A unit is KSEG consecutive pixels of a row, the
+// K of the products.  A = the rows (s, co) of dY, its three shifted copies one after another (each a
+// TMA copy of the same pixels at another x), packed into M blocks of 128 -- 96 of 128 rows used for
+// 32 output channels, where one tap per product would use 32.  B = the channels of the X rows
+// y - 1 .. y + 1 (one copy), each row a product of its own with N = cin.  So dY and X are fetched
+// three times per pixel instead of once per tap, and a unit takes 3 products per M block instead of 9.
+// The bias gradient (the column sums of dY) rides along: the row of dy = 0 has 16 more columns of
+// ones behind its channels.  Both operands are MN-major (the channel runs along the 16-byte row).
+// A CTA keeps every accumulator in TMEM: M blocks x (rows x cin + 16) columns; where that exceeds
+// 512 the grid's y takes one dy each, and its z one M block each (wgrad_config in isti_unet.cu).
+// 1x1 layers: one row, no shift, the image a single row of pixels.
+//
+// Bound by shared-memory operand reads (4 KB of A per K = 16 step, 32 cycles) and latency; 8 images
+// of 480x272: 32 -> 32 channels 407 -> 134 us, 16 -> 32 358 -> 99, 64 -> 64 at half size 154 -> 68;
+// the bias gradients had passes over dY of their own, 0.7 ms of a 3.0 ms step.
 struct WgradParams
 {
-    float *partial; // [splits][cout][TAPS][cin]
+    float *partial;  // [splits][cout][TAPS][cin]
+    float *bpartial; // [splits][cout], or null: no bias gradient
     int32_t *status;
     int w, h, b;
     int cin, cout;
-    int tiles_x, tiles_y, n_tiles, tiles_per_split;
+    int kseg, segs, n_units, units_per_split;
+    int n_dy, n_mb; // X rows and M blocks of one CTA
+    int box_chunks; // channel chunks (of 8) per TMA box of dY: cout / 8, or 1 where an M block may start inside a shift
     int stages;
 };
 
-__host__ __device__ constexpr uint32_t wgrad_a_bytes() { return 16u * BOX_BYTES; } // M = 128 output channels
-__host__ __device__ constexpr uint32_t wgrad_stage_bytes(int cin) { return wgrad_a_bytes() + (uint32_t)(cin / 8) * BOX_BYTES; }
+__host__ __device__ constexpr uint32_t wgrad_a_bytes(int n_mb, int kseg) { return (uint32_t)n_mb * 16u * kseg * 16u; }
+__host__ __device__ constexpr uint32_t wgrad_stage_bytes(int cin, int n_dy, int n_mb, int kseg)
+{
+    return wgrad_a_bytes(n_mb, kseg) + (uint32_t)(cin / 8 + 2) * n_dy * kseg * 16u; // two chunks of ones behind X's
+}
+__host__ __device__ constexpr int wgrad_mb_cols(int cin, int n_dy) { return n_dy * cin + 16; }
+
+constexpr int WGRAD_THREADS = 128; // warp 0 producer, warp 1 MMA, all four epilogue
 
 template <int TAPS>
-__global__ void __launch_bounds__(CONV_THREADS) wgrad_kernel(const __grid_constant__ WgradParams p, const __grid_constant__ CUtensorMap dymap,
-                                                             const __grid_constant__ CUtensorMap xmap)
+__global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_constant__ WgradParams p, const __grid_constant__ CUtensorMap dymap,
+                                                              const __grid_constant__ CUtensorMap xmap)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
+    constexpr int SHIFTS = TAPS == 9 ? 3 : 1;
     const int S = p.stages;
-    const uint32_t a_bytes = wgrad_a_bytes(), stage_bytes = wgrad_stage_bytes(p.cin);
+    const uint32_t px_bytes = (uint32_t)p.kseg * 16u; // one channel chunk of a unit's pixels
+    const uint32_t a_bytes = wgrad_a_bytes(p.n_mb, p.kseg), stage_bytes = wgrad_stage_bytes(p.cin, p.n_dy, p.n_mb, p.kseg);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)S * stage_bytes);
     uint64_t *empty = full + S;
     uint64_t *done = empty + S;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int tap = blockIdx.y, split = blockIdx.x;
-    const int dy = TAPS == 9 ? tap / 3 - 1 : 0, dx = TAPS == 9 ? tap % 3 - 1 : 0;
-    const int t_begin = split * p.tiles_per_split;
-    const int t_end = min(p.n_tiles, t_begin + p.tiles_per_split);
-    const uint32_t ncols = tmem_cols(p.cin);
+    const int split = blockIdx.x, dy0 = TAPS == 9 ? (int)blockIdx.y : 1, mb0 = (int)blockIdx.z * p.n_mb; // dy0: first row, 0..2
+    const int u_begin = split * p.units_per_split, u_end = min(p.n_units, u_begin + p.units_per_split);
+    const int iters = max(0, u_end - u_begin);
+    const int co_chunks = p.cout / 8;
+    const int boxes = min(p.n_mb * 16, SHIFTS * co_chunks - mb0 * 16) / p.box_chunks; // dY boxes of this CTA
+    const uint32_t ncols = tmem_cols(p.n_mb * wgrad_mb_cols(p.cin, p.n_dy));
+    const uint32_t b_rows_bytes = (uint32_t)p.n_dy * px_bytes; // one channel chunk of X
+    // columns of row d within an M block: the row of dy = 0 has 16 more
+    auto row_col = [&](int d) { return d * p.cin + (dy0 + d > 1 && d > 0 ? 16 : 0); };
 
-    // the output-channel boxes beyond cout are never loaded: zero once, for every stage
-    for (uint32_t i = threadIdx.x * 16u; i < (uint32_t)S * stage_bytes; i += CONV_THREADS * 16u)
-        *reinterpret_cast<uint4 *>(smem + i) = make_uint4(0, 0, 0, 0);
+    // rows of A past the last channel and the ones behind X's channels are never loaded: set once,
+    // for every stage
+    for (uint32_t i = threadIdx.x * 16u; i < (uint32_t)S * stage_bytes; i += WGRAD_THREADS * 16u)
+    {
+        const uint32_t v = i % stage_bytes >= a_bytes + (uint32_t)(p.cin / 8) * b_rows_bytes ? 0x3f803f80u : 0u;
+        *reinterpret_cast<uint4 *>(smem + i) = make_uint4(v, v, v, v);
+    }
     fence_proxy_async();
     if (threadIdx.x == 0)
     {
@@ -574,28 +607,26 @@ __global__ void __launch_bounds__(CONV_THREADS) wgrad_kernel(const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const int iters = t_end > t_begin ? t_end - t_begin : 0;
-    const uint32_t tx_bytes = (uint32_t)(p.cout / 8 + p.cin / 8) * BOX_BYTES;
 
     if (warp == 0 && lane == 0)
     {
+        const uint32_t tx_bytes = (uint32_t)(boxes * p.box_chunks) * px_bytes + (uint32_t)(p.cin / 8) * b_rows_bytes;
         int issued = 0;
         for (int it = 0; it < iters; it++)
         {
             const int s = it % S, r = it / S;
             if (r > 0 && !mbar_wait(&empty[s], (uint32_t)((r - 1) & 1), p.status))
                 break;
-            int t = t_begin + it;
-            const int tx = t % p.tiles_x;
-            t /= p.tiles_x;
-            const int ty = t % p.tiles_y;
-            const int bi = t / p.tiles_y;
+            const int u = u_begin + it;
+            const int x0 = (u % p.segs) * p.kseg, row = (u / p.segs) % p.h, bi = u / (p.segs * p.h);
             uint8_t *st = smem + (size_t)s * stage_bytes;
             mbar_expect_tx(&full[s], tx_bytes);
-            for (int j = 0; j < p.cout / 8; j++)
-                tma_load_4d(st + j * BOX_BYTES, &dymap, 8 * j, tx * TILE_W, ty * TILE_H, bi, &full[s]);
-            for (int j = 0; j < p.cin / 8; j++)
-                tma_load_4d(st + a_bytes + j * BOX_BYTES, &xmap, 8 * j, tx * TILE_W + dx, ty * TILE_H + dy, bi, &full[s]);
+            for (int b = 0; b < boxes; b++)
+            {
+                const int gc = mb0 * 16 + b * p.box_chunks, shift = TAPS == 9 ? gc / co_chunks - 1 : 0;
+                tma_load_5d(st + (uint32_t)(b * p.box_chunks) * px_bytes, &dymap, 0, x0 + shift, row, gc % co_chunks, bi, &full[s]);
+            }
+            tma_load_5d(st + a_bytes, &xmap, 0, x0, row + dy0 - 1, 0, bi, &full[s]);
             issued = it + 1;
         }
         for (int it = issued > S ? issued - S : 0; it < issued; it++)
@@ -604,11 +635,8 @@ __global__ void __launch_bounds__(CONV_THREADS) wgrad_kernel(const __grid_consta
     }
     else if (warp == 1 && lane == 0)
     {
-        const uint32_t idesc = idesc_bf16(TILE_M, (uint32_t)p.cin, 1, 1);
         // MN-major operands: LBO = distance between core matrices adjacent in K (the next 8
-        // pixels, 128 bytes on), SBO = between core matrices adjacent in M/N (the next 8
-        // channels, the next box)
-        const uint32_t lbo = 128u, sbo = BOX_BYTES;
+        // pixels, 128 bytes on), SBO = between core matrices adjacent in M/N (the next 8 channels)
         for (int it = 0; it < iters; it++)
         {
             const int s = it % S, r = it / S;
@@ -616,9 +644,19 @@ __global__ void __launch_bounds__(CONV_THREADS) wgrad_kernel(const __grid_consta
                 break;
             tc_fence_after();
             const uint32_t a0 = smem_u32(smem + (size_t)s * stage_bytes), b0 = a0 + a_bytes;
-            // K = 16 pixels per MMA: two 8-pixel core-matrix groups, 256 bytes on
-            for (int k = 0; k < TILE_M / 16; k++)
-                mma_bf16(tmem, smem_desc(a0 + k * 256, lbo, sbo), smem_desc(b0 + k * 256, lbo, sbo), idesc, it > 0 || k > 0);
+            for (int d = 0; d < p.n_dy; d++)
+            {
+                const bool ones = p.bpartial && dy0 + d == 1;
+                const uint32_t idesc = idesc_bf16(128, (uint32_t)p.cin + (ones ? 16u : 0u), 1, 1);
+                for (int mb = 0; mb < p.n_mb; mb++)
+                {
+                    const uint32_t acc = tmem + (uint32_t)(mb * wgrad_mb_cols(p.cin, p.n_dy) + row_col(d));
+                    // K = 16 pixels per MMA: two 8-pixel core-matrix groups, 256 bytes on
+                    for (int k = 0; k < p.kseg / 16; k++)
+                        mma_bf16(acc, smem_desc(a0 + (uint32_t)mb * 16u * px_bytes + k * 256, 128u, px_bytes),
+                                 smem_desc(b0 + (uint32_t)d * px_bytes + k * 256, 128u, b_rows_bytes), idesc, it > 0 || k > 0);
+                }
+            }
             mma_commit(&empty[s]);
         }
         mma_commit(done);
@@ -627,21 +665,36 @@ __global__ void __launch_bounds__(CONV_THREADS) wgrad_kernel(const __grid_consta
 
     const bool ok = mbar_wait(done, 0, p.status);
     tc_fence_after();
-    const int co = warp * 32 + lane;
     if (ok)
-        for (int c0 = 0; c0 < p.cin; c0 += 16)
+        for (int mb = 0; mb < p.n_mb; mb++)
         {
-            uint32_t r[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
-            tmem_ld_wait();
-            if (co >= p.cout)
-                continue;
-            float4 *dst = reinterpret_cast<float4 *>(p.partial + (((size_t)split * p.cout + co) * TAPS + tap) * p.cin + c0);
+            const int m = (mb0 + mb) * 128 + warp * 32 + lane; // row (shift, co)
+            const int shift = m / p.cout, co = m % p.cout;
+            for (int d = 0; d < p.n_dy; d++)
+            {
+                const int tap = TAPS == 9 ? (dy0 + d) * 3 + (2 - shift) : 0;
+                const bool ones = p.bpartial && dy0 + d == 1;
+                for (int c0 = 0; c0 < p.cin + (ones ? 16 : 0); c0 += 16)
+                {
+                    uint32_t r[16];
+                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mb * wgrad_mb_cols(p.cin, p.n_dy) + row_col(d) + c0), r);
+                    tmem_ld_wait();
+                    if (shift >= SHIFTS)
+                        continue;
+                    if (c0 == p.cin)
+                    {
+                        if (shift == SHIFTS / 2)
+                            p.bpartial[(size_t)split * p.cout + co] = iters > 0 ? __uint_as_float(r[0]) : 0.0f;
+                        continue;
+                    }
+                    float4 *dst = reinterpret_cast<float4 *>(p.partial + (((size_t)split * p.cout + co) * TAPS + tap) * p.cin + c0);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-                dst[i] = iters > 0 ? make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
-                                                 __uint_as_float(r[4 * i + 3]))
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int i = 0; i < 4; i++)
+                        dst[i] = iters > 0 ? make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
+                                                         __uint_as_float(r[4 * i + 3]))
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
         }
     tc_fence_before();
     __syncthreads();
@@ -649,16 +702,34 @@ __global__ void __launch_bounds__(CONV_THREADS) wgrad_kernel(const __grid_consta
         tmem_dealloc(tmem, ncols);
 }
 
-// dW (+)= sum over splits of the partials, in split order.
-__global__ void wgrad_reduce_kernel(const float *partial, int splits, size_t n, float *dw, int accumulate)
+// dW (+)= sum over splits of the partials, in a fixed order: eight threads per value add every
+// eighth split, then their sums are added.  The bias gradients db follow the n weights (db may be null).
+constexpr int WREDUCE_PARTS = 8;
+__global__ void __launch_bounds__(32 * WREDUCE_PARTS) wgrad_reduce_kernel(const float *partial, const float *bpartial, int splits, int n, int nb,
+                                                                          float *dw, float *db, int accumulate)
 {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
+    __shared__ float part[WREDUCE_PARTS][32];
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    const bool weight = i < n, used = weight || (db && i < n + nb);
+    float s = 0.0f;
+    if (used)
+    {
+        const float *src = weight ? partial + i : bpartial + (i - n);
+        const size_t stride = weight ? n : nb;
+#pragma unroll 4
+        for (int k = threadIdx.y; k < splits; k += WREDUCE_PARTS)
+            s += src[k * stride];
+    }
+    part[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y != 0 || !used)
         return;
-    float s = accumulate ? dw[i] : 0.0f;
-    for (int k = 0; k < splits; k++)
-        s += partial[(size_t)k * n + i];
-    dw[i] = s;
+    float *out = weight ? dw + i : db + (i - n);
+    float total = accumulate ? *out : 0.0f;
+#pragma unroll
+    for (int k = 0; k < WREDUCE_PARTS; k++)
+        total += part[k][threadIdx.x];
+    *out = total;
 }
 
 // Packs f32 weights [cout][taps][cin] into the bf16 operand image of conv_kernel:
