@@ -82,113 +82,109 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8])
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// y[n, h/2, w/2] = mean of the 2x2 block of x[n, h, w]
-__global__ void pool_kernel(const bf16 *x, int n, int h, int w, int c, bf16 *y)
+// The elementwise kernels work on tensors in planes of 8 channels ([n][c / 8][h][w][8],
+// isti_unet_conv.cuh): a thread takes one 16-byte group of a half-resolution pixel and the 2x2
+// block of the full resolution under it.  planes = n * c / 8; ho, wo: the half resolution.
+// f(index of the half-resolution group, index of the block's first group, the full row's groups).
+constexpr int EW_X = 64, EW_Y = 4;
+template <class F>
+__device__ __forceinline__ void for_each_block(uint32_t planes, uint32_t ho, uint32_t wo, F f)
+{
+    for (uint32_t r = blockIdx.x * EW_Y + threadIdx.y; r < planes * ho; r += gridDim.x * EW_Y)
+    {
+        const uint32_t plane = r / ho, yo = r - plane * ho;
+        for (uint32_t x = threadIdx.x; x < wo; x += EW_X)
+            f((size_t)r * wo + x, ((size_t)plane * ho + yo) * 4 * wo + 2 * x, (size_t)2 * wo);
+    }
+}
+
+__device__ __forceinline__ void add8(float (&acc)[8], const bf16 *x, size_t group)
+{
+    float f[8];
+    unpack8(reinterpret_cast<const uint4 *>(x)[group], f); // plain load: the previous kernel may still run at launch
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        acc[k] += f[k];
+}
+
+// r = scale * the sum of x over 2x2 blocks: average pooling (0.25), gradient of nearest upsampling (1)
+__global__ void __launch_bounds__(EW_X * EW_Y) blocksum_kernel(const bf16 *x, uint32_t planes, uint32_t ho, uint32_t wo, float scale, bf16 *r)
 {
     isti_tc::griddep_launch_dependents();
     isti_tc::griddep_wait();
-    const int cg = c / 8, ho = h / 2, wo = w / 2;
-    const size_t total = (size_t)n * ho * wo * cg;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
-    {
-        const int g = (int)(i % cg);
-        size_t pix = i / cg;
-        const int xo = (int)(pix % wo);
-        pix /= wo;
-        const int yo = (int)(pix % ho);
-        const int b = (int)(pix / ho);
+    for_each_block(planes, ho, wo, [&](size_t half, size_t full, size_t row) {
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int dy = 0; dy < 2; dy++)
-            for (int dx = 0; dx < 2; dx++)
-            {
-                float f[8];
-                unpack8(*reinterpret_cast<const uint4 *>(x + ((((size_t)b * h + 2 * yo + dy) * w + 2 * xo + dx) * c + 8 * g)), f);
-#pragma unroll
-                for (int k = 0; k < 8; k++)
-                    acc[k] += f[k];
-            }
+        add8(acc, x, full);
+        add8(acc, x, full + 1);
+        add8(acc, x, full + row);
+        add8(acc, x, full + row + 1);
 #pragma unroll
         for (int k = 0; k < 8; k++)
-            acc[k] *= 0.25f;
-        *reinterpret_cast<uint4 *>(y + (((size_t)b * ho + yo) * wo + xo) * c + 8 * g) = pack8(acc);
-    }
+            acc[k] *= scale;
+        reinterpret_cast<uint4 *>(r)[half] = pack8(acc);
+    });
 }
 
-// s[n, h, w] = a[n, h/2, w/2] (nearest upsampling) + b[n, h, w]
-__global__ void upadd_kernel(const bf16 *a, const bf16 *b, int n, int h, int w, int c, bf16 *s)
+// s[h, w] = a[h/2, w/2] (nearest upsampling) + b[h, w]
+__global__ void __launch_bounds__(EW_X * EW_Y) upadd_kernel(const bf16 *a, const bf16 *b, uint32_t planes, uint32_t ho, uint32_t wo, bf16 *s)
 {
     isti_tc::griddep_launch_dependents();
     isti_tc::griddep_wait();
-    const int cg = c / 8;
-    const size_t total = (size_t)n * h * w * cg;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
-    {
-        const int g = (int)(i % cg);
-        size_t pix = i / cg;
-        const int x = (int)(pix % w);
-        pix /= w;
-        const int y = (int)(pix % h);
-        const int bi = (int)(pix / h);
-        float fa[8], fb[8];
-        unpack8(*reinterpret_cast<const uint4 *>(a + (((size_t)bi * (h / 2) + y / 2) * (w / 2) + x / 2) * c + 8 * g), fa);
-        unpack8(*reinterpret_cast<const uint4 *>(b + i * 8), fb);
+    for_each_block(planes, ho, wo, [&](size_t half, size_t full, size_t row) {
+        const uint4 ua = reinterpret_cast<const uint4 *>(a)[half];
+        uint4 ub[4];
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-            fa[k] += fb[k];
-        *reinterpret_cast<uint4 *>(s + i * 8) = pack8(fa);
-    }
+        for (int q = 0; q < 4; q++)
+            ub[q] = reinterpret_cast<const uint4 *>(b)[full + (q / 2) * row + q % 2];
+        float fa[8];
+        unpack8(ua, fa);
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+        {
+            float fb[8];
+            unpack8(ub[q], fb);
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                fb[k] = fa[k] + fb[k];
+            reinterpret_cast<uint4 *>(s)[full + (q / 2) * row + q % 2] = pack8(fb);
+        }
+    });
 }
 
-// r[n, h/2, w/2] = sum of the 2x2 block of g[n, h, w] (gradient of nearest upsampling)
-__global__ void downsum_kernel(const bf16 *g, int n, int h, int w, int c, bf16 *r)
-{
-    const int cg = c / 8, ho = h / 2, wo = w / 2;
-    const size_t total = (size_t)n * ho * wo * cg;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
-    {
-        const int gi = (int)(i % cg);
-        size_t pix = i / cg;
-        const int xo = (int)(pix % wo);
-        pix /= wo;
-        const int yo = (int)(pix % ho);
-        const int b = (int)(pix / ho);
-        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int dy = 0; dy < 2; dy++)
-            for (int dx = 0; dx < 2; dx++)
-            {
-                float f[8];
-                unpack8(*reinterpret_cast<const uint4 *>(g + ((((size_t)b * h + 2 * yo + dy) * w + 2 * xo + dx) * c + 8 * gi)), f);
-#pragma unroll
-                for (int k = 0; k < 8; k++)
-                    acc[k] += f[k];
-            }
-        *reinterpret_cast<uint4 *>(r + (((size_t)b * ho + yo) * wo + xo) * c + 8 * gi) = pack8(acc);
-    }
-}
-
-// ge[n, h, w] = (gskip[n, h, w] + gq[n, h/2, w/2] / 4) * (act > 0): the gradient of an encoder
+// ge[h, w] = (gskip[h, w] + gq[h/2, w/2] / 4) * (act > 0): the gradient of an encoder
 // activation that feeds both a skip connection and the 2x2 average pool, through its ReLU
-__global__ void poolback_kernel(const bf16 *gskip, const bf16 *gq, const bf16 *act, int n, int h, int w, int c, bf16 *ge)
+__global__ void __launch_bounds__(EW_X * EW_Y) poolback_kernel(const bf16 *gskip, const bf16 *gq, const bf16 *act, uint32_t planes, uint32_t ho,
+                                                               uint32_t wo, bf16 *ge)
 {
-    const int cg = c / 8;
-    const size_t total = (size_t)n * h * w * cg;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
-    {
-        const int g = (int)(i % cg);
-        size_t pix = i / cg;
-        const int x = (int)(pix % w);
-        pix /= w;
-        const int y = (int)(pix % h);
-        const int bi = (int)(pix / h);
-        float fs[8], fq[8], fa[8];
-        unpack8(*reinterpret_cast<const uint4 *>(gskip + i * 8), fs);
-        unpack8(*reinterpret_cast<const uint4 *>(gq + (((size_t)bi * (h / 2) + y / 2) * (w / 2) + x / 2) * c + 8 * g), fq);
-        unpack8(*reinterpret_cast<const uint4 *>(act + i * 8), fa);
+    for_each_block(planes, ho, wo, [&](size_t half, size_t full, size_t row) {
+        uint4 us[4], ua[4];
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-            fs[k] = fa[k] > 0.0f ? fs[k] + 0.25f * fq[k] : 0.0f;
-        *reinterpret_cast<uint4 *>(ge + i * 8) = pack8(fs);
-    }
+        for (int q = 0; q < 4; q++)
+        {
+            us[q] = reinterpret_cast<const uint4 *>(gskip)[full + (q / 2) * row + q % 2];
+            ua[q] = reinterpret_cast<const uint4 *>(act)[full + (q / 2) * row + q % 2];
+        }
+        float fq[8];
+        unpack8(reinterpret_cast<const uint4 *>(gq)[half], fq);
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+        {
+            float fs[8], fa[8];
+            unpack8(us[q], fs);
+            unpack8(ua[q], fa);
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                fs[k] = fa[k] > 0.0f ? fs[k] + 0.25f * fq[k] : 0.0f;
+            reinterpret_cast<uint4 *>(ge)[full + (q / 2) * row + q % 2] = pack8(fs);
+        }
+    });
+}
+
+// 16-byte group q of pixel p (of all images) of a tensor in planes with `groups` groups
+__device__ __forceinline__ size_t plane_group(size_t p, size_t image, int groups, int q)
+{
+    const size_t b = p / image;
+    return (b * groups + q) * image + (p - b * image);
 }
 
 // out[i] = sum over blocks of partial[block][i] (fixed order)
@@ -204,7 +200,7 @@ __global__ void sum_partials_kernel(const float *partial, int blocks, int n, flo
 }
 
 // flow[p][0..3] = hb + hw . d1[p]  (the 1x1 output head, f32); optionally also f16
-__global__ void head_kernel(const bf16 *d1, size_t npix, const float *hw, const float *hb, float *flow, __half *flow16)
+__global__ void head_kernel(const bf16 *d1, size_t npix, size_t image, const float *hw, const float *hb, float *flow, __half *flow16)
 {
     __shared__ float sw[HEAD_COUT * HEAD_CIN + HEAD_COUT];
     for (int i = threadIdx.x; i < HEAD_COUT * HEAD_CIN; i += blockDim.x)
@@ -217,12 +213,12 @@ __global__ void head_kernel(const bf16 *d1, size_t npix, const float *hw, const 
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (size_t)gridDim.x * blockDim.x)
     {
         float f[HEAD_CIN];
-        const uint4 *src = reinterpret_cast<const uint4 *>(d1 + p * HEAD_CIN);
+        const uint4 *src = reinterpret_cast<const uint4 *>(d1) + plane_group(p, image, HEAD_CIN / 8, 0);
 #pragma unroll
         for (int q = 0; q < HEAD_CIN / 8; q++)
         {
             float t[8];
-            unpack8(src[q], t); // plain load: written by the previous kernel, which may still run at launch
+            unpack8(src[q * image], t); // plain load: written by the previous kernel, which may still run at launch
 #pragma unroll
             for (int k = 0; k < 8; k++)
                 f[8 * q + k] = t[k];
@@ -255,7 +251,7 @@ __global__ void head_kernel(const bf16 *d1, size_t npix, const float *hw, const 
 // Writes the gradient of the head's input through d1's ReLU (bf16), and per-block partials
 // of the loss [block][1] and of the head's weight/bias gradients [block][4 * 32 + 4].
 constexpr int HEAD_GRADS = HEAD_COUT * HEAD_CIN + HEAD_COUT;
-__global__ void head_back_kernel(const bf16 *d1, size_t npix, const float *hw, const float *hb, const float *label, float inv_norm, bf16 *g_d1,
+__global__ void head_back_kernel(const bf16 *d1, size_t npix, size_t image, const float *hw, const float *hb, const float *label, float inv_norm, bf16 *g_d1,
                                  float *loss_partial, float *hgrad_partial)
 {
     __shared__ float sw[HEAD_GRADS];
@@ -275,12 +271,13 @@ __global__ void head_back_kernel(const bf16 *d1, size_t npix, const float *hw, c
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (size_t)gridDim.x * blockDim.x)
     {
         float f[HEAD_CIN];
-        const uint4 *src = reinterpret_cast<const uint4 *>(d1 + p * HEAD_CIN);
+        const size_t group = plane_group(p, image, HEAD_CIN / 8, 0);
+        const uint4 *src = reinterpret_cast<const uint4 *>(d1) + group;
 #pragma unroll
         for (int q = 0; q < HEAD_CIN / 8; q++)
         {
             float t[8];
-            unpack8(__ldg(src + q), t);
+            unpack8(__ldg(src + q * image), t);
 #pragma unroll
             for (int k = 0; k < 8; k++)
                 f[8 * q + k] = t[k];
@@ -320,7 +317,7 @@ __global__ void head_back_kernel(const bf16 *d1, size_t npix, const float *hw, c
                 my_g[j * HEAD_CIN + k] += go[j] * f[k];
             my_g[HEAD_COUT * HEAD_CIN + j] += go[j];
         }
-        uint4 *dst = reinterpret_cast<uint4 *>(g_d1 + p * HEAD_CIN);
+        uint4 *dst = reinterpret_cast<uint4 *>(g_d1) + group;
 #pragma unroll
         for (int q = 0; q < HEAD_CIN / 8; q++)
         {
@@ -328,7 +325,7 @@ __global__ void head_back_kernel(const bf16 *d1, size_t npix, const float *hw, c
 #pragma unroll
             for (int k = 0; k < 8; k++)
                 t[k] = gi[8 * q + k];
-            dst[q] = pack8(t);
+            dst[q * image] = pack8(t);
         }
     }
     // block reduction: warp shuffles, then one shared-memory add per warp and value
@@ -373,6 +370,9 @@ __global__ void adam_kernel(float *w, const float *g, float *m, float *v, size_t
 }
 
 unsigned grid_for(size_t work) { return (unsigned)std::max<size_t>(1, std::min<size_t>((work + 255) / 256, 152 * 8)); }
+
+// grid of the elementwise kernels over `rows` half-resolution rows of all planes
+dim3 rows_grid(int rows) { return dim3((unsigned)std::max(1, std::min((rows + EW_Y - 1) / EW_Y, 152 * 8))); }
 
 constexpr int REDUCE_BLOCKS = 256;
 } // namespace
@@ -478,22 +478,26 @@ isti_status conv(isti_flownet *net, int l, const bf16 *x, int n, int h, int w, c
                  const isti_unet::ConvHead *head = nullptr, bool *head_fused = nullptr)
 {
     const LayerDef &d = LAYERS[l];
+    // every tensor but the network's input (NHWC) is in planes
     return isti_unet::conv_launch(d.taps, x, n, h, w, d.cin, net->packs + net->pk_off[l], net->params + net->b_off[l], mask, d.relu, out, d.cout,
-                                  net->status, s, pdl, head, head_fused);
+                                  net->status, s, l == 0 ? isti_unet::OUT_PLANES : isti_unet::IN_PLANES | isti_unet::OUT_PLANES, pdl, head,
+                                  head_fused);
 }
 
 // data gradient of layer l: g_in = conv(g_out, W^T flipped), masked by (mask > 0) when given
 isti_status dgrad(isti_flownet *net, int l, const bf16 *g_out, int n, int h, int w, const bf16 *mask, bf16 *g_in, cudaStream_t s)
 {
     const LayerDef &d = LAYERS[l];
-    return isti_unet::conv_launch(d.taps, g_out, n, h, w, d.cout, net->packs + net->pkt_off[l], nullptr, mask, 0, g_in, d.cin, net->status, s);
+    return isti_unet::conv_launch(d.taps, g_out, n, h, w, d.cout, net->packs + net->pkt_off[l], nullptr, mask, 0, g_in, d.cin, net->status, s,
+                                  isti_unet::IN_PLANES | isti_unet::OUT_PLANES);
 }
 
 isti_status wgrad(isti_flownet *net, int l, const bf16 *g_out, const bf16 *x, int n, int h, int w, Buffers &b, cudaStream_t s)
 {
     const LayerDef &d = LAYERS[l];
     return isti_unet::wgrad_launch(d.taps, g_out, x, n, h, w, d.cin, d.cout, net->grads + net->w_off[l], net->grads + net->b_off[l], 0, b.wscratch,
-                                   b.wscratch_bytes, net->status, s);
+                                   b.wscratch_bytes, net->status, s,
+                                   l == 0 ? isti_unet::OUT_PLANES : isti_unet::IN_PLANES | isti_unet::OUT_PLANES);
 }
 
 #define ISTI_TRY(x)                                                                                                                             \
@@ -511,7 +515,7 @@ isti_status forward(isti_flownet *net, const bf16 *x0, int n, int h, int w, Buff
 {
     using isti_unet::launch_kernel;
     const int h2 = h / 2, w2 = w / 2, h4 = h / 4, w4 = w / 4, h8 = h / 8, w8 = w / 8;
-    const dim3 blk(256);
+    const dim3 blk(EW_X, EW_Y);
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t x) {
         if (e == cudaSuccess)
@@ -519,22 +523,22 @@ isti_status forward(isti_flownet *net, const bf16 *x0, int n, int h, int w, Buff
         return e == cudaSuccess;
     };
     ISTI_TRY(conv(net, 0, x0, n, h, w, nullptr, b.e1, s, pdl));
-    ok(launch_kernel(pool_kernel, dim3(grid_for((size_t)n * h2 * w2 * 4)), blk, 0, s, pdl, (const bf16 *)b.e1, n, h, w, 32, b.q1));
+    ok(launch_kernel(blocksum_kernel, rows_grid(n * 4 * h2), blk, 0, s, pdl, (const bf16 *)b.e1, (uint32_t)(n * 4), (uint32_t)h2, (uint32_t)w2, 0.25f, b.q1));
     ISTI_TRY(conv(net, 1, b.q1, n, h2, w2, nullptr, b.e2, s, pdl));
-    ok(launch_kernel(pool_kernel, dim3(grid_for((size_t)n * h4 * w4 * 8)), blk, 0, s, pdl, (const bf16 *)b.e2, n, h2, w2, 64, b.q2));
+    ok(launch_kernel(blocksum_kernel, rows_grid(n * 8 * h4), blk, 0, s, pdl, (const bf16 *)b.e2, (uint32_t)(n * 8), (uint32_t)h4, (uint32_t)w4, 0.25f, b.q2));
     ISTI_TRY(conv(net, 2, b.q2, n, h4, w4, nullptr, b.e3, s, pdl));
-    ok(launch_kernel(pool_kernel, dim3(grid_for((size_t)n * h8 * w8 * 12)), blk, 0, s, pdl, (const bf16 *)b.e3, n, h4, w4, 96, b.q3));
+    ok(launch_kernel(blocksum_kernel, rows_grid(n * 12 * h8), blk, 0, s, pdl, (const bf16 *)b.e3, (uint32_t)(n * 12), (uint32_t)h8, (uint32_t)w8, 0.25f, b.q3));
     ISTI_TRY(conv(net, 3, b.q3, n, h8, w8, nullptr, b.e4, s, pdl));
     ISTI_TRY(conv(net, 4, b.e4, n, h8, w8, nullptr, b.p3, s, pdl));
-    ok(launch_kernel(upadd_kernel, dim3(grid_for((size_t)n * h4 * w4 * 12)), blk, 0, s, pdl, (const bf16 *)b.p3, (const bf16 *)b.e3, n, h4, w4,
-                     96, b.s3));
+    ok(launch_kernel(upadd_kernel, rows_grid(n * 12 * h8), blk, 0, s, pdl, (const bf16 *)b.p3, (const bf16 *)b.e3, (uint32_t)(n * 12), (uint32_t)h8, (uint32_t)w8,
+                     b.s3));
     ISTI_TRY(conv(net, 5, b.s3, n, h4, w4, nullptr, b.d3, s, pdl));
     ISTI_TRY(conv(net, 6, b.d3, n, h4, w4, nullptr, b.p2, s, pdl));
-    ok(launch_kernel(upadd_kernel, dim3(grid_for((size_t)n * h2 * w2 * 8)), blk, 0, s, pdl, (const bf16 *)b.p2, (const bf16 *)b.e2, n, h2, w2,
-                     64, b.s2));
+    ok(launch_kernel(upadd_kernel, rows_grid(n * 8 * h4), blk, 0, s, pdl, (const bf16 *)b.p2, (const bf16 *)b.e2, (uint32_t)(n * 8), (uint32_t)h4, (uint32_t)w4,
+                     b.s2));
     ISTI_TRY(conv(net, 7, b.s2, n, h2, w2, nullptr, b.d2, s, pdl));
     ISTI_TRY(conv(net, 8, b.d2, n, h2, w2, nullptr, b.p1, s, pdl));
-    ok(launch_kernel(upadd_kernel, dim3(grid_for((size_t)n * h * w * 4)), blk, 0, s, pdl, (const bf16 *)b.p1, (const bf16 *)b.e1, n, h, w, 32,
+    ok(launch_kernel(upadd_kernel, rows_grid(n * 4 * h2), blk, 0, s, pdl, (const bf16 *)b.p1, (const bf16 *)b.e1, (uint32_t)(n * 4), (uint32_t)h2, (uint32_t)w2,
                      b.s1));
     // inference: the 1x1 head in d1's epilogue where the row-tile kernel runs d1 (d1 itself is
     // then not stored), else its own kernel
@@ -542,7 +546,7 @@ isti_status forward(isti_flownet *net, const bf16 *x0, int n, int h, int w, Buff
     bool fused = false;
     ISTI_TRY(conv(net, 9, b.s1, n, h, w, nullptr, b.d1, s, pdl, pdl && (flow || flow16) ? &head : nullptr, &fused));
     if ((flow || flow16) && !fused)
-        ok(launch_kernel(head_kernel, dim3(grid_for((size_t)n * h * w)), blk, 0, s, pdl, (const bf16 *)b.d1, (size_t)n * h * w,
+        ok(launch_kernel(head_kernel, dim3(grid_for((size_t)n * h * w)), dim3(256), 0, s, pdl, (const bf16 *)b.d1, (size_t)n * h * w, (size_t)h * w,
                          (const float *)(net->params + net->w_off[N_CONV]), (const float *)(net->params + net->b_off[N_CONV]), flow, flow16));
     if (e == cudaSuccess)
         e = cudaGetLastError();
@@ -553,38 +557,38 @@ isti_status backward(isti_flownet *net, const bf16 *x0, const float *label, int 
 {
     const int h2 = h / 2, w2 = w / 2, h4 = h / 4, w4 = w / 4, h8 = h / 8, w8 = w / 8;
     const size_t npix = (size_t)n * h * w;
-    head_back_kernel<<<REDUCE_BLOCKS, 256, 0, s>>>(b.d1, npix, net->params + net->w_off[N_CONV], net->params + net->b_off[N_CONV], label,
+    head_back_kernel<<<REDUCE_BLOCKS, 256, 0, s>>>(b.d1, npix, (size_t)h * w, net->params + net->w_off[N_CONV], net->params + net->b_off[N_CONV], label,
                                                   1.0f / (float)npix, b.g_d1, b.partial, b.partial + REDUCE_BLOCKS);
     sum_partials_kernel<<<1, 32, 0, s>>>(b.partial, REDUCE_BLOCKS, 1, net->loss);
     sum_partials_kernel<<<1, 256, 0, s>>>(b.partial + REDUCE_BLOCKS, REDUCE_BLOCKS, HEAD_GRADS, net->grads + net->w_off[N_CONV]);
     // level 1 decoder
     ISTI_TRY(wgrad(net, 9, b.g_d1, b.s1, n, h, w, b, s));
     ISTI_TRY(dgrad(net, 9, b.g_d1, n, h, w, nullptr, b.g_s1, s));
-    downsum_kernel<<<grid_for((size_t)n * h2 * w2 * 4), 256, 0, s>>>(b.g_s1, n, h, w, 32, b.g_p1);
+    blocksum_kernel<<<rows_grid(n * 4 * h2), dim3(EW_X, EW_Y), 0, s>>>(b.g_s1, n * 4, h2, w2, 1.0f, b.g_p1);
     ISTI_TRY(wgrad(net, 8, b.g_p1, b.d2, n, h2, w2, b, s));
     ISTI_TRY(dgrad(net, 8, b.g_p1, n, h2, w2, b.d2, b.g_d2, s));
     // level 2 decoder
     ISTI_TRY(wgrad(net, 7, b.g_d2, b.s2, n, h2, w2, b, s));
     ISTI_TRY(dgrad(net, 7, b.g_d2, n, h2, w2, nullptr, b.g_s2, s));
-    downsum_kernel<<<grid_for((size_t)n * h4 * w4 * 8), 256, 0, s>>>(b.g_s2, n, h2, w2, 64, b.g_p2);
+    blocksum_kernel<<<rows_grid(n * 8 * h4), dim3(EW_X, EW_Y), 0, s>>>(b.g_s2, n * 8, h4, w4, 1.0f, b.g_p2);
     ISTI_TRY(wgrad(net, 6, b.g_p2, b.d3, n, h4, w4, b, s));
     ISTI_TRY(dgrad(net, 6, b.g_p2, n, h4, w4, b.d3, b.g_d3, s));
     // level 3 decoder
     ISTI_TRY(wgrad(net, 5, b.g_d3, b.s3, n, h4, w4, b, s));
     ISTI_TRY(dgrad(net, 5, b.g_d3, n, h4, w4, nullptr, b.g_s3, s));
-    downsum_kernel<<<grid_for((size_t)n * h8 * w8 * 12), 256, 0, s>>>(b.g_s3, n, h4, w4, 96, b.g_p3);
+    blocksum_kernel<<<rows_grid(n * 12 * h8), dim3(EW_X, EW_Y), 0, s>>>(b.g_s3, n * 12, h8, w8, 1.0f, b.g_p3);
     ISTI_TRY(wgrad(net, 4, b.g_p3, b.e4, n, h8, w8, b, s));
     ISTI_TRY(dgrad(net, 4, b.g_p3, n, h8, w8, b.e4, b.g_e4, s));
     // bottleneck and encoder
     ISTI_TRY(wgrad(net, 3, b.g_e4, b.q3, n, h8, w8, b, s));
     ISTI_TRY(dgrad(net, 3, b.g_e4, n, h8, w8, nullptr, b.g_q3, s));
-    poolback_kernel<<<grid_for((size_t)n * h4 * w4 * 12), 256, 0, s>>>(b.g_s3, b.g_q3, b.e3, n, h4, w4, 96, b.g_e3);
+    poolback_kernel<<<rows_grid(n * 12 * h8), dim3(EW_X, EW_Y), 0, s>>>(b.g_s3, b.g_q3, b.e3, n * 12, h8, w8, b.g_e3);
     ISTI_TRY(wgrad(net, 2, b.g_e3, b.q2, n, h4, w4, b, s));
     ISTI_TRY(dgrad(net, 2, b.g_e3, n, h4, w4, nullptr, b.g_q2, s));
-    poolback_kernel<<<grid_for((size_t)n * h2 * w2 * 8), 256, 0, s>>>(b.g_s2, b.g_q2, b.e2, n, h2, w2, 64, b.g_e2);
+    poolback_kernel<<<rows_grid(n * 8 * h4), dim3(EW_X, EW_Y), 0, s>>>(b.g_s2, b.g_q2, b.e2, n * 8, h4, w4, b.g_e2);
     ISTI_TRY(wgrad(net, 1, b.g_e2, b.q1, n, h2, w2, b, s));
     ISTI_TRY(dgrad(net, 1, b.g_e2, n, h2, w2, nullptr, b.g_q1, s));
-    poolback_kernel<<<grid_for((size_t)n * h * w * 4), 256, 0, s>>>(b.g_s1, b.g_q1, b.e1, n, h, w, 32, b.g_e1);
+    poolback_kernel<<<rows_grid(n * 4 * h2), dim3(EW_X, EW_Y), 0, s>>>(b.g_s1, b.g_q1, b.e1, n * 4, h2, w2, b.g_e1);
     ISTI_TRY(wgrad(net, 0, b.g_e1, x0, n, h, w, b, s));
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "flownet backward");

@@ -54,36 +54,34 @@ isti_status nhwc_map(CUtensorMap &m, const void *base, int n, int h, int w, int 
     return ISTI_OK;
 }
 
-// 5-D map over an NHWC bf16 tensor with the channels split as (8, c / 8) and the chunk index
-// outermost: dims (c_lo, w, h, c_hi, n), box {8, 16 x, 8 y, ck / 8 chunks, 1}, so one copy lands
-// a stage's channel chunks one after another (the layout of ck / 8 separate 4-D boxes).
-// Returns false when the driver does not accept the strides.
-bool nhwc_chunked_map(CUtensorMap &m, const void *base, int n, int h, int w, int c, int ck)
+// Map of a box of `px` x `rows` pixels x `groups` channel groups of 8.  NHWC: 5-D over (8, w, h,
+// c / 8, n); planes: 4-D over (2 w, h, c / 8, n) 64-bit elements, so that a box row is one run of
+// px * 16 bytes.  Either lands the groups one after another, pixels of 16 bytes within.
+isti_status box_map(CUtensorMap &m, const void *base, bool planes, int n, int h, int w, int c, int px, int rows, int groups)
 {
     EncodeTiledFn enc = encode_tiled();
-    if (!enc || ((uintptr_t)base & 15u) || c % 8 || ck % 8)
-        return false;
-    const cuuint64_t dims[5] = {8, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)(c / 8), (cuuint64_t)n};
-    const cuuint64_t strides[4] = {(cuuint64_t)c * 2u, (cuuint64_t)w * c * 2u, 16u, (cuuint64_t)h * w * c * 2u};
-    const cuuint32_t box[5] = {8, (cuuint32_t)TILE_W, (cuuint32_t)TILE_H, (cuuint32_t)(ck / 8), 1};
+    if (!enc)
+        return isti::set_error(ISTI_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
+    if (((uintptr_t)base & 15u) || c % 8)
+        return isti::set_error(ISTI_ERR_INVALID_ARG, "activation tensor: base 16-byte aligned, channels a multiple of 8");
+    const cuuint64_t W = (cuuint64_t)w, H = (cuuint64_t)h, G = (cuuint64_t)(c / 8), N = (cuuint64_t)n;
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    return enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// 5-D map for row_conv_kernel: box {8, 130 x, 3 y, ck / 8 chunks, 1} (a 128-pixel row segment
-// with its halo).
-bool nhwc_row_map(CUtensorMap &m, const void *base, int n, int h, int w, int c, int ck)
-{
-    EncodeTiledFn enc = encode_tiled();
-    if (!enc || ((uintptr_t)base & 15u) || c % 8 || ck % 8)
-        return false;
-    const cuuint64_t dims[5] = {8, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)(c / 8), (cuuint64_t)n};
-    const cuuint64_t strides[4] = {(cuuint64_t)c * 2u, (cuuint64_t)w * c * 2u, 16u, (cuuint64_t)h * w * c * 2u};
-    const cuuint32_t box[5] = {8, (cuuint32_t)ROW_HALO, 3, (cuuint32_t)(ck / 8), 1};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    return enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    CUresult r;
+    if (planes)
+    {
+        const cuuint64_t dims[4] = {2 * W, H, G, N}, strides[3] = {16 * W, 16 * W * H, 16 * W * H * G};
+        const cuuint32_t box[4] = {2 * (cuuint32_t)px, (cuuint32_t)rows, (cuuint32_t)groups, 1};
+        r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
+    else
+    {
+        const cuuint64_t dims[5] = {8, W, H, G, N}, strides[4] = {16 * G, 16 * G * W, 16u, 16 * G * W * H};
+        const cuuint32_t box[5] = {8, (cuuint32_t)px, (cuuint32_t)rows, (cuuint32_t)groups, 1};
+        r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
+    return r == CUDA_SUCCESS ? ISTI_OK : isti::set_error(ISTI_ERR_INVALID_ARG, "cuTensorMapEncodeTiled rejected an activation tensor");
 }
 
 int sm_count()
@@ -162,7 +160,7 @@ namespace isti_unet
 {
 // Launch of conv_kernel<taps> (shared with the network code in isti_flownet.cu).
 isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, const void *wpack, const float *bias, const void *mask, int relu,
-                        void *out, int cout, int32_t *status, cudaStream_t stream, bool pdl, const ConvHead *head, bool *head_fused)
+                        void *out, int cout, int32_t *status, cudaStream_t stream, int planes, bool pdl, const ConvHead *head, bool *head_fused)
 {
     if (head_fused)
         *head_fused = false;
@@ -187,16 +185,29 @@ isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, c
     p.cin = cin;
     p.cout = cout;
     p.ck = cin % 32 == 0 ? 32 : 16;
-    p.tiles_x = (w + TILE_W - 1) / TILE_W;
-    p.tiles_y = (h + TILE_H - 1) / TILE_H;
+    p.in_planes = (planes & IN_PLANES) != 0;
+    p.out_planes = (planes & OUT_PLANES) != 0;
+    p.halo = p.in_planes ? ROW_M : ROW_HALO;
+    p.seg_out = p.halo - 2;
+    p.tile_shift = 4;
+    // 1x1 layers in planes: an image is one row of pixels, a tile 128 of them
+    if (taps == 1 && p.in_planes && p.out_planes && (size_t)h * w <= (size_t)INT32_MAX / 2)
+    {
+        p.tile_shift = 7;
+        p.w = w = h * w;
+        p.h = h = 1;
+    }
+    const int tile_w = 1 << p.tile_shift, tile_h = TILE_M / tile_w;
+    p.tiles_x = (w + tile_w - 1) / tile_w;
+    p.tiles_y = (h + tile_h - 1) / tile_h;
     p.n_tiles = n * p.tiles_x * p.tiles_y;
     p.relu = relu;
     CUtensorMap xmap;
     // wide, thin 3x3 layers: row-tile kernel with a loaded-once halo and resident weights
     const uint32_t w_bytes = 9u * (uint32_t)cin * cout * 2u;
-    if (taps == 9 && w >= ROW_M && w_bytes <= 96u * 1024u && nhwc_row_map(xmap, x, n, h, w, cin, p.ck))
+    if (taps == 9 && w >= ROW_M && w_bytes <= 96u * 1024u && box_map(xmap, x, p.in_planes, n, h, w, cin, p.halo, 3, p.ck / 8) == ISTI_OK)
     {
-        const size_t w_region = (w_bytes + 1023) / 1024 * 1024, sb = row_stage_bytes(p.ck), tail = 16 * 8 + 16;
+        const size_t w_region = (w_bytes + 1023) / 1024 * 1024, sb = row_stage_bytes(p.ck, p.halo), tail = 16 * 8 + 16;
         int per_sm = 2;
         size_t stages = w_region + 2 * sb + 2 * 16 + tail <= 100 * 1024 ? (100 * 1024 - w_region - tail) / (sb + 16) : 0;
         if (stages < 2)
@@ -215,7 +226,7 @@ isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, c
                 p.head_flow16 = static_cast<__half *>(head->flow16);
             }
             const size_t smem = w_region + (size_t)p.stages * sb + (2 * p.stages + 6) * 8 + 16;
-            const int units = n * h * ((w + ROW_M - 1) / ROW_M);
+            const int units = n * h * ((w + p.seg_out - 1) / p.seg_out);
             const int grid = std::min(units, sm_count() * per_sm);
             cudaError_t e = smem_limit(row_conv_kernel<0>, smem);
             if (e == cudaSuccess)
@@ -225,8 +236,9 @@ isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, c
             return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "isti_unet_conv launch");
         }
     }
-    p.chunked_map = nhwc_chunked_map(xmap, x, n, h, w, cin, p.ck) ? 1 : 0;
-    if (!p.chunked_map && (st = nhwc_map(xmap, x, n, h, w, cin)) != ISTI_OK)
+    st = box_map(xmap, x, p.in_planes, n, h, w, cin, tile_w, tile_h, p.ck / 8);
+    p.chunked_map = !p.in_planes && st == ISTI_OK;
+    if (st != ISTI_OK && (p.in_planes || (st = nhwc_map(xmap, x, n, h, w, cin)) != ISTI_OK))
         return st;
     // ring: about 100 KB, so that two CTAs share an SM; the ring runs across tiles
     const uint32_t sb = conv_stage_bytes(p.ck, cout);
@@ -258,7 +270,7 @@ isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, c
 // The weight gradient's work split (wgrad_kernel) and its scratch.
 struct WgradConfig
 {
-    int n, h, w;              // the image, 1x1 layers as one row of pixels
+    int n, h, w;              // the images, those of 1x1 layers as one row of pixels each
     int kseg, segs, n_units;
     int n_dy, n_mb;           // per CTA
     int grid_y, grid_z, splits, units_per_split, stages;
@@ -268,10 +280,10 @@ struct WgradConfig
 bool wgrad_config(int taps, int n, int h, int w, int cin, int cout, WgradConfig &c)
 {
     c = WgradConfig{};
-    c.n = taps == 9 ? n : 1;
+    c.n = n;
     c.h = taps == 9 ? h : 1;
-    const long long row = taps == 9 ? w : (long long)n * h * w;
-    if (row > INT32_MAX - 256)
+    const long long row = taps == 9 ? w : (long long)h * w;
+    if (row > INT32_MAX / 2 - 256)
         return false;
     c.w = (int)row;
     const int mblocks = ((taps == 9 ? 3 : 1) * cout + 127) / 128;
@@ -311,27 +323,8 @@ size_t wgrad_scratch(int taps, int n, int h, int w, int cin, int cout)
     return (size_t)c.splits * cout * ((size_t)taps * cin + 1) * sizeof(float);
 }
 
-// 5-D map over an NHWC bf16 tensor, the channels split as (8, c / 8) and the chunk index
-// outermost: box {8, kseg x, rows, chunks, 1}.
-isti_status nhwc_segment_map(CUtensorMap &m, const void *base, int n, int h, int w, int c, int kseg, int rows, int chunks)
-{
-    EncodeTiledFn enc = encode_tiled();
-    if (!enc)
-        return isti::set_error(ISTI_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
-    if (((uintptr_t)base & 15u) || c % 8)
-        return isti::set_error(ISTI_ERR_INVALID_ARG, "NHWC tensor: base 16-byte aligned, channels a multiple of 8");
-    const cuuint64_t dims[5] = {8, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)(c / 8), (cuuint64_t)n};
-    const cuuint64_t strides[4] = {(cuuint64_t)c * 2u, (cuuint64_t)w * c * 2u, 16u, (cuuint64_t)h * w * c * 2u};
-    const cuuint32_t box[5] = {8, (cuuint32_t)kseg, (cuuint32_t)rows, (cuuint32_t)chunks, 1};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    if (enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return isti::set_error(ISTI_ERR_INVALID_ARG, "cuTensorMapEncodeTiled rejected an NHWC tensor");
-    return ISTI_OK;
-}
-
 isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, int w, int cin, int cout, float *dw, float *db, int accumulate,
-                         void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream)
+                         void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream, int planes)
 {
     if ((taps != 9 && taps != 1) || n < 1 || h < 1 || w < 1 || cin % 16 || cout % 16 || cin < 16 || cin > 256 || cout < 16 || cout > 128 || !dy ||
         !x || !dw || !scratch || (db && cin > 240))
@@ -361,9 +354,11 @@ isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, 
     p.n_mb = c.n_mb;
     p.box_chunks = c.grid_z == 1 ? cout / 8 : 1;
     p.stages = c.stages;
+    p.dy_planes = (planes & OUT_PLANES) != 0;
+    p.x_planes = (planes & IN_PLANES) != 0;
     CUtensorMap dymap, xmap;
-    if ((st = nhwc_segment_map(dymap, dy, c.n, c.h, c.w, cout, c.kseg, 1, p.box_chunks)) != ISTI_OK ||
-        (st = nhwc_segment_map(xmap, x, c.n, c.h, c.w, cin, c.kseg, c.n_dy, cin / 8)) != ISTI_OK)
+    if ((st = box_map(dymap, dy, p.dy_planes, c.n, c.h, c.w, cout, c.kseg, 1, p.box_chunks)) != ISTI_OK ||
+        (st = box_map(xmap, x, p.x_planes, c.n, c.h, c.w, cin, c.kseg, c.n_dy, cin / 8)) != ISTI_OK)
         return st;
     const dim3 grid((unsigned)c.splits, (unsigned)c.grid_y, (unsigned)c.grid_z);
     auto kernel = taps == 9 ? wgrad_kernel<9> : wgrad_kernel<1>;

@@ -1,6 +1,10 @@
 // Implicit-GEMM convolutions of the learned flow initialiser on the tcgen05 tensor core.
 //
-// Activations are NHWC bf16 (channels innermost, a multiple of 16); weights are kept as
+// Activations are bf16, their channels a multiple of 16, in one of two layouts: NHWC, or in planes
+// of 8 channels, [n][c / 8][h][w][8].  The products read 8 channels of a pixel as one 16-byte row;
+// a TMA box of NHWC data is made of such rows, at about 1.6 cycles each the bound of the wide
+// layers, while a box of planes has rows of as many pixels as it is wide (seen as pairs of 64-bit
+// elements).  The network keeps its tensors in planes (LAYOUT_MEASURED).  Weights are kept as
 // f32 masters [cout][tap][cin] (tap = 3 * (dy + 1) + (dx + 1) for 3x3, 0 for 1x1) and
 // packed to bf16 operand images by pack_kernel.
 //
@@ -57,9 +61,12 @@ struct ConvParams
     int w, h, b;
     int cin, cout, ck;          // ck: input channels per stage (16 or 32)
     int tiles_x, tiles_y, n_tiles;
+    int tile_shift;             // conv_kernel: log2 of the tile's width (4: 16 x 8 pixels; 7: 128 x 1, 1x1 layers in planes)
     int relu;
     int stages;                 // depth of the shared-memory ring
-    int chunked_map;            // 1: one 5-D box per stage (channel chunks outermost); 0: ck / 8 4-D boxes
+    int in_planes, out_planes;  // layouts of the input; of the output and the mask
+    int chunked_map;            // NHWC input: 1: one 5-D box per stage (channel chunks outermost); 0: ck / 8 4-D boxes
+    int halo, seg_out;          // row_conv_kernel: pixels per fetched row and outputs per unit
     // 1x1 output head fused into the epilogue (row_conv_kernel, inference): when head_w is
     // set, each pixel's bf16 outputs feed HEAD outputs = head_b + head_w . out (f32, fused
     // multiply-adds in channel order) written to head_flow (f32) and/or head_flow16 (f16),
@@ -84,6 +91,14 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, i
                      smem_u32(dst)),
                  "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
                  : "memory");
+}
+
+// The 16-byte groups of channels c0 .. c0 + 7 and c0 + 8 .. c0 + 15 of a pixel (image bi, pixel
+// `pix` of the image) of an output-shaped tensor.
+__device__ __forceinline__ size_t channel_group(const ConvParams &p, int bi, size_t pix, int c0, int half)
+{
+    const size_t image = (size_t)p.h * p.w;
+    return p.out_planes ? ((size_t)bi * (p.cout / 8) + c0 / 8 + half) * image + pix : (((size_t)bi * image + pix) * p.cout + c0) / 8 + half;
 }
 
 constexpr int PCONV_THREADS = 192; // warp 0: TMA producer, warp 1: MMA issuer, warps 2-5: epilogue
@@ -145,7 +160,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
             tt /= p.tiles_x;
             const int ty = tt % p.tiles_y;
             const int bi = tt / p.tiles_y;
-            const int x0 = tx * TILE_W, y0 = ty * TILE_H;
+            const int x0 = tx << p.tile_shift, y0 = ty * (TILE_M >> p.tile_shift);
             for (int it = 0; it < iters; it++, g++)
             {
                 const uint32_t s = g % (uint32_t)S, r = g / (uint32_t)S;
@@ -158,7 +173,9 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
                 mbar_expect_tx(&full[s], stage_bytes);
                 const int tap = it / chunks, c = it % chunks;
                 const int dy = TAPS == 9 ? tap / 3 - 1 : 0, dx = TAPS == 9 ? tap % 3 - 1 : 0;
-                if (p.chunked_map)
+                if (p.in_planes)
+                    tma_load_4d(st, &xmap, 2 * (x0 + dx), y0 + dy, c * (p.ck / 8), bi, &full[s]);
+                else if (p.chunked_map)
                     tma_load_5d(st, &xmap, 0, x0 + dx, y0 + dy, c * (p.ck / 8), bi, &full[s]);
                 else
                     for (int j = 0; j < p.ck / 8; j++)
@@ -220,9 +237,9 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
             tt /= p.tiles_x;
             const int ty = tt % p.tiles_y;
             const int bi = tt / p.tiles_y;
-            const int px = tx * TILE_W + (m % TILE_W), py = ty * TILE_H + (m / TILE_W);
+            const int px = (tx << p.tile_shift) + (m & ((1 << p.tile_shift) - 1)), py = ty * (TILE_M >> p.tile_shift) + (m >> p.tile_shift);
             const bool inb = px < p.w && py < p.h;
-            const size_t pix = ((size_t)bi * p.h + (inb ? py : 0)) * p.w + (inb ? px : 0);
+            const size_t pix = (size_t)(inb ? py : 0) * p.w + (inb ? px : 0); // of image bi
             for (int c0 = 0; c0 < p.cout; c0 += 16)
             {
                 uint32_t r[16];
@@ -242,8 +259,8 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
                 }
                 if (p.mask)
                 {
-                    const uint4 *mk = reinterpret_cast<const uint4 *>(p.mask + pix * p.cout + c0);
-                    const uint4 m0 = __ldg(mk), m1 = __ldg(mk + 1);
+                    const uint4 *mk = reinterpret_cast<const uint4 *>(p.mask);
+                    const uint4 m0 = __ldg(mk + channel_group(p, bi, pix, c0, 0)), m1 = __ldg(mk + channel_group(p, bi, pix, c0, 1));
                     const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
 #pragma unroll
                     for (int j = 0; j < 16; j++)
@@ -257,9 +274,9 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
                     const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
                     o[j] = *reinterpret_cast<const uint32_t *>(&h2);
                 }
-                uint4 *dst = reinterpret_cast<uint4 *>(p.out + pix * p.cout + c0);
-                dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-                dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+                uint4 *dst = reinterpret_cast<uint4 *>(p.out);
+                dst[channel_group(p, bi, pix, c0, 0)] = make_uint4(o[0], o[1], o[2], o[3]);
+                dst[channel_group(p, bi, pix, c0, 1)] = make_uint4(o[4], o[5], o[6], o[7]);
             }
             tc_fence_before();
             __syncwarp();
@@ -285,16 +302,19 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
 
 // ---- row-tile 3x3 convolution for the wide, thin layers ----
 //
-// A unit is 128 consecutive output pixels of one row (M = 128).  Per chunk of ck input
-// channels one TMA copy (5-D map, box {8, 130 x, 3 y, ck / 8 chunks, 1}) lands the unit's
-// halo -- 3 input rows of 130 pixels, chunk-major -- and the 9 taps are 9 descriptor start
-// offsets into it ((dy + 1) rows and (dx + 1) pixels on, 16 bytes per pixel and chunk), so
-// every input pixel is fetched for 3 units instead of 9 taps.  The weights of all taps and
-// chunks stay in shared memory for the CTA's lifetime (one bulk copy).  Roles and the
-// double-buffered TMEM accumulators are those of conv_kernel.
+// A unit is up to 128 consecutive output pixels of one row (M = 128).  Per chunk of ck input
+// channels one TMA copy lands the unit's halo -- 3 input rows, channel groups of 8 outermost -- and
+// the 9 taps are 9 descriptor start offsets into it ((dy + 1) rows and (dx + 1) pixels on, 16
+// bytes per pixel and group), so every input pixel is fetched for 3 units instead of 9 taps.  From
+// planes the copy is 128 pixels wide (a TMA box has at most 256 elements) for 126 outputs: the
+// products of the last two pixels read past their row and are not stored.  From NHWC it is 130
+// pixels wide for 128 outputs.  The weights of all taps and chunks stay in shared memory for the
+// CTA's lifetime (one bulk copy).  Roles and the double-buffered TMEM accumulators are those of
+// conv_kernel.
 constexpr int ROW_M = 128, ROW_HALO = ROW_M + 2;
-__host__ __device__ constexpr uint32_t row_chunk_bytes() { return 3u * ROW_HALO * 16u; }          // one 8-channel chunk
-__host__ __device__ constexpr uint32_t row_stage_bytes(int ck) { return ((uint32_t)(ck / 8) * row_chunk_bytes() + 1023u) / 1024u * 1024u; }
+__host__ __device__ constexpr uint32_t row_chunk_bytes(int halo) { return 3u * halo * 16u; } // one 8-channel group
+// (32 bytes more than the groups: the unstored products read that far)
+__host__ __device__ constexpr uint32_t row_stage_bytes(int ck, int halo) { return ((uint32_t)(ck / 8) * row_chunk_bytes(halo) + 32u + 1023u) / 1024u * 1024u; }
 
 template <int UNUSED = 0>
 __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid_constant__ ConvParams p, const __grid_constant__ CUtensorMap xmap)
@@ -304,7 +324,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     const int chunks = p.cin / p.ck;
     const uint32_t w_bytes = 9u * (uint32_t)p.cin * p.cout * 2u; // every tap and chunk, packed
     const uint32_t w_region = (w_bytes + 1023u) / 1024u * 1024u;
-    const uint32_t a_bytes = (uint32_t)(p.ck / 8) * row_chunk_bytes(), stage_bytes = row_stage_bytes(p.ck);
+    const uint32_t chunk_bytes = row_chunk_bytes(p.halo), a_bytes = (uint32_t)(p.ck / 8) * chunk_bytes, stage_bytes = row_stage_bytes(p.ck, p.halo);
     uint8_t *wsm = smem;
     uint8_t *ring = smem + w_region;
     uint64_t *full = reinterpret_cast<uint64_t *>(ring + (size_t)S * stage_bytes);
@@ -316,7 +336,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(wbar + 1);
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t acc_cols = tmem_cols(p.cout), ncols = 2 * acc_cols;
-    const int segs = (p.w + ROW_M - 1) / ROW_M;
+    const int segs = (p.w + p.seg_out - 1) / p.seg_out;
     const int n_units = p.b * p.h * segs;
 
     if (threadIdx.x == 0)
@@ -365,7 +385,10 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
                     break;
                 }
                 mbar_expect_tx(&full[s], a_bytes);
-                tma_load_5d(ring + (size_t)s * stage_bytes, &xmap, 0, seg * ROW_M - 1, row - 1, c * (p.ck / 8), bi, &full[s]);
+                if (p.in_planes)
+                    tma_load_4d(ring + (size_t)s * stage_bytes, &xmap, 2 * (seg * p.seg_out - 1), row - 1, c * (p.ck / 8), bi, &full[s]);
+                else
+                    tma_load_5d(ring + (size_t)s * stage_bytes, &xmap, 0, seg * p.seg_out - 1, row - 1, c * (p.ck / 8), bi, &full[s]);
             }
         }
         for (uint32_t q = g > (uint32_t)S ? g - (uint32_t)S : 0u; q < g; q++)
@@ -400,10 +423,10 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
                 const uint32_t a0 = smem_u32(ring + (size_t)s * stage_bytes);
                 for (int tap = 0; tap < 9; tap++)
                 {
-                    const uint32_t shift = (uint32_t)((tap / 3) * ROW_HALO + (tap % 3)) * 16u;
+                    const uint32_t shift = (uint32_t)((tap / 3) * p.halo + (tap % 3)) * 16u;
                     const uint32_t b0 = wbase + (uint32_t)(tap * chunks + c) * (uint32_t)p.ck * p.cout * 2u;
                     for (int k = 0; k < p.ck / 16; k++)
-                        mma_bf16(d, smem_desc(a0 + (uint32_t)(2 * k) * row_chunk_bytes() + shift, row_chunk_bytes(), 128),
+                        mma_bf16(d, smem_desc(a0 + (uint32_t)(2 * k) * chunk_bytes + shift, chunk_bytes, 128),
                                  smem_desc(b0 + k * 2 * lbo_b, lbo_b, 128), idesc, c > 0 || tap > 0 || k > 0);
                 }
                 mma_commit(&empty[s]);
@@ -425,9 +448,9 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
                 break;
             tc_fence_after();
             const int seg = u % segs, row = (u / segs) % p.h, bi = u / (segs * p.h);
-            const int px = seg * ROW_M + m;
-            const bool inb = px < p.w;
-            const size_t pix = ((size_t)bi * p.h + row) * p.w + (inb ? px : 0);
+            const int px = seg * p.seg_out + m;
+            const bool inb = m < p.seg_out && px < p.w;
+            const size_t pix = (size_t)row * p.w + (inb ? px : 0); // of image bi
             float hacc[CONV_HEAD];
             if (p.head_w)
 #pragma unroll
@@ -452,8 +475,8 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
                 }
                 if (p.mask)
                 {
-                    const uint4 *mk = reinterpret_cast<const uint4 *>(p.mask + pix * p.cout + c0);
-                    const uint4 m0 = __ldg(mk), m1 = __ldg(mk + 1);
+                    const uint4 *mk = reinterpret_cast<const uint4 *>(p.mask);
+                    const uint4 m0 = __ldg(mk + channel_group(p, bi, pix, c0, 0)), m1 = __ldg(mk + channel_group(p, bi, pix, c0, 1));
                     const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
 #pragma unroll
                     for (int j = 0; j < 16; j++)
@@ -482,18 +505,19 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
                     }
                     continue;
                 }
-                uint4 *dst = reinterpret_cast<uint4 *>(p.out + pix * p.cout + c0);
-                dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-                dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+                uint4 *dst = reinterpret_cast<uint4 *>(p.out);
+                dst[channel_group(p, bi, pix, c0, 0)] = make_uint4(o[0], o[1], o[2], o[3]);
+                dst[channel_group(p, bi, pix, c0, 1)] = make_uint4(o[4], o[5], o[6], o[7]);
             }
             if (p.head_w && inb)
             {
+                const size_t hp = (size_t)bi * p.h * p.w + pix;
                 if (p.head_flow)
-                    *reinterpret_cast<float4 *>(p.head_flow + pix * CONV_HEAD) = make_float4(hacc[0], hacc[1], hacc[2], hacc[3]);
+                    *reinterpret_cast<float4 *>(p.head_flow + hp * CONV_HEAD) = make_float4(hacc[0], hacc[1], hacc[2], hacc[3]);
                 if (p.head_flow16)
                 {
                     const __half2 h0 = __floats2half2_rn(hacc[0], hacc[1]), h1 = __floats2half2_rn(hacc[2], hacc[3]);
-                    *reinterpret_cast<uint2 *>(p.head_flow16 + pix * CONV_HEAD) =
+                    *reinterpret_cast<uint2 *>(p.head_flow16 + hp * CONV_HEAD) =
                         make_uint2(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1));
                 }
             }
@@ -532,7 +556,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
 // ones behind its channels.  Both operands are MN-major (the channel runs along the 16-byte row).
 // A CTA keeps every accumulator in TMEM: M blocks x (rows x cin + 16) columns; where that exceeds
 // 512 the grid's y takes one dy each, and its z one M block each (wgrad_config in isti_unet.cu).
-// 1x1 layers: one row, no shift, the image a single row of pixels.
+// 1x1 layers: one row, no shift, an image one row of pixels.
 //
 // Bound by shared-memory operand reads (4 KB of A per K = 16 step, 32 cycles) and latency; 8 images
 // of 480x272: 32 -> 32 channels 407 -> 134 us, 16 -> 32 358 -> 99, 64 -> 64 at half size 154 -> 68;
@@ -546,6 +570,7 @@ struct WgradParams
     int cin, cout;
     int kseg, segs, n_units, units_per_split;
     int n_dy, n_mb; // X rows and M blocks of one CTA
+    int dy_planes, x_planes; // layouts
     int box_chunks; // channel chunks (of 8) per TMA box of dY: cout / 8, or 1 where an M block may start inside a shift
     int stages;
 };
@@ -624,9 +649,16 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
             for (int b = 0; b < boxes; b++)
             {
                 const int gc = mb0 * 16 + b * p.box_chunks, shift = TAPS == 9 ? gc / co_chunks - 1 : 0;
-                tma_load_5d(st + (uint32_t)(b * p.box_chunks) * px_bytes, &dymap, 0, x0 + shift, row, gc % co_chunks, bi, &full[s]);
+                uint8_t *dst = st + (uint32_t)(b * p.box_chunks) * px_bytes;
+                if (p.dy_planes)
+                    tma_load_4d(dst, &dymap, 2 * (x0 + shift), row, gc % co_chunks, bi, &full[s]);
+                else
+                    tma_load_5d(dst, &dymap, 0, x0 + shift, row, gc % co_chunks, bi, &full[s]);
             }
-            tma_load_5d(st + a_bytes, &xmap, 0, x0, row + dy0 - 1, 0, bi, &full[s]);
+            if (p.x_planes)
+                tma_load_4d(st + a_bytes, &xmap, 2 * x0, row + dy0 - 1, 0, bi, &full[s]);
+            else
+                tma_load_5d(st + a_bytes, &xmap, 0, x0, row + dy0 - 1, 0, bi, &full[s]);
             issued = it + 1;
         }
         for (int it = issued > S ? issued - S : 0; it < issued; it++)

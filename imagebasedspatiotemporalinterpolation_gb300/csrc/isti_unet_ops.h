@@ -21,13 +21,18 @@ struct ConvHead
     void *flow16;
 };
 
+// planes: which tensors are in planes of 8 channels ([n][c / 8][h][w][8], isti_unet_conv.cuh) rather
+// than NHWC -- IN_PLANES the layer's input (x, of the weight gradient too), OUT_PLANES its output
+// (out and mask; dy of the weight gradient).
+constexpr int IN_PLANES = 1, OUT_PLANES = 2;
+
 // pdl: launch as a programmatic dependent of the previous kernel in `stream` (it prepares
 // while that kernel finishes; see griddep_wait in isti_tc.cuh).  head: fuse that head into
 // the epilogue where the row-tile kernel runs the layer (then `out` is not written and
 // *head_fused is set); otherwise the layer runs as usual and *head_fused is cleared.
 isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, const void *wpack, const float *bias, const void *mask, int relu,
-                        void *out, int cout, int32_t *status, cudaStream_t stream, bool pdl = false, const ConvHead *head = nullptr,
-                        bool *head_fused = nullptr);
+                        void *out, int cout, int32_t *status, cudaStream_t stream, int planes = 0, bool pdl = false,
+                        const ConvHead *head = nullptr, bool *head_fused = nullptr);
 
 // <<<grid, block, smem, stream>>> with, when `pdl`, the programmatic-dependent-launch
 // attribute; the kernel must call griddep_wait before it touches the previous kernel's data
@@ -48,7 +53,7 @@ cudaError_t launch_kernel(void (*kernel)(K...), dim3 grid, dim3 block, size_t sm
 }
 // db (may be null): the bias gradient, the column sums of dy
 isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, int w, int cin, int cout, float *dw, float *db, int accumulate,
-                         void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream);
+                         void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream, int planes = 0);
 isti_status pack_launch(int taps, const float *w, int cin, int cout, int transpose, void *wpack, cudaStream_t stream);
 size_t wgrad_scratch(int taps, int n, int h, int w, int cin, int cout);
 } // namespace isti_unet
