@@ -133,12 +133,34 @@ __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t m, uint32_t n, uint32
            | ((m >> 4) << 24);  // M >> 4
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate)
+// A descriptor's low word holds the start address (in units of 16 bytes, below 2^14) and LBO, so
+// moving it within shared memory is one 32-bit addition; the high word (SBO, version) stays.  One
+// thread issues the MMAs, and what it computes for each of them is what bounds narrow ones
+// (N = 32: about 190 cycles an MMA with descriptors built from scratch).
+struct Desc
 {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-                 "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate)
+    uint32_t lo, hi;
+    __device__ __forceinline__ Desc(uint32_t saddr, uint32_t lbo, uint32_t sbo)
+    {
+        const uint64_t d = smem_desc(saddr, lbo, sbo);
+        lo = (uint32_t)d;
+        hi = (uint32_t)(d >> 32);
+    }
+    // start address + bytes (a multiple of 16)
+    __device__ __forceinline__ Desc operator+(uint32_t bytes) const
+    {
+        Desc d = *this;
+        d.lo += bytes >> 4;
+        return d;
+    }
+};
+
+// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, Desc a, Desc b, uint32_t idesc, bool accumulate)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(tmem_d),
+                 "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"((uint32_t)accumulate)
                  : "memory");
 }
 

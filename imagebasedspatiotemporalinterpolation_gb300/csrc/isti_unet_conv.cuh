@@ -93,12 +93,163 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, i
                  : "memory");
 }
 
-// The 16-byte groups of channels c0 .. c0 + 7 and c0 + 8 .. c0 + 15 of a pixel (image bi, pixel
-// `pix` of the image) of an output-shaped tensor.
-__device__ __forceinline__ size_t channel_group(const ConvParams &p, int bi, size_t pix, int c0, int half)
+// The producer, MMA and epilogue loops run on one thread or four warps of a CTA, at the latency of
+// every instruction: divisions are done once and positions then stepped along.
+
+// Position in a ring of S stages: stage and phase (how often the ring wrapped, mod 2).
+struct RingPos
 {
-    const size_t image = (size_t)p.h * p.w;
-    return p.out_planes ? ((size_t)bi * (p.cout / 8) + c0 / 8 + half) * image + pix : (((size_t)bi * image + pix) * p.cout + c0) / 8 + half;
+    uint32_t s = 0, phase = 0;
+    __device__ __forceinline__ void next(uint32_t S)
+    {
+        if (++s == S)
+        {
+            s = 0;
+            phase ^= 1u;
+        }
+    }
+};
+
+// Unit u = (bi * ny + y) * nx + x, stepped by `step` units at a time.
+struct UnitPos
+{
+    int x, y, b, dx, dy, db, nx, ny;
+    __device__ __forceinline__ UnitPos(int u, int step, int nx_, int ny_) : nx(nx_), ny(ny_)
+    {
+        x = u % nx, u /= nx, y = u % ny, b = u / ny;
+        dx = step % nx, step /= nx, dy = step % ny, db = step / ny;
+    }
+    __device__ __forceinline__ void next()
+    {
+        x += dx, y += dy, b += db;
+        if (x >= nx)
+            x -= nx, y++;
+        if (y >= ny)
+            y -= ny, b++;
+    }
+};
+
+// What the epilogue reads for every pixel: bias, and the weights and bias of a fused head.
+constexpr int CONV_MAX_COUT = 256;
+struct EpilogueTable
+{
+    float bias[CONV_MAX_COUT];
+    float head[CONV_HEAD * CONV_MAX_COUT], head_bias[CONV_HEAD];
+    __device__ __forceinline__ void fill(const ConvParams &p) // whole block; parameters only, no previous kernel's output
+    {
+        for (int i = threadIdx.x; i < p.cout; i += blockDim.x)
+            bias[i] = p.bias ? __ldg(p.bias + i) : 0.0f;
+        if (!p.head_w)
+            return;
+        for (int i = threadIdx.x; i < CONV_HEAD * p.cout; i += blockDim.x)
+            head[i] = __ldg(p.head_w + i);
+        if (threadIdx.x < CONV_HEAD)
+            head_bias[threadIdx.x] = __ldg(p.head_b + threadIdx.x);
+    }
+};
+
+// Drains the accumulator of one pixel per lane (warp-collective; columns taddr .. taddr + cout - 1):
+// bias, ReLU, gradient mask, bf16, 16-byte stores or the fused head.  pix: the pixel within image bi;
+// store: whether this lane's pixel exists.
+__device__ __forceinline__ void epilogue_pixel(const ConvParams &p, const EpilogueTable &t, uint32_t taddr, int bi, uint32_t pix, bool store)
+{
+    // 16-byte groups of 8 channels: the pixel's first, and the distance to the next
+    const size_t image = (size_t)p.h * p.w, groups = (size_t)(p.cout / 8);
+    size_t group = p.out_planes ? (size_t)bi * groups * image + pix : ((size_t)bi * image + pix) * groups;
+    const size_t step = p.out_planes ? image : 1;
+    float hacc[CONV_HEAD];
+    if (p.head_w)
+#pragma unroll
+        for (int q = 0; q < CONV_HEAD; q++)
+            hacc[q] = t.head_bias[q];
+#pragma unroll 1
+    for (int c0 = 0; c0 < p.cout; c0 += 32)
+    {
+        uint32_t r[2][16];
+        const int halves = c0 + 16 < p.cout ? 2 : 1;
+        tmem_ld16(taddr + (uint32_t)c0, r[0]);
+        if (halves == 2)
+            tmem_ld16(taddr + (uint32_t)c0 + 16u, r[1]);
+        tmem_ld_wait();
+        if (!store)
+            continue;
+#pragma unroll
+        for (int half = 0; half < 2; half++)
+        {
+            if (half == halves)
+                break;
+            const int c = c0 + 16 * half;
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++)
+                v[j] = __uint_as_float(r[half][j]);
+            if (p.bias)
+#pragma unroll
+                for (int j = 0; j < 16; j += 4)
+                {
+                    const float4 b = *reinterpret_cast<const float4 *>(t.bias + c + j);
+                    v[j] += b.x, v[j + 1] += b.y, v[j + 2] += b.z, v[j + 3] += b.w;
+                }
+            if (p.relu)
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    v[j] = fmaxf(v[j], 0.0f);
+            if (p.mask)
+            {
+                const uint4 *mk = reinterpret_cast<const uint4 *>(p.mask) + group;
+                const uint4 m0 = __ldg(mk), m1 = __ldg(mk + step);
+                const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (!bf16_positive((uint16_t)(mw[j / 2] >> (16 * (j % 2)))))
+                        v[j] = 0.0f;
+            }
+            uint32_t o[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+            {
+                const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                o[j] = *reinterpret_cast<const uint32_t *>(&h2);
+            }
+            if (p.head_w)
+            {
+#pragma unroll
+                for (int j = 0; j < 8; j += 2)
+                {
+                    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&o[j]));
+                    const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&o[j + 1]));
+#pragma unroll
+                    for (int q = 0; q < CONV_HEAD; q++)
+                    {
+                        const float4 w = *reinterpret_cast<const float4 *>(t.head + q * p.cout + c + 2 * j);
+                        hacc[q] = fmaf(w.x, f.x, hacc[q]);
+                        hacc[q] = fmaf(w.y, f.y, hacc[q]);
+                        hacc[q] = fmaf(w.z, g.x, hacc[q]);
+                        hacc[q] = fmaf(w.w, g.y, hacc[q]);
+                    }
+                }
+            }
+            else
+            {
+                uint4 *dst = reinterpret_cast<uint4 *>(p.out) + group;
+                dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                dst[step] = make_uint4(o[4], o[5], o[6], o[7]);
+            }
+            group += 2 * step;
+        }
+    }
+    if (p.head_w && store)
+    {
+        const size_t hp = (size_t)bi * image + pix;
+        if (p.head_flow)
+            *reinterpret_cast<float4 *>(p.head_flow + hp * CONV_HEAD) = make_float4(hacc[0], hacc[1], hacc[2], hacc[3]);
+        if (p.head_flow16)
+        {
+            const __half2 h0 = __floats2half2_rn(hacc[0], hacc[1]), h1 = __floats2half2_rn(hacc[2], hacc[3]);
+            *reinterpret_cast<uint2 *>(p.head_flow16 + hp * CONV_HEAD) =
+                make_uint2(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1));
+        }
+    }
 }
 
 constexpr int PCONV_THREADS = 192; // warp 0: TMA producer, warp 1: MMA issuer, warps 2-5: epilogue
@@ -111,6 +262,7 @@ template <int TAPS>
 __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_constant__ ConvParams p, const __grid_constant__ CUtensorMap xmap)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(16) EpilogueTable table;
     const int S = p.stages;
     const uint32_t a_bytes = (uint32_t)p.ck * 256u, b_bytes = (uint32_t)p.ck * p.cout * 2u, stage_bytes = a_bytes + b_bytes;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)S * stage_bytes);
@@ -122,6 +274,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t acc_cols = tmem_cols(p.cout), ncols = 2 * acc_cols;
 
+    table.fill(p);
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < S; s++)
@@ -143,7 +296,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const int chunks = p.cin / p.ck, iters = TAPS * chunks;
+    const int chunks = p.cin / p.ck;
     if (threadIdx.x == 0)
         griddep_launch_dependents(); // the next layer may set up while this one runs
 
@@ -151,36 +304,36 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     {
         griddep_wait(); // the previous layer's output is complete (every load below is later)
         fence_proxy_async_global();
-        uint32_t g = 0;
+        uint32_t g = 0; // stages filled
+        RingPos ring;
+        UnitPos at(blockIdx.x, gridDim.x, p.tiles_x, p.tiles_y);
         bool stop = false;
-        for (int t = blockIdx.x; t < p.n_tiles && !stop; t += gridDim.x)
+        for (int t = blockIdx.x; t < p.n_tiles && !stop; t += gridDim.x, at.next())
         {
-            int tt = t;
-            const int tx = tt % p.tiles_x;
-            tt /= p.tiles_x;
-            const int ty = tt % p.tiles_y;
-            const int bi = tt / p.tiles_y;
-            const int x0 = tx << p.tile_shift, y0 = ty * (TILE_M >> p.tile_shift);
-            for (int it = 0; it < iters; it++, g++)
+            const int x0 = at.x << p.tile_shift, y0 = at.y * (TILE_M >> p.tile_shift);
+            const __nv_bfloat16 *weights = p.wpack;
+            for (int tap = 0; tap < TAPS && !stop; tap++)
             {
-                const uint32_t s = g % (uint32_t)S, r = g / (uint32_t)S;
-                if (r > 0 && !mbar_wait(&empty[s], (r - 1) & 1u, p.status))
-                {
-                    stop = true;
-                    break;
-                }
-                uint8_t *st = smem + (size_t)s * stage_bytes;
-                mbar_expect_tx(&full[s], stage_bytes);
-                const int tap = it / chunks, c = it % chunks;
                 const int dy = TAPS == 9 ? tap / 3 - 1 : 0, dx = TAPS == 9 ? tap % 3 - 1 : 0;
-                if (p.in_planes)
-                    tma_load_4d(st, &xmap, 2 * (x0 + dx), y0 + dy, c * (p.ck / 8), bi, &full[s]);
-                else if (p.chunked_map)
-                    tma_load_5d(st, &xmap, 0, x0 + dx, y0 + dy, c * (p.ck / 8), bi, &full[s]);
-                else
-                    for (int j = 0; j < p.ck / 8; j++)
-                        tma_load_4d(st + j * BOX_BYTES, &xmap, c * p.ck + 8 * j, x0 + dx, y0 + dy, bi, &full[s]);
-                bulk_load(st + a_bytes, p.wpack + (size_t)it * p.ck * p.cout, b_bytes, &full[s]);
+                for (int c = 0; c < chunks; c++, g++, ring.next(S), weights += p.ck * p.cout)
+                {
+                    const uint32_t s = ring.s;
+                    if (!mbar_wait(&empty[s], ring.phase ^ 1u, p.status)) // (the first round's waits return at once)
+                    {
+                        stop = true;
+                        break;
+                    }
+                    uint8_t *st = smem + (size_t)s * stage_bytes;
+                    mbar_expect_tx(&full[s], stage_bytes);
+                    if (p.in_planes)
+                        tma_load_4d(st, &xmap, 2 * (x0 + dx), y0 + dy, c * (p.ck / 8), at.b, &full[s]);
+                    else if (p.chunked_map)
+                        tma_load_5d(st, &xmap, 0, x0 + dx, y0 + dy, c * (p.ck / 8), at.b, &full[s]);
+                    else
+                        for (int j = 0; j < p.ck / 8; j++)
+                            tma_load_4d(st + j * BOX_BYTES, &xmap, c * p.ck + 8 * j, x0 + dx, y0 + dy, at.b, &full[s]);
+                    bulk_load(st + a_bytes, weights, b_bytes, &full[s]);
+                }
             }
         }
         for (uint32_t q = g > (uint32_t)S ? g - (uint32_t)S : 0u; q < g; q++) // copies still landing
@@ -191,7 +344,8 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     {
         const uint32_t idesc = idesc_bf16(TILE_M, (uint32_t)p.cout, 0, 0);
         const uint32_t lbo_b = (uint32_t)(p.cout / 8) * 128u;
-        uint32_t g = 0;
+        const int iters = TAPS * chunks;
+        RingPos ring;
         int i = 0;
         bool stop = false;
         for (int t = blockIdx.x; t < p.n_tiles && !stop; t += gridDim.x, i++)
@@ -201,19 +355,20 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
                 break;
             tc_fence_after();
             const uint32_t d = tmem + (uint32_t)buf * acc_cols;
-            for (int it = 0; it < iters; it++, g++)
+            for (int it = 0; it < iters; it++, ring.next(S))
             {
-                const uint32_t s = g % (uint32_t)S, r = g / (uint32_t)S;
-                if (!mbar_wait(&full[s], r & 1u, p.status))
+                const uint32_t s = ring.s;
+                if (!mbar_wait(&full[s], ring.phase, p.status))
                 {
                     stop = true;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t a0 = smem_u32(smem + (size_t)s * stage_bytes), b0 = a0 + a_bytes;
-                for (int k = 0; k < p.ck / 16; k++)
-                    mma_bf16(d, smem_desc(a0 + k * 2 * BOX_BYTES, BOX_BYTES, 128), smem_desc(b0 + k * 2 * lbo_b, lbo_b, 128), idesc,
-                             it > 0 || k > 0);
+                const uint32_t a0 = smem_u32(smem) + s * stage_bytes;
+                const Desc da(a0, BOX_BYTES, 128), db(a0 + a_bytes, lbo_b, 128);
+                mma_bf16(d, da, db, idesc, it > 0);
+                if (p.ck == 32)
+                    mma_bf16(d, da + 2u * BOX_BYTES, db + 2u * lbo_b, idesc, true);
                 mma_commit(&empty[s]);
             }
             if (!stop)
@@ -224,60 +379,18 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     else if (warp >= 2)
     {
         const int q = warp % 4; // the TMEM lane quadrant this warp may read
-        const int m = q * 32 + lane;
+        const int m = q * 32 + lane, mx = m & ((1 << p.tile_shift) - 1), my = m >> p.tile_shift;
+        UnitPos at(blockIdx.x, gridDim.x, p.tiles_x, p.tiles_y);
         int i = 0;
-        for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, i++)
+        for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, i++, at.next())
         {
             const int buf = i & 1;
             if (!mbar_wait(&acc_full[buf], (uint32_t)((i >> 1) & 1), p.status))
                 break;
             tc_fence_after();
-            int tt = t;
-            const int tx = tt % p.tiles_x;
-            tt /= p.tiles_x;
-            const int ty = tt % p.tiles_y;
-            const int bi = tt / p.tiles_y;
-            const int px = (tx << p.tile_shift) + (m & ((1 << p.tile_shift) - 1)), py = ty * (TILE_M >> p.tile_shift) + (m >> p.tile_shift);
-            const bool inb = px < p.w && py < p.h;
-            const size_t pix = (size_t)(inb ? py : 0) * p.w + (inb ? px : 0); // of image bi
-            for (int c0 = 0; c0 < p.cout; c0 += 16)
-            {
-                uint32_t r[16];
-                tmem_ld16(tmem + (uint32_t)buf * acc_cols + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
-                tmem_ld_wait();
-                if (!inb)
-                    continue;
-                float v[16];
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                {
-                    v[j] = __uint_as_float(r[j]);
-                    if (p.bias)
-                        v[j] += __ldg(p.bias + c0 + j);
-                    if (p.relu)
-                        v[j] = fmaxf(v[j], 0.0f);
-                }
-                if (p.mask)
-                {
-                    const uint4 *mk = reinterpret_cast<const uint4 *>(p.mask);
-                    const uint4 m0 = __ldg(mk + channel_group(p, bi, pix, c0, 0)), m1 = __ldg(mk + channel_group(p, bi, pix, c0, 1));
-                    const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (!bf16_positive((uint16_t)(mw[j / 2] >> (16 * (j % 2)))))
-                            v[j] = 0.0f;
-                }
-                uint32_t o[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                {
-                    const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                    o[j] = *reinterpret_cast<const uint32_t *>(&h2);
-                }
-                uint4 *dst = reinterpret_cast<uint4 *>(p.out);
-                dst[channel_group(p, bi, pix, c0, 0)] = make_uint4(o[0], o[1], o[2], o[3]);
-                dst[channel_group(p, bi, pix, c0, 1)] = make_uint4(o[4], o[5], o[6], o[7]);
-            }
+            const int px = (at.x << p.tile_shift) + mx, py = at.y * (TILE_M >> p.tile_shift) + my;
+            epilogue_pixel(p, table, tmem + (uint32_t)buf * acc_cols + ((uint32_t)(q * 32) << 16), at.b, (uint32_t)py * (uint32_t)p.w + (uint32_t)px,
+                           px < p.w && py < p.h);
             tc_fence_before();
             __syncwarp();
             if (lane == 0)
@@ -320,6 +433,7 @@ template <int UNUSED = 0>
 __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid_constant__ ConvParams p, const __grid_constant__ CUtensorMap xmap)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(16) EpilogueTable table;
     const int S = p.stages;
     const int chunks = p.cin / p.ck;
     const uint32_t w_bytes = 9u * (uint32_t)p.cin * p.cout * 2u; // every tap and chunk, packed
@@ -339,6 +453,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     const int segs = (p.w + p.seg_out - 1) / p.seg_out;
     const int n_units = p.b * p.h * segs;
 
+    table.fill(p);
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < S; s++)
@@ -372,25 +487,24 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
         griddep_wait(); // the previous layer's output is complete (every activation load below is later)
         fence_proxy_async_global();
         uint32_t g = 0;
+        RingPos pos;
+        UnitPos at(blockIdx.x, gridDim.x, segs, p.h);
         bool stop = false;
-        for (int u = blockIdx.x; u < n_units && !stop; u += gridDim.x)
-        {
-            const int seg = u % segs, row = (u / segs) % p.h, bi = u / (segs * p.h);
-            for (int c = 0; c < chunks; c++, g++)
+        for (int u = blockIdx.x; u < n_units && !stop; u += gridDim.x, at.next())
+            for (int c = 0; c < chunks; c++, g++, pos.next(S))
             {
-                const uint32_t s = g % (uint32_t)S, r = g / (uint32_t)S;
-                if (r > 0 && !mbar_wait(&empty[s], (r - 1) & 1u, p.status))
+                const uint32_t s = pos.s;
+                if (!mbar_wait(&empty[s], pos.phase ^ 1u, p.status))
                 {
                     stop = true;
                     break;
                 }
                 mbar_expect_tx(&full[s], a_bytes);
                 if (p.in_planes)
-                    tma_load_4d(ring + (size_t)s * stage_bytes, &xmap, 2 * (seg * p.seg_out - 1), row - 1, c * (p.ck / 8), bi, &full[s]);
+                    tma_load_4d(ring + (size_t)s * stage_bytes, &xmap, 2 * (at.x * p.seg_out - 1), at.y - 1, c * (p.ck / 8), at.b, &full[s]);
                 else
-                    tma_load_5d(ring + (size_t)s * stage_bytes, &xmap, 0, seg * p.seg_out - 1, row - 1, c * (p.ck / 8), bi, &full[s]);
+                    tma_load_5d(ring + (size_t)s * stage_bytes, &xmap, 0, at.x * p.seg_out - 1, at.y - 1, c * (p.ck / 8), at.b, &full[s]);
             }
-        }
         for (uint32_t q = g > (uint32_t)S ? g - (uint32_t)S : 0u; q < g; q++)
             if (!mbar_wait(&full[q % (uint32_t)S], (q / (uint32_t)S) & 1u, p.status))
                 break;
@@ -400,8 +514,9 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     {
         const uint32_t idesc = idesc_bf16(ROW_M, (uint32_t)p.cout, 0, 0);
         const uint32_t lbo_b = (uint32_t)(p.cout / 8) * 128u;
-        const uint32_t wbase = smem_u32(wsm);
-        uint32_t g = 0;
+        const uint32_t wtap_bytes = (uint32_t)p.ck * p.cout * 2u; // packed weights of one tap and chunk
+        const Desc db0(smem_u32(wsm), lbo_b, 128);
+        RingPos pos;
         int i = 0;
         bool stop = !mbar_wait(wbar, 0, p.status);
         for (int u = blockIdx.x; u < n_units && !stop; u += gridDim.x, i++)
@@ -411,23 +526,24 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
                 break;
             tc_fence_after();
             const uint32_t d = tmem + (uint32_t)buf * acc_cols;
-            for (int c = 0; c < chunks; c++, g++)
+            for (int c = 0; c < chunks; c++, pos.next(S))
             {
-                const uint32_t s = g % (uint32_t)S, r = g / (uint32_t)S;
-                if (!mbar_wait(&full[s], r & 1u, p.status))
+                const uint32_t s = pos.s;
+                if (!mbar_wait(&full[s], pos.phase, p.status))
                 {
                     stop = true;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t a0 = smem_u32(ring + (size_t)s * stage_bytes);
-                for (int tap = 0; tap < 9; tap++)
+                const Desc da(smem_u32(ring) + s * stage_bytes, chunk_bytes, 128);
+                Desc db = db0 + (uint32_t)c * wtap_bytes;
+#pragma unroll
+                for (int tap = 0; tap < 9; tap++, db = db + (uint32_t)chunks * wtap_bytes)
                 {
-                    const uint32_t shift = (uint32_t)((tap / 3) * p.halo + (tap % 3)) * 16u;
-                    const uint32_t b0 = wbase + (uint32_t)(tap * chunks + c) * (uint32_t)p.ck * p.cout * 2u;
-                    for (int k = 0; k < p.ck / 16; k++)
-                        mma_bf16(d, smem_desc(a0 + (uint32_t)(2 * k) * chunk_bytes + shift, chunk_bytes, 128),
-                                 smem_desc(b0 + k * 2 * lbo_b, lbo_b, 128), idesc, c > 0 || tap > 0 || k > 0);
+                    const Desc dt = da + (uint32_t)((tap / 3) * p.halo + (tap % 3)) * 16u;
+                    mma_bf16(d, dt, db, idesc, c > 0 || tap > 0);
+                    if (p.ck == 32)
+                        mma_bf16(d, dt + 2u * chunk_bytes, db + 2u * lbo_b, idesc, true);
                 }
                 mma_commit(&empty[s]);
             }
@@ -440,87 +556,17 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     {
         const int q = warp % 4;
         const int m = q * 32 + lane;
+        UnitPos at(blockIdx.x, gridDim.x, segs, p.h);
         int i = 0;
-        for (int u = blockIdx.x; u < n_units; u += gridDim.x, i++)
+        for (int u = blockIdx.x; u < n_units; u += gridDim.x, i++, at.next())
         {
             const int buf = i & 1;
             if (!mbar_wait(&acc_full[buf], (uint32_t)((i >> 1) & 1), p.status))
                 break;
             tc_fence_after();
-            const int seg = u % segs, row = (u / segs) % p.h, bi = u / (segs * p.h);
-            const int px = seg * p.seg_out + m;
-            const bool inb = m < p.seg_out && px < p.w;
-            const size_t pix = (size_t)row * p.w + (inb ? px : 0); // of image bi
-            float hacc[CONV_HEAD];
-            if (p.head_w)
-#pragma unroll
-                for (int q = 0; q < CONV_HEAD; q++)
-                    hacc[q] = __ldg(p.head_b + q);
-            for (int c0 = 0; c0 < p.cout; c0 += 16)
-            {
-                uint32_t r[16];
-                tmem_ld16(tmem + (uint32_t)buf * acc_cols + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
-                tmem_ld_wait();
-                if (!inb)
-                    continue;
-                float v[16];
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                {
-                    v[j] = __uint_as_float(r[j]);
-                    if (p.bias)
-                        v[j] += __ldg(p.bias + c0 + j);
-                    if (p.relu)
-                        v[j] = fmaxf(v[j], 0.0f);
-                }
-                if (p.mask)
-                {
-                    const uint4 *mk = reinterpret_cast<const uint4 *>(p.mask);
-                    const uint4 m0 = __ldg(mk + channel_group(p, bi, pix, c0, 0)), m1 = __ldg(mk + channel_group(p, bi, pix, c0, 1));
-                    const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (!bf16_positive((uint16_t)(mw[j / 2] >> (16 * (j % 2)))))
-                            v[j] = 0.0f;
-                }
-                uint32_t o[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                {
-                    const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                    o[j] = *reinterpret_cast<const uint32_t *>(&h2);
-                }
-                if (p.head_w)
-                {
-#pragma unroll
-                    for (int j = 0; j < 8; j++)
-                    {
-                        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&o[j]));
-#pragma unroll
-                        for (int q = 0; q < CONV_HEAD; q++)
-                        {
-                            hacc[q] = fmaf(__ldg(p.head_w + q * p.cout + c0 + 2 * j), f.x, hacc[q]);
-                            hacc[q] = fmaf(__ldg(p.head_w + q * p.cout + c0 + 2 * j + 1), f.y, hacc[q]);
-                        }
-                    }
-                    continue;
-                }
-                uint4 *dst = reinterpret_cast<uint4 *>(p.out);
-                dst[channel_group(p, bi, pix, c0, 0)] = make_uint4(o[0], o[1], o[2], o[3]);
-                dst[channel_group(p, bi, pix, c0, 1)] = make_uint4(o[4], o[5], o[6], o[7]);
-            }
-            if (p.head_w && inb)
-            {
-                const size_t hp = (size_t)bi * p.h * p.w + pix;
-                if (p.head_flow)
-                    *reinterpret_cast<float4 *>(p.head_flow + hp * CONV_HEAD) = make_float4(hacc[0], hacc[1], hacc[2], hacc[3]);
-                if (p.head_flow16)
-                {
-                    const __half2 h0 = __floats2half2_rn(hacc[0], hacc[1]), h1 = __floats2half2_rn(hacc[2], hacc[3]);
-                    *reinterpret_cast<uint2 *>(p.head_flow16 + hp * CONV_HEAD) =
-                        make_uint2(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1));
-                }
-            }
+            const int px = at.x * p.seg_out + m;
+            epilogue_pixel(p, table, tmem + (uint32_t)buf * acc_cols + ((uint32_t)(q * 32) << 16), at.b, (uint32_t)at.y * (uint32_t)p.w + (uint32_t)px,
+                           m < p.seg_out && px < p.w);
             tc_fence_before();
             __syncwarp();
             if (lane == 0)
@@ -636,29 +682,34 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     if (warp == 0 && lane == 0)
     {
         const uint32_t tx_bytes = (uint32_t)(boxes * p.box_chunks) * px_bytes + (uint32_t)(p.cin / 8) * b_rows_bytes;
+        const int shift0 = mb0 * 16 / co_chunks, group0 = mb0 * 16 % co_chunks; // of the first box
+        RingPos ring;
+        UnitPos at(u_begin, 1, p.segs, p.h);
         int issued = 0;
-        for (int it = 0; it < iters; it++)
+        for (int it = 0; it < iters; it++, ring.next(S), at.next())
         {
-            const int s = it % S, r = it / S;
-            if (r > 0 && !mbar_wait(&empty[s], (uint32_t)((r - 1) & 1), p.status))
+            const uint32_t s = ring.s;
+            if (!mbar_wait(&empty[s], ring.phase ^ 1u, p.status)) // (the first round's waits return at once)
                 break;
-            const int u = u_begin + it;
-            const int x0 = (u % p.segs) * p.kseg, row = (u / p.segs) % p.h, bi = u / (p.segs * p.h);
+            const int x0 = at.x * p.kseg;
             uint8_t *st = smem + (size_t)s * stage_bytes;
             mbar_expect_tx(&full[s], tx_bytes);
+            int shift = TAPS == 9 ? shift0 - 1 : 0, group = group0;
             for (int b = 0; b < boxes; b++)
             {
-                const int gc = mb0 * 16 + b * p.box_chunks, shift = TAPS == 9 ? gc / co_chunks - 1 : 0;
                 uint8_t *dst = st + (uint32_t)(b * p.box_chunks) * px_bytes;
                 if (p.dy_planes)
-                    tma_load_4d(dst, &dymap, 2 * (x0 + shift), row, gc % co_chunks, bi, &full[s]);
+                    tma_load_4d(dst, &dymap, 2 * (x0 + shift), at.y, group, at.b, &full[s]);
                 else
-                    tma_load_5d(dst, &dymap, 0, x0 + shift, row, gc % co_chunks, bi, &full[s]);
+                    tma_load_5d(dst, &dymap, 0, x0 + shift, at.y, group, at.b, &full[s]);
+                group += p.box_chunks;
+                if (group >= co_chunks)
+                    group = 0, shift++;
             }
             if (p.x_planes)
-                tma_load_4d(st + a_bytes, &xmap, 2 * x0, row + dy0 - 1, 0, bi, &full[s]);
+                tma_load_4d(st + a_bytes, &xmap, 2 * x0, at.y + dy0 - 1, 0, at.b, &full[s]);
             else
-                tma_load_5d(st + a_bytes, &xmap, 0, x0, row + dy0 - 1, 0, bi, &full[s]);
+                tma_load_5d(st + a_bytes, &xmap, 0, x0, at.y + dy0 - 1, 0, at.b, &full[s]);
             issued = it + 1;
         }
         for (int it = issued > S ? issued - S : 0; it < issued; it++)
@@ -669,24 +720,28 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     {
         // MN-major operands: LBO = distance between core matrices adjacent in K (the next 8
         // pixels, 128 bytes on), SBO = between core matrices adjacent in M/N (the next 8 channels)
-        for (int it = 0; it < iters; it++)
+        RingPos ring;
+        for (int it = 0; it < iters; it++, ring.next(S))
         {
-            const int s = it % S, r = it / S;
-            if (!mbar_wait(&full[s], (uint32_t)(r & 1), p.status))
+            const uint32_t s = ring.s;
+            if (!mbar_wait(&full[s], ring.phase, p.status))
                 break;
             tc_fence_after();
-            const uint32_t a0 = smem_u32(smem + (size_t)s * stage_bytes), b0 = a0 + a_bytes;
+            const uint32_t a0 = smem_u32(smem) + s * stage_bytes, b0 = a0 + a_bytes;
             for (int d = 0; d < p.n_dy; d++)
             {
-                const bool ones = p.bpartial && dy0 + d == 1;
-                const uint32_t idesc = idesc_bf16(128, (uint32_t)p.cin + (ones ? 16u : 0u), 1, 1);
+                const uint32_t idesc = idesc_bf16(128, (uint32_t)p.cin + (p.bpartial && dy0 + d == 1 ? 16u : 0u), 1, 1);
                 for (int mb = 0; mb < p.n_mb; mb++)
                 {
                     const uint32_t acc = tmem + (uint32_t)(mb * wgrad_mb_cols(p.cin, p.n_dy) + row_col(d));
+                    Desc da(a0 + (uint32_t)mb * 16u * px_bytes, 128u, px_bytes), db(b0 + (uint32_t)d * px_bytes, 128u, b_rows_bytes);
                     // K = 16 pixels per MMA: two 8-pixel core-matrix groups, 256 bytes on
-                    for (int k = 0; k < p.kseg / 16; k++)
-                        mma_bf16(acc, smem_desc(a0 + (uint32_t)mb * 16u * px_bytes + k * 256, 128u, px_bytes),
-                                 smem_desc(b0 + (uint32_t)d * px_bytes + k * 256, 128u, b_rows_bytes), idesc, it > 0 || k > 0);
+                    for (int k = 0; k < p.kseg; k += 64, da = da + 1024u, db = db + 1024u)
+                    {
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; q++)
+                            mma_bf16(acc, da + q * 256u, db + q * 256u, idesc, it > 0 || k > 0 || q > 0);
+                    }
                 }
             }
             mma_commit(&empty[s]);
