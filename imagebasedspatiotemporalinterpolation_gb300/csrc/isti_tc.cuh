@@ -48,6 +48,29 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
+// ---- warp-collective forms ----
+//
+// The producer and the MMA issuer are whole warps in step: every lane computes the same addresses,
+// descriptors and coordinates, and one elected lane executes the copy, MMA or arrival (predicated,
+// no branch).  The compiler then keeps those values on the uniform datapath, where the tensor
+// instructions take them from; issued from a branch for one lane, each of them moved five or six
+// registers over first, at the latency of the move.
+
+// 1 in one lane of the warp (whole warp)
+__device__ __forceinline__ uint32_t elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n}" : "=r"(e));
+    return e;
+}
+
+__device__ __forceinline__ void mbar_expect_tx_if(uint32_t leader, uint64_t *bar, uint32_t bytes)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}" ::"r"(smem_u32(bar)),
+                 "r"(bytes), "r"(leader)
+                 : "memory");
+}
+
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -74,24 +97,46 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int32_
     return false;
 }
 
+// mbar_wait by a whole warp in step
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, int32_t *status)
+{
+    for (uint32_t i = 0; i < WAIT_LIMIT; i++)
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity)))
+            return true;
+    atomicExch(status, ERR_TIMEOUT);
+    return false;
+}
+
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// 4-D tiled TMA load (c, x, y, n) of a tensor map into shared memory; completion on `bar`.
+// 4-D tiled TMA load (c, x, y, n) of a tensor map into shared memory (address dst); completion on `bar`.
 // c * 2 bytes must be a multiple of 16 (c a multiple of 8 for bf16); x and y may be
 // negative or past the end (zero fill).
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c, int x, int y, int n, uint64_t *bar)
+__device__ __forceinline__ void tma_load_4d(uint32_t leader, uint32_t dst, const CUtensorMap *map, int c, int x, int y, int n, uint64_t *bar)
 {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(map), "r"(c), "r"(x), "r"(y), "r"(n), "r"(smem_u32(bar))
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %7, 0;\n\t"
+                 "@p cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n}" ::"r"(dst),
+                 "l"(map), "r"(c), "r"(x), "r"(y), "r"(n), "r"(smem_u32(bar)), "r"(leader)
+                 : "memory");
+}
+
+// 5-D form
+__device__ __forceinline__ void tma_load_5d(uint32_t leader, uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4,
+                                            uint64_t *bar)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %8, 0;\n\t"
+                 "@p cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];\n}" ::"r"(
+                     dst),
+                 "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar)), "r"(leader)
                  : "memory");
 }
 
 // Untiled bulk copy global -> shared (both 16-byte aligned, size a multiple of 16).
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
+__device__ __forceinline__ void bulk_load(uint32_t leader, uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar)
 {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "@p cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar)), "r"(leader)
                  : "memory");
 }
 
@@ -135,8 +180,8 @@ __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t m, uint32_t n, uint32
 
 // A descriptor's low word holds the start address (in units of 16 bytes, below 2^14) and LBO, so
 // moving it within shared memory is one 32-bit addition; the high word (SBO, version) stays.  One
-// thread issues the MMAs, and what it computes for each of them is what bounds narrow ones
-// (N = 32: about 190 cycles an MMA with descriptors built from scratch).
+// warp issues the MMAs, and what it computes for each of them is what bounds narrow ones
+// (N = 32: about 190 cycles an MMA with descriptors built from scratch in a branch for one lane).
 struct Desc
 {
     uint32_t lo, hi;
@@ -155,19 +200,22 @@ struct Desc
     }
 };
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, Desc a, Desc b, uint32_t idesc, bool accumulate)
+// D[tmem] (+)= A[smem] * B[smem]^T, issued by the elected lane.
+__device__ __forceinline__ void mma_bf16(uint32_t leader, uint32_t tmem_d, Desc a, Desc b, uint32_t idesc, bool accumulate)
 {
-    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(tmem_d),
-                 "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"((uint32_t)accumulate)
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+                 "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(tmem_d),
+                 "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader)
                  : "memory");
 }
 
-// Arrives on `bar` once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void mma_commit(uint64_t *bar)
+// Arrives on `bar` once every MMA issued so far by the elected lane has completed.
+__device__ __forceinline__ void mma_commit(uint32_t leader, uint64_t *bar)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(smem_u32(bar)), "r"(leader)
+                 : "memory");
 }
 
 // 32 lanes x 16 columns of 32-bit TMEM words: thread i of the warp gets lane (base lane + i),

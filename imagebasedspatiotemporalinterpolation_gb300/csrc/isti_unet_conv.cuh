@@ -84,15 +84,6 @@ __host__ __device__ constexpr uint32_t conv_stage_bytes(int ck, int cout) { retu
 // bf16 > 0 (positive, non-zero, not NaN)
 __device__ __forceinline__ bool bf16_positive(uint16_t b) { return (b & 0x8000u) == 0 && (b & 0x7fffu) != 0 && (b & 0x7fffu) <= 0x7f80u; }
 
-// 5-D tiled TMA load (c_lo, x, y, c_hi, n): the channel chunks of a box land one after another
-__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4, uint64_t *bar)
-{
-    asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
-                 : "memory");
-}
-
 // The producer, MMA and epilogue loops run on one thread or four warps of a CTA, at the latency of
 // every instruction: divisions are done once and positions then stepped along.
 
@@ -271,7 +262,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     uint64_t *acc_empty = acc_full + 2;
     uint64_t *mma_done = acc_empty + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x / 32, 0), lane = threadIdx.x % 32; // warp: known to be uniform
     const uint32_t acc_cols = tmem_cols(p.cout), ncols = 2 * acc_cols;
 
     table.fill(p);
@@ -300,8 +291,9 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     if (threadIdx.x == 0)
         griddep_launch_dependents(); // the next layer may set up while this one runs
 
-    if (warp == 0 && lane == 0)
+    if (warp == 0)
     {
+        const uint32_t leader = elect_one();
         griddep_wait(); // the previous layer's output is complete (every load below is later)
         fence_proxy_async_global();
         uint32_t g = 0; // stages filled
@@ -318,30 +310,31 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
                 for (int c = 0; c < chunks; c++, g++, ring.next(S), weights += p.ck * p.cout)
                 {
                     const uint32_t s = ring.s;
-                    if (!mbar_wait(&empty[s], ring.phase ^ 1u, p.status)) // (the first round's waits return at once)
+                    if (!mbar_wait_warp(&empty[s], ring.phase ^ 1u, p.status)) // (the first round's waits return at once)
                     {
                         stop = true;
                         break;
                     }
-                    uint8_t *st = smem + (size_t)s * stage_bytes;
-                    mbar_expect_tx(&full[s], stage_bytes);
+                    const uint32_t st = smem_u32(smem) + s * stage_bytes;
+                    mbar_expect_tx_if(leader, &full[s], stage_bytes);
                     if (p.in_planes)
-                        tma_load_4d(st, &xmap, 2 * (x0 + dx), y0 + dy, c * (p.ck / 8), at.b, &full[s]);
+                        tma_load_4d(leader, st, &xmap, 2 * (x0 + dx), y0 + dy, c * (p.ck / 8), at.b, &full[s]);
                     else if (p.chunked_map)
-                        tma_load_5d(st, &xmap, 0, x0 + dx, y0 + dy, c * (p.ck / 8), at.b, &full[s]);
+                        tma_load_5d(leader, st, &xmap, 0, x0 + dx, y0 + dy, c * (p.ck / 8), at.b, &full[s]);
                     else
                         for (int j = 0; j < p.ck / 8; j++)
-                            tma_load_4d(st + j * BOX_BYTES, &xmap, c * p.ck + 8 * j, x0 + dx, y0 + dy, at.b, &full[s]);
-                    bulk_load(st + a_bytes, weights, b_bytes, &full[s]);
+                            tma_load_4d(leader, st + j * BOX_BYTES, &xmap, c * p.ck + 8 * j, x0 + dx, y0 + dy, at.b, &full[s]);
+                    bulk_load(leader, st + a_bytes, weights, b_bytes, &full[s]);
                 }
             }
         }
         for (uint32_t q = g > (uint32_t)S ? g - (uint32_t)S : 0u; q < g; q++) // copies still landing
-            if (!mbar_wait(&full[q % (uint32_t)S], (q / (uint32_t)S) & 1u, p.status))
+            if (!mbar_wait_warp(&full[q % (uint32_t)S], (q / (uint32_t)S) & 1u, p.status))
                 break;
     }
-    else if (warp == 1 && lane == 0)
+    else if (warp == 1)
     {
+        const uint32_t leader = elect_one();
         const uint32_t idesc = idesc_bf16(TILE_M, (uint32_t)p.cout, 0, 0);
         const uint32_t lbo_b = (uint32_t)(p.cout / 8) * 128u;
         const int iters = TAPS * chunks;
@@ -351,14 +344,14 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
         for (int t = blockIdx.x; t < p.n_tiles && !stop; t += gridDim.x, i++)
         {
             const int buf = i & 1;
-            if (i >= 2 && !mbar_wait(&acc_empty[buf], (uint32_t)(((i >> 1) - 1) & 1), p.status))
+            if (i >= 2 && !mbar_wait_warp(&acc_empty[buf], (uint32_t)(((i >> 1) - 1) & 1), p.status))
                 break;
             tc_fence_after();
             const uint32_t d = tmem + (uint32_t)buf * acc_cols;
             for (int it = 0; it < iters; it++, ring.next(S))
             {
                 const uint32_t s = ring.s;
-                if (!mbar_wait(&full[s], ring.phase, p.status))
+                if (!mbar_wait_warp(&full[s], ring.phase, p.status))
                 {
                     stop = true;
                     break;
@@ -366,15 +359,15 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
                 tc_fence_after();
                 const uint32_t a0 = smem_u32(smem) + s * stage_bytes;
                 const Desc da(a0, BOX_BYTES, 128), db(a0 + a_bytes, lbo_b, 128);
-                mma_bf16(d, da, db, idesc, it > 0);
+                mma_bf16(leader, d, da, db, idesc, it > 0);
                 if (p.ck == 32)
-                    mma_bf16(d, da + 2u * BOX_BYTES, db + 2u * lbo_b, idesc, true);
-                mma_commit(&empty[s]);
+                    mma_bf16(leader, d, da + 2u * BOX_BYTES, db + 2u * lbo_b, idesc, true);
+                mma_commit(leader, &empty[s]);
             }
             if (!stop)
-                mma_commit(&acc_full[buf]);
+                mma_commit(leader, &acc_full[buf]);
         }
-        mma_commit(mma_done);
+        mma_commit(leader, mma_done);
     }
     else if (warp >= 2)
     {
@@ -448,7 +441,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     uint64_t *mma_done = acc_empty + 2;
     uint64_t *wbar = mma_done + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(wbar + 1);
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x / 32, 0), lane = threadIdx.x % 32; // warp: known to be uniform
     const uint32_t acc_cols = tmem_cols(p.cout), ncols = 2 * acc_cols;
     const int segs = (p.w + p.seg_out - 1) / p.seg_out;
     const int n_units = p.b * p.h * segs;
@@ -479,11 +472,12 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
 
     if (threadIdx.x == 0)
         griddep_launch_dependents(); // the next layer may set up while this one runs
-    if (warp == 0 && lane == 0)
+    if (warp == 0)
     {
-        mbar_expect_tx(wbar, w_bytes);
+        const uint32_t leader = elect_one();
+        mbar_expect_tx_if(leader, wbar, w_bytes);
         for (uint32_t o = 0; o < w_bytes; o += 32768u) // pieces of at most 32 KiB (weights: no previous kernel writes them)
-            bulk_load(wsm + o, reinterpret_cast<const uint8_t *>(p.wpack) + o, min(32768u, w_bytes - o), wbar);
+            bulk_load(leader, smem_u32(wsm) + o, reinterpret_cast<const uint8_t *>(p.wpack) + o, min(32768u, w_bytes - o), wbar);
         griddep_wait(); // the previous layer's output is complete (every activation load below is later)
         fence_proxy_async_global();
         uint32_t g = 0;
@@ -494,42 +488,43 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
             for (int c = 0; c < chunks; c++, g++, pos.next(S))
             {
                 const uint32_t s = pos.s;
-                if (!mbar_wait(&empty[s], pos.phase ^ 1u, p.status))
+                if (!mbar_wait_warp(&empty[s], pos.phase ^ 1u, p.status))
                 {
                     stop = true;
                     break;
                 }
-                mbar_expect_tx(&full[s], a_bytes);
+                mbar_expect_tx_if(leader, &full[s], a_bytes);
                 if (p.in_planes)
-                    tma_load_4d(ring + (size_t)s * stage_bytes, &xmap, 2 * (at.x * p.seg_out - 1), at.y - 1, c * (p.ck / 8), at.b, &full[s]);
+                    tma_load_4d(leader, smem_u32(ring) + s * stage_bytes, &xmap, 2 * (at.x * p.seg_out - 1), at.y - 1, c * (p.ck / 8), at.b, &full[s]);
                 else
-                    tma_load_5d(ring + (size_t)s * stage_bytes, &xmap, 0, at.x * p.seg_out - 1, at.y - 1, c * (p.ck / 8), at.b, &full[s]);
+                    tma_load_5d(leader, smem_u32(ring) + s * stage_bytes, &xmap, 0, at.x * p.seg_out - 1, at.y - 1, c * (p.ck / 8), at.b, &full[s]);
             }
         for (uint32_t q = g > (uint32_t)S ? g - (uint32_t)S : 0u; q < g; q++)
-            if (!mbar_wait(&full[q % (uint32_t)S], (q / (uint32_t)S) & 1u, p.status))
+            if (!mbar_wait_warp(&full[q % (uint32_t)S], (q / (uint32_t)S) & 1u, p.status))
                 break;
-        mbar_wait(wbar, 0, p.status);
+        mbar_wait_warp(wbar, 0, p.status);
     }
-    else if (warp == 1 && lane == 0)
+    else if (warp == 1)
     {
+        const uint32_t leader = elect_one();
         const uint32_t idesc = idesc_bf16(ROW_M, (uint32_t)p.cout, 0, 0);
         const uint32_t lbo_b = (uint32_t)(p.cout / 8) * 128u;
         const uint32_t wtap_bytes = (uint32_t)p.ck * p.cout * 2u; // packed weights of one tap and chunk
         const Desc db0(smem_u32(wsm), lbo_b, 128);
         RingPos pos;
         int i = 0;
-        bool stop = !mbar_wait(wbar, 0, p.status);
+        bool stop = !mbar_wait_warp(wbar, 0, p.status);
         for (int u = blockIdx.x; u < n_units && !stop; u += gridDim.x, i++)
         {
             const int buf = i & 1;
-            if (i >= 2 && !mbar_wait(&acc_empty[buf], (uint32_t)(((i >> 1) - 1) & 1), p.status))
+            if (i >= 2 && !mbar_wait_warp(&acc_empty[buf], (uint32_t)(((i >> 1) - 1) & 1), p.status))
                 break;
             tc_fence_after();
             const uint32_t d = tmem + (uint32_t)buf * acc_cols;
             for (int c = 0; c < chunks; c++, pos.next(S))
             {
                 const uint32_t s = pos.s;
-                if (!mbar_wait(&full[s], pos.phase, p.status))
+                if (!mbar_wait_warp(&full[s], pos.phase, p.status))
                 {
                     stop = true;
                     break;
@@ -541,16 +536,16 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
                 for (int tap = 0; tap < 9; tap++, db = db + (uint32_t)chunks * wtap_bytes)
                 {
                     const Desc dt = da + (uint32_t)((tap / 3) * p.halo + (tap % 3)) * 16u;
-                    mma_bf16(d, dt, db, idesc, c > 0 || tap > 0);
+                    mma_bf16(leader, d, dt, db, idesc, c > 0 || tap > 0);
                     if (p.ck == 32)
-                        mma_bf16(d, dt + 2u * chunk_bytes, db + 2u * lbo_b, idesc, true);
+                        mma_bf16(leader, d, dt + 2u * chunk_bytes, db + 2u * lbo_b, idesc, true);
                 }
-                mma_commit(&empty[s]);
+                mma_commit(leader, &empty[s]);
             }
             if (!stop)
-                mma_commit(&acc_full[buf]);
+                mma_commit(leader, &acc_full[buf]);
         }
-        mma_commit(mma_done);
+        mma_commit(leader, mma_done);
     }
     else if (warp >= 2)
     {
@@ -643,7 +638,7 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     uint64_t *empty = full + S;
     uint64_t *done = empty + S;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x / 32, 0), lane = threadIdx.x % 32; // warp: known to be uniform
     const int split = blockIdx.x, dy0 = TAPS == 9 ? (int)blockIdx.y : 1, mb0 = (int)blockIdx.z * p.n_mb; // dy0: first row, 0..2
     const int u_begin = split * p.units_per_split, u_end = min(p.n_units, u_begin + p.units_per_split);
     const int iters = max(0, u_end - u_begin);
@@ -679,8 +674,9 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == 0 && lane == 0)
+    if (warp == 0)
     {
+        const uint32_t leader = elect_one();
         const uint32_t tx_bytes = (uint32_t)(boxes * p.box_chunks) * px_bytes + (uint32_t)(p.cin / 8) * b_rows_bytes;
         const int shift0 = mb0 * 16 / co_chunks, group0 = mb0 * 16 % co_chunks; // of the first box
         RingPos ring;
@@ -689,42 +685,43 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
         for (int it = 0; it < iters; it++, ring.next(S), at.next())
         {
             const uint32_t s = ring.s;
-            if (!mbar_wait(&empty[s], ring.phase ^ 1u, p.status)) // (the first round's waits return at once)
+            if (!mbar_wait_warp(&empty[s], ring.phase ^ 1u, p.status)) // (the first round's waits return at once)
                 break;
             const int x0 = at.x * p.kseg;
-            uint8_t *st = smem + (size_t)s * stage_bytes;
-            mbar_expect_tx(&full[s], tx_bytes);
+            const uint32_t st = smem_u32(smem) + s * stage_bytes;
+            mbar_expect_tx_if(leader, &full[s], tx_bytes);
             int shift = TAPS == 9 ? shift0 - 1 : 0, group = group0;
             for (int b = 0; b < boxes; b++)
             {
-                uint8_t *dst = st + (uint32_t)(b * p.box_chunks) * px_bytes;
+                const uint32_t dst = st + (uint32_t)(b * p.box_chunks) * px_bytes;
                 if (p.dy_planes)
-                    tma_load_4d(dst, &dymap, 2 * (x0 + shift), at.y, group, at.b, &full[s]);
+                    tma_load_4d(leader, dst, &dymap, 2 * (x0 + shift), at.y, group, at.b, &full[s]);
                 else
-                    tma_load_5d(dst, &dymap, 0, x0 + shift, at.y, group, at.b, &full[s]);
+                    tma_load_5d(leader, dst, &dymap, 0, x0 + shift, at.y, group, at.b, &full[s]);
                 group += p.box_chunks;
                 if (group >= co_chunks)
                     group = 0, shift++;
             }
             if (p.x_planes)
-                tma_load_4d(st + a_bytes, &xmap, 2 * x0, at.y + dy0 - 1, 0, at.b, &full[s]);
+                tma_load_4d(leader, st + a_bytes, &xmap, 2 * x0, at.y + dy0 - 1, 0, at.b, &full[s]);
             else
-                tma_load_5d(st + a_bytes, &xmap, 0, x0, at.y + dy0 - 1, 0, at.b, &full[s]);
+                tma_load_5d(leader, st + a_bytes, &xmap, 0, x0, at.y + dy0 - 1, 0, at.b, &full[s]);
             issued = it + 1;
         }
         for (int it = issued > S ? issued - S : 0; it < issued; it++)
-            if (!mbar_wait(&full[it % S], (uint32_t)((it / S) & 1), p.status))
+            if (!mbar_wait_warp(&full[it % S], (uint32_t)((it / S) & 1), p.status))
                 break;
     }
-    else if (warp == 1 && lane == 0)
+    else if (warp == 1)
     {
+        const uint32_t leader = elect_one();
         // MN-major operands: LBO = distance between core matrices adjacent in K (the next 8
         // pixels, 128 bytes on), SBO = between core matrices adjacent in M/N (the next 8 channels)
         RingPos ring;
         for (int it = 0; it < iters; it++, ring.next(S))
         {
             const uint32_t s = ring.s;
-            if (!mbar_wait(&full[s], ring.phase, p.status))
+            if (!mbar_wait_warp(&full[s], ring.phase, p.status))
                 break;
             tc_fence_after();
             const uint32_t a0 = smem_u32(smem) + s * stage_bytes, b0 = a0 + a_bytes;
@@ -740,13 +737,13 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
                     {
 #pragma unroll
                         for (uint32_t q = 0; q < 4; q++)
-                            mma_bf16(acc, da + q * 256u, db + q * 256u, idesc, it > 0 || k > 0 || q > 0);
+                            mma_bf16(leader, acc, da + q * 256u, db + q * 256u, idesc, it > 0 || k > 0 || q > 0);
                     }
                 }
             }
-            mma_commit(&empty[s]);
+            mma_commit(leader, &empty[s]);
         }
-        mma_commit(done);
+        mma_commit(leader, done);
     }
     __syncwarp();
 
