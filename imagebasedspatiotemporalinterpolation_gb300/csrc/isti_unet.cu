@@ -350,8 +350,6 @@ isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, 
     p.segs = c.segs;
     p.n_units = c.n_units;
     p.units_per_split = c.units_per_split;
-    p.n_dy = c.n_dy;
-    p.n_mb = c.n_mb;
     p.box_chunks = c.grid_z == 1 ? cout / 8 : 1;
     p.stages = c.stages;
     p.dy_planes = (planes & OUT_PLANES) != 0;
@@ -361,7 +359,10 @@ isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, 
         (st = box_map(xmap, x, p.x_planes, c.n, c.h, c.w, cin, c.kseg, c.n_dy, cin / 8)) != ISTI_OK)
         return st;
     const dim3 grid((unsigned)c.splits, (unsigned)c.grid_y, (unsigned)c.grid_z);
-    auto kernel = taps == 9 ? wgrad_kernel<9> : wgrad_kernel<1>;
+    using Kernel = void (*)(WgradParams, CUtensorMap, CUtensorMap);
+    constexpr Kernel rows3[3] = {wgrad_kernel<9, 3, 1>, wgrad_kernel<9, 3, 2>, wgrad_kernel<9, 3, 3>};
+    constexpr Kernel rows1[3] = {wgrad_kernel<9, 1, 1>, wgrad_kernel<9, 1, 2>, wgrad_kernel<9, 1, 3>};
+    const Kernel kernel = taps == 1 ? wgrad_kernel<1, 1, 1> : (c.n_dy == 3 ? rows3 : rows1)[c.n_mb - 1];
     cudaError_t e = smem_limit(kernel, c.smem);
     if (e == cudaSuccess)
     {

@@ -596,12 +596,14 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
 // The bias gradient (the column sums of dY) rides along: the row of dy = 0 has 16 more columns of
 // ones behind its channels.  Both operands are MN-major (the channel runs along the 16-byte row).
 // A CTA keeps every accumulator in TMEM: M blocks x (rows x cin + 16) columns; where that exceeds
-// 512 the grid's y takes one dy each, and its z one M block each (wgrad_config in isti_unet.cu).
+// 512 the grid's y takes one dy each, and its z one M block each (wgrad_config in isti_unet.cu;
+// N_DY X rows and N_MB M blocks per CTA).
 // 1x1 layers: one row, no shift, an image one row of pixels.
 //
-// Bound by shared-memory operand reads (4 KB of A per K = 16 step, 32 cycles) and latency; 8 images
-// of 480x272: 32 -> 32 channels 407 -> 134 us, 16 -> 32 358 -> 99, 64 -> 64 at half size 154 -> 68;
-// the bias gradients had passes over dY of their own, 0.7 ms of a 3.0 ms step.
+// Bound by the issue of narrow MMAs (about 75 cycles each) and by shared-memory operand reads (4 KB
+// of A per K = 16 step).  8 images of 480x272: 32 -> 32 channels 407 -> 50 us, 16 -> 32 358 -> 41,
+// 64 -> 64 at half size 154 -> 37; the bias gradients had passes over dY of their own, 0.7 ms of a
+// 3.0 ms step.
 struct WgradParams
 {
     float *partial;  // [splits][cout][TAPS][cin]
@@ -610,7 +612,6 @@ struct WgradParams
     int w, h, b;
     int cin, cout;
     int kseg, segs, n_units, units_per_split;
-    int n_dy, n_mb; // X rows and M blocks of one CTA
     int dy_planes, x_planes; // layouts
     int box_chunks; // channel chunks (of 8) per TMA box of dY: cout / 8, or 1 where an M block may start inside a shift
     int stages;
@@ -625,7 +626,7 @@ __host__ __device__ constexpr int wgrad_mb_cols(int cin, int n_dy) { return n_dy
 
 constexpr int WGRAD_THREADS = 128; // warp 0 producer, warp 1 MMA, all four epilogue
 
-template <int TAPS>
+template <int TAPS, int N_DY, int N_MB>
 __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_constant__ WgradParams p, const __grid_constant__ CUtensorMap dymap,
                                                               const __grid_constant__ CUtensorMap xmap)
 {
@@ -633,19 +634,19 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     constexpr int SHIFTS = TAPS == 9 ? 3 : 1;
     const int S = p.stages;
     const uint32_t px_bytes = (uint32_t)p.kseg * 16u; // one channel chunk of a unit's pixels
-    const uint32_t a_bytes = wgrad_a_bytes(p.n_mb, p.kseg), stage_bytes = wgrad_stage_bytes(p.cin, p.n_dy, p.n_mb, p.kseg);
+    const uint32_t a_bytes = wgrad_a_bytes(N_MB, p.kseg), stage_bytes = wgrad_stage_bytes(p.cin, N_DY, N_MB, p.kseg);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)S * stage_bytes);
     uint64_t *empty = full + S;
     uint64_t *done = empty + S;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x / 32, 0), lane = threadIdx.x % 32; // warp: known to be uniform
-    const int split = blockIdx.x, dy0 = TAPS == 9 ? (int)blockIdx.y : 1, mb0 = (int)blockIdx.z * p.n_mb; // dy0: first row, 0..2
+    const int split = blockIdx.x, dy0 = TAPS == 9 ? (int)blockIdx.y : 1, mb0 = (int)blockIdx.z * N_MB; // dy0: first row, 0..2
     const int u_begin = split * p.units_per_split, u_end = min(p.n_units, u_begin + p.units_per_split);
     const int iters = max(0, u_end - u_begin);
     const int co_chunks = p.cout / 8;
-    const int boxes = min(p.n_mb * 16, SHIFTS * co_chunks - mb0 * 16) / p.box_chunks; // dY boxes of this CTA
-    const uint32_t ncols = tmem_cols(p.n_mb * wgrad_mb_cols(p.cin, p.n_dy));
-    const uint32_t b_rows_bytes = (uint32_t)p.n_dy * px_bytes; // one channel chunk of X
+    const int boxes = min(N_MB * 16, SHIFTS * co_chunks - mb0 * 16) / p.box_chunks; // dY boxes of this CTA
+    const uint32_t ncols = tmem_cols(N_MB * wgrad_mb_cols(p.cin, N_DY));
+    const uint32_t b_rows_bytes = (uint32_t)N_DY * px_bytes; // one channel chunk of X
     // columns of row d within an M block: the row of dy = 0 has 16 more
     auto row_col = [&](int d) { return d * p.cin + (dy0 + d > 1 && d > 0 ? 16 : 0); };
 
@@ -717,6 +718,13 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
         const uint32_t leader = elect_one();
         // MN-major operands: LBO = distance between core matrices adjacent in K (the next 8
         // pixels, 128 bytes on), SBO = between core matrices adjacent in M/N (the next 8 channels)
+        const uint32_t idesc_side = idesc_bf16(128, (uint32_t)p.cin, 1, 1);
+        const uint32_t idesc_centre = idesc_bf16(128, (uint32_t)p.cin + (p.bpartial ? 16u : 0u), 1, 1);
+        const uint32_t mb_cols = (uint32_t)wgrad_mb_cols(p.cin, N_DY);
+        uint32_t row_cols[N_DY];
+#pragma unroll
+        for (int d = 0; d < N_DY; d++)
+            row_cols[d] = (uint32_t)row_col(d);
         RingPos ring;
         for (int it = 0; it < iters; it++, ring.next(S))
         {
@@ -725,21 +733,22 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
                 break;
             tc_fence_after();
             const uint32_t a0 = smem_u32(smem) + s * stage_bytes, b0 = a0 + a_bytes;
-            for (int d = 0; d < p.n_dy; d++)
+            const Desc da(a0, 128u, px_bytes), db(b0, 128u, b_rows_bytes);
+            // K = 16 pixels per MMA: two 8-pixel core-matrix groups, 256 bytes on.  The accumulators in
+            // turn, an MMA into the one before's waits for it; unrolled, the loop costs more than that
+            for (uint32_t k0 = 0; k0 < px_bytes; k0 += 1024u)
             {
-                const uint32_t idesc = idesc_bf16(128, (uint32_t)p.cin + (p.bpartial && dy0 + d == 1 ? 16u : 0u), 1, 1);
-                for (int mb = 0; mb < p.n_mb; mb++)
-                {
-                    const uint32_t acc = tmem + (uint32_t)(mb * wgrad_mb_cols(p.cin, p.n_dy) + row_col(d));
-                    Desc da(a0 + (uint32_t)mb * 16u * px_bytes, 128u, px_bytes), db(b0 + (uint32_t)d * px_bytes, 128u, b_rows_bytes);
-                    // K = 16 pixels per MMA: two 8-pixel core-matrix groups, 256 bytes on
-                    for (int k = 0; k < p.kseg; k += 64, da = da + 1024u, db = db + 1024u)
-                    {
 #pragma unroll
-                        for (uint32_t q = 0; q < 4; q++)
-                            mma_bf16(leader, acc, da + q * 256u, db + q * 256u, idesc, it > 0 || k > 0 || q > 0);
-                    }
-                }
+                for (int q = 0; q < 4; q++)
+#pragma unroll
+                    for (int mb = 0; mb < N_MB; mb++)
+#pragma unroll
+                        for (int d = 0; d < N_DY; d++)
+                        {
+                            const uint32_t k = k0 + 256u * q;
+                            mma_bf16(leader, tmem + (uint32_t)mb * mb_cols + row_cols[d], da + (uint32_t)mb * 16u * px_bytes + k,
+                                     db + (uint32_t)d * px_bytes + k, dy0 + d == 1 ? idesc_centre : idesc_side, it > 0 || k0 > 0 || q > 0);
+                        }
             }
             mma_commit(leader, &empty[s]);
         }
@@ -750,18 +759,18 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     const bool ok = mbar_wait(done, 0, p.status);
     tc_fence_after();
     if (ok)
-        for (int mb = 0; mb < p.n_mb; mb++)
+        for (int mb = 0; mb < N_MB; mb++)
         {
             const int m = (mb0 + mb) * 128 + warp * 32 + lane; // row (shift, co)
             const int shift = m / p.cout, co = m % p.cout;
-            for (int d = 0; d < p.n_dy; d++)
+            for (int d = 0; d < N_DY; d++)
             {
                 const int tap = TAPS == 9 ? (dy0 + d) * 3 + (2 - shift) : 0;
                 const bool ones = p.bpartial && dy0 + d == 1;
                 for (int c0 = 0; c0 < p.cin + (ones ? 16 : 0); c0 += 16)
                 {
                     uint32_t r[16];
-                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mb * wgrad_mb_cols(p.cin, p.n_dy) + row_col(d) + c0), r);
+                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mb * wgrad_mb_cols(p.cin, N_DY) + row_col(d) + c0), r);
                     tmem_ld_wait();
                     if (shift >= SHIFTS)
                         continue;
