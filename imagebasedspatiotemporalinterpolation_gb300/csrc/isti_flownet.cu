@@ -156,6 +156,8 @@ __global__ void __launch_bounds__(EW_X * EW_Y) upadd_kernel(const bf16 *a, const
 __global__ void __launch_bounds__(EW_X * EW_Y) poolback_kernel(const bf16 *gskip, const bf16 *gq, const bf16 *act, uint32_t planes, uint32_t ho,
                                                                uint32_t wo, bf16 *ge)
 {
+    isti_tc::griddep_launch_dependents();
+    isti_tc::griddep_wait();
     for_each_block(planes, ho, wo, [&](size_t half, size_t full, size_t row) {
         uint4 us[4], ua[4];
 #pragma unroll
@@ -255,6 +257,8 @@ __global__ void __launch_bounds__(HEAD_TILE, 2) head_back_kernel(const bf16 *d1,
         sw[i] = hw[i];
     if (threadIdx.x < HEAD_COUT)
         sw[HEAD_COUT * HEAD_CIN + threadIdx.x] = hb[threadIdx.x];
+    isti_tc::griddep_launch_dependents();
+    isti_tc::griddep_wait(); // the weights above are no previous kernel's output; d1 is
     __syncthreads();
     const bool label_vec = (reinterpret_cast<uintptr_t>(label) & 15u) == 0;
     const int q = threadIdx.x / HEAD_LANES, lane = threadIdx.x % HEAD_LANES; // second step: channel group, pixel lane
@@ -283,7 +287,7 @@ __global__ void __launch_bounds__(HEAD_TILE, 2) head_back_kernel(const bf16 *d1,
             for (int g = 0; g < HEAD_GROUPS; g++)
             {
                 float t[8];
-                unpack8(__ldg(src + g * image), t);
+                unpack8(src[g * image], t);
 #pragma unroll
                 for (int k = 0; k < 8; k++)
                     f[8 * g + k] = t[k];
@@ -331,7 +335,7 @@ __global__ void __launch_bounds__(HEAD_TILE, 2) head_back_kernel(const bf16 *d1,
             const float4 g4 = gout[buf][t];
             const float g[HEAD_COUT] = {g4.x, g4.y, g4.z, g4.w};
             float f[8];
-            unpack8(__ldg(reinterpret_cast<const uint4 *>(d1) + plane_group(p0 + t, image, HEAD_GROUPS, q)), f);
+            unpack8(reinterpret_cast<const uint4 *>(d1)[plane_group(p0 + t, image, HEAD_GROUPS, q)], f);
 #pragma unroll
             for (int j = 0; j < HEAD_COUT; j++)
             {
@@ -380,6 +384,8 @@ constexpr int SUM_PARTS = 8;
 __global__ void __launch_bounds__(32 * SUM_PARTS) head_sums_kernel(const float *partial, int blocks, float *grads, float *loss)
 {
     __shared__ float part[SUM_PARTS][32];
+    isti_tc::griddep_launch_dependents();
+    isti_tc::griddep_wait();
     const int i = blockIdx.x * 32 + threadIdx.x;
     float s = 0.0f;
     if (i < HEAD_VALUES)
@@ -530,7 +536,7 @@ isti_status dgrad(isti_flownet *net, int l, const bf16 *g_out, int n, int h, int
 {
     const LayerDef &d = LAYERS[l];
     return isti_unet::conv_launch(d.taps, g_out, n, h, w, d.cout, net->packs + net->pkt_off[l], nullptr, mask, 0, g_in, d.cin, net->status, s,
-                                  isti_unet::IN_PLANES | isti_unet::OUT_PLANES);
+                                  isti_unet::IN_PLANES | isti_unet::OUT_PLANES, true);
 }
 
 isti_status wgrad(isti_flownet *net, int l, const bf16 *g_out, const bf16 *x, int n, int h, int w, Buffers &b, cudaStream_t s)
@@ -538,7 +544,7 @@ isti_status wgrad(isti_flownet *net, int l, const bf16 *g_out, const bf16 *x, in
     const LayerDef &d = LAYERS[l];
     return isti_unet::wgrad_launch(d.taps, g_out, x, n, h, w, d.cin, d.cout, net->grads + net->w_off[l], net->grads + net->b_off[l], 0, b.wscratch,
                                    b.wscratch_bytes, net->status, s,
-                                   l == 0 ? isti_unet::OUT_PLANES : isti_unet::IN_PLANES | isti_unet::OUT_PLANES);
+                                   l == 0 ? isti_unet::OUT_PLANES : isti_unet::IN_PLANES | isti_unet::OUT_PLANES, true);
 }
 
 #define ISTI_TRY(x)                                                                                                                             \
@@ -549,11 +555,13 @@ isti_status wgrad(isti_flownet *net, int l, const bf16 *g_out, const bf16 *x, in
             return st_;                                                                                                                         \
     } while (0)
 
-// pdl: every launch after the first is a programmatic dependent of the one before (each
-// kernel sets up while its predecessor finishes; inference only)
+// Every launch is a programmatic dependent of the one before (each kernel sets up while its
+// predecessor finishes); the first one only with first_pdl (inference), in training it follows in full
+// order what may have written the weights.
 isti_status forward(isti_flownet *net, const bf16 *x0, int n, int h, int w, Buffers &b, float *flow, __half *flow16, cudaStream_t s,
-                    bool pdl = false)
+                    bool first_pdl = false)
 {
+    const bool pdl = true;
     using isti_unet::launch_kernel;
     const int h2 = h / 2, w2 = w / 2, h4 = h / 4, w4 = w / 4, h8 = h / 8, w8 = w / 8;
     const dim3 blk(EW_X, EW_Y);
@@ -563,7 +571,7 @@ isti_status forward(isti_flownet *net, const bf16 *x0, int n, int h, int w, Buff
             e = x;
         return e == cudaSuccess;
     };
-    ISTI_TRY(conv(net, 0, x0, n, h, w, nullptr, b.e1, s, pdl));
+    ISTI_TRY(conv(net, 0, x0, n, h, w, nullptr, b.e1, s, first_pdl));
     ok(launch_kernel(blocksum_kernel, rows_grid(n * 4 * h2), blk, 0, s, pdl, (const bf16 *)b.e1, (uint32_t)(n * 4), (uint32_t)h2, (uint32_t)w2, 0.25f, b.q1));
     ISTI_TRY(conv(net, 1, b.q1, n, h2, w2, nullptr, b.e2, s, pdl));
     ok(launch_kernel(blocksum_kernel, rows_grid(n * 8 * h4), blk, 0, s, pdl, (const bf16 *)b.e2, (uint32_t)(n * 8), (uint32_t)h4, (uint32_t)w4, 0.25f, b.q2));
@@ -599,39 +607,48 @@ isti_status backward(isti_flownet *net, const bf16 *x0, const float *label, int 
     const int h2 = h / 2, w2 = w / 2, h4 = h / 4, w4 = w / 4, h8 = h / 8, w8 = w / 8;
     const size_t npix = (size_t)n * h * w;
     const int blocks = (int)std::min<size_t>(HEAD_BLOCKS, (npix + HEAD_TILE - 1) / HEAD_TILE);
-    head_back_kernel<<<blocks, HEAD_TILE, 0, s>>>(b.d1, npix, (size_t)h * w, net->params + net->w_off[N_CONV], net->params + net->b_off[N_CONV], label,
-                                                  1.0f / (float)npix, b.g_d1, b.partial);
-    head_sums_kernel<<<(HEAD_VALUES + 31) / 32, dim3(32, SUM_PARTS), 0, s>>>(b.partial, blocks, net->grads + net->w_off[N_CONV], net->loss);
+    cudaError_t e = cudaSuccess;
+    // every launch a programmatic dependent of the one before
+    auto launch = [&](auto kernel, dim3 grid, dim3 block, auto... args) {
+        const cudaError_t x = isti_unet::launch_kernel(kernel, grid, block, 0, s, true, args...);
+        if (e == cudaSuccess)
+            e = x;
+    };
+    const dim3 blk(EW_X, EW_Y);
+    launch(head_back_kernel, dim3(blocks), dim3(HEAD_TILE), b.d1, npix, (size_t)h * w, net->params + net->w_off[N_CONV],
+           net->params + net->b_off[N_CONV], label, 1.0f / (float)npix, b.g_d1, b.partial);
+    launch(head_sums_kernel, dim3((HEAD_VALUES + 31) / 32), dim3(32, SUM_PARTS), b.partial, blocks, net->grads + net->w_off[N_CONV], net->loss);
     // level 1 decoder
     ISTI_TRY(wgrad(net, 9, b.g_d1, b.s1, n, h, w, b, s));
     ISTI_TRY(dgrad(net, 9, b.g_d1, n, h, w, nullptr, b.g_s1, s));
-    blocksum_kernel<<<rows_grid(n * 4 * h2), dim3(EW_X, EW_Y), 0, s>>>(b.g_s1, n * 4, h2, w2, 1.0f, b.g_p1);
+    launch(blocksum_kernel, rows_grid(n * 4 * h2), blk, b.g_s1, n * 4, h2, w2, 1.0f, b.g_p1);
     ISTI_TRY(wgrad(net, 8, b.g_p1, b.d2, n, h2, w2, b, s));
     ISTI_TRY(dgrad(net, 8, b.g_p1, n, h2, w2, b.d2, b.g_d2, s));
     // level 2 decoder
     ISTI_TRY(wgrad(net, 7, b.g_d2, b.s2, n, h2, w2, b, s));
     ISTI_TRY(dgrad(net, 7, b.g_d2, n, h2, w2, nullptr, b.g_s2, s));
-    blocksum_kernel<<<rows_grid(n * 8 * h4), dim3(EW_X, EW_Y), 0, s>>>(b.g_s2, n * 8, h4, w4, 1.0f, b.g_p2);
+    launch(blocksum_kernel, rows_grid(n * 8 * h4), blk, b.g_s2, n * 8, h4, w4, 1.0f, b.g_p2);
     ISTI_TRY(wgrad(net, 6, b.g_p2, b.d3, n, h4, w4, b, s));
     ISTI_TRY(dgrad(net, 6, b.g_p2, n, h4, w4, b.d3, b.g_d3, s));
     // level 3 decoder
     ISTI_TRY(wgrad(net, 5, b.g_d3, b.s3, n, h4, w4, b, s));
     ISTI_TRY(dgrad(net, 5, b.g_d3, n, h4, w4, nullptr, b.g_s3, s));
-    blocksum_kernel<<<rows_grid(n * 12 * h8), dim3(EW_X, EW_Y), 0, s>>>(b.g_s3, n * 12, h8, w8, 1.0f, b.g_p3);
+    launch(blocksum_kernel, rows_grid(n * 12 * h8), blk, b.g_s3, n * 12, h8, w8, 1.0f, b.g_p3);
     ISTI_TRY(wgrad(net, 4, b.g_p3, b.e4, n, h8, w8, b, s));
     ISTI_TRY(dgrad(net, 4, b.g_p3, n, h8, w8, b.e4, b.g_e4, s));
     // bottleneck and encoder
     ISTI_TRY(wgrad(net, 3, b.g_e4, b.q3, n, h8, w8, b, s));
     ISTI_TRY(dgrad(net, 3, b.g_e4, n, h8, w8, nullptr, b.g_q3, s));
-    poolback_kernel<<<rows_grid(n * 12 * h8), dim3(EW_X, EW_Y), 0, s>>>(b.g_s3, b.g_q3, b.e3, n * 12, h8, w8, b.g_e3);
+    launch(poolback_kernel, rows_grid(n * 12 * h8), blk, b.g_s3, b.g_q3, b.e3, n * 12, h8, w8, b.g_e3);
     ISTI_TRY(wgrad(net, 2, b.g_e3, b.q2, n, h4, w4, b, s));
     ISTI_TRY(dgrad(net, 2, b.g_e3, n, h4, w4, nullptr, b.g_q2, s));
-    poolback_kernel<<<rows_grid(n * 8 * h4), dim3(EW_X, EW_Y), 0, s>>>(b.g_s2, b.g_q2, b.e2, n * 8, h4, w4, b.g_e2);
+    launch(poolback_kernel, rows_grid(n * 8 * h4), blk, b.g_s2, b.g_q2, b.e2, n * 8, h4, w4, b.g_e2);
     ISTI_TRY(wgrad(net, 1, b.g_e2, b.q1, n, h2, w2, b, s));
     ISTI_TRY(dgrad(net, 1, b.g_e2, n, h2, w2, nullptr, b.g_q1, s));
-    poolback_kernel<<<rows_grid(n * 4 * h2), dim3(EW_X, EW_Y), 0, s>>>(b.g_s1, b.g_q1, b.e1, n * 4, h2, w2, b.g_e1);
+    launch(poolback_kernel, rows_grid(n * 4 * h2), blk, b.g_s1, b.g_q1, b.e1, n * 4, h2, w2, b.g_e1);
     ISTI_TRY(wgrad(net, 0, b.g_e1, x0, n, h, w, b, s));
-    const cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cudaGetLastError();
     return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "flownet backward");
 }
 

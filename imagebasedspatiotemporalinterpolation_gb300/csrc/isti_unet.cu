@@ -324,7 +324,7 @@ size_t wgrad_scratch(int taps, int n, int h, int w, int cin, int cout)
 }
 
 isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, int w, int cin, int cout, float *dw, float *db, int accumulate,
-                         void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream, int planes)
+                         void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream, int planes, bool pdl)
 {
     if ((taps != 9 && taps != 1) || n < 1 || h < 1 || w < 1 || cin % 16 || cout % 16 || cin < 16 || cin > 256 || cout < 16 || cout > 128 || !dy ||
         !x || !dw || !scratch || (db && cin > 240))
@@ -366,10 +366,14 @@ isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, 
     cudaError_t e = smem_limit(kernel, c.smem);
     if (e == cudaSuccess)
     {
-        kernel<<<grid, WGRAD_THREADS, c.smem, stream>>>(p, dymap, xmap);
+        e = launch_kernel(kernel, grid, dim3(WGRAD_THREADS), c.smem, stream, pdl, p, dymap, xmap);
         const int nw = cout * taps * cin;
-        wgrad_reduce_kernel<<<(unsigned)((nw + (db ? cout : 0) + 31) / 32), dim3(32, WREDUCE_PARTS), 0, stream>>>(p.partial, p.bpartial, c.splits, nw,
-                                                                                                              cout, dw, db, accumulate);
+        if (e == cudaSuccess)
+            e = launch_kernel(wgrad_reduce_kernel, dim3((unsigned)((nw + (db ? cout : 0) + 31) / 32)), dim3(32, WREDUCE_PARTS), 0, stream, pdl,
+                              (const float *)p.partial, (const float *)p.bpartial, c.splits, nw, cout, dw, db, accumulate);
+    }
+    if (e == cudaSuccess)
+    {
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "isti_unet_wgrad launch");

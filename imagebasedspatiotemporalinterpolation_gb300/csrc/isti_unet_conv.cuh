@@ -188,7 +188,7 @@ __device__ __forceinline__ void epilogue_pixel(const ConvParams &p, const Epilog
             if (p.mask)
             {
                 const uint4 *mk = reinterpret_cast<const uint4 *>(p.mask) + group;
-                const uint4 m0 = __ldg(mk), m1 = __ldg(mk + step);
+                const uint4 m0 = mk[0], m1 = mk[step]; // plain loads: a previous kernel wrote them, perhaps after this launch
                 const uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
 #pragma unroll
                 for (int j = 0; j < 16; j++)
@@ -675,9 +675,13 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
+    if (threadIdx.x == 0)
+        griddep_launch_dependents();
     if (warp == 0)
     {
         const uint32_t leader = elect_one();
+        griddep_wait(); // dY and X are complete (every load below is later), and the scratch is free
+        fence_proxy_async_global();
         const uint32_t tx_bytes = (uint32_t)(boxes * p.box_chunks) * px_bytes + (uint32_t)(p.cin / 8) * b_rows_bytes;
         const int shift0 = mb0 * 16 / co_chunks, group0 = mb0 * 16 % co_chunks; // of the first box
         RingPos ring;
@@ -802,6 +806,8 @@ __global__ void __launch_bounds__(32 * WREDUCE_PARTS) wgrad_reduce_kernel(const 
                                                                           float *dw, float *db, int accumulate)
 {
     __shared__ float part[WREDUCE_PARTS][32];
+    griddep_launch_dependents();
+    griddep_wait();
     const int i = blockIdx.x * 32 + threadIdx.x;
     const bool weight = i < n, used = weight || (db && i < n + nb);
     float s = 0.0f;

@@ -53,7 +53,7 @@ cudaError_t launch_kernel(void (*kernel)(K...), dim3 grid, dim3 block, size_t sm
 }
 // db (may be null): the bias gradient, the column sums of dy
 isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, int w, int cin, int cout, float *dw, float *db, int accumulate,
-                         void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream, int planes = 0);
+                         void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream, int planes = 0, bool pdl = false);
 isti_status pack_launch(int taps, const float *w, int cin, int cout, int transpose, void *wpack, cudaStream_t stream);
 size_t wgrad_scratch(int taps, int n, int h, int w, int cin, int cout);
 } // namespace isti_unet
