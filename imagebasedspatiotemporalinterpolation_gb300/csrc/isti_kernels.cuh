@@ -113,6 +113,7 @@ struct alignas(16) FrameParams
     int32_t *status;   // device status word: 0 ok, ISTI_ERR_TIMEOUT after a bounded wait gave up
     uint32_t out_w, out_h;
     int32_t n_views, n_aux, n_frames, linear, chain;
+    int32_t keep_status;      // the init kernel leaves the status word as it is (further batches of one call)
     int32_t use_tma;          // key tiles fetched by TMA (every view's row pitch a multiple of 16 bytes)
     int32_t row_pairs;        // pairs of output rows per reprojection block
     int32_t group_frames;     // frames whose results a reprojection block holds at a time
@@ -268,7 +269,9 @@ __device__ __forceinline__ void init_part(const FrameParams &p, size_t t, size_t
 __global__ void __launch_bounds__(256) init_kernel(const __grid_constant__ FrameParams p)
 {
     dependents_may_launch();
-    init_part(p, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
+    init_part(p, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, !p.keep_status);
+    wait_for_prerequisites(); // launched early only where the kernels before it use other keys and tables: nothing to wait
+                              // for, but its completion has to mean theirs
 }
 
 // ---- computeFlowFields_sortedSplatting_kernel, src/renderer.cu:76-146 ----
@@ -1102,6 +1105,7 @@ __global__ void __maxnreg__(reproj_regs(SW, REGS, NV)) reproj_kernel(const __gri
     }
     __syncthreads();
     wait_for_prerequisites();
+    dependents_may_launch(); // (after the wait: what starts early then may rely on all earlier kernels)
     int round = 0;
     reproj_block<SW, SI, MAV, REGS, NV, HOOK>(p, km.m, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x, smem, bars, round, aborted);
 }

@@ -326,8 +326,9 @@ cudaError_t launch_reproj_mode(isti::FrameParams &p, int mode, cudaStream_t stre
 }
 
 // Enqueues the three kernels of one batch; events (optional) are recorded after init and splat.
+// early: the kernel enqueued just before is another batch's reprojection, with keys of its own.
 cudaError_t launch_batch(isti::FrameParams &p, int mode, cudaStream_t stream, cudaEvent_t after_init, cudaEvent_t after_splat,
-                         ReprojChoice choice)
+                         ReprojChoice choice, bool early = false)
 {
     uint32_t max_w = 0, max_h = 0;
     for (int k = 0; k < p.n_views; k++)
@@ -341,11 +342,13 @@ cudaError_t launch_batch(isti::FrameParams &p, int mode, cudaStream_t stream, cu
         init_blocks = 256;
     if (init_blocks > 152 * 64)
         init_blocks = 152 * 64;
-    isti::init_kernel<<<(unsigned)init_blocks, 256, 0, stream>>>(p);
+    cudaError_t e = launch_after(early, isti::init_kernel, (unsigned)init_blocks, 256, 0, stream, p);
+    if (e != cudaSuccess)
+        return e;
     if (after_init)
         cudaEventRecord(after_init, stream);
     const dim3 gs((max_w + 31) / 32, (max_h + 7) / 8, p.n_views);
-    const cudaError_t e = launch_after(!after_init, isti::splat_kernel, gs, dim3(32, 8), 0, stream, p);
+    e = launch_after(!after_init, isti::splat_kernel, gs, dim3(32, 8), 0, stream, p);
     if (e != cudaSuccess)
         return e;
     if (after_splat)

@@ -41,8 +41,14 @@ constexpr int LT_W = 32, LT_H = 8; // learned / fallback tile (one block)
 struct LearnedParams
 {
     FrameParams fp;             // views 0 (fwd) and 1 (bwd), frames, outputs, client matrices
-    float4 *ws[2];              // per source pixel: ws_from (x, y, z, w)
-    float4 *dws[2];             // per source pixel: ws_to - ws_from
+    // Per source pixel, the client-independent part of its projection: ws_from (x, y, z) and the x of
+    // ws_to - ws_from; its y and z.  The w of ws_from is 1 and that of the difference 0 wherever they
+    // are not NaN (w / w, include/util/helper_common.h:77-87); a NaN is carried by wa's x, which
+    // makes every projected component NaN just as the w would.
+    float4 *wa[2];
+    float2 *wb[2];
+    int32_t reset;              // the keyframe kernel clears the call's counters (render calls)
+    uint32_t cell_total;        // words of cell_bits
     const __half *guess;        // [frame][hq][wq][4] source offsets (fwd dx, dy, bwd dx, dy), quarter pixels; null = none
     __nv_bfloat16 *net_in;      // [frame][hq][wq][16] network input
     int32_t hq, wq;             // network grid (multiples of 8, covering ceil(h / 4) x ceil(w / 4))
@@ -64,10 +70,10 @@ __device__ __forceinline__ float4 learned_project(const LearnedParams &p, int v,
 {
     const DevView &dv = p.fp.v[v];
     const uint32_t i = sy * dv.w + sx;
-    const float4 a = __ldg(p.ws[v] + i), d = __ldg(p.dws[v] + i);
+    const float4 a = p.wa[v][i];
+    const float2 b = p.wb[v][i];
     const float wg = dv.forward ? p.fp.f[k].alpha : xsub(1.0f, p.fp.f[k].alpha);
-    const float4 scaled = make_float4(xadd(a.x, xmul(wg, d.x)), xadd(a.y, xmul(wg, d.y)), xadd(a.z, xmul(wg, d.z)), xadd(a.w, xmul(wg, d.w)));
-    return project(p.fp.cam_vp[k], scaled);
+    return project(p.fp.cam_vp[k], make_float4(xadd(a.x, xmul(wg, a.w)), xadd(a.y, xmul(wg, b.x)), xadd(a.z, xmul(wg, b.y)), 1.0f));
 }
 
 // client-camera flow (xyz) of that pixel (full_motion_cam, src/renderer.cu:117), and its z in w
@@ -81,15 +87,29 @@ __device__ __forceinline__ float4 learned_camflow(const LearnedParams &p, int v,
 
 // ---- per keyframe pair ----
 
-__global__ void __launch_bounds__(256) keyframe_kernel(const __grid_constant__ LearnedParams p)
+// Bound by issue and by HBM alike: 10 to 20 bytes read and 40 written per source pixel, three IEEE
+// projections (two 1080p keyframes: 53 us).
+__global__ void __launch_bounds__(256, 7) keyframe_kernel(const __grid_constant__ LearnedParams p)
 {
+    dependents_may_launch();
     const int v = blockIdx.z;
     const DevView &dv = p.fp.v[v];
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    const uint32_t t = threadIdx.y * blockDim.x + threadIdx.x;
+    const uint32_t x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+    const uint32_t t = threadIdx.y * 32 + threadIdx.x;
     if (blockIdx.x == 0 && blockIdx.y == 0) // pixel->clip tables, as init_kernel writes them
-        for (uint32_t j = t; j < dv.w + dv.h; j += blockDim.x * blockDim.y)
+        for (uint32_t j = t; j < dv.w + dv.h; j += 256)
             dv.lut[j] = j < dv.w ? pixel2cs(j, 0, dv.w, 1).x : pixel2cs(0, j - dv.w, 1, dv.h).y;
+    if (p.reset && v == 0)
+    {
+        const uint32_t i = (blockIdx.y * gridDim.x + blockIdx.x) * 256 + t; // every pixel's thread: more than cell words
+        if (i < p.cell_total)
+            p.cell_bits[i] = 0u;
+        if (i == 0)
+        {
+            *p.fallback_count = 0;
+            *p.fp.status = 0;
+        }
+    }
     if (x >= dv.w || y >= dv.h)
         return;
     const uint32_t idx = y * dv.w + x;
@@ -105,8 +125,9 @@ __global__ void __launch_bounds__(256) keyframe_kernel(const __grid_constant__ L
     const bool visible = quotient_inside(cm.x, cm.w, lim) && quotient_inside(cm.y, cm.w, lim) && quotient_inside(cm.z, cm.w, lim);
     const float4 cs_to = project(dv.vp_to, ws_to);
     dv.full_ff[idx] = make_float4(xsub(cs_to.x, cs_from.x), xsub(cs_to.y, cs_from.y), xsub(cs_to.z, cs_from.z), visible ? 1.0f : 0.0f);
-    p.ws[v][idx] = ws_from;
-    p.dws[v][idx] = make_float4(xsub(ws_to.x, ws_from.x), xsub(ws_to.y, ws_from.y), xsub(ws_to.z, ws_from.z), xsub(ws_to.w, ws_from.w));
+    const float dw = xsub(ws_to.w, ws_from.w); // 0, or NaN when either w is
+    p.wa[v][idx] = make_float4(isnan(dw) ? dw : ws_from.x, ws_from.y, ws_from.z, xsub(ws_to.x, ws_from.x));
+    p.wb[v][idx] = make_float2(xsub(ws_to.y, ws_from.y), xsub(ws_to.z, ws_from.z));
 }
 
 // ---- per frame: the network input ----
@@ -119,6 +140,8 @@ __device__ __forceinline__ uint32_t bf16x2(float a, float b)
 
 __global__ void __launch_bounds__(256) input_kernel(const __grid_constant__ LearnedParams p)
 {
+    dependents_may_launch();
+    wait_for_prerequisites();
     const int k = blockIdx.z;
     const int qx = blockIdx.x * blockDim.x + threadIdx.x, qy = blockIdx.y * blockDim.y + threadIdx.y;
     if (qx >= p.wq || qy >= p.hq)
@@ -208,13 +231,14 @@ __device__ __forceinline__ void learned_step_approx(const LearnedParams &p, int 
 {
     const DevView &dv = p.fp.v[v];
     const uint32_t i = sy * dv.w + sx;
-    const float4 a = __ldg(p.ws[v] + i), d = __ldg(p.dws[v] + i);
+    const float4 a = p.wa[v][i];
+    const float2 b = p.wb[v][i];
     const float wg = dv.forward ? p.fp.f[k].alpha : 1.0f - p.fp.f[k].alpha;
     const float *m = p.fp.cam_vp[k];
-    const float x = fmaf(wg, d.x, a.x), y = fmaf(wg, d.y, a.y), z = fmaf(wg, d.z, a.z), w = fmaf(wg, d.w, a.w);
-    const float cx = fmaf(m[0], x, fmaf(m[4], y, fmaf(m[8], z, m[12] * w)));
-    const float cy = fmaf(m[1], x, fmaf(m[5], y, fmaf(m[9], z, m[13] * w)));
-    const float cw = fmaf(m[3], x, fmaf(m[7], y, fmaf(m[11], z, m[15] * w)));
+    const float x = fmaf(wg, a.w, a.x), y = fmaf(wg, b.x, a.y), z = fmaf(wg, b.y, a.z);
+    const float cx = fmaf(m[0], x, fmaf(m[4], y, fmaf(m[8], z, m[12])));
+    const float cy = fmaf(m[1], x, fmaf(m[5], y, fmaf(m[9], z, m[13])));
+    const float cw = fmaf(m[3], x, fmaf(m[7], y, fmaf(m[11], z, m[15])));
     const float mx = __fdividef(cx, cw) - __ldg(dv.lut + sx), my = __fdividef(cy, cw) - __ldg(dv.lut + dv.w + sy);
     const int2 t = cs2pixel(qx - mx, qy - my, dv.w, dv.h);
     if (in_range(t, dv.w, dv.h))
@@ -230,6 +254,8 @@ __device__ __forceinline__ void learned_step_approx(const LearnedParams &p, int 
 // the kernel waits on dependent gathers, so resident warps count
 __global__ void __launch_bounds__(LT_W *LT_H, 6) learned_kernel(const __grid_constant__ LearnedParams p)
 {
+    dependents_may_launch();
+    wait_for_prerequisites();
     const uint32_t x = blockIdx.x * LT_W + threadIdx.x, y = blockIdx.y * LT_H + threadIdx.y;
     const bool inb = x < p.fp.out_w && y < p.fp.out_h;
     const DevView &a = p.fp.v[0], &b = p.fp.v[1];
@@ -330,7 +356,7 @@ __device__ __forceinline__ bool marked_within(const LearnedParams &p, int k, int
         return false;
     for (int ty = y0 / LT_H; ty <= y1 / LT_H; ty++)
         for (int tx = x0 / LT_W; tx <= x1 / LT_W; tx++)
-            if (__ldg(p.tile_flags + ((size_t)k * p.tiles_y + ty) * p.tiles_x + tx) != 0u)
+            if (p.tile_flags[((size_t)k * p.tiles_y + ty) * p.tiles_x + tx] != 0u)
                 return true;
     return false;
 }
@@ -365,12 +391,14 @@ constexpr int FB_MARGIN = FB_RING + 2;
 __global__ void __launch_bounds__(LT_W *LT_H) fallback_init_kernel(const __grid_constant__ LearnedParams p)
 {
     constexpr int RW = LT_W + 2 * FB_RING, RH = LT_H + 2 * FB_RING;
+    dependents_may_launch();
+    wait_for_prerequisites();
     const int n = *p.fallback_count;
     const int cells_x = ((int)p.fp.out_w + FB_CELL - 1) / FB_CELL;
     for (int i = blockIdx.x; i < n; i += gridDim.x)
     {
         int k, x0, y0;
-        tile_origin(p, __ldg(p.tile_list + i), k, x0, y0);
+        tile_origin(p, p.tile_list[i], k, x0, y0);
         const int t = threadIdx.y * LT_W + threadIdx.x;
         {
             // cells overlapping [x0 - FB_MARGIN, x0 + LT_W + FB_MARGIN) x [y0 - FB_MARGIN, y0 + LT_H + FB_MARGIN)
@@ -400,9 +428,14 @@ __global__ void __launch_bounds__(LT_W *LT_H) fallback_init_kernel(const __grid_
 // approximate projection (contracted multiply-adds, fast division) first rejects targets
 // farther than 2 pixels beyond every tile's ring -- its error is orders of magnitude below
 // that margin; a w near zero or a non-finite value is never rejected -- and only candidates
-// take the exact projection of the plain path.
-__global__ void __launch_bounds__(256) fallback_splat_kernel(const __grid_constant__ LearnedParams p)
+// take the exact projection of the plain path.  The loop over the frames is unrolled over the
+// batch limit, so that the client matrices are constant operands.
+// Bound by issue (the rejection of every pixel and frame) and by its 24 bytes per source pixel
+// (1080p, 3 frames: 52 -> 43 us).
+__global__ void __launch_bounds__(256, 8) fallback_splat_kernel(const __grid_constant__ LearnedParams p)
 {
+    dependents_may_launch();
+    wait_for_prerequisites();
     if (*p.fallback_count == 0)
         return;
     const int v = blockIdx.z;
@@ -411,33 +444,35 @@ __global__ void __launch_bounds__(256) fallback_splat_kernel(const __grid_consta
     if (x >= dv.w || y >= dv.h)
         return;
     const uint32_t i = y * dv.w + x;
-    const float4 a = __ldg(p.ws[v] + i), d = __ldg(p.dws[v] + i);
-    for (int k = 0; k < p.fp.n_frames; k++)
+    const float4 a = p.wa[v][i];
+    const float2 b = p.wb[v][i];
+    const float half_w = (float)dv.w * 0.5f, half_h = (float)dv.h * 0.5f;
+#pragma unroll
+    for (int k = 0; k < MAX_FRAMES; k++)
     {
+        if (k >= p.fp.n_frames)
+            break;
         const float *m = p.fp.cam_vp[k];
         const float wg = dv.forward ? p.fp.f[k].alpha : xsub(1.0f, p.fp.f[k].alpha);
         // approximate target pixel
-        const float sx = fmaf(wg, d.x, a.x), sy = fmaf(wg, d.y, a.y), sz = fmaf(wg, d.z, a.z), sw = fmaf(wg, d.w, a.w);
-        const float qx = fmaf(m[0], sx, fmaf(m[4], sy, fmaf(m[8], sz, m[12] * sw)));
-        const float qy = fmaf(m[1], sx, fmaf(m[5], sy, fmaf(m[9], sz, m[13] * sw)));
-        const float qw = fmaf(m[3], sx, fmaf(m[7], sy, fmaf(m[11], sz, m[15] * sw)));
+        const float sx = fmaf(wg, a.w, a.x), sy = fmaf(wg, b.x, a.y), sz = fmaf(wg, b.y, a.z);
+        const float qx = fmaf(m[0], sx, fmaf(m[4], sy, fmaf(m[8], sz, m[12])));
+        const float qy = fmaf(m[1], sx, fmaf(m[5], sy, fmaf(m[9], sz, m[13])));
+        const float qw = fmaf(m[3], sx, fmaf(m[7], sy, fmaf(m[11], sz, m[15])));
+        const float rw = __fdividef(1.0f, qw);
+        const float fx = fmaf(qx * rw, half_w, half_w), fy = fmaf(qy * rw, half_h, half_h);
         bool candidate = true;
-        if (isfinite(qx) && isfinite(qy) && fabsf(qw) > 1e-6f)
+        if (fabsf(qw) > 1e-6f && fabsf(fx) < 1e30f && fabsf(fy) < 1e30f) // (NaN: a candidate)
         {
-            const float fx = (__fdividef(qx, qw) + 1.0f) * (float)dv.w * 0.5f, fy = (__fdividef(qy, qw) + 1.0f) * (float)dv.h * 0.5f;
-            if (isfinite(fx) && isfinite(fy))
+            // a marked tile within FB_MARGIN pixels of (ix, iy) (the box clipped to the image) is
+            // within FB_MARGIN of the nearest pixel of the image too, whose cell is then marked:
+            // the cell test keeps every candidate the box test would keep
+            const int ix = __float2int_rd(fx), iy = __float2int_rd(fy);
+            candidate = (uint32_t)ix + FB_MARGIN < dv.w + 2 * FB_MARGIN && (uint32_t)iy + FB_MARGIN < dv.h + 2 * FB_MARGIN;
+            if (candidate)
             {
-                // a marked tile within FB_MARGIN pixels of (ix, iy) (the box clipped to the image) is
-                // within FB_MARGIN of the nearest pixel of the image too, whose cell is then marked:
-                // the cell test keeps every candidate the box test would keep
-                const int ix = (int)floorf(fminf(fmaxf(fx, -1e6f), 1e6f)), iy = (int)floorf(fminf(fmaxf(fy, -1e6f), 1e6f));
-                if (ix < -FB_MARGIN || iy < -FB_MARGIN || ix >= (int)dv.w + FB_MARGIN || iy >= (int)dv.h + FB_MARGIN)
-                    candidate = false;
-                else
-                {
-                    const int cx = min(max(ix, 0), (int)dv.w - 1) / FB_CELL, cy = min(max(iy, 0), (int)dv.h - 1) / FB_CELL;
-                    candidate = (__ldg(p.cell_bits + ((size_t)k * p.cells_y + cy) * p.cell_words + cx / 32) >> (cx % 32)) & 1u;
-                }
+                const int cx = min(max(ix, 0), (int)dv.w - 1) / FB_CELL, cy = min(max(iy, 0), (int)dv.h - 1) / FB_CELL;
+                candidate = (p.cell_bits[((uint32_t)k * (uint32_t)p.cells_y + (uint32_t)cy) * (uint32_t)p.cell_words + (uint32_t)cx / 32u] >> (cx % 32)) & 1u;
             }
         }
         if (!candidate)
@@ -475,13 +510,15 @@ __device__ __forceinline__ unsigned long long window_key_global(const unsigned l
 
 __global__ void __launch_bounds__(LT_W *LT_H) fallback_reproj_kernel(const __grid_constant__ LearnedParams p)
 {
+    dependents_may_launch();
+    wait_for_prerequisites();
     const int n = *p.fallback_count;
     const DevView &a = p.fp.v[0];
     for (int i = blockIdx.x; i < n; i += gridDim.x)
     {
         int k;
         uint32_t x, y;
-        tile_of(p, __ldg(p.tile_list + i), k, x, y);
+        tile_of(p, p.tile_list[i], k, x, y);
         if (x >= p.fp.out_w || y >= p.fp.out_h)
             continue;
         const float qx = __ldg(a.lut + x), qy = __ldg(a.lut + a.w + y);
@@ -513,6 +550,7 @@ __global__ void __launch_bounds__(LT_W *LT_H) fallback_reproj_kernel(const __gri
 // out[k] after frame k.
 __global__ void __launch_bounds__(256) learned_chain_kernel(const __grid_constant__ LearnedParams p)
 {
+    wait_for_prerequisites();
     const size_t n = (size_t)p.fp.out_w * p.fp.out_h;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     {

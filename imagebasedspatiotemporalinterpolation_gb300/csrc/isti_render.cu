@@ -778,6 +778,17 @@ cudaError_t launch_pairs_mode(int mode, int regs, const isti::BatchParams &bp, s
     return cudaErrorInvalidValue;
 }
 
+// Whether isti_render_pairs renders its pairs as batches, one after the other, rather than in the
+// persistent launch.  A batch's kernels run at their own block shapes and registers (the persistent
+// kernel splats with the reprojection's) but cost a pair 12 us of launches; so the persistent launch
+// is left to many small pairs.  Per pair, persistent / batches: 32 pairs of 160x96 7.9 / 12.5 us (one
+// frame), 12.5 / 17.7 (three); of 320x180 25 / 15 and 40 / 28; 8 pairs of 96x64 8.5 / 14, 2 pairs
+// 24 / 19; 6 pairs of 1280x720 to 2064x2208, three frames, 508 / 329.
+bool pairs_as_batches(size_t source_pixels, int n_pairs)
+{
+    return n_pairs <= 2 || source_pixels >= (size_t)50000 * n_pairs;
+}
+
 template <int SW>
 bool pair_maps(const isti::FrameParams &p, isti::KeyMaps &km)
 {
@@ -813,6 +824,7 @@ extern "C" isti_status isti_render_pairs(isti_renderer *r, int32_t n_pairs, cons
         return fail(ISTI_ERR_INVALID_ARG, "renderer was created on another device");
     // validation and the arena layout: every pair's intermediates, then the parameter block
     std::vector<Layout> layouts(n_pairs);
+    size_t source_pixels = 0;
     std::vector<std::vector<const isti_view *>> views(n_pairs);
     int mode = -1, nv = 0;
     size_t data_bytes = 0;
@@ -838,6 +850,8 @@ extern "C" isti_status isti_render_pairs(isti_renderer *r, int32_t n_pairs, cons
         views[i].assign(vv, vv + n_views);
         layouts[i] = layout_of(vv, n_views, pf.n_frames);
         data_bytes += align_up(layouts[i].total, 256);
+        for (int k = 0; k < n_views; k++)
+            source_pixels += (size_t)vv[k]->width * vv[k]->height;
     }
     const size_t fp_bytes = align_up(sizeof(isti::FrameParams) * n_pairs, 256);
     const size_t map_bytes = align_up(sizeof(CUtensorMap) * isti::MAX_VIEWS * n_pairs, 256);
@@ -861,6 +875,27 @@ extern "C" isti_status isti_render_pairs(isti_renderer *r, int32_t n_pairs, cons
         if (e != cudaSuccess)
             return e == cudaErrorMemoryAllocation ? fail(ISTI_ERR_OOM, "cudaMalloc of the multi-pair arena failed") : cuda_fail(e, "cudaMalloc");
         r->multi_bytes = total;
+    }
+    // One batch after the other (unless the caller asks for the persistent launch's units)
+    if (r->stall_pair < 0 && !r->pair_splat_rows && !r->pair_init_kib && pairs_as_batches(source_pixels, n_pairs))
+    {
+        char *at = static_cast<char *>(r->multi_arena);
+        for (int i = 0; i < n_pairs; i++)
+        {
+            const isti_pair_frames &pf = pairs[i];
+            isti::FrameParams p;
+            fill_params(p, pf.n_frames, pf.out_rgba, pf.infos, pf.frame, views[i].data(), nv, layouts[i], at, pf.chain_outputs != 0);
+            at += align_up(layouts[i].total, 256);
+            if (i > 0)
+                p.status = r->last.status; // one status word for the call, reset by the first batch
+            p.keep_status = i > 0 ? 1 : 0;
+            if ((e = isti::launch_batch(p, mode, stream, nullptr, nullptr, isti::ReprojChoice{}, i > 0)) != cudaSuccess)
+                return cuda_fail(e, "isti_render_pairs launch");
+            if (i == 0)
+                r->last = p;
+        }
+        r->has_frame = true;
+        return ISTI_OK;
     }
     if (!r->multi_copied && (e = cudaEventCreateWithFlags(&r->multi_copied, cudaEventDisableTiming)) != cudaSuccess)
         return cuda_fail(e, "cudaEventCreate");
@@ -1011,34 +1046,32 @@ extern "C" isti_status isti_render_learned(isti_renderer *r, isti_flownet *net, 
     const cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
     isti::LearnedParams &p = r->learned;
     const uint32_t w = infos[0].width, h = infos[0].height;
-    cudaError_t e = cudaMemsetAsync(p.fallback_count, 0, 4, stream);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(p.fp.status, 0, 4, stream);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(p.cell_bits, 0, (size_t)n_frames * p.cells_y * p.cell_words * 4, stream);
-    if (e != cudaSuccess)
-        return cuda_fail(e, "cudaMemsetAsync");
-    const dim3 b2(32, 8);
+    p.reset = 1;
+    const dim3 b2(32, 8), tile(isti::LT_W, isti::LT_H);
+    // each kernel after the first a programmatic dependent of the one before (the network's too)
     isti::keyframe_kernel<<<dim3((w + 31) / 32, (h + 7) / 8, 2), b2, 0, stream>>>(p);
-    if (net)
+    cudaError_t e = cudaGetLastError();
+    if (net && e == cudaSuccess)
     {
-        isti::input_kernel<<<dim3((p.wq + 31) / 32, (p.hq + 7) / 8, n_frames), b2, 0, stream>>>(p);
-        e = cudaGetLastError();
+        e = isti::launch_after(true, isti::input_kernel, dim3((p.wq + 31) / 32, (p.hq + 7) / 8, n_frames), b2, 0, stream, p);
         if (e != cudaSuccess)
             return cuda_fail(e, "learned input launch");
         st = isti_flownet_forward(net, p.net_in, n_frames, p.hq, p.wq, nullptr, guess, stream);
         if (st != ISTI_OK)
             return st;
     }
-    isti::learned_kernel<<<dim3(p.tiles_x, p.tiles_y), dim3(isti::LT_W, isti::LT_H), 0, stream>>>(p);
+    auto launch = [&](auto kernel, dim3 grid, dim3 block) {
+        if (e == cudaSuccess)
+            e = isti::launch_after(true, kernel, grid, block, 0, stream, p);
+    };
+    launch(isti::learned_kernel, dim3(p.tiles_x, p.tiles_y), tile);
     // the fallback kernels walk the list of marked tiles (none: they return at once)
     const unsigned list_blocks = (unsigned)std::min(p.tiles_x * p.tiles_y * n_frames, 152 * 4);
-    isti::fallback_init_kernel<<<list_blocks, dim3(isti::LT_W, isti::LT_H), 0, stream>>>(p);
-    isti::fallback_splat_kernel<<<dim3((w + 31) / 32, (h + 7) / 8, 2), b2, 0, stream>>>(p);
-    isti::fallback_reproj_kernel<<<list_blocks, dim3(isti::LT_W, isti::LT_H), 0, stream>>>(p);
+    launch(isti::fallback_init_kernel, list_blocks, tile);
+    launch(isti::fallback_splat_kernel, dim3((w + 31) / 32, (h + 7) / 8, 2), b2);
+    launch(isti::fallback_reproj_kernel, list_blocks, tile);
     if (chain_outputs && n_frames > 1)
-        isti::learned_chain_kernel<<<(unsigned)std::min<size_t>(((size_t)w * h + 255) / 256, 152 * 8), 256, 0, stream>>>(p);
-    e = cudaGetLastError();
+        launch(isti::learned_chain_kernel, (unsigned)std::min<size_t>(((size_t)w * h + 255) / 256, 152 * 8), 256);
     if (e != cudaSuccess)
         return cuda_fail(e, "learned render launch");
     r->has_learned = true;
@@ -1121,7 +1154,7 @@ isti_status learned_setup(isti_renderer *r, isti_flownet *net, int32_t n_frames,
     const int hq = quarter_grid(h), wq = quarter_grid(w);
     const int tiles_x = (int)((w + isti::LT_W - 1) / isti::LT_W), tiles_y = (int)((h + isti::LT_H - 1) / isti::LT_H);
     // [keys: frames x 2 views][full flow: 2 views][lut: 2 views][status] (fill_params' layout, no cam flow)
-    // then [ws: 2 views][dws: 2 views][network input][network output][tile flags][fallback count]
+    // then [wa: 2 views][wb: 2 views][network input][network output][tile flags][fallback count]
     Layout l{};
     for (int k = 0; k < 2; k++)
     {
@@ -1131,7 +1164,7 @@ isti_status learned_setup(isti_renderer *r, isti_flownet *net, int32_t n_frames,
     l.ff_bytes = 2 * align_up(px * 16, 256);
     l.key_bytes = l.key_frame_bytes * n_frames;
     l.total = l.key_bytes + l.ff_bytes + l.lut_bytes + STATUS_BYTES;
-    const size_t ws_bytes = align_up(px * 16, 256);
+    const size_t wa_bytes = align_up(px * 16, 256), wb_bytes = align_up(px * 8, 256), w_bytes = 2 * (wa_bytes + wb_bytes);
     const size_t in_bytes = align_up((size_t)n_frames * hq * wq * 16 * 2, 256);
     const size_t guess_bytes = align_up((size_t)n_frames * hq * wq * 4 * 2, 256);
     const size_t flag_bytes = 2 * align_up((size_t)n_frames * tiles_x * tiles_y * 4, 256); // flags, then the marked-tile list
@@ -1139,7 +1172,7 @@ isti_status learned_setup(isti_renderer *r, isti_flownet *net, int32_t n_frames,
     const int cells_y = (int)((h + isti::FB_CELL - 1) / isti::FB_CELL);
     const int cell_words = (int)(((w + isti::FB_CELL - 1) / isti::FB_CELL + 31) / 32);
     const size_t cell_bytes = align_up((size_t)n_frames * cells_y * cell_words * 4, 256);
-    const size_t total = l.total + 4 * ws_bytes + in_bytes + guess_bytes + flag_bytes + 256 + valid_bytes + cell_bytes;
+    const size_t total = l.total + w_bytes + in_bytes + guess_bytes + flag_bytes + 256 + valid_bytes + cell_bytes;
     if (total > r->learned_bytes)
     {
         if (r->learned_arena)
@@ -1158,19 +1191,21 @@ isti_status learned_setup(isti_renderer *r, isti_flownet *net, int32_t n_frames,
     char *extra = base + l.total;
     for (int v = 0; v < 2; v++)
     {
-        p.ws[v] = reinterpret_cast<float4 *>(extra + v * ws_bytes);
-        p.dws[v] = reinterpret_cast<float4 *>(extra + (2 + v) * ws_bytes);
+        p.wa[v] = reinterpret_cast<float4 *>(extra + v * wa_bytes);
+        p.wb[v] = reinterpret_cast<float2 *>(extra + 2 * wa_bytes + v * wb_bytes);
     }
-    p.net_in = reinterpret_cast<__nv_bfloat16 *>(extra + 4 * ws_bytes);
-    __half *guess = reinterpret_cast<__half *>(extra + 4 * ws_bytes + in_bytes);
+    p.net_in = reinterpret_cast<__nv_bfloat16 *>(extra + w_bytes);
+    __half *guess = reinterpret_cast<__half *>(extra + w_bytes + in_bytes);
     p.guess = net ? guess : nullptr;
-    p.tile_flags = reinterpret_cast<uint32_t *>(extra + 4 * ws_bytes + in_bytes + guess_bytes);
-    p.tile_list = reinterpret_cast<uint32_t *>(extra + 4 * ws_bytes + in_bytes + guess_bytes + flag_bytes / 2);
-    p.fallback_count = reinterpret_cast<int32_t *>(extra + 4 * ws_bytes + in_bytes + guess_bytes + flag_bytes);
-    p.valid = reinterpret_cast<uint8_t *>(extra + 4 * ws_bytes + in_bytes + guess_bytes + flag_bytes + 256);
-    p.cell_bits = reinterpret_cast<uint32_t *>(extra + 4 * ws_bytes + in_bytes + guess_bytes + flag_bytes + 256 + valid_bytes);
+    p.tile_flags = reinterpret_cast<uint32_t *>(extra + w_bytes + in_bytes + guess_bytes);
+    p.tile_list = reinterpret_cast<uint32_t *>(extra + w_bytes + in_bytes + guess_bytes + flag_bytes / 2);
+    p.fallback_count = reinterpret_cast<int32_t *>(extra + w_bytes + in_bytes + guess_bytes + flag_bytes);
+    p.valid = reinterpret_cast<uint8_t *>(extra + w_bytes + in_bytes + guess_bytes + flag_bytes + 256);
+    p.cell_bits = reinterpret_cast<uint32_t *>(extra + w_bytes + in_bytes + guess_bytes + flag_bytes + 256 + valid_bytes);
     p.cells_y = cells_y;
     p.cell_words = cell_words;
+    p.reset = 0;
+    p.cell_total = (uint32_t)n_frames * (uint32_t)cells_y * (uint32_t)cell_words;
     p.hq = hq;
     p.wq = wq;
     p.learned_iters = iterations;

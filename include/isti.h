@@ -153,20 +153,21 @@ isti_status isti_render(isti_renderer *r, void *out_rgba, const isti_render_info
 isti_status isti_render_batch(isti_renderer *r, int32_t n_frames, void *const *out_rgba, const isti_render_info *infos,
                               const isti_frame_data *frame, int32_t chain_outputs, void *stream);
 
-/* The frames of several keyframe pairs in ONE persistent launch (no counterpart in the
- * reference, which renders frame by frame, src/main.cu:152-190).  pairs[i] renders
- * n_frames client frames of pairs[i].frame exactly as isti_render_batch would (same
- * chain_outputs meaning, same bits): key initialisation, splatting and reprojection of every
- * pair are units of one cooperative kernel that takes them from a device work queue, the
- * next pair's initialisation and splatting ahead of the previous pair's reprojection.  All
- * pairs share the render mode (not timewarp) and the number of source views.
- * 1 <= n_pairs <= ISTI_MAX_PAIRS.  The kernel parameters travel through pinned staging
- * buffers of the renderer, one for uncaptured and one for captured calls: a call captured
- * into a CUDA graph reads its buffer when the graph runs, so capture no other
- * isti_render_pairs call on that renderer while the graph is in use, and make one call of
- * the same size outside any capture first (a capture allocates nothing; a larger one is
- * refused with ISTI_ERR_INVALID_ARG).  isti_renderer_device_status reports the call's
- * status word. */
+/* The frames of several keyframe pairs in one call (no counterpart in the reference, which
+ * renders frame by frame, src/main.cu:152-190).  pairs[i] renders n_frames client frames of
+ * pairs[i].frame exactly as isti_render_batch would (same chain_outputs meaning, same bits).
+ * Many small pairs are rendered in ONE persistent launch: key initialisation, splatting and
+ * reprojection of every pair are units of one cooperative kernel that takes them from a device
+ * work queue, the next pair's initialisation and splatting ahead of the previous pair's
+ * reprojection.  Larger pairs follow each other as batches, which is faster for them; a unit
+ * size set by isti_renderer_set_pair_units asks for the persistent launch.  All pairs share
+ * the render mode (not timewarp) and the number of source views.  1 <= n_pairs <=
+ * ISTI_MAX_PAIRS.  The persistent kernel's parameters travel through pinned staging buffers
+ * of the renderer, one for uncaptured and one for captured calls: a call captured into a CUDA
+ * graph reads its buffer when the graph runs, so capture no other isti_render_pairs call on
+ * that renderer while the graph is in use, and make one call of the same size outside any
+ * capture first (a capture allocates nothing; a larger one is refused with
+ * ISTI_ERR_INVALID_ARG).  isti_renderer_device_status reports the call's status word. */
 #define ISTI_MAX_PAIRS 64
 typedef struct isti_pair_frames
 {
@@ -178,9 +179,10 @@ typedef struct isti_pair_frames
 } isti_pair_frames;
 isti_status isti_render_pairs(isti_renderer *r, int32_t n_pairs, const isti_pair_frames *pairs, void *stream);
 
-/* Work-unit sizes of isti_render_pairs on this renderer: source rows per splat unit
- * (32 columns of one view, every frame; 1..256) and KiB of splat keys per init unit
- * (16..4096); 0 keeps a default (32 rows, 256 KiB).  The output does not depend on them. */
+/* Work-unit sizes of isti_render_pairs' persistent launch on this renderer: source rows per
+ * splat unit (32 columns of one view, every frame; 1..256) and KiB of splat keys per init
+ * unit (16..4096); 0 keeps a default (32 rows, 256 KiB).  With either set, pairs of every
+ * size take the persistent launch.  The output does not depend on them. */
 isti_status isti_renderer_set_pair_units(isti_renderer *r, int32_t splat_rows, int32_t init_unit_kib);
 
 /* Device pointers to the intermediates of the last render call for view

@@ -89,8 +89,9 @@ def test_mixed_pairs_chained_equal_render_batch(cuda, mode, units):
     ref.close()
 
 
+@pytest.mark.parametrize("units", [(0, 0), (32, 256)], ids=["rule", "persistent"])
 @pytest.mark.parametrize("mode", [0, 1])
-def test_pairs_with_tma_and_plain_key_tiles_equal_render_batch(cuda, mode):
+def test_pairs_with_tma_and_plain_key_tiles_equal_render_batch(cuda, mode, units):
     """Pairs whose key tiles come by TMA (even widths) and by plain loads (odd widths) in one
     call, an odd number of tile rounds per reprojection block: the units of the former must
     not lose step with their barrier over the units of the latter."""
@@ -106,12 +107,41 @@ def test_pairs_with_tma_and_plain_key_tiles_equal_render_batch(cuda, mode):
         ref.render_batch(want, clients, frame, chain=False)
         wants.append(want)
     r = Renderer()
+    r.set_pair_units(*units)
     r.render_pairs(jobs)
     torch.cuda.synchronize()
     assert r.device_status() == native.ISTI_OK
     for i, ((outs, _, _), want) in enumerate(zip(jobs, wants)):
         for k, (a, b) in enumerate(zip(outs, want)):
             assert torch.equal(a, b), f"pair {i} frame {k}: {int((a != b).any(-1).sum())} pixels differ"
+    r.close()
+    ref.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 9])
+@pytest.mark.parametrize("size", [(96, 64), (158, 158), (158, 159), (333, 197)], ids=lambda s: f"{s[0]}x{s[1]}")
+def test_small_pairs_either_side_of_the_batch_rule(cuda, size, n):
+    """Pairs around the sizes and counts at which the call turns from the persistent launch to
+    batches, chained, twice on one renderer."""
+    import torch
+    w, h = size
+    seq = scene.Sequence(w, h, n + 1, seed=4600, max_speed=2.0)
+    ref, r = Renderer(), Renderer()
+    for turn in range(2):
+        jobs, wants = [], []
+        for i in range(n):
+            clients = [seq.client(i, b) for b in (1, 2, 3)]
+            frame = DeviceFrame.from_host(seq.frame(i))
+            want = [torch.full((h, w, 4), 9 + turn, dtype=torch.uint8, device="cuda") for _ in clients]
+            jobs.append(([o.clone() for o in want], clients, frame))
+            ref.render_batch(want, clients, frame, chain=True)
+            wants.append(want)
+        r.render_pairs(jobs, chain=True)
+        torch.cuda.synchronize()
+        assert r.device_status() == native.ISTI_OK
+        for (outs, _, _), want in zip(jobs, wants):
+            for a, b in zip(outs, want):
+                assert torch.equal(a, b)
     r.close()
     ref.close()
 
