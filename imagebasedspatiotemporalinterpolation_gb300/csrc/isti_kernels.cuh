@@ -199,12 +199,12 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
 
 // ---- programmatic dependent launch ----
 //
-// The kernels of a call depend on each other one after the other.  Each lets the next one's blocks
-// take SMs as soon as its own blocks have all started (launch_dependents), and waits for the
-// kernels before it to complete, writes visible, before it touches what they wrote (wait; returns
-// at once in an ordinary launch).  That hides the launch latency between them: about 3 of 4.8 us
-// per kernel, most of a small frame (640x360: 24.6 -> 19.0 us a call).  A call's first kernel is launched in full
-// order, so everything before the call is complete by then.
+// The kernels of a call depend on each other one after the other, and on what was in the stream
+// before.  Each lets the next one's blocks take SMs as soon as its own blocks have all started
+// (launch_dependents), and waits for the kernel before it to complete, writes visible, before it
+// touches anything (wait; returns at once in an ordinary launch, or after work that is not a
+// kernel).  That hides the launch latency between them: about 3 of 4.8 us per kernel, most of a
+// small frame (640x360: 24.6 -> 19.0 us a call from within the call, 17.2 with the first kernel too).
 __device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -269,9 +269,13 @@ __device__ __forceinline__ void init_part(const FrameParams &p, size_t t, size_t
 __global__ void __launch_bounds__(256) init_kernel(const __grid_constant__ FrameParams p)
 {
     dependents_may_launch();
+    // a further batch of a call has keys and tables of its own, and the reprojection before it let it start only after
+    // waiting for all that was before the call: it writes at once, but its completion has to mean theirs
+    if (!p.keep_status)
+        wait_for_prerequisites();
     init_part(p, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, !p.keep_status);
-    wait_for_prerequisites(); // launched early only where the kernels before it use other keys and tables: nothing to wait
-                              // for, but its completion has to mean theirs
+    if (p.keep_status)
+        wait_for_prerequisites();
 }
 
 // ---- computeFlowFields_sortedSplatting_kernel, src/renderer.cu:76-146 ----
@@ -1180,6 +1184,7 @@ __device__ __forceinline__ void tw_block_reduce(double &sum, uint32_t &zmax, uin
 __global__ void __launch_bounds__(TW_THREADS) timewarp_rowsum_kernel(const __grid_constant__ FrameParams p)
 {
     dependents_may_launch();
+    wait_for_prerequisites();
     const DevView &v = p.v[0];
     const float *row = v.z + (size_t)blockIdx.x * v.w;
     double acc = 0.0;
@@ -1364,6 +1369,8 @@ __global__ void depth_to_z_kernel(float *__restrict__ z, size_t n)
 template <bool VEC>
 __global__ void rgb8_to_rgba8_kernel(uint32_t *__restrict__ dst, const uint8_t *__restrict__ src, size_t n)
 {
+    dependents_may_launch();
+    wait_for_prerequisites();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t groups = 0;
@@ -1391,6 +1398,8 @@ __global__ void rgb8_to_rgba8_kernel(uint32_t *__restrict__ dst, const uint8_t *
 __global__ void unpack_shadows_kernel(uint32_t *__restrict__ info, uint32_t *__restrict__ a, uint32_t *__restrict__ b, size_t n_pixels,
                                       const uint4 *__restrict__ entries, size_t n_entries)
 {
+    dependents_may_launch();
+    wait_for_prerequisites();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n_entries; e += stride)
     {
@@ -1408,6 +1417,8 @@ __global__ void unpack_shadows_kernel(uint32_t *__restrict__ info, uint32_t *__r
 __global__ void clear_shadows_kernel(uint32_t *__restrict__ info, uint32_t *__restrict__ a, uint32_t *__restrict__ b, size_t n_pixels,
                                      const uint4 *__restrict__ entries, size_t n_entries)
 {
+    dependents_may_launch();
+    wait_for_prerequisites();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n_entries; e += stride)
     {

@@ -16,8 +16,8 @@
 
 namespace isti
 {
-// Launches a kernel whose prerequisite is the kernel enqueued just before it; `early`: as a
-// programmatic dependent launch (the kernel waits by itself), otherwise in full order.
+// Launches a kernel after what was enqueued before it; `early`: as a programmatic dependent launch
+// (the kernel waits by itself), otherwise in full order (around timing events).
 template <class... P, class... A>
 cudaError_t launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A &...args)
 {
@@ -40,8 +40,9 @@ cudaError_t launch_timewarp(isti::FrameParams &p, char *base, cudaStream_t strea
 {
     p.tw_rows = reinterpret_cast<isti::TwRow *>(base);
     p.tw_plane = reinterpret_cast<float4 *>(base + ((size_t)p.v[0].h * sizeof(isti::TwRow) + 255) / 256 * 256);
-    isti::timewarp_rowsum_kernel<<<p.v[0].h, isti::TW_THREADS, 0, stream>>>(p);
-    cudaError_t e = launch_after(true, isti::timewarp_mean_kernel, 1, isti::TW_THREADS, 0, stream, p);
+    cudaError_t e = launch_after(true, isti::timewarp_rowsum_kernel, p.v[0].h, isti::TW_THREADS, 0, stream, p);
+    if (e == cudaSuccess)
+        e = launch_after(true, isti::timewarp_mean_kernel, 1, isti::TW_THREADS, 0, stream, p);
     if (e != cudaSuccess)
         return e;
     if (after_mean)
@@ -326,9 +327,8 @@ cudaError_t launch_reproj_mode(isti::FrameParams &p, int mode, cudaStream_t stre
 }
 
 // Enqueues the three kernels of one batch; events (optional) are recorded after init and splat.
-// early: the kernel enqueued just before is another batch's reprojection, with keys of its own.
 cudaError_t launch_batch(isti::FrameParams &p, int mode, cudaStream_t stream, cudaEvent_t after_init, cudaEvent_t after_splat,
-                         ReprojChoice choice, bool early = false)
+                         ReprojChoice choice)
 {
     uint32_t max_w = 0, max_h = 0;
     for (int k = 0; k < p.n_views; k++)
@@ -342,7 +342,7 @@ cudaError_t launch_batch(isti::FrameParams &p, int mode, cudaStream_t stream, cu
         init_blocks = 256;
     if (init_blocks > 152 * 64)
         init_blocks = 152 * 64;
-    cudaError_t e = launch_after(early, isti::init_kernel, (unsigned)init_blocks, 256, 0, stream, p);
+    cudaError_t e = launch_after(!after_init, isti::init_kernel, (unsigned)init_blocks, 256, 0, stream, p);
     if (e != cudaSuccess)
         return e;
     if (after_init)

@@ -92,6 +92,7 @@ __device__ __forceinline__ float4 learned_camflow(const LearnedParams &p, int v,
 __global__ void __launch_bounds__(256, 7) keyframe_kernel(const __grid_constant__ LearnedParams p)
 {
     dependents_may_launch();
+    wait_for_prerequisites();
     const int v = blockIdx.z;
     const DevView &dv = p.fp.v[v];
     const uint32_t x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;

@@ -889,7 +889,7 @@ extern "C" isti_status isti_render_pairs(isti_renderer *r, int32_t n_pairs, cons
             if (i > 0)
                 p.status = r->last.status; // one status word for the call, reset by the first batch
             p.keep_status = i > 0 ? 1 : 0;
-            if ((e = isti::launch_batch(p, mode, stream, nullptr, nullptr, isti::ReprojChoice{}, i > 0)) != cudaSuccess)
+            if ((e = isti::launch_batch(p, mode, stream, nullptr, nullptr, isti::ReprojChoice{})) != cudaSuccess)
                 return cuda_fail(e, "isti_render_pairs launch");
             if (i == 0)
                 r->last = p;
@@ -1048,9 +1048,8 @@ extern "C" isti_status isti_render_learned(isti_renderer *r, isti_flownet *net, 
     const uint32_t w = infos[0].width, h = infos[0].height;
     p.reset = 1;
     const dim3 b2(32, 8), tile(isti::LT_W, isti::LT_H);
-    // each kernel after the first a programmatic dependent of the one before (the network's too)
-    isti::keyframe_kernel<<<dim3((w + 31) / 32, (h + 7) / 8, 2), b2, 0, stream>>>(p);
-    cudaError_t e = cudaGetLastError();
+    // each kernel a programmatic dependent of the one before (the network's too)
+    cudaError_t e = isti::launch_after(true, isti::keyframe_kernel, dim3((w + 31) / 32, (h + 7) / 8, 2), b2, 0, stream, p);
     if (net && e == cudaSuccess)
     {
         e = isti::launch_after(true, isti::input_kernel, dim3((p.wq + 31) / 32, (p.hq + 7) / 8, n_frames), b2, 0, stream, p);
@@ -1350,11 +1349,8 @@ extern "C" isti_status isti_rgb8_to_rgba8(void *dst_rgba, const void *src_rgb, s
     cudaStream_t st = static_cast<cudaStream_t>(stream_ptr);
     uint32_t *dst = static_cast<uint32_t *>(dst_rgba);
     const uint8_t *src = static_cast<const uint8_t *>(src_rgb);
-    if (vec)
-        isti::rgb8_to_rgba8_kernel<true><<<blocks, 256, 0, st>>>(dst, src, n_pixels);
-    else
-        isti::rgb8_to_rgba8_kernel<false><<<blocks, 256, 0, st>>>(dst, src, n_pixels);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = isti::launch_after(true, vec ? isti::rgb8_to_rgba8_kernel<true> : isti::rgb8_to_rgba8_kernel<false>, blocks, 256, 0, st,
+                                             dst, src, n_pixels);
     return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "isti_rgb8_to_rgba8");
 }
 
@@ -1389,18 +1385,16 @@ extern "C" isti_status isti_unpack_shadows(void *info_rgba, void *a_rgba, void *
     else if (n_clear)
     {
         const unsigned blocks = (unsigned)std::min<size_t>((n_clear + 255) / 256, 152 * 8);
-        isti::clear_shadows_kernel<<<blocks, 256, 0, st>>>(static_cast<uint32_t *>(info_rgba), static_cast<uint32_t *>(a_rgba),
-                                                           static_cast<uint32_t *>(b_rgba), n_pixels, static_cast<const uint4 *>(clear_entries),
-                                                           n_clear);
-        e = cudaGetLastError();
+        e = isti::launch_after(true, isti::clear_shadows_kernel, blocks, 256, 0, st, static_cast<uint32_t *>(info_rgba),
+                               static_cast<uint32_t *>(a_rgba), static_cast<uint32_t *>(b_rgba), n_pixels,
+                               static_cast<const uint4 *>(clear_entries), n_clear);
     }
     if (e == cudaSuccess && n_entries)
     {
         const unsigned blocks = (unsigned)std::min<size_t>((n_entries + 255) / 256, 152 * 8);
-        isti::unpack_shadows_kernel<<<blocks, 256, 0, st>>>(static_cast<uint32_t *>(info_rgba), static_cast<uint32_t *>(a_rgba),
-                                                            static_cast<uint32_t *>(b_rgba), n_pixels, static_cast<const uint4 *>(entries),
-                                                            n_entries);
-        e = cudaGetLastError();
+        e = isti::launch_after(true, isti::unpack_shadows_kernel, blocks, 256, 0, st, static_cast<uint32_t *>(info_rgba),
+                               static_cast<uint32_t *>(a_rgba), static_cast<uint32_t *>(b_rgba), n_pixels, static_cast<const uint4 *>(entries),
+                               n_entries);
     }
     return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "isti_unpack_shadows");
 }

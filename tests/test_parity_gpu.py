@@ -106,6 +106,8 @@ def test_timewarp_mean_is_summed_in_order_where_order_matters(cuda, size, kind):
     w, h = size
     seq = Sequence(w, h, 2, seed=708)
     frame = seq.frame(0)
+    # a general matrix: the plane's normal (and with it the frame) depends on the mean depth
+    frame.fwd.inv_viewproj = np.random.default_rng(9).uniform(-1, 1, (4, 4)).astype(np.float32)
     z = np.random.default_rng(5).uniform(0.2, 0.95, (h, w)).astype(np.float32)
     big = np.float32(2.0 ** 60)
     if kind == "row":      # every row: what lies between +2^60 and -2^60 is absorbed
