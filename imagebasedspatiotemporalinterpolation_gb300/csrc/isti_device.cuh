@@ -175,6 +175,18 @@ __device__ __forceinline__ float4 project(const float *m, float4 v)
 __device__ __forceinline__ float z_to_depth(float z) { return xmul(xadd(z, 1.0f), 0.5f); } // :89-91
 __device__ __forceinline__ float depth_to_z(float d) { return xsub(xmul(d, 2.0f), 1.0f); } // :93-95
 
+// x / D, correctly rounded for D = 116, 200, 255 and 500 and normal quotients: the product with RN(1 / D)
+// corrected by its remainder (P. Markstein's division step, 1990; equal to the division for every
+// significand, tests/cpp/divided_by_test.cu).  4 operations instead of a division's 10 or so.
+template <int D>
+__host__ __device__ __forceinline__ float divided_by(float x)
+{
+    static_assert(D == 116 || D == 200 || D == 255 || D == 500, "another divisor has to be checked first");
+    constexpr float r = 1.0f / (float)D;
+    const float q = x * r;
+    return fmaf(fmaf(-q, (float)D, x), r, q);
+}
+
 // Byte c of a packed colour as a float, exact: the byte becomes the low mantissa bits of 2^23
 // (a byte permute and an addition; the integer conversion runs on a slower unit).
 __device__ __forceinline__ float byte_to_float(uint32_t color, int c)

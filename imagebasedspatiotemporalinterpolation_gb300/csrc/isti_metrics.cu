@@ -12,6 +12,9 @@
 // quality_final_kernel: one block adds the partial sums in a fixed order.
 #include "isti_metrics.h"
 #include "host/isti_error.hpp"
+#include "isti_device.cuh"
+#include "isti_tc.cuh"
+#include "isti_unet_ops.h"
 
 #include <cuda_runtime.h>
 
@@ -48,12 +51,10 @@ struct PairSum
     __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
 
-// v / 255 for an integer v in 0..255, correctly rounded: the product with RN(1 / 255) corrected
-// by its exact remainder (Markstein's division step; equal to the division for all 256 values).
+// v / 255 for an integer v in 0..255, correctly rounded
 __device__ __forceinline__ float byte_to_unit(uint32_t v)
 {
-    const float f = (float)v, q = __fmul_rn(f, 1.0f / 255.0f);
-    return fmaf(fmaf(-q, 255.0f, f), 1.0f / 255.0f, q);
+    return isti::divided_by<255>((float)v);
 }
 
 // Both passes are bound by FMA issue and shared-memory reads, so a thread filters several
@@ -73,6 +74,8 @@ __global__ void __launch_bounds__(Q_THREADS) quality_tile_kernel(const uint32_t 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
 
+    isti_tc::griddep_launch_dependents();
+    isti_tc::griddep_wait();
     uint32_t pa[PER], pb[PER]; // this thread's staged pixels, read once for the three channels
     uint32_t sq = 0;
 #pragma unroll
@@ -209,6 +212,8 @@ __global__ void __launch_bounds__(THREADS) quality_final_kernel(const double *__
 {
     __shared__ double ss[THREADS], sq[THREADS];
     double s = 0.0, q = 0.0;
+    isti_tc::griddep_launch_dependents();
+    isti_tc::griddep_wait();
     for (size_t i = threadIdx.x; i < n_blocks; i += THREADS) // fixed assignment and order: deterministic
     {
         s += partials[2 * i];
@@ -270,19 +275,29 @@ struct FlipFilters
     float2 tap[N_FLIP_FILTERS][4 * FGROUPS_MAX]; // tap k (offset k - r) twice, for the packed operations; zeros past 2 r
 };
 
-// Shared memory of a FLIP tile: three input planes (Y or the normalised Y, Cx, Cz) of (reference,
-// test) pairs, two buffers of horizontally filtered rows, the sRGB table.
+// Shared memory of a FLIP tile: the (reference, test) pixels, one plane of them at a time (Cz, Cx, Y,
+// the normalised Y) as pairs, two buffers of horizontally filtered rows, the sRGB table.  The third
+// buffer of the feature detectors lies over the pixels, not needed by then.
 struct FlipTile
 {
-    int sh, pitch, hrows; // input rows; input pitch; rows of a filtered buffer (padded taps read past sh)
-    __host__ __device__ explicit FlipTile(int r, int groups) : sh(FTH + 2 * r), pitch(FTW + 4 * groups + 2), hrows(FTH + 4 * groups) {}
+    int sh, sw, pitch, hrows; // input rows and columns; input pitch; rows of a filtered buffer (padded taps read past sh)
+    __host__ __device__ explicit FlipTile(int r, int groups)
+        : sh(FTH + 2 * r), sw(FTW + 2 * r), pitch(sw + (sw % 4 == 0 ? 2 : 0)), hrows(FTH + 4 * groups)
+    {
+    }
     __host__ __device__ int plane() const { return sh * pitch; }
     __host__ __device__ int hplane() const { return hrows * FH_PITCH; }
-    __host__ __device__ size_t bytes() const { return (size_t)(3 * plane() + 2 * hplane()) * sizeof(float2) + 256 * sizeof(float); }
+    __host__ __device__ int pixels() const { return plane() > hplane() ? plane() : hplane(); }
+    __host__ __device__ int padded_plane() const { return plane() + ROW_SLACK; }
+    __host__ __device__ size_t bytes() const
+    {
+        return (size_t)(pixels() + padded_plane() + 2 * hplane()) * sizeof(float2) + 256 * sizeof(float);
+    }
     static constexpr int FH_PITCH = FTW + 2;
+    static constexpr int ROW_SLACK = 4; // padded (zero) taps read up to 4 pairs past a row
 };
 
-constexpr float FLIP_QC = 0.7f, FLIP_QF = 0.5f, FLIP_PC = 0.4f, FLIP_PT = 0.95f, FLIP_EPS = 1e-15f;
+constexpr float FLIP_QC = 0.7f, FLIP_PC = 0.4f, FLIP_PT = 0.95f, FLIP_EPS = 1e-15f;
 
 // linear RGB -> XYZ (D65), the reference's rational constants rounded to float
 __constant__ float L2X[3][3] = {{(float)(10135552.0 / 24577794.0), (float)(8788810.0 / 24577794.0), (float)(4435075.0 / 24577794.0)},
@@ -303,18 +318,25 @@ __device__ __forceinline__ float srgb8_to_linear(uint32_t byte)
     return v > 0.04045f ? powf((fmaxf(v, 0.04045f) + 0.055f) / 1.055f, 2.4f) : v / 12.92f;
 }
 
-// sRGB pixel -> YCxCz (color_space_transform 'srgb2ycxcz'): Y, Cx, Cz; lin: srgb8_to_linear of every byte
-__device__ __forceinline__ float3 srgb8_to_ycxcz(uint32_t p, const float *lin)
+// sRGB pixel -> one component of YCxCz (color_space_transform 'srgb2ycxcz'); lin: srgb8_to_linear of every byte
+enum FlipPlane
+{
+    PLANE_Y,
+    PLANE_CX,
+    PLANE_CZ
+};
+template <FlipPlane C>
+__device__ __forceinline__ float srgb8_to_ycxcz(uint32_t p, const float *lin)
 {
     const float3 xyz = lin_to_xyz_scaled(lin[p & 255u], lin[(p >> 8) & 255u], lin[(p >> 16) & 255u]);
-    return make_float3(116.0f * xyz.y - 16.0f, 500.0f * (xyz.x - xyz.y), 200.0f * (xyz.y - xyz.z));
+    return C == PLANE_Y ? 116.0f * xyz.y - 16.0f : C == PLANE_CX ? 500.0f * (xyz.x - xyz.y) : 200.0f * (xyz.y - xyz.z);
 }
 
 // filtered YCxCz -> linear RGB clamped to the unit cube -> L*a*b* -> Hunt-adjusted
 __device__ __forceinline__ float3 ycxcz_to_hunt_lab(float Y, float Cx, float Cz)
 {
-    const float yy = (Y + 16.0f) / 116.0f;
-    const float X = (yy + Cx / 500.0f) * 0.950428545f, Yv = yy, Z = (yy - Cz / 200.0f) * 1.088900371f;
+    const float yy = isti::divided_by<116>(Y + 16.0f);
+    const float X = (yy + isti::divided_by<500>(Cx)) * 0.950428545f, Yv = yy, Z = (yy - isti::divided_by<200>(Cz)) * 1.088900371f;
     float rgb[3] = {3.241003275f * X - 1.537398934f * Yv - 0.498615861f * Z, -0.969224334f * X + 1.875930071f * Yv + 0.041554224f * Z,
                     0.055639423f * X - 0.204011202f * Yv + 1.057148933f * Z};
 #pragma unroll
@@ -424,22 +446,23 @@ __device__ __forceinline__ void flip_columns(const FlipFilters &f, const float2 
 }
 
 // One block per 32x32 output tile.  Both images travel together as (reference, test) pairs:
-// every filter step is one packed fma.rn.f32x2 for both.  The tile and an R-pixel
-// replicate-padded halo are staged as Y, Cx, Cz; plane by plane, rows are filtered into shared
-// memory, then columns per output pixel.  Cz and Cx go first: the feature detectors (three
-// filters over the normalised Y, computed in place) reuse the space of Cz as a third buffer, so
-// two blocks of a 21-tap tile share an SM.
-// Bound by FMA issue and shared-memory reads (not by HBM: 2 x 4 bytes a pixel): the register
-// windows read each staged value once per 4 outputs.  1080p: 510 -> 238 us (the images in turn,
-// one output per thread and pass, a power per staged colour value before).
-__global__ void __launch_bounds__(THREADS, 2) flip_tile_kernel(const uint32_t *__restrict__ test, const uint32_t *__restrict__ ref, int w,
+// every filter step is one packed fma.rn.f32x2 for both.  The tile's pixels and an R-pixel
+// replicate-padded halo are staged once; plane by plane they are converted, rows are filtered into
+// shared memory, then columns per output pixel, while the next plane is converted.
+// Bound by issue and its latencies (8 powers a pixel, the filters' FMAs and shared-memory reads; not by
+// HBM: 2 x 4 bytes a pixel): the register windows read each staged value once per 4 outputs, and a
+// 21-tap tile takes a third of an SM.  1080p: 510 us with the images in turn, one output per thread
+// and pass and a power per staged colour value; 238 with all three planes staged and two tiles per
+// SM; 211 with three tiles, 198 with divisions by constants and roots instead of powers.
+__global__ void __launch_bounds__(THREADS, 3) flip_tile_kernel(const uint32_t *__restrict__ test, const uint32_t *__restrict__ ref, int w,
                                                                int h, const __grid_constant__ FlipFilters f,
                                                                double *__restrict__ partials, float *__restrict__ map)
 {
     extern __shared__ __align__(16) float2 fsm[];
     const FlipTile t(f.r, f.groups);
-    float2 *pz = fsm, *px = pz + t.plane(), *py = px + t.plane(); // Cz, Cx, Y
-    float2 *h0 = py + t.plane(), *h1 = h0 + t.hplane(), *h2 = pz;
+    uint2 *pixels = reinterpret_cast<uint2 *>(fsm); // (reference, test)
+    float2 *plane = fsm + t.pixels();
+    float2 *h0 = plane + t.padded_plane(), *h1 = h0 + t.hplane(), *h2 = fsm;
     float *lin = reinterpret_cast<float *>(h1 + t.hplane());
     const int tid = threadIdx.x;
     const int x0 = blockIdx.x * FTW, y0 = blockIdx.y * FTH;
@@ -453,40 +476,52 @@ __global__ void __launch_bounds__(THREADS, 2) flip_tile_kernel(const uint32_t *_
     lin[tid] = srgb8_to_linear((uint32_t)tid);
     clear_tail(h0);
     clear_tail(h1);
-    __syncthreads();
-    const int sw = FTW + 2 * f.r;
-    for (int i = tid; i < t.plane(); i += THREADS)
+    if (tid < FlipTile::ROW_SLACK)
+        plane[t.plane() + tid] = zero;
+    isti_tc::griddep_launch_dependents();
+    isti_tc::griddep_wait();
+    const int step_y = THREADS / t.pitch, step_x = THREADS - step_y * t.pitch;
+    for (int i = tid, yy = tid / t.pitch, xx = tid - yy * t.pitch; i < t.plane(); i += THREADS)
     {
-        const int yy = i / t.pitch, xx = i - yy * t.pitch;
-        float3 cr = make_float3(0.f, 0.f, 0.f), ct = cr;
-        if (xx < sw)
+        const int gx = min(max(x0 + xx - f.r, 0), w - 1), gy = min(max(y0 + yy - f.r, 0), h - 1);
+        const size_t idx = (size_t)gy * w + gx;
+        pixels[i] = make_uint2(__ldg(ref + idx), __ldg(test + idx));
+        xx += step_x;
+        yy += step_y;
+        if (xx >= t.pitch)
         {
-            const int gx = min(max(x0 + xx - f.r, 0), w - 1), gy = min(max(y0 + yy - f.r, 0), h - 1);
-            const size_t idx = (size_t)gy * w + gx;
-            cr = srgb8_to_ycxcz(__ldg(ref + idx), lin);
-            ct = srgb8_to_ycxcz(__ldg(test + idx), lin);
+            xx -= t.pitch;
+            yy++;
         }
-        py[i] = make_float2(cr.x, ct.x);
-        px[i] = make_float2(cr.y, ct.y);
-        pz[i] = make_float2(cr.z, ct.z);
     }
+    __syncthreads();
+    // (a thread converts the pixels that it staged)
+    auto convert = [&]<FlipPlane C>() {
+        for (int i = tid; i < t.plane(); i += THREADS)
+            plane[i] = make_float2(srgb8_to_ycxcz<C>(pixels[i].x, lin), srgb8_to_ycxcz<C>(pixels[i].y, lin));
+    };
+    convert.template operator()<PLANE_CZ>();
     __syncthreads();
 
     float2 by[1][F_ROWS_EACH] = {}, rg[1][F_ROWS_EACH] = {}, la[1][F_ROWS_EACH] = {};
-    flip_rows<2>(f, t, pz, {CSF_BY1, CSF_BY2}, {h0, h1});
+    flip_rows<2>(f, t, plane, {CSF_BY1, CSF_BY2}, {h0, h1});
     __syncthreads();
     flip_columns<2, 2>(f, {h0, h1}, {0, 1}, {CSF_BY1, CSF_BY2}, {0, 0}, by);
+    convert.template operator()<PLANE_CX>();
     __syncthreads();
-    flip_rows<1>(f, t, px, {CSF_RG}, {h0});
-    flip_rows<1>(f, t, py, {CSF_A}, {h1});
-    clear_tail(h2);
+    flip_rows<1>(f, t, plane, {CSF_RG}, {h0});
     __syncthreads();
     flip_columns<1, 1>(f, {h0}, {0}, {CSF_RG}, {0}, rg);
+    convert.template operator()<PLANE_Y>();
+    __syncthreads();
+    flip_rows<1>(f, t, plane, {CSF_A}, {h1});
+    clear_tail(h2);
+    __syncthreads();
     flip_columns<1, 1>(f, {h1}, {0}, {CSF_A}, {0}, la);
     for (int i = tid; i < t.plane(); i += THREADS)
-        py[i] = make_float2((py[i].x + 16.0f) / 116.0f, (py[i].y + 16.0f) / 116.0f);
+        plane[i] = make_float2(isti::divided_by<116>(plane[i].x + 16.0f), isti::divided_by<116>(plane[i].y + 16.0f));
     __syncthreads();
-    flip_rows<3>(f, t, py, {GAUSS, EDGE, POINT}, {h0, h1, h2});
+    flip_rows<3>(f, t, plane, {GAUSS, EDGE, POINT}, {h0, h1, h2});
     __syncthreads();
     float2 gy[2][F_ROWS_EACH] = {}, ex[1][F_ROWS_EACH] = {}, fx[1][F_ROWS_EACH] = {}; // gy: edge and point along y
     flip_columns<1, 2>(f, {h0}, {0, 0}, {EDGE, POINT}, {0, 1}, gy);
@@ -505,7 +540,8 @@ __global__ void __launch_bounds__(THREADS, 2) flip_tile_kernel(const uint32_t *_
         const float3 lr = ycxcz_to_hunt_lab(la[0][r].x, rg[0][r].x, by[0][r].x), lt = ycxcz_to_hunt_lab(la[0][r].y, rg[0][r].y, by[0][r].y);
         // color pipeline: HyAB(reference, test) of the Hunt-adjusted colours
         const float dL = lr.x - lt.x, da = lr.y - lt.y, db = lr.z - lt.z;
-        const float hy = sqrtf(fmaxf(dL * dL, FLIP_EPS)) + sqrtf(da * da + db * db);
+        // (the root of a rounded square is the number again)
+        const float hy = (dL * dL > FLIP_EPS ? fabsf(dL) : sqrtf(FLIP_EPS)) + sqrtf(da * da + db * db);
         const float power = powf(hy, FLIP_QC);
         const float dec = power < pccmax ? (FLIP_PT / pccmax) * power
                                          : FLIP_PT + ((power - pccmax) / (f.cmax - pccmax)) * (1.0f - FLIP_PT);
@@ -514,7 +550,7 @@ __global__ void __launch_bounds__(THREADS, 2) flip_tile_kernel(const uint32_t *_
         const float pr = sqrtf(fx[0][r].x * fx[0][r].x + gy[1][r].x * gy[1][r].x), pt = sqrtf(fx[0][r].y * fx[0][r].y + gy[1][r].y * gy[1][r].y);
         float def = fmaxf(fabsf(er - et), fabsf(pt - pr));
         def = fmaxf(def, FLIP_EPS);
-        def = powf(0.70710678f * def, FLIP_QF);
+        def = sqrtf(0.70710678f * def); // to the power qf = 1/2
         const float v = powf(dec, 1.0f - def);
         sum_v.add(v);
         if (map)
@@ -541,6 +577,8 @@ __global__ void __launch_bounds__(THREADS) flip_final_kernel(const double *__res
 {
     __shared__ double ss[THREADS];
     double s = 0.0;
+    isti_tc::griddep_launch_dependents();
+    isti_tc::griddep_wait();
     for (size_t i = threadIdx.x; i < n_blocks; i += THREADS)
         s += partials[i];
     ss[threadIdx.x] = s;
@@ -677,11 +715,12 @@ isti_status isti_quality_rgba8(const void *a, const void *b, int32_t width, int3
     static const Gauss gw = make_gauss();
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid((width + TW - 1) / TW, (height + TH - 1) / TH);
-    quality_tile_kernel<<<grid, Q_THREADS, 0, s>>>(static_cast<const uint32_t *>(a), static_cast<const uint32_t *>(b),
-                                                    width, height, static_cast<double *>(scratch), gw);
-    quality_final_kernel<<<1, THREADS, 0, s>>>(static_cast<const double *>(scratch), n_tiles(width, height),
-                                               3.0 * (double)width * (double)height, out);
-    const cudaError_t e = cudaGetLastError();
+    // (every launch a programmatic dependent of what was before it)
+    cudaError_t e = isti_unet::launch_kernel(quality_tile_kernel, grid, Q_THREADS, 0, s, true, static_cast<const uint32_t *>(a),
+                                             static_cast<const uint32_t *>(b), width, height, static_cast<double *>(scratch), gw);
+    if (e == cudaSuccess)
+        e = isti_unet::launch_kernel(quality_final_kernel, 1, THREADS, 0, s, true, static_cast<const double *>(scratch),
+                                     n_tiles(width, height), 3.0 * (double)width * (double)height, out);
     if (e != cudaSuccess)
         return isti::set_error(ISTI_ERR_CUDA, std::string("isti_quality_rgba8: ") + cudaGetErrorString(e));
     return ISTI_OK;
@@ -716,11 +755,11 @@ isti_status isti_flip_rgba8(const void *test, const void *reference, int32_t wid
         return isti::set_error(ISTI_ERR_CUDA, std::string("isti_flip_rgba8: ") + cudaGetErrorString(attr_err));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid((width + FTW - 1) / FTW, (height + FTH - 1) / FTH);
-    flip_tile_kernel<<<grid, THREADS, smem, s>>>(static_cast<const uint32_t *>(test), static_cast<const uint32_t *>(reference), width,
-                                                     height, f, static_cast<double *>(scratch), out_map);
-    flip_final_kernel<<<1, THREADS, 0, s>>>(static_cast<const double *>(scratch), flip_tiles(width, height),
-                                            (double)width * (double)height, out_mean);
-    const cudaError_t e = cudaGetLastError();
+    cudaError_t e = isti_unet::launch_kernel(flip_tile_kernel, grid, THREADS, smem, s, true, static_cast<const uint32_t *>(test),
+                                             static_cast<const uint32_t *>(reference), width, height, f, static_cast<double *>(scratch), out_map);
+    if (e == cudaSuccess)
+        e = isti_unet::launch_kernel(flip_final_kernel, 1, THREADS, 0, s, true, static_cast<const double *>(scratch),
+                                     flip_tiles(width, height), (double)width * (double)height, out_mean);
     if (e != cudaSuccess)
         return isti::set_error(ISTI_ERR_CUDA, std::string("isti_flip_rgba8: ") + cudaGetErrorString(e));
     return ISTI_OK;
