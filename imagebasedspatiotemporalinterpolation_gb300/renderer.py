@@ -25,6 +25,15 @@ def _torch():
     return torch
 
 
+def _stream_ptr(stream) -> int:
+    """The stream's handle, or that of the current stream (asked for by itself: building the
+    current stream's object takes 2.9 us, more than a kernel launch)."""
+    if stream:
+        return stream.cuda_stream
+    torch = _torch()
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
 def _dptr(t) -> int | None:
     if t is None:
         return None
@@ -171,7 +180,7 @@ class Renderer:
         ri = info if isinstance(info, IstiRenderInfo) else render_info(info)
         if tuple(render_buffer.shape) != (ri.height, ri.width, 4) or render_buffer.dtype != torch.uint8:
             raise ValueError("render_buffer must be a (H, W, 4) uint8 tensor of the render resolution")
-        s = (stream or torch.cuda.current_stream()).cuda_stream
+        s = _stream_ptr(stream)
         check(self._lib.isti_render(self._h, _dptr(render_buffer), C.byref(ri), C.byref(frame_data.to_c()), C.c_void_p(s)))
 
     def render_batch(self, render_buffers, infos, frame_data: DeviceFrame, chain: bool = True, stream=None) -> None:
@@ -188,14 +197,13 @@ class Renderer:
             if tuple(b.shape) != (ris[0].height, ris[0].width, 4) or b.dtype != torch.uint8:
                 raise ValueError("render buffers must be (H, W, 4) uint8 tensors of the render resolution")
         outs = (C.c_void_p * n)(*[_dptr(b) for b in render_buffers])
-        s = (stream or torch.cuda.current_stream()).cuda_stream
+        s = _stream_ptr(stream)
         check(self._lib.isti_render_batch(self._h, n, outs, ris, C.byref(frame_data.to_c()), int(chain), C.c_void_p(s)))
 
     def render_pairs(self, jobs, chain: bool = False, stream=None) -> None:
         """isti_render_pairs: jobs = [(render_buffers, infos, frame_data), ...], the frames of
         several keyframe pairs in one persistent launch; each job's result equals
         render_batch(render_buffers, infos, frame_data, chain)."""
-        torch = _torch()
         if not 1 <= len(jobs) <= native.MAX_PAIRS:
             raise ValueError(f"need 1..{native.MAX_PAIRS} keyframe pairs")
         keep = []
@@ -210,7 +218,7 @@ class Renderer:
             keep += [ris, outs, fdc]
             arr[i] = native.IstiPairFrames(C.pointer(fdc), n, C.cast(outs, C.POINTER(C.c_void_p)), C.cast(ris, C.POINTER(IstiRenderInfo)),
                                            int(chain))
-        s = (stream or torch.cuda.current_stream()).cuda_stream
+        s = _stream_ptr(stream)
         self._keep_pairs = (arr, keep)  # the structs must outlive the call
         check(self._lib.isti_render_pairs(self._h, len(jobs), arr, C.c_void_p(s)))
 
@@ -230,13 +238,12 @@ class Renderer:
         output pixel) and `iterations` search steps; tiles left unresolved are rendered by
         the plain method.  chain: as render_batch's (one persistent buffer across the frames);
         otherwise each buffer is updated in place like isti_render."""
-        torch = _torch()
         n = len(infos)
         if n != len(render_buffers) or not 1 <= n <= native.MAX_BATCH_FRAMES:
             raise ValueError(f"need 1..{native.MAX_BATCH_FRAMES} frames and one buffer per frame")
         ris = (IstiRenderInfo * n)(*[i if isinstance(i, IstiRenderInfo) else render_info(i) for i in infos])
         outs = (C.c_void_p * n)(*[_dptr(b) for b in render_buffers])
-        s = (stream or torch.cuda.current_stream()).cuda_stream
+        s = _stream_ptr(stream)
         check(self._lib.isti_render_learned(self._h, net.handle if net is not None else None, n, outs, ris,
                                             C.byref(frame_data.to_c()), int(iterations), int(chain), C.c_void_p(s)))
 
@@ -336,7 +343,7 @@ def render_noalloc(render_buffer, info, frame_data: DeviceFrame, stream=None) ->
     ri = info if isinstance(info, IstiRenderInfo) else render_info(info)
     if tuple(render_buffer.shape) != (ri.height, ri.width, 4) or render_buffer.dtype != torch.uint8:
         raise ValueError("render_buffer must be a (H, W, 4) uint8 tensor of the render resolution")
-    s = (stream or torch.cuda.current_stream()).cuda_stream
+    s = _stream_ptr(stream)
     check(lib.isti_render_noalloc(_dptr(render_buffer), C.byref(ri), C.byref(frame_data.to_c()), C.c_void_p(s)))
 
 
@@ -345,12 +352,11 @@ def rgb8_to_rgba8(dst, src, stream=None) -> None:
     (..., 4) uint8 the renderer reads, alpha 255.  For images whose alpha the renderer
     never reads (shadow colour A/B, shadow info): uploading them as RGB moves 3/4 of the
     bytes over the host link."""
-    torch = _torch()
-    if src.dtype != torch.uint8 or dst.dtype != torch.uint8 or src.shape[-1] != 3 or dst.shape[-1] != 4 \
-            or src.shape[:-1] != dst.shape[:-1] or not src.is_contiguous() or not dst.is_contiguous():
+    u8, to, of = _torch().uint8, dst.shape, src.shape
+    if src.dtype != u8 or dst.dtype != u8 or of[-1] != 3 or to[-1] != 4 or to[:-1] != of[:-1] \
+            or not src.is_contiguous() or not dst.is_contiguous():
         raise ValueError("rgb8_to_rgba8 expects contiguous uint8 (..., 3) -> (..., 4) tensors of the same pixel count")
-    s = (stream or torch.cuda.current_stream()).cuda_stream
-    check(native.load().isti_rgb8_to_rgba8(_dptr(dst), _dptr(src), C.c_size_t(src.numel() // 3), C.c_void_p(s)))
+    check(native.load().isti_rgb8_to_rgba8(_dptr(dst), _dptr(src), src.numel() // 3, _stream_ptr(stream)))
 
 
 SHADOW_ENTRY_BYTES = 16  # ISTI_SHADOW_ENTRY_BYTES
@@ -384,14 +390,11 @@ def unpack_shadows(info, a, b, entries, n_entries=None, clear_entries=None, n_cl
     <- zero, then the listed pixels of `entries` (a device uint8 tensor of n x 16 bytes, as
     pack_shadow_entries makes them).  clear_entries: the entries of the previous unpack into
     the same images, whose pixels alone are then cleared."""
-    torch = _torch()
-    for t in (info, a, b):
-        if t.dtype != torch.uint8 or t.shape[-1] != 4 or not t.is_contiguous() or t.shape != info.shape:
-            raise ValueError("unpack_shadows expects three contiguous uint8 (..., 4) tensors of one shape")
+    u8, shape = _torch().uint8, info.shape
+    if shape[-1] != 4 or a.shape != shape or b.shape != shape or info.dtype != u8 or a.dtype != u8 or b.dtype != u8 \
+            or not (info.is_contiguous() and a.is_contiguous() and b.is_contiguous()):
+        raise ValueError("unpack_shadows expects three contiguous uint8 (..., 4) tensors of one shape")
     n = entries.numel() // SHADOW_ENTRY_BYTES if n_entries is None else int(n_entries)
     nc = 0 if clear_entries is None else (clear_entries.numel() // SHADOW_ENTRY_BYTES if n_clear is None else int(n_clear))
-    s = (stream or torch.cuda.current_stream()).cuda_stream
-    check(native.load().isti_unpack_shadows(_dptr(info), _dptr(a), _dptr(b), C.c_size_t(info.numel() // 4),
-                                            C.c_void_p(_dptr(entries) if n else None), C.c_size_t(n),
-                                            C.c_void_p(_dptr(clear_entries) if clear_entries is not None else None), C.c_size_t(nc),
-                                            C.c_void_p(s)))
+    check(native.load().isti_unpack_shadows(_dptr(info), _dptr(a), _dptr(b), info.numel() // 4, _dptr(entries) if n else None, n,
+                                            _dptr(clear_entries), nc, _stream_ptr(stream)))
