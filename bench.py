@@ -851,12 +851,14 @@ def run_graph_batch(args, dev, rank):
     single.close()
     r.close()
 
-    # the same batch as ONE persistent launch (isti_render_pairs: a cooperative kernel over a
-    # device work queue of init / splat / reprojection units), captured once and replayed; its
+    # the same batch as ONE persistent launch (isti_render_pairs with unit sizes set, which asks for
+    # it: a cooperative kernel over a device work queue of init / splat / reprojection units; without
+    # them pairs of this size are rendered as batches), captured once and replayed; its
     # frames must equal the 48-launch graph's bit for bit
     persistent = None
     try:
         rp = Renderer()
+        rp.set_pair_units(32, 256)
         pouts = [[torch.zeros_like(o) for o in os_] for os_ in outs]
         pjobs = [(po, infos, frame) for po, (w, h, frame, infos) in zip(pouts, jobs)]
         with torch.cuda.stream(stream):

@@ -11,7 +11,7 @@ learned one learned-initialiser call (isti_render_learned, trained weights, 1 it
         1920x1080, main camera only, 3 frames: the network's conv kernels, keyframe_kernel,
         learned_kernel and the fallback kernels.
 pairs   one isti_render_pairs call over 4 keyframe pairs at 1920x1080 (main camera, 3 frames
-        each): one launch of batch_kernel.
+        each), with unit sizes set, which asks for the persistent launch: one of batch_kernel.
 
 Each case runs once after one untimed warm-up call of the same case, so a profiler selects
 the second launch of a kernel with `-s 1 -c 1` (learned: the network runs once per call).
@@ -64,6 +64,7 @@ def _pairs(torch, seq_cls, frame_cls, renderer_cls, arith):
         outs = [torch.zeros((1080, 1920, 4), dtype=torch.uint8, device="cuda") for _ in clients]
         jobs.append((outs, clients, frame))
     r = renderer_cls()
+    r.set_pair_units(32, 256)
     for _ in range(2):
         r.render_pairs(jobs)
     torch.cuda.synchronize()
