@@ -114,3 +114,43 @@ def test_uploads_and_renders_in_one_chain(cuda, captured):
         assert torch.equal(out, wants[turn % 2]), f"turn {turn}"
     assert r.device_status() == native.ISTI_OK
     r.close()
+
+
+@pytest.mark.parametrize("render_on_default", [True, False])
+def test_implicit_order_with_the_default_stream(cuda, render_on_default):
+    """A stream made by cudaStreamCreate and the default stream wait for each other without events.  The
+    keyframes' colour arrives on one of them behind a delay, the render runs on the other, where the
+    kernel before it was enqueued earlier than that, and the output is read on the first."""
+    import ctypes
+    import torch
+    handle = ctypes.c_void_p()
+    assert torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(handle)) == torch.cuda.cudart().cudaError.success
+    default, blocking = torch.cuda.default_stream(), torch.cuda.ExternalStream(handle.value)
+    at, other = (default, blocking) if render_on_default else (blocking, default)
+    seq = Sequence(162, 98, 2, seed=921, aux_offsets=(0.3,), shadows=True, max_speed=3.0)
+    frame, client = DeviceFrame.from_host(seq.frame(0)), seq.client(0, 2)
+    colors = [frame.fwd.color.clone(), 255 - frame.fwd.color]
+    r = Renderer()
+    out = torch.zeros((98, 162, 4), dtype=torch.uint8, device="cuda")
+    wants = []
+    for c in colors:
+        for view in frame.views():
+            view.color.copy_(c)
+        r.render(out.zero_(), client, frame)
+        torch.cuda.synchronize()
+        wants.append(out.clone())
+    torch.cuda.synchronize()
+    for turn in range(6):
+        with torch.cuda.stream(at):
+            out.zero_()
+        with torch.cuda.stream(other):
+            torch.cuda._sleep(4_000_000)  # about 2 ms
+            for view in frame.views():
+                view.color.copy_(colors[turn % 2])
+        r.render(out, client, frame, at)
+        with torch.cuda.stream(other):
+            got = out.clone()
+        torch.cuda.synchronize()
+        assert torch.equal(got, wants[turn % 2]), f"turn {turn}"
+    r.close()
+    torch.cuda.cudart().cudaStreamDestroy(handle.value)
