@@ -1127,13 +1127,16 @@ __global__ void __maxnreg__(reproj_regs(SW, REGS, NV)) reproj_kernel(const __gri
 // n * max|z|; with n * max|z| <= 2^53 u every partial sum is a multiple of u that a double
 // holds exactly.  NDC depths of a 1080p frame meet that for |z| >= 2^-18 (rows) and 2^-9
 // (total); a row or total that does not (and NaN or infinity) is summed in order by one warp.
-// Whether sums of n values of at most |zmax| that are multiples of 2^(e_min - 150) are exact.
-__device__ __forceinline__ bool sums_exact(double n, uint32_t zmax, uint32_t e_min)
+// Whether sums of n (or up to n) values of at most |zmax| that are multiples of u = 2^(e_min - 150) stay
+// below 2^53 u (no non-zero value: e_min 255; e_min 0: not known).  In float, rounded up: the FP64
+// unit takes a lane a clock.
+__device__ __forceinline__ bool sums_exact(float n, uint32_t zmax, uint32_t e_min)
 {
-    if (zmax >= 0x7f800000u || e_min == 0u)
+    if (zmax == 0u && e_min != 0u)
+        return true;
+    if (zmax >= 0x7f800000u || e_min - 1u >= 224u)
         return false;
-    const double unit53 = __hiloint2double((int)((min(e_min, 255u) - 150u + 53u + 1023u) << 20), 0); // 2^53 units
-    return n * (double)__uint_as_float(zmax) <= unit53;
+    return __fmul_ru(n, __uint_as_float(zmax)) <= __uint_as_float((e_min + 53u - 150u + 127u) << 23);
 }
 
 // Adds `count` doubles to acc one after the other; called by a whole warp, element i from
@@ -1154,6 +1157,7 @@ __device__ double warp_sum_in_order(double acc, uint32_t count, Get get)
 
 // Sum, largest |z| and smallest exponent over the block (TW_THREADS threads); valid in thread 0.
 constexpr int TW_THREADS = 128;
+constexpr int TW_LOADS = 16; // loads a thread has in flight
 __device__ __forceinline__ void tw_block_reduce(double &sum, uint32_t &zmax, uint32_t &e_min)
 {
     __shared__ double s_sum[TW_THREADS / 32];
@@ -1179,40 +1183,89 @@ __device__ __forceinline__ void tw_block_reduce(double &sum, uint32_t &zmax, uin
 }
 
 // One block per row, so that a row's loads are coalesced and in flight together (4 bytes a
-// pixel, each read once).  With one thread per row summing in order the two sums took 235 and
-// 65 us of a 1080p call; the whole call went from 289 to 43 us.
+// pixel, each read once).  What bounded the double sums is the FP64 unit (a lane a clock): a
+// thread's sum is a float and the sum of its additions' rounding errors (Knuth's two-sum) where
+// that holds it exactly, and a block's the integer sum of those in units of u.  With n values per
+// thread an error is at most n max|z| 2^-24, a multiple of u, and their sum a multiple of u below
+// n^2 max|z| 2^-24 (to a few rounding errors): with n^2 max|z| <= 2^47 u a float holds every
+// partial sum of them.
+// With one thread per row summing in order the two sums took 235 and 65 us of a 1080p call (289 us);
+// this kernel 16 us in double, 5.9 us so, the call 37.2 and 27.7 us.
 __global__ void __launch_bounds__(TW_THREADS) timewarp_rowsum_kernel(const __grid_constant__ FrameParams p)
 {
     dependents_may_launch();
     wait_for_prerequisites();
     const DevView &v = p.v[0];
     const float *row = v.z + (size_t)blockIdx.x * v.w;
-    double acc = 0.0;
+    float hi = 0.0f, lo = 0.0f;
     uint32_t zmax = 0u, e_min = 255u;
-#pragma unroll 4
-    for (uint32_t x = threadIdx.x; x < v.w; x += TW_THREADS)
+    for (uint32_t x0 = threadIdx.x; x0 < v.w; x0 += TW_THREADS * TW_LOADS)
     {
-        const float z = __ldg(row + x);
-        const uint32_t a = __float_as_uint(z) & 0x7fffffffu;
-        acc = __dadd_rn(acc, (double)z);
-        zmax = max(zmax, a);
-        if (a != 0u)
-            e_min = min(e_min, max(1u, a >> 23));
+        float z[TW_LOADS]; // past the row: 0, which changes nothing
+#pragma unroll
+        for (int i = 0; i < TW_LOADS; i++)
+            z[i] = x0 + i * TW_THREADS < v.w ? __ldg(row + x0 + i * TW_THREADS) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < TW_LOADS; i++)
+        {
+            const uint32_t a = __float_as_uint(z[i]) & 0x7fffffffu;
+            const float s = __fadd_rn(hi, z[i]), t = __fsub_rn(s, hi);
+            lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(z[i], t)));
+            hi = s;
+            zmax = max(zmax, a);
+            if (a != 0u)
+                e_min = min(e_min, max(1u, a >> 23));
+        }
     }
-    tw_block_reduce(acc, zmax, e_min);
-    __shared__ bool exact;
-    if (threadIdx.x == 0)
+    __shared__ uint32_t s_zmax[TW_THREADS / 32], s_e_min[TW_THREADS / 32];
+    __shared__ long long s_units[TW_THREADS / 32];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    zmax = __reduce_max_sync(0xffffffffu, zmax);
+    e_min = __reduce_min_sync(0xffffffffu, e_min);
+    if (lane == 0u)
     {
-        exact = sums_exact((double)v.w, zmax, e_min);
-        if (exact)
-            p.tw_rows[blockIdx.x] = TwRow{acc, zmax, e_min};
+        s_zmax[warp] = zmax;
+        s_e_min[warp] = e_min;
     }
     __syncthreads();
-    if (exact || threadIdx.x >= 32)
-        return;
-    acc = warp_sum_in_order(0.0, v.w, [&](uint32_t x) { return (double)__ldg(row + x); });
-    if (threadIdx.x == 0)
-        p.tw_rows[blockIdx.x] = TwRow{acc, 0u, 0u};
+#pragma unroll
+    for (int k = 0; k < TW_THREADS / 32; k++)
+    {
+        zmax = max(zmax, s_zmax[k]);
+        e_min = min(e_min, s_e_min[k]);
+    }
+    const float n = (float)((v.w + TW_THREADS - 1) / TW_THREADS);
+    double acc = 0.0;
+    if (!sums_exact((float)v.w, zmax, e_min))
+    {
+        if (warp != 0u)
+            return;
+        acc = warp_sum_in_order(0.0, v.w, [&](uint32_t x) { return (double)__ldg(row + x); });
+        zmax = e_min = 0u;
+    }
+    else if (e_min >= 64u && sums_exact(n * n * 64.0f, zmax, e_min)) // (from 2^-63 on no rounding error is flushed to zero)
+    {
+        const float per_unit = zmax == 0u ? 1.0f : __uint_as_float((127u + 150u - e_min) << 23);
+        long long units = __float2ll_rn(hi * per_unit) + __float2ll_rn(lo * per_unit);
+        for (int o = 16; o > 0; o >>= 1)
+            units += __shfl_down_sync(0xffffffffu, units, o);
+        if (lane == 0u)
+            s_units[warp] = units;
+        __syncthreads();
+        if (threadIdx.x != 0u)
+            return;
+        for (int k = 1; k < TW_THREADS / 32; k++)
+            units += s_units[k];
+        acc = __ll2double_rn(units) * __hiloint2double((int)((e_min + 1023u - 150u) << 20), 0);
+    }
+    else
+    {
+        for (uint32_t x = threadIdx.x; x < v.w; x += TW_THREADS)
+            acc = __dadd_rn(acc, (double)__ldg(row + x));
+        tw_block_reduce(acc, zmax, e_min); // (the largest and smallest as before)
+    }
+    if (threadIdx.x == 0u)
+        p.tw_rows[blockIdx.x] = TwRow{acc, zmax, e_min};
 }
 
 __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz)
@@ -1229,18 +1282,24 @@ __global__ void __launch_bounds__(TW_THREADS) timewarp_mean_kernel(const __grid_
     const DevView &to = p.v[0];
     double acc = 0.0;
     uint32_t zmax = 0u, e_min = 255u;
-#pragma unroll 4
-    for (uint32_t y = threadIdx.x; y < to.h; y += TW_THREADS)
+    for (uint32_t y0 = threadIdx.x; y0 < to.h; y0 += TW_THREADS * TW_LOADS)
     {
-        const TwRow r = p.tw_rows[y];
-        acc = __dadd_rn(acc, r.sum);
-        zmax = max(zmax, r.zmax);
-        e_min = min(e_min, r.e_min);
+        TwRow r[TW_LOADS];
+#pragma unroll
+        for (int i = 0; i < TW_LOADS; i++)
+            r[i] = y0 + i * TW_THREADS < to.h ? p.tw_rows[y0 + i * TW_THREADS] : TwRow{0.0, 0u, 255u};
+#pragma unroll
+        for (int i = 0; i < TW_LOADS; i++)
+        {
+            acc = __dadd_rn(acc, r[i].sum);
+            zmax = max(zmax, r[i].zmax);
+            e_min = min(e_min, r[i].e_min);
+        }
     }
     tw_block_reduce(acc, zmax, e_min);
     __shared__ bool exact;
     if (threadIdx.x == 0)
-        exact = sums_exact((double)to.w * (double)to.h, zmax, e_min);
+        exact = sums_exact(__fmul_ru((float)to.w, (float)to.h), zmax, e_min);
     __syncthreads();
     if (threadIdx.x >= 32)
         return;

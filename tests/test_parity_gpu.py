@@ -97,8 +97,8 @@ def test_timewarp_matches_oracle_1080p(cuda, aux):
     r.close()
 
 
-@pytest.mark.parametrize("size", [(333, 197), (96, 64), (31, 5), (640, 1)], ids=lambda s: f"{s[0]}x{s[1]}")
-@pytest.mark.parametrize("kind", ["exact", "row", "total", "zeros"])
+@pytest.mark.parametrize("size", [(333, 197), (96, 64), (31, 5), (640, 1), (5000, 3)], ids=lambda s: f"{s[0]}x{s[1]}")
+@pytest.mark.parametrize("kind", ["exact", "row", "total", "zeros", "small"])
 def test_timewarp_mean_is_summed_in_order_where_order_matters(cuda, size, kind):
     """The mean depth is the in-order double sum: rows and totals whose additions round (values
     that absorb others and cancel later) give what the oracle's order gives, not another order's."""
@@ -116,6 +116,8 @@ def test_timewarp_mean_is_summed_in_order_where_order_matters(cuda, size, kind):
         z[0], z[-1 - h // 8] = big, -big
     elif kind == "zeros":
         z[:] = np.where(z > 0.5, np.float32(0.0), np.float32(-0.0))
+    elif kind == "small":  # rows of ever smaller units: first a float pair per thread, then double, then only the order sums them
+        z *= np.float32(2.0) ** -np.random.default_rng(6).integers(0, 3 + np.arange(h)[:, None] % 40, (h, w)).astype(np.float32)
     frame.fwd.z = z
     client = seq.client(0, 2, mode=native.MODE_TIMEWARP)
     prev = np.full((h, w, 4), 11, np.uint8)
