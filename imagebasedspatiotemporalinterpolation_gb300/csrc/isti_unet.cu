@@ -135,7 +135,6 @@ cudaError_t smem_limit(K kernel, size_t bytes)
     return e;
 }
 
-constexpr size_t SMEM_BUDGET = 200 * 1024;
 int32_t *g_null_status = nullptr; // device word for callers that pass no status
 
 isti_status status_word(int32_t *&status)
@@ -267,54 +266,7 @@ isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, c
     return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "isti_unet_conv launch");
 }
 
-// The weight gradient's work split (wgrad_kernel) and its scratch.
-struct WgradConfig
-{
-    int n, h, w;              // the images, those of 1x1 layers as one row of pixels each
-    int kseg, segs, n_units;
-    int n_dy, n_mb;           // per CTA
-    int grid_y, grid_z, splits, units_per_split, stages;
-    size_t smem;
-};
-
-bool wgrad_config(int taps, int n, int h, int w, int cin, int cout, WgradConfig &c)
-{
-    c = WgradConfig{};
-    c.n = n;
-    c.h = taps == 9 ? h : 1;
-    const long long row = taps == 9 ? w : (long long)h * w;
-    if (row > INT32_MAX / 2 - 256)
-        return false;
-    c.w = (int)row;
-    const int mblocks = ((taps == 9 ? 3 : 1) * cout + 127) / 128;
-    c.n_dy = taps == 9 ? 3 : 1;
-    c.n_mb = mblocks;
-    // all accumulators of a CTA in the 512 TMEM columns: else one row (dy) per CTA, then one M block
-    if (c.n_dy == 3 && c.n_mb * wgrad_mb_cols(cin, 3) > 512)
-        c.n_dy = 1;
-    if (c.n_mb * wgrad_mb_cols(cin, c.n_dy) > 512)
-        c.n_mb = 1;
-    c.grid_y = taps == 9 && c.n_dy == 1 ? 3 : 1;
-    c.grid_z = mblocks / c.n_mb;
-    // 128 pixels per unit where three stages of them fit and the rows are that long, else 64
-    for (c.kseg = 128;; c.kseg = 64)
-    {
-        const size_t sb = wgrad_stage_bytes(cin, c.n_dy, c.n_mb, c.kseg);
-        c.stages = (int)std::min<size_t>(6, (SMEM_BUDGET - 256) / sb);
-        if (c.kseg == 64 || (c.stages >= 3 && c.w > 64))
-        {
-            c.smem = c.stages * sb + (2 * c.stages + 1) * 8 + 16;
-            break;
-        }
-    }
-    c.segs = (c.w + c.kseg - 1) / c.kseg;
-    c.n_units = c.n * c.h * c.segs;
-    // one CTA per SM, at least 4 units each
-    c.splits = std::max(1, std::min(152 / (c.grid_y * c.grid_z), (c.n_units + 3) / 4));
-    c.units_per_split = (c.n_units + c.splits - 1) / c.splits;
-    return c.stages >= 2;
-}
-
+// Bytes of scratch: every split's partial sums.
 size_t wgrad_scratch(int taps, int n, int h, int w, int cin, int cout)
 {
     WgradConfig c;

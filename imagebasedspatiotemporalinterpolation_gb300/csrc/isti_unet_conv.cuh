@@ -36,10 +36,13 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 namespace isti_unet
 {
 using namespace isti_tc;
 
+constexpr size_t SMEM_BUDGET = 200 * 1024; // shared memory of a CTA that has the SM to itself
 constexpr int TILE_W = 16, TILE_H = 8, TILE_M = TILE_W * TILE_H;
 constexpr uint32_t BOX_BYTES = TILE_M * 16; // one TMA box: 8 channels x 128 pixels
 
@@ -371,6 +374,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     }
     else if (warp >= 2)
     {
+        griddep_wait(); // the mask is complete
         const int q = warp % 4; // the TMEM lane quadrant this warp may read
         const int m = q * 32 + lane, mx = m & ((1 << p.tile_shift) - 1), my = m >> p.tile_shift;
         UnitPos at(blockIdx.x, gridDim.x, p.tiles_x, p.tiles_y);
@@ -549,6 +553,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     }
     else if (warp >= 2)
     {
+        griddep_wait(); // the mask is complete
         const int q = warp % 4;
         const int m = q * 32 + lane;
         UnitPos at(blockIdx.x, gridDim.x, segs, p.h);
@@ -624,6 +629,56 @@ __host__ __device__ constexpr uint32_t wgrad_stage_bytes(int cin, int n_dy, int 
 }
 __host__ __device__ constexpr int wgrad_mb_cols(int cin, int n_dy) { return n_dy * cin + 16; }
 
+// The work split of wgrad_kernel.  Every split has units (tests/cpp/wgrad_splits_test.cu): one without
+// would write its zeros, and be added up, for nothing.
+struct WgradConfig
+{
+    int n, h, w;              // the images, those of 1x1 layers as one row of pixels each
+    int kseg, segs, n_units;
+    int n_dy, n_mb;           // per CTA
+    int grid_y, grid_z, splits, units_per_split, stages;
+    size_t smem;
+};
+
+inline bool wgrad_config(int taps, int n, int h, int w, int cin, int cout, WgradConfig &c)
+{
+    c = WgradConfig{};
+    c.n = n;
+    c.h = taps == 9 ? h : 1;
+    const long long row = taps == 9 ? w : (long long)h * w;
+    if (row > INT32_MAX / 2 - 256)
+        return false;
+    c.w = (int)row;
+    const int mblocks = ((taps == 9 ? 3 : 1) * cout + 127) / 128;
+    c.n_dy = taps == 9 ? 3 : 1;
+    c.n_mb = mblocks;
+    // all accumulators of a CTA in the 512 TMEM columns: else one row (dy) per CTA, then one M block
+    if (c.n_dy == 3 && c.n_mb * wgrad_mb_cols(cin, 3) > 512)
+        c.n_dy = 1;
+    if (c.n_mb * wgrad_mb_cols(cin, c.n_dy) > 512)
+        c.n_mb = 1;
+    c.grid_y = taps == 9 && c.n_dy == 1 ? 3 : 1;
+    c.grid_z = mblocks / c.n_mb;
+    // 128 pixels per unit where three stages of them fit and the rows are that long, else 64
+    for (c.kseg = 128;; c.kseg = 64)
+    {
+        const size_t sb = wgrad_stage_bytes(cin, c.n_dy, c.n_mb, c.kseg);
+        c.stages = (int)std::min<size_t>(6, (SMEM_BUDGET - 256) / sb);
+        if (c.kseg == 64 || (c.stages >= 3 && c.w > 64))
+        {
+            c.smem = c.stages * sb + (2 * c.stages + 1) * 8 + 16;
+            break;
+        }
+    }
+    c.segs = (c.w + c.kseg - 1) / c.kseg;
+    c.n_units = c.n * c.h * c.segs;
+    // at most one CTA per SM, at least 4 units each (the last one takes what is left)
+    const int most = std::max(1, std::min(152 / (c.grid_y * c.grid_z), (c.n_units + 3) / 4));
+    c.units_per_split = (c.n_units + most - 1) / most;
+    c.splits = (c.n_units + c.units_per_split - 1) / c.units_per_split;
+    return c.stages >= 2;
+}
+
 constexpr int WGRAD_THREADS = 128; // warp 0 producer, warp 1 MMA, all four epilogue
 
 template <int TAPS, int N_DY, int N_MB>
@@ -680,7 +735,7 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     if (warp == 0)
     {
         const uint32_t leader = elect_one();
-        griddep_wait(); // dY and X are complete (every load below is later), and the scratch is free
+        griddep_wait(); // dY and X are complete (every load below is later)
         fence_proxy_async_global();
         const uint32_t tx_bytes = (uint32_t)(boxes * p.box_chunks) * px_bytes + (uint32_t)(p.cin / 8) * b_rows_bytes;
         const int shift0 = mb0 * 16 / co_chunks, group0 = mb0 * 16 % co_chunks; // of the first box
@@ -760,6 +815,10 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     }
     __syncwarp();
 
+    // The scratch is one for all layers, and the kernels between let this one start before they
+    // waited themselves: the reduction of the layer before may still read it.  (Warp 0's wait
+    // orders a CTA's stores by way of its copies and products only where it has units.)
+    griddep_wait();
     const bool ok = mbar_wait(done, 0, p.status);
     tc_fence_after();
     if (ok)
