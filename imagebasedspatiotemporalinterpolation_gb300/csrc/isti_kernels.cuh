@@ -205,6 +205,11 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
 // touches anything (wait; returns at once in an ordinary launch, or after work that is not a
 // kernel).  That hides the launch latency between them: about 3 of 4.8 us per kernel, most of a
 // small frame (640x360: 24.6 -> 19.0 us a call from within the call, 17.2 with the first kernel too).
+//
+// So a kernel may be resident while others still write what it will read, and not only the one
+// before it.  The read-only path (__ldg, const __restrict__ parameters) is for data that nobody
+// writes meanwhile: what earlier kernels or the caller's may have written -- every image, table and
+// intermediate -- is read by ordinary loads.
 __device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -212,21 +217,21 @@ __device__ __forceinline__ void wait_for_prerequisites() { asm volatile("griddep
 
 __device__ __forceinline__ float ld_f(const float *img, uint32_t x, uint32_t y, uint32_t w, uint32_t h)
 {
-    return (x < w && y < h) ? __ldg(img + (y * w + x)) : 0.0f;
+    return (x < w && y < h) ? img[y * w + x] : 0.0f;
 }
 __device__ __forceinline__ float4 ld_f4(const float4 *img, uint32_t x, uint32_t y, uint32_t w, uint32_t h)
 {
-    return (x < w && y < h) ? __ldg(img + (y * w + x)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return (x < w && y < h) ? img[y * w + x] : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 __device__ __forceinline__ uint32_t ld_c(const uint32_t *img, uint32_t x, uint32_t y, uint32_t w, uint32_t h)
 {
-    return (x < w && y < h) ? __ldg(img + (y * w + x)) : 0u;
+    return (x < w && y < h) ? img[y * w + x] : 0u;
 }
 
 __device__ __forceinline__ float4 load_motion(const DevView &v, uint32_t idx)
 {
     if (v.motion_fmt == ISTI_MOTION_F32X4)
-        return __ldg(static_cast<const float4 *>(v.motion) + idx);
+        return static_cast<const float4 *>(v.motion)[idx];
     if (v.motion_fmt == ISTI_MOTION_F16X3)
     {
         const __half *m = static_cast<const __half *>(v.motion) + 3 * (size_t)idx;
@@ -240,7 +245,7 @@ template <class V>
 __device__ __forceinline__ float2 view_pixel2cs(const V &v, uint32_t x, uint32_t y)
 {
     if (x < v.w && y < v.h)
-        return make_float2(__ldg(v.lut + x), __ldg(v.lut + v.w + y));
+        return make_float2(v.lut[x], v.lut[v.w + y]);
     return pixel2cs(x, y, v.w, v.h);
 }
 
@@ -291,9 +296,9 @@ __device__ __forceinline__ void splat_pixel(const FrameParams &p, int view, uint
     const uint32_t idx = y * v.w + x;
 
     // keyframe part, independent of the client camera
-    const float z_from = __ldg(v.z + idx);
+    const float z_from = v.z[idx];
     const float4 om = load_motion(v, idx);
-    const float pcx = __ldg(v.lut + x), pcy = __ldg(v.lut + v.w + y); // pixel2CS(idx2D, resolution)
+    const float pcx = v.lut[x], pcy = v.lut[v.w + y]; // pixel2CS(idx2D, resolution)
     const float4 cs_from = make_float4(pcx, pcy, z_from, 1.0f);
     const float4 ws_from = project(v.inv_vp, cs_from);
     const float4 moved = make_float4(xadd(pcx, om.x), xadd(pcy, om.y), xadd(z_from, om.z), 1.0f);
@@ -378,9 +383,9 @@ __device__ __forceinline__ PixelShade load_shade(const V &v, uint32_t px, uint32
     PixelShade s;
     const bool in = px < v.w && py < v.h;
     const uint32_t idx = py * v.w + px;
-    s.color = in ? __ldg(v.color + idx) : 0u;
+    s.color = in ? v.color[idx] : 0u;
     s.sha = s.shb = 0u;
-    const uint32_t si = (shadows && in) ? __ldg(v.shi + idx) : 0u;
+    const uint32_t si = (shadows && in) ? v.shi[idx] : 0u;
     s.bf = ((si & 255u) << 16) | (((si >> 8) & 255u) << 8) | ((si >> 16) & 255u);
     s.levels = shadows && v.shb != nullptr && s.bf != 0;
     s.init = (int32_t)(s.bf & SOFTSHADOW_VAL_MASK);
@@ -397,9 +402,9 @@ __device__ __forceinline__ PixelShade load_shade(const V &v, uint32_t px, uint32
         // colour A / B are read only where a level differs from the initial one
         // (colorFromShadow uses the pixel's own colour otherwise)
         if (s.mn != s.init)
-            s.sha = __ldg(v.sha + idx);
+            s.sha = v.sha[idx];
         if (s.mx != s.init)
-            s.shb = __ldg(v.shb + idx);
+            s.shb = v.shb[idx];
     }
     return s;
 }
@@ -498,8 +503,8 @@ __device__ uint32_t second_chance(float weight, const ShadowFrames &sf, const Fr
     {
         const bool on_to = shadows_on(sf, c, to);
         const uint32_t pi = (uint32_t)pp.y * to.w + (uint32_t)pp.x;
-        const float az = __ldg(to.z + pi);
-        const float4 m_tf = __ldg(to.full_ff + pi);
+        const float az = to.z[pi];
+        const float4 m_tf = to.full_ff[pi];
         const PixelShade s_to = load_shade(to, (uint32_t)pp.x, (uint32_t)pp.y, on_to, c.sfpa);
         const float dx = xsub(m_ft.x, -m_tf.x), dy = xsub(m_ft.y, -m_tf.y), dz = xsub(m_ft.z, -m_tf.z);
         if (sqrt_less(xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz)), EPS_3) &&
@@ -895,8 +900,8 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
         // pixel2CS of the output pixels in the main view (the search target) and in this view (the error)
         const DevView &v0 = p.v[0];
         const uint32_t xc = min(x, p.out_w - 1);
-        const float qx = __ldg(v0.lut + xc);
-        const float pcx = __ldg(v.lut + min(ix, v.w - 1));
+        const float qx = v0.lut[xc];
+        const float pcx = v.lut[min(ix, v.w - 1)];
         const uint32_t vwid = v.w, vhei = v.h;
         const float half_w = (float)vwid * 0.5f, half_h = (float)vhei * 0.5f;
         // the scale res / min(res) (src/renderer.cu:213): the host's IEEE quotient, or under the
@@ -911,8 +916,8 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
             const uint32_t iy0 = v.sy == 1 ? y0 : y0 / v.sy, iy1 = v.sy == 1 ? y0 + 1 : (y0 + 1) / v.sy;
             const bool rok[ROWS] = {xok && y0 < p.out_h, xok && y0 + 1 < p.out_h};
             const uint32_t y0c = min(y0, p.out_h - 1), y1c = min(y0 + 1, p.out_h - 1);
-            const float qy[ROWS] = {__ldg(v0.lut + v0.w + y0c), __ldg(v0.lut + v0.w + y1c)};
-            const float pcy[ROWS] = {__ldg(v.lut + v.w + min(iy0, vhei - 1)), __ldg(v.lut + v.w + min(iy1, vhei - 1))};
+            const float qy[ROWS] = {v0.lut[v0.w + y0c], v0.lut[v0.w + y1c]};
+            const float pcy[ROWS] = {v.lut[v.w + min(iy0, vhei - 1)], v.lut[v.w + min(iy1, vhei - 1)]};
 #pragma unroll 1
             for (int j = 0; j < gn; j++)
             {
@@ -943,7 +948,7 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                         for (int c = lane; c < T::W; c += 32)
                         {
                             const uint32_t gx = (uint32_t)(xs + c);
-                            tg[r * T::W + c] = (row_ok && gx < vwid) ? __ldg(keys + (gy * vwid + gx)) : 0ull;
+                            tg[r * T::W + c] = (row_ok && gx < vwid) ? keys[gy * vwid + gx] : 0ull;
                         }
                     }
                     __syncwarp();
@@ -983,7 +988,7 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                     float2 m[ROWS];
 #pragma unroll
                     for (int r = 0; r < ROWS; r++)
-                        m[r] = __ldg(cam + (ay[r] * vwid + ax[r]));
+                        m[r] = cam[ay[r] * vwid + ax[r]];
 #pragma unroll
                     for (int r = 0; r < ROWS; r++)
                     {
@@ -1003,11 +1008,11 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                 for (int r = 0; r < ROWS; r++)
                 {
                     const uint32_t si = ay[r] * vwid + ax[r];
-                    m[r] = __ldg(cam + si);
-                    dz[r] = __ldg(cdep + si);
-                    vs[r] = __ldg(v.vis + si);
-                    fx[r] = __ldg(v.lut + ax[r]);
-                    fy[r] = __ldg(v.lut + vwid + ay[r]);
+                    m[r] = cam[si];
+                    dz[r] = cdep[si];
+                    vs[r] = v.vis[si];
+                    fx[r] = v.lut[ax[r]];
+                    fy[r] = v.lut[vwid + ay[r]];
                 }
 #pragma unroll
                 for (int r = 0; r < ROWS; r++)
@@ -1204,7 +1209,7 @@ __global__ void __launch_bounds__(TW_THREADS) timewarp_rowsum_kernel(const __gri
         float z[TW_LOADS]; // past the row: 0, which changes nothing
 #pragma unroll
         for (int i = 0; i < TW_LOADS; i++)
-            z[i] = x0 + i * TW_THREADS < v.w ? __ldg(row + x0 + i * TW_THREADS) : 0.0f;
+            z[i] = x0 + i * TW_THREADS < v.w ? row[x0 + i * TW_THREADS] : 0.0f;
 #pragma unroll
         for (int i = 0; i < TW_LOADS; i++)
         {
@@ -1240,7 +1245,7 @@ __global__ void __launch_bounds__(TW_THREADS) timewarp_rowsum_kernel(const __gri
     {
         if (warp != 0u)
             return;
-        acc = warp_sum_in_order(0.0, v.w, [&](uint32_t x) { return (double)__ldg(row + x); });
+        acc = warp_sum_in_order(0.0, v.w, [&](uint32_t x) { return (double)row[x]; });
         zmax = e_min = 0u;
     }
     else if (e_min >= 64u && sums_exact(n * n * 64.0f, zmax, e_min)) // (from 2^-63 on no rounding error is flushed to zero)
@@ -1261,7 +1266,7 @@ __global__ void __launch_bounds__(TW_THREADS) timewarp_rowsum_kernel(const __gri
     else
     {
         for (uint32_t x = threadIdx.x; x < v.w; x += TW_THREADS)
-            acc = __dadd_rn(acc, (double)__ldg(row + x));
+            acc = __dadd_rn(acc, (double)row[x]);
         tw_block_reduce(acc, zmax, e_min); // (the largest and smallest as before)
     }
     if (threadIdx.x == 0u)
@@ -1347,7 +1352,7 @@ __device__ __forceinline__ bool timewarp_pixel(const float *cam_ivp, const DevVi
     }
     pix.x = min(max(pix.x, 0), (int)src->w - 1);
     pix.y = min(max(pix.y, 0), (int)src->h - 1);
-    color = __ldg(src->color + ((uint32_t)pix.y * src->w + (uint32_t)pix.x));
+    color = src->color[(uint32_t)pix.y * src->w + (uint32_t)pix.x];
     return true;
 }
 
@@ -1399,7 +1404,7 @@ __global__ void __launch_bounds__(256) timewarp_kernel(const __grid_constant__ F
 __device__ __forceinline__ float unity_depth_to_z(float d) { return xsub(xmul(2.0f, xsub(1.0f, d)), 1.0f); }
 
 template <bool VEC>
-__global__ void depth_to_z_kernel(float *__restrict__ z, size_t n)
+__global__ void depth_to_z_kernel(float *z, size_t n)
 {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     if (!VEC)
@@ -1426,7 +1431,7 @@ __global__ void depth_to_z_kernel(float *__restrict__ z, size_t n)
 // Packed RGB8 -> RGBA8 with alpha 255.  VEC (src 4-byte and dst 16-byte aligned): a thread
 // turns 3 source words (4 pixels, byte 0 = R of the first) into one 16-byte store.
 template <bool VEC>
-__global__ void rgb8_to_rgba8_kernel(uint32_t *__restrict__ dst, const uint8_t *__restrict__ src, size_t n)
+__global__ void rgb8_to_rgba8_kernel(uint32_t *dst, const uint8_t *src, size_t n)
 {
     dependents_may_launch();
     wait_for_prerequisites();
@@ -1439,7 +1444,7 @@ __global__ void rgb8_to_rgba8_kernel(uint32_t *__restrict__ dst, const uint8_t *
         const uint32_t *s32 = reinterpret_cast<const uint32_t *>(src);
         for (size_t g = t; g < groups; g += stride)
         {
-            const uint32_t w0 = __ldg(s32 + 3 * g), w1 = __ldg(s32 + 3 * g + 1), w2 = __ldg(s32 + 3 * g + 2);
+            const uint32_t w0 = s32[3 * g], w1 = s32[3 * g + 1], w2 = s32[3 * g + 2];
             uint4 o;
             o.x = (w0 & 0xffffffu) | 0xff000000u;
             o.y = (w0 >> 24) | ((w1 & 0xffffu) << 8) | 0xff000000u;
@@ -1449,20 +1454,19 @@ __global__ void rgb8_to_rgba8_kernel(uint32_t *__restrict__ dst, const uint8_t *
         }
     }
     for (size_t i = groups * 4 + t; i < n; i += stride)
-        dst[i] = (uint32_t)__ldg(src + 3 * i) | (uint32_t)__ldg(src + 3 * i + 1) << 8 | (uint32_t)__ldg(src + 3 * i + 2) << 16 | 0xff000000u;
+        dst[i] = (uint32_t)src[3 * i] | (uint32_t)src[3 * i + 1] << 8 | (uint32_t)src[3 * i + 2] << 16 | 0xff000000u;
 }
 
 // Sparse shadow entries -> the three RGBA8 shadow images (zeroed before): one thread per
 // entry {pixel index, info RGB, A RGB, B RGB, pad} (16 bytes).
-__global__ void unpack_shadows_kernel(uint32_t *__restrict__ info, uint32_t *__restrict__ a, uint32_t *__restrict__ b, size_t n_pixels,
-                                      const uint4 *__restrict__ entries, size_t n_entries)
+__global__ void unpack_shadows_kernel(uint32_t *info, uint32_t *a, uint32_t *b, size_t n_pixels, const uint4 *entries, size_t n_entries)
 {
     dependents_may_launch();
     wait_for_prerequisites();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n_entries; e += stride)
     {
-        const uint4 v = __ldg(entries + e);
+        const uint4 v = entries[e];
         if (v.x >= n_pixels)
             continue;
         // bytes 4..15: info R G B, A R G B, B R G B, pad (little-endian words y, z, w)
@@ -1473,15 +1477,14 @@ __global__ void unpack_shadows_kernel(uint32_t *__restrict__ info, uint32_t *__r
 }
 
 // The pixels of sparse shadow entries <- 0 in the three shadow images.
-__global__ void clear_shadows_kernel(uint32_t *__restrict__ info, uint32_t *__restrict__ a, uint32_t *__restrict__ b, size_t n_pixels,
-                                     const uint4 *__restrict__ entries, size_t n_entries)
+__global__ void clear_shadows_kernel(uint32_t *info, uint32_t *a, uint32_t *b, size_t n_pixels, const uint4 *entries, size_t n_entries)
 {
     dependents_may_launch();
     wait_for_prerequisites();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n_entries; e += stride)
     {
-        const uint32_t i = __ldg(&entries[e].x);
+        const uint32_t i = entries[e].x;
         if (i < n_pixels)
             info[i] = a[i] = b[i] = 0u;
     }

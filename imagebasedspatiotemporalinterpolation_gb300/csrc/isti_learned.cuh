@@ -81,8 +81,8 @@ __device__ __forceinline__ float4 learned_camflow(const LearnedParams &p, int v,
 {
     const DevView &dv = p.fp.v[v];
     const float4 pc = learned_project(p, v, k, sx, sy);
-    const float z = __ldg(dv.z + (sy * dv.w + sx));
-    return make_float4(xsub(pc.x, __ldg(dv.lut + sx)), xsub(pc.y, __ldg(dv.lut + dv.w + sy)), xsub(pc.z, z), z);
+    const float z = dv.z[sy * dv.w + sx];
+    return make_float4(xsub(pc.x, dv.lut[sx]), xsub(pc.y, dv.lut[dv.w + sy]), xsub(pc.z, z), z);
 }
 
 // ---- per keyframe pair ----
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(256, 7) keyframe_kernel(const __grid_constant_
     if (x >= dv.w || y >= dv.h)
         return;
     const uint32_t idx = y * dv.w + x;
-    const float z_from = __ldg(dv.z + idx);
+    const float z_from = dv.z[idx];
     const float4 om = load_motion(dv, idx);
     const float2 pcs = pixel2cs(x, y, dv.w, dv.h);
     const float4 cs_from = make_float4(pcs.x, pcs.y, z_from, 1.0f);
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(256) input_kernel(const __grid_constant__ Lear
     {
         const float sx = 0.125f * (float)a.w, sy = 0.125f * (float)a.h; // NDC -> quarter pixels
         const uint32_t i = y * a.w + x;
-        const float za = __ldg(a.z + i), zb = __ldg(b.z + i);
+        const float za = a.z[i], zb = b.z[i];
         f[0] = 10.0f * (1.0f - za); // ~ 2 near / depth: inverse depth
         f[1] = 10.0f * (1.0f - zb);
         const float4 ma = load_motion(a, i), mb = load_motion(b, i);
@@ -199,11 +199,11 @@ __device__ __forceinline__ DirRes learned_dir(const LearnedParams &p, int v, int
         }
     }
     const float4 m = learned_camflow(p, v, k, sx, sy);
-    const float vis = __ldg(dv.full_ff + (sy * dv.w + sx)).w;
+    const float vis = dv.full_ff[sy * dv.w + sx].w;
     DirRes d;
     d.depth = z_to_depth(xadd(m.w, m.z));
-    const float ex = xmul(xsub(xadd(__ldg(dv.lut + sx), m.x), pcx), esx);
-    const float ey = xmul(xsub(xadd(__ldg(dv.lut + dv.w + sy), m.y), pcy), esy);
+    const float ex = xmul(xsub(xadd(dv.lut[sx], m.x), pcx), esx);
+    const float ey = xmul(xsub(xadd(dv.lut[dv.w + sy], m.y), pcy), esy);
     d.error_vis = pack_error_vis<SQ>(xadd(xmul(ex, ex), xmul(ey, ey)), vis > 0.0f);
     d.src = (sx << 16) | sy;
     return d;
@@ -240,7 +240,7 @@ __device__ __forceinline__ void learned_step_approx(const LearnedParams &p, int 
     const float cx = fmaf(m[0], x, fmaf(m[4], y, fmaf(m[8], z, m[12])));
     const float cy = fmaf(m[1], x, fmaf(m[5], y, fmaf(m[9], z, m[13])));
     const float cw = fmaf(m[3], x, fmaf(m[7], y, fmaf(m[11], z, m[15])));
-    const float mx = __fdividef(cx, cw) - __ldg(dv.lut + sx), my = __fdividef(cy, cw) - __ldg(dv.lut + dv.w + sy);
+    const float mx = __fdividef(cx, cw) - dv.lut[sx], my = __fdividef(cy, cw) - dv.lut[dv.w + sy];
     const int2 t = cs2pixel(qx - mx, qy - my, dv.w, dv.h);
     if (in_range(t, dv.w, dv.h))
     {
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(LT_W *LT_H, 6) learned_kernel(const __grid_con
     const uint32_t x = blockIdx.x * LT_W + threadIdx.x, y = blockIdx.y * LT_H + threadIdx.y;
     const bool inb = x < p.fp.out_w && y < p.fp.out_h;
     const DevView &a = p.fp.v[0], &b = p.fp.v[1];
-    const float qx = inb ? __ldg(a.lut + x) : 0.0f, qy = inb ? __ldg(a.lut + a.w + y) : 0.0f; // pixel2CS of the output pixel
+    const float qx = inb ? a.lut[x] : 0.0f, qy = inb ? a.lut[a.w + y] : 0.0f; // pixel2CS of the output pixel
     const uint32_t qxi = min(x / 4, (uint32_t)p.wq - 1), qyi = min(y / 4, (uint32_t)p.hq - 1);
     for (int k = 0; k < p.fp.n_frames; k++)
     {
@@ -311,8 +311,8 @@ __global__ void __launch_bounds__(LT_W *LT_H, 6) learned_kernel(const __grid_con
             {
                 // sources on the far plane (z = 1: sky) in both keyframes are left to the temporal
                 // hole filling, as the plain method mostly leaves them
-                const float z0 = __ldg(a.z + (sy[0] * a.w + sx[0]));
-                const float z1 = __ldg(b.z + (sy[1] * b.w + sx[1]));
+                const float z0 = a.z[sy[0] * a.w + sx[0]];
+                const float z1 = b.z[sy[1] * b.w + sx[1]];
                 fail = !(z0 >= 1.0f && z1 >= 1.0f);
             }
             else
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(LT_W *LT_H) fallback_reproj_kernel(const __gri
         tile_of(p, p.tile_list[i], k, x, y);
         if (x >= p.fp.out_w || y >= p.fp.out_h)
             continue;
-        const float qx = __ldg(a.lut + x), qy = __ldg(a.lut + a.w + y);
+        const float qx = a.lut[x], qy = a.lut[a.w + y];
         DirRes d[2];
 #pragma unroll
         for (int v = 0; v < 2; v++)
@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(256) label_kernel(const __grid_constant__ Fram
     if (x < p.out_w && y < p.out_h)
     {
         const DevView &a = p.v[0];
-        const float qxc = __ldg(a.lut + x), qyc = __ldg(a.lut + a.w + y);
+        const float qxc = a.lut[x], qyc = a.lut[a.w + y];
         for (int v = 0; v < 2; v++)
         {
             const DevView &dv = p.v[v];
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(256) label_kernel(const __grid_constant__ Fram
             const float2 *cam = dv.cam_xy + k * p.cam_stride;
             for (int i = 0; i < 3; i++)
             {
-                const float2 m = __ldg(cam + (sy * dv.w + sx));
+                const float2 m = cam[sy * dv.w + sx];
                 const int2 t = cs2pixel(xsub(qxc, m.x), xsub(qyc, m.y), dv.w, dv.h);
                 if (in_range(t, dv.w, dv.h))
                 {
@@ -604,9 +604,9 @@ __global__ void __launch_bounds__(256) label_kernel(const __grid_constant__ Fram
                     sy = (uint32_t)t.y;
                 }
             }
-            const float2 m = __ldg(cam + (sy * dv.w + sx));
-            const float ex = xmul(xsub(xadd(__ldg(dv.lut + sx), m.x), qxc), dv.err_sx);
-            const float ey = xmul(xsub(xadd(__ldg(dv.lut + dv.w + sy), m.y), qyc), dv.err_sy);
+            const float2 m = cam[sy * dv.w + sx];
+            const float ex = xmul(xsub(xadd(dv.lut[sx], m.x), qxc), dv.err_sx);
+            const float ey = xmul(xsub(xadd(dv.lut[dv.w + sy], m.y), qyc), dv.err_sy);
             if (err_below<true>(err_pack<true>(xadd(xmul(ex, ex), xmul(ey, ey))), ERR_EPS_1_FULL_RES<true>))
             {
                 out[2 * v] = 0.25f * ((float)sx - (float)x);

@@ -64,8 +64,8 @@ __device__ __forceinline__ float byte_to_unit(uint32_t v)
 // 9 for the single plane) are odd, so their 16-byte accesses meet no bank conflict.
 // 1080p: 112 -> 66 us (one output per thread and pass, 32x16 tiles, scalar operations before).
 constexpr int Q_PITCH = TW + 2, Q_PITCH1 = TW + 4;
-__global__ void __launch_bounds__(Q_THREADS) quality_tile_kernel(const uint32_t *__restrict__ a, const uint32_t *__restrict__ b, int w,
-                                                                 int h, double *__restrict__ partials, const __grid_constant__ Gauss gw)
+__global__ void __launch_bounds__(Q_THREADS) quality_tile_kernel(const uint32_t *a, const uint32_t *b, int w, int h, double *partials,
+                                                                 const __grid_constant__ Gauss gw)
 {
     __shared__ __align__(16) float2 xy[SH * SW];
     __shared__ __align__(16) float2 hm[SH * Q_PITCH], hq[SH * Q_PITCH]; // horizontally filtered (x, y) and (x^2, y^2)
@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(Q_THREADS) quality_tile_kernel(const uint32_t 
         if (e < SH * SW && gx >= 0 && gx < w && gy >= 0 && gy < h)
         {
             const size_t idx = (size_t)gy * w + gx;
-            pa[i] = __ldg(a + idx);
-            pb[i] = __ldg(b + idx);
+            pa[i] = a[idx];
+            pb[i] = b[idx];
             if (xx >= R && xx < R + TW && yy >= R && yy < R + TH)
             {
                 const uint32_t d = __vabsdiffu4(pa[i], pb[i]) & 0xffffffu;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(Q_THREADS) quality_tile_kernel(const uint32_t 
     }
 }
 
-__global__ void __launch_bounds__(THREADS) quality_final_kernel(const double *__restrict__ partials, size_t n_blocks,
+__global__ void __launch_bounds__(THREADS) quality_final_kernel(const double *partials, size_t n_blocks,
                                                                 double n_values, isti_quality *out)
 {
     __shared__ double ss[THREADS], sq[THREADS];
@@ -454,9 +454,8 @@ __device__ __forceinline__ void flip_columns(const FlipFilters &f, const float2 
 // 21-tap tile takes a third of an SM.  1080p: 510 us with the images in turn, one output per thread
 // and pass and a power per staged colour value; 238 with all three planes staged and two tiles per
 // SM; 211 with three tiles, 198 with divisions by constants and roots instead of powers.
-__global__ void __launch_bounds__(THREADS, 3) flip_tile_kernel(const uint32_t *__restrict__ test, const uint32_t *__restrict__ ref, int w,
-                                                               int h, const __grid_constant__ FlipFilters f,
-                                                               double *__restrict__ partials, float *__restrict__ map)
+__global__ void __launch_bounds__(THREADS, 3) flip_tile_kernel(const uint32_t *test, const uint32_t *ref, int w, int h,
+                                                               const __grid_constant__ FlipFilters f, double *partials, float *map)
 {
     extern __shared__ __align__(16) float2 fsm[];
     const FlipTile t(f.r, f.groups);
@@ -485,7 +484,7 @@ __global__ void __launch_bounds__(THREADS, 3) flip_tile_kernel(const uint32_t *_
     {
         const int gx = min(max(x0 + xx - f.r, 0), w - 1), gy = min(max(y0 + yy - f.r, 0), h - 1);
         const size_t idx = (size_t)gy * w + gx;
-        pixels[i] = make_uint2(__ldg(ref + idx), __ldg(test + idx));
+        pixels[i] = make_uint2(ref[idx], test[idx]);
         xx += step_x;
         yy += step_y;
         if (xx >= t.pitch)
@@ -572,7 +571,7 @@ __global__ void __launch_bounds__(THREADS, 3) flip_tile_kernel(const uint32_t *_
     }
 }
 
-__global__ void __launch_bounds__(THREADS) flip_final_kernel(const double *__restrict__ partials, size_t n_blocks, double n_px,
+__global__ void __launch_bounds__(THREADS) flip_final_kernel(const double *partials, size_t n_blocks, double n_px,
                                                              double *out)
 {
     __shared__ double ss[THREADS];
