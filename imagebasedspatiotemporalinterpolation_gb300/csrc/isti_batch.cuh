@@ -74,7 +74,8 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p)
     return v;
 }
 
-template <int SW, int SI, bool MAV, int REGS>
+// HOOK: built with the failure-detection test hook (FrameParams::withhold_block, pair 0)
+template <int SW, int SI, bool MAV, int REGS, bool HOOK = false>
 __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchParams bp)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -100,7 +101,7 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
         ctrl[5] = 0u;
     }
     __syncthreads();
-    int round = 0;        // TMA rounds of this warp's barrier (its phase carries across units)
+    int round = 0;        // TMA rounds of this warp's barrier (its phase carries across units; -1: out of use)
     uint32_t slot = 0;    // ctrl word holding the current ticket
     // the segment of the current ticket; a block's tickets only grow, so the search resumes
     // where the previous unit's ended
@@ -124,7 +125,9 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
             status_seen = *(volatile int32_t *)bp.status;
         }
         // once a wait has given up (status word set) the remaining units only count themselves
-        // done: the failed block's TMA barrier is out of step, and the call's outputs are void
+        // done: the call's outputs are void.  The word was read while the unit before this one ran, so
+        // the unit after one that gave up still runs here: reproj_block announces nothing on a barrier
+        // that is out of step (`round`) and leaves again (ctrl[5])
         const bool failed = ctrl[2 + slot] != 0;
         const uint32_t old_pair = seg_pair;
         while (t >= seg_end)
@@ -194,7 +197,7 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
             else
             {
                 const uint32_t bx = u % bpair.reproj_gx, by = u / bpair.reproj_gx;
-                reproj_block<SW, SI, MAV, REGS>(p, bpair.maps, bx, by, u, region, bars, round, *reinterpret_cast<volatile uint32_t *>(ctrl + 5));
+                reproj_block<SW, SI, MAV, REGS, 0, HOOK>(p, bpair.maps, bx, by, u, region, bars, round, *reinterpret_cast<volatile uint32_t *>(ctrl + 5));
             }
         }
         if (helper)

@@ -848,7 +848,9 @@ __host__ __device__ __forceinline__ void window_keys(const unsigned long long *t
 // threads: the body of reproj_kernel, also run as a work unit of batch_kernel.  `maps`: the
 // views' key-tile tensor maps; `bars`: the warps' TMA completion barriers, initialised once per
 // thread block; `round`: TMA rounds this warp's barrier has completed so far (its phase carries
-// over from unit to unit, also across units whose tiles came by plain loads); `aborted`: a
+// over from unit to unit, also across units whose tiles came by plain loads), or -1 once a wait of
+// this warp gave up: the barrier's phase did not complete then, and another arrival would overrun
+// its count, so the warp announces nothing more, in this unit or a later one; `aborted`: a
 // shared word, 0 when the block starts, that a warp whose wait for a key tile gave up sets to 1;
 // `block_id`: the index the test hook `withhold_block` refers to, compiled in only where HOOK is
 // set.  Every thread returns together (early exits are block-uniform or come after the last
@@ -895,7 +897,7 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
             const uint32_t y0 = yb + (uint32_t)rp * ROWS;
             tma_load_3d(tg, &maps[vw], xs, (int)(v.sy == 1 ? y0 : y0 / v.sy) - SW, k, bar);
         };
-        if (p.use_tma && lane == 0)
+        if (p.use_tma && round >= 0 && lane == 0)
             fetch(0, g0);
         // pixel2CS of the output pixels in the main view (the search target) and in this view (the error)
         const DevView &v0 = p.v[0];
@@ -924,13 +926,14 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                 const int k = g0 + j, u = j * np + rp;
                 if (p.use_tma)
                 {
-                    // A warp whose copy did not arrive reads nothing more, starts no further copy (an
-                    // arrival on a barrier whose phase did not complete would overrun its count) and
-                    // marks the block, which then leaves after the barrier that ends phase 1, writing
-                    // nothing (the mark is written before that barrier and read after it, by every thread).
-                    arrived = __all_sync(0xffffffffu, mbar_wait_bounded(bar, (uint32_t)(round & 1), p.status, p.wait_limit));
+                    // A warp whose copy did not arrive reads nothing more, starts no further copy (see
+                    // `round`) and marks the block, which then leaves after the barrier that ends phase 1,
+                    // writing nothing of this group (the mark is written before that barrier and read
+                    // after it, by every thread).
+                    arrived = round >= 0 && __all_sync(0xffffffffu, mbar_wait_bounded(bar, (uint32_t)(round & 1), p.status, p.wait_limit));
                     if (!arrived)
                     {
+                        round = -1;
                         aborted = 1u;
                         break;
                     }

@@ -719,10 +719,10 @@ isti_status isti_renderer_view_depth(const isti_renderer *r, int32_t view, const
 
 namespace
 {
-template <int SW, int SI, bool MAV, int REGS>
+template <int SW, int SI, bool MAV, int REGS, bool HOOK = false>
 cudaError_t launch_pairs_kernel(const isti::BatchParams &bp, size_t smem, unsigned threads_y, cudaStream_t stream)
 {
-    auto kernel = isti::batch_kernel<SW, SI, MAV, REGS>;
+    auto kernel = isti::batch_kernel<SW, SI, MAV, REGS, HOOK>;
     static std::mutex mu;
     static size_t set_bytes[64] = {};
     int dev = 0;
@@ -761,8 +761,11 @@ cudaError_t launch_pairs_kernel(const isti::BatchParams &bp, size_t smem, unsign
     return cudaLaunchKernelEx(&cfg, kernel, bp);
 }
 
-cudaError_t launch_pairs_mode(int mode, int regs, const isti::BatchParams &bp, size_t smem, unsigned threads_y, cudaStream_t stream)
+// withheld: the failure-detection test hook is armed (built for mode 0 with the main camera only)
+cudaError_t launch_pairs_mode(int mode, int regs, const isti::BatchParams &bp, size_t smem, unsigned threads_y, cudaStream_t stream, bool withheld)
 {
+    if (withheld)
+        return launch_pairs_kernel<1, 3, false, isti::REPROJ_REGS, true>(bp, smem, threads_y, stream);
     switch (mode)
     {
     case ISTI_MODE_OURS:
@@ -975,6 +978,12 @@ extern "C" isti_status isti_render_pairs(isti_renderer *r, int32_t n_pairs, cons
         bpair.reproj_gx = (p.out_w + 31) / 32;
         const uint32_t block_rows = (uint32_t)(isti::ROWS * p.row_pairs);
         bpair.reproj_units = bpair.reproj_gx * ((p.out_h + block_rows - 1) / block_rows);
+        // the test hook: a tile of pair 0
+        if (i == 0 && r->withhold_x >= 0 && r->withhold_y >= 0 && (uint32_t)r->withhold_x < p.out_w && (uint32_t)r->withhold_y < p.out_h &&
+            mode == ISTI_MODE_OURS && regs == isti::REPROJ_REGS)
+            p.withhold_block = (int32_t)((uint32_t)r->withhold_y / block_rows * bpair.reproj_gx + (uint32_t)r->withhold_x / 32u);
+        if (hfp[0].withhold_block >= 0)
+            p.wait_limit = r->wait_limit;
     }
     // the queue: I0 S0 I1 S1 R0 I2 S2 R1 ... R(n-1)
     int ns = 0;
@@ -1014,7 +1023,7 @@ extern "C" isti_status isti_render_pairs(isti_renderer *r, int32_t n_pairs, cons
             e = cudaEventRecord(r->multi_copied, stream);
     }
     if (e == cudaSuccess)
-        e = launch_pairs_mode(mode, regs, bp, smem, (unsigned)nv, stream);
+        e = launch_pairs_mode(mode, regs, bp, smem, (unsigned)nv, stream, hfp[0].withhold_block >= 0);
     if (e != cudaSuccess)
         return cuda_fail(e, "isti_render_pairs launch");
     r->last = hfp[0];

@@ -243,7 +243,9 @@ isti_status isti_renderer_set_arithmetic(isti_renderer *r, int32_t arith);
  * `wait_limit` polls (0: the default limit, seconds at most): the block sets
  * ISTI_ERR_TIMEOUT in the device status word and leaves without reading a tile or
  * writing a pixel; every other block renders normally.  Only renders that fetch
- * their tiles by TMA have such a wait.  x < 0 switches the hook off. */
+ * their tiles by TMA have such a wait.  isti_render_pairs' persistent launch has
+ * the hook for its first pair in mode 0 without aux cameras (the call's outputs are
+ * then void).  x < 0 switches the hook off. */
 isti_status isti_renderer_test_withhold_tile(isti_renderer *r, int32_t x, int32_t y, uint32_t wait_limit);
 
 /* Failure-detection test hook for isti_render_pairs (no counterpart in the reference).
