@@ -129,7 +129,7 @@ struct EpilogueTable
 {
     float bias[CONV_MAX_COUT];
     float head[CONV_HEAD * CONV_MAX_COUT], head_bias[CONV_HEAD];
-    __device__ __forceinline__ void fill(const ConvParams &p) // whole block; parameters only, no previous kernel's output
+    __device__ __forceinline__ void fill(const ConvParams &p) // whole block; complete before the kernel started (forward in isti_flownet.cu)
     {
         for (int i = threadIdx.x; i < p.cout; i += blockDim.x)
             bias[i] = p.bias ? __ldg(p.bias + i) : 0.0f;
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     {
         const uint32_t leader = elect_one();
         mbar_expect_tx_if(leader, wbar, w_bytes);
-        for (uint32_t o = 0; o < w_bytes; o += 32768u) // pieces of at most 32 KiB (weights: no previous kernel writes them)
+        for (uint32_t o = 0; o < w_bytes; o += 32768u) // pieces of at most 32 KiB (the weights are complete, forward in isti_flownet.cu)
             bulk_load(leader, smem_u32(wsm) + o, reinterpret_cast<const uint8_t *>(p.wpack) + o, min(32768u, w_bytes - o), wbar);
         griddep_wait(); // the previous layer's output is complete (every activation load below is later)
         fence_proxy_async_global();

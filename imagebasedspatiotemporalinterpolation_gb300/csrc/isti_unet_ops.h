@@ -27,7 +27,8 @@ struct ConvHead
 constexpr int IN_PLANES = 1, OUT_PLANES = 2;
 
 // pdl: launch as a programmatic dependent of the previous kernel in `stream` (it prepares
-// while that kernel finishes; see griddep_wait in isti_tc.cuh).  head: fuse that head into
+// while that kernel finishes; see griddep_wait in isti_tc.cuh).  It then reads wpack, bias and the
+// head before it waits: only behind a kernel that was itself launched after they were complete.  head: fuse that head into
 // the epilogue where the row-tile kernel runs the layer (then `out` is not written and
 // *head_fused is set); otherwise the layer runs as usual and *head_fused is cleared.
 isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, const void *wpack, const float *bias, const void *mask, int relu,

@@ -140,3 +140,41 @@ def test_metrics_right_behind_the_render_they_measure(cuda):
         assert m.tolist() == [w[0]["mse"], w[0]["psnr"], w[0]["ssim"]]
         assert f == w[1]
     r.close()
+
+
+@pytest.mark.gpu
+def test_network_right_behind_its_weights(cuda):
+    """Training steps, each followed at once by an inference and a learned render with the new weights (a
+    dependent launch in between), against the same steps waited for one by one."""
+    import torch
+    seq, frame, shape = _scenes(())[0]
+    clients = [seq.client(0, b) for b in (1, 2)]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(2, 48, 136, 16, generator=g, device="cuda").bfloat16()
+    label = torch.randn(2, 48, 136, 4, generator=g, device="cuda")
+
+    def steps(waits):
+        net, r, got = FlowNet(seed=9), Renderer(), []
+        wait = torch.cuda.synchronize if waits else lambda: None
+        wait()
+        for _ in range(8):
+            net.backward(x, label)
+            wait()
+            net.adam(1e-2)
+            wait()
+            flow = net.forward(x)
+            wait()
+            net.adam(1e-2)
+            wait()
+            outs = [torch.full(shape, 5, dtype=torch.uint8, device="cuda") for _ in clients]
+            wait()
+            r.render_learned(outs, clients, frame, net, iterations=1)
+            wait()
+            got += [flow, *outs]
+        torch.cuda.synchronize()
+        r.close()
+        net.close()
+        return got
+
+    for i, (a, b) in enumerate(zip(steps(False), steps(True))):
+        assert torch.equal(a, b), f"output {i}"
