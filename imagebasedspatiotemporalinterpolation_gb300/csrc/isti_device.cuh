@@ -187,6 +187,25 @@ __host__ __device__ __forceinline__ float divided_by(float x)
     return fmaf(fmaf(-q, (float)D, x), r, q);
 }
 
+// Sum of up to 32 floats of magnitude below 4 without the few FP64 units (two lanes a clock), rounded once,
+// to double: each value is split, exactly, into multiples of 2^-20 and of 2^-43 -- the mantissa bits of its sum
+// with 1.5 times a power of two -- which are added as integers, and what is left, at most 2^-44, whose float
+// sum is exact too unless values below 2^-40 are in it.
+struct ExactSum
+{
+    int32_t hi = 0, lo = 0;
+    float rest = 0.0f;
+    __host__ __device__ __forceinline__ void add(float v)
+    {
+        constexpr float A = 0x1.8p3f, B = 0x1.8p-20f;
+        const float a = v + A, r = v - (a - A), b = r + B;
+        hi += __builtin_bit_cast(int32_t, a) - __builtin_bit_cast(int32_t, A);
+        lo += __builtin_bit_cast(int32_t, b) - __builtin_bit_cast(int32_t, B);
+        rest += r - (b - B);
+    }
+    __host__ __device__ __forceinline__ double value() const { return ((double)hi * 0x1p-20 + (double)lo * 0x1p-43) + (double)rest; }
+};
+
 // Byte c of a packed colour as a float, exact: the byte becomes the low mantissa bits of 2^23
 // (a byte permute and an addition; the integer conversion runs on a slower unit).
 __device__ __forceinline__ float byte_to_float(uint32_t color, int c)

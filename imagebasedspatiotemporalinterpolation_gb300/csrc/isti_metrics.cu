@@ -37,20 +37,6 @@ struct Gauss
     float2 g[WIN]; // each tap twice: the packed operations take a pair
 };
 
-// Running sum of floats as an unevaluated pair: the rounding error of every addition is kept
-// (Knuth's two-sum), so the pair is as exact as a double sum without the few FP64 units.
-struct PairSum
-{
-    float hi = 0.0f, lo = 0.0f;
-    __device__ __forceinline__ void add(float v)
-    {
-        const float s = __fadd_rn(hi, v), t = __fsub_rn(s, hi);
-        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(v, t)));
-        hi = s;
-    }
-    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
-};
-
 // v / 255 for an integer v in 0..255, correctly rounded
 __device__ __forceinline__ float byte_to_unit(uint32_t v)
 {
@@ -96,7 +82,7 @@ __global__ void __launch_bounds__(Q_THREADS) quality_tile_kernel(const uint32_t 
             }
         }
     }
-    PairSum ssim;
+    isti::ExactSum ssim;
 #pragma unroll 1
     for (int c = 0; c < 3; c++)
     {
@@ -173,7 +159,7 @@ __global__ void __launch_bounds__(Q_THREADS) quality_tile_kernel(const uint32_t 
             const float v1 = q[j].x - m1s, v2 = q[j].y - m2s, v12 = x12[j] - m12;
             const float num = (2.0f * m12 + C1) * (2.0f * v12 + C2);
             const float den = (m1s + m2s + C1) * (v1 + v2 + C2);
-            ssim.add(__fdiv_rn(num, den));
+            ssim.add(__fdiv_rn(num, den)); // (about -1..1)
         }
         // the next channel's staging writes xy, which every thread has read before the last
         // barrier; its horizontal pass writes hm, hq and hc after the next one
@@ -527,7 +513,7 @@ __global__ void __launch_bounds__(THREADS, 3) flip_tile_kernel(const uint32_t *t
     flip_columns<1, 1>(f, {h1}, {0}, {GAUSS}, {0}, ex);
     flip_columns<1, 1>(f, {h2}, {0}, {GAUSS}, {0}, fx);
 
-    PairSum sum_v;
+    isti::ExactSum sum_v;
     const float pccmax = FLIP_PC * f.cmax;
     const int lane = tid & 31, warp = tid >> 5;
 #pragma unroll
@@ -551,7 +537,7 @@ __global__ void __launch_bounds__(THREADS, 3) flip_tile_kernel(const uint32_t *t
         def = fmaxf(def, FLIP_EPS);
         def = sqrtf(0.70710678f * def); // to the power qf = 1/2
         const float v = powf(dec, 1.0f - def);
-        sum_v.add(v);
+        sum_v.add(v); // (about 0..1)
         if (map)
             map[(size_t)gyy * w + gx] = v;
     }
