@@ -14,6 +14,7 @@
 //   s1 = up2(conv1x1 64->32 (d2)) + e1     d1 = relu(conv3x3 32->32)(s1)
 //   flow = conv1x1 32->4 (d1)              [H,W,4] f32
 // 10 tensor-core layers + the head: 339,268 parameters.
+#include "isti_pdl.cuh"
 #include "isti_tc.cuh"
 #include "isti_unet.h"
 #include "isti_unet_ops.h"
@@ -55,7 +56,7 @@ constexpr int IN_CH = 16;
 
 isti_status cuda_fail(cudaError_t e, const char *what) { return isti::set_error(ISTI_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)); }
 
-// ---- elementwise kernels on NHWC bf16, 8 channels (16 bytes) per thread ----
+// ---- elementwise kernels on bf16, 8 channels (16 bytes) at a time ----
 
 __device__ __forceinline__ void unpack8(uint4 u, float (&f)[8])
 {
@@ -110,8 +111,8 @@ __device__ __forceinline__ void add8(float (&acc)[8], const bf16 *x, size_t grou
 // r = scale * the sum of x over 2x2 blocks: average pooling (0.25), gradient of nearest upsampling (1)
 __global__ void __launch_bounds__(EW_X * EW_Y) blocksum_kernel(const bf16 *x, uint32_t planes, uint32_t ho, uint32_t wo, float scale, bf16 *r)
 {
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait();
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites();
     for_each_block(planes, ho, wo, [&](size_t half, size_t full, size_t row) {
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         add8(acc, x, full);
@@ -128,8 +129,8 @@ __global__ void __launch_bounds__(EW_X * EW_Y) blocksum_kernel(const bf16 *x, ui
 // s[h, w] = a[h/2, w/2] (nearest upsampling) + b[h, w]
 __global__ void __launch_bounds__(EW_X * EW_Y) upadd_kernel(const bf16 *a, const bf16 *b, uint32_t planes, uint32_t ho, uint32_t wo, bf16 *s)
 {
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait();
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites();
     for_each_block(planes, ho, wo, [&](size_t half, size_t full, size_t row) {
         const uint4 ua = reinterpret_cast<const uint4 *>(a)[half];
         uint4 ub[4];
@@ -156,8 +157,8 @@ __global__ void __launch_bounds__(EW_X * EW_Y) upadd_kernel(const bf16 *a, const
 __global__ void __launch_bounds__(EW_X * EW_Y) poolback_kernel(const bf16 *gskip, const bf16 *gq, const bf16 *act, uint32_t planes, uint32_t ho,
                                                                uint32_t wo, bf16 *ge)
 {
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait();
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites();
     for_each_block(planes, ho, wo, [&](size_t half, size_t full, size_t row) {
         uint4 us[4], ua[4];
 #pragma unroll
@@ -197,8 +198,8 @@ __global__ void head_kernel(const bf16 *d1, size_t npix, size_t image, const flo
         sw[i] = hw[i];
     if (threadIdx.x < HEAD_COUT)
         sw[HEAD_COUT * HEAD_CIN + threadIdx.x] = hb[threadIdx.x];
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait(); // the weights above are no previous kernel's output; d1 is
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites(); // the weights above are no previous kernel's output; d1 is
     __syncthreads();
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (size_t)gridDim.x * blockDim.x)
     {
@@ -257,8 +258,8 @@ __global__ void __launch_bounds__(HEAD_TILE, 2) head_back_kernel(const bf16 *d1,
         sw[i] = hw[i];
     if (threadIdx.x < HEAD_COUT)
         sw[HEAD_COUT * HEAD_CIN + threadIdx.x] = hb[threadIdx.x];
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait(); // the weights above are no previous kernel's output; d1 is
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites(); // the weights above are no previous kernel's output; d1 is
     __syncthreads();
     const bool label_vec = (reinterpret_cast<uintptr_t>(label) & 15u) == 0;
     const int q = threadIdx.x / HEAD_LANES, lane = threadIdx.x % HEAD_LANES; // second step: channel group, pixel lane
@@ -384,8 +385,8 @@ constexpr int SUM_PARTS = 8;
 __global__ void __launch_bounds__(32 * SUM_PARTS) head_sums_kernel(const float *partial, int blocks, float *grads, float *loss)
 {
     __shared__ float part[SUM_PARTS][32];
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait();
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites();
     const int i = blockIdx.x * 32 + threadIdx.x;
     float s = 0.0f;
     if (i < HEAD_VALUES)
@@ -563,7 +564,6 @@ isti_status wgrad(isti_flownet *net, int l, const bf16 *g_out, const bf16 *x, in
 isti_status forward(isti_flownet *net, const bf16 *x0, int n, int h, int w, Buffers &b, float *flow, __half *flow16, cudaStream_t s)
 {
     constexpr bool pdl = true;
-    using isti_unet::launch_kernel;
     const int h2 = h / 2, w2 = w / 2, h4 = h / 4, w4 = w / 4, h8 = h / 8, w8 = w / 8;
     const dim3 blk(EW_X, EW_Y);
     cudaError_t e = cudaSuccess;
@@ -573,22 +573,22 @@ isti_status forward(isti_flownet *net, const bf16 *x0, int n, int h, int w, Buff
         return e == cudaSuccess;
     };
     ISTI_TRY(conv(net, 0, x0, n, h, w, nullptr, b.e1, s));
-    ok(launch_kernel(blocksum_kernel, rows_grid(n * 4 * h2), blk, 0, s, pdl, (const bf16 *)b.e1, (uint32_t)(n * 4), (uint32_t)h2, (uint32_t)w2, 0.25f, b.q1));
+    ok(isti::launch_after(pdl, blocksum_kernel, rows_grid(n * 4 * h2), blk, 0, s, (const bf16 *)b.e1, (uint32_t)(n * 4), (uint32_t)h2, (uint32_t)w2, 0.25f, b.q1));
     ISTI_TRY(conv(net, 1, b.q1, n, h2, w2, nullptr, b.e2, s, pdl));
-    ok(launch_kernel(blocksum_kernel, rows_grid(n * 8 * h4), blk, 0, s, pdl, (const bf16 *)b.e2, (uint32_t)(n * 8), (uint32_t)h4, (uint32_t)w4, 0.25f, b.q2));
+    ok(isti::launch_after(pdl, blocksum_kernel, rows_grid(n * 8 * h4), blk, 0, s, (const bf16 *)b.e2, (uint32_t)(n * 8), (uint32_t)h4, (uint32_t)w4, 0.25f, b.q2));
     ISTI_TRY(conv(net, 2, b.q2, n, h4, w4, nullptr, b.e3, s, pdl));
-    ok(launch_kernel(blocksum_kernel, rows_grid(n * 12 * h8), blk, 0, s, pdl, (const bf16 *)b.e3, (uint32_t)(n * 12), (uint32_t)h8, (uint32_t)w8, 0.25f, b.q3));
+    ok(isti::launch_after(pdl, blocksum_kernel, rows_grid(n * 12 * h8), blk, 0, s, (const bf16 *)b.e3, (uint32_t)(n * 12), (uint32_t)h8, (uint32_t)w8, 0.25f, b.q3));
     ISTI_TRY(conv(net, 3, b.q3, n, h8, w8, nullptr, b.e4, s, pdl));
     ISTI_TRY(conv(net, 4, b.e4, n, h8, w8, nullptr, b.p3, s, pdl));
-    ok(launch_kernel(upadd_kernel, rows_grid(n * 12 * h8), blk, 0, s, pdl, (const bf16 *)b.p3, (const bf16 *)b.e3, (uint32_t)(n * 12), (uint32_t)h8, (uint32_t)w8,
+    ok(isti::launch_after(pdl, upadd_kernel, rows_grid(n * 12 * h8), blk, 0, s, (const bf16 *)b.p3, (const bf16 *)b.e3, (uint32_t)(n * 12), (uint32_t)h8, (uint32_t)w8,
                      b.s3));
     ISTI_TRY(conv(net, 5, b.s3, n, h4, w4, nullptr, b.d3, s, pdl));
     ISTI_TRY(conv(net, 6, b.d3, n, h4, w4, nullptr, b.p2, s, pdl));
-    ok(launch_kernel(upadd_kernel, rows_grid(n * 8 * h4), blk, 0, s, pdl, (const bf16 *)b.p2, (const bf16 *)b.e2, (uint32_t)(n * 8), (uint32_t)h4, (uint32_t)w4,
+    ok(isti::launch_after(pdl, upadd_kernel, rows_grid(n * 8 * h4), blk, 0, s, (const bf16 *)b.p2, (const bf16 *)b.e2, (uint32_t)(n * 8), (uint32_t)h4, (uint32_t)w4,
                      b.s2));
     ISTI_TRY(conv(net, 7, b.s2, n, h2, w2, nullptr, b.d2, s, pdl));
     ISTI_TRY(conv(net, 8, b.d2, n, h2, w2, nullptr, b.p1, s, pdl));
-    ok(launch_kernel(upadd_kernel, rows_grid(n * 4 * h2), blk, 0, s, pdl, (const bf16 *)b.p1, (const bf16 *)b.e1, (uint32_t)(n * 4), (uint32_t)h2, (uint32_t)w2,
+    ok(isti::launch_after(pdl, upadd_kernel, rows_grid(n * 4 * h2), blk, 0, s, (const bf16 *)b.p1, (const bf16 *)b.e1, (uint32_t)(n * 4), (uint32_t)h2, (uint32_t)w2,
                      b.s1));
     // inference: the 1x1 head in d1's epilogue where the row-tile kernel runs d1 (d1 itself is
     // then not stored), else its own kernel
@@ -596,7 +596,7 @@ isti_status forward(isti_flownet *net, const bf16 *x0, int n, int h, int w, Buff
     bool fused = false;
     ISTI_TRY(conv(net, 9, b.s1, n, h, w, nullptr, b.d1, s, pdl, flow || flow16 ? &head : nullptr, &fused));
     if ((flow || flow16) && !fused)
-        ok(launch_kernel(head_kernel, dim3(grid_for((size_t)n * h * w)), dim3(256), 0, s, pdl, (const bf16 *)b.d1, (size_t)n * h * w, (size_t)h * w,
+        ok(isti::launch_after(pdl, head_kernel, dim3(grid_for((size_t)n * h * w)), dim3(256), 0, s, (const bf16 *)b.d1, (size_t)n * h * w, (size_t)h * w,
                          (const float *)(net->params + net->w_off[N_CONV]), (const float *)(net->params + net->b_off[N_CONV]), flow, flow16));
     if (e == cudaSuccess)
         e = cudaGetLastError();
@@ -611,7 +611,7 @@ isti_status backward(isti_flownet *net, const bf16 *x0, const float *label, int 
     cudaError_t e = cudaSuccess;
     // every launch a programmatic dependent of the one before
     auto launch = [&](auto kernel, dim3 grid, dim3 block, auto... args) {
-        const cudaError_t x = isti_unet::launch_kernel(kernel, grid, block, 0, s, true, args...);
+        const cudaError_t x = isti::launch_after(true, kernel, grid, block, 0, s, args...);
         if (e == cudaSuccess)
             e = x;
     };

@@ -30,6 +30,7 @@
 #include "isti.h"
 #include "isti_device.cuh"
 #include "isti_error_cmp.cuh"
+#include "isti_pdl.cuh"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -196,22 +197,6 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
                  "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
                  : "memory");
 }
-
-// ---- programmatic dependent launch ----
-//
-// The kernels of a call depend on each other one after the other, and on what was in the stream
-// before.  Each lets the next one's blocks take SMs as soon as its own blocks have all started
-// (launch_dependents), and waits for the kernel before it to complete, writes visible, before it
-// touches anything (wait; returns at once in an ordinary launch, or after work that is not a
-// kernel).  That hides the launch latency between them: about 3 of 4.8 us per kernel, most of a
-// small frame (640x360: 24.6 -> 19.0 us a call from within the call, 17.2 with the first kernel too).
-//
-// So a kernel may be resident while others still write what it will read, and not only the one
-// before it.  The read-only path (__ldg, const __restrict__ parameters) is for data that nobody
-// writes meanwhile: what earlier kernels or the caller's may have written -- every image, table and
-// intermediate -- is read by ordinary loads.
-__device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- border-addressed loads: zero outside the image (cudaAddressModeBorder) ----
 
@@ -527,9 +512,11 @@ struct DirRes
     uint32_t src;       // source pixel, x << 16 | y
 };
 
-// Squared errors save the square root, but the freer schedule spills at 40 registers, where
-// the roots are faster (1080p, 3 frames, 6 views: 0.537 ms roots, 0.548 squared; 2 views at
-// 48 registers 0.238 -> 0.222 ms squared; 7x7 window at 56, 6 views 1.116 -> 1.092 ms).
+// Squared errors save the square root, but under the cap of 40 registers, which is for many views,
+// the freer schedule spills and the roots are faster (1080p, 3 frames, 6 views: 0.537 ms roots, 0.548
+// squared); under the other caps squares are (2 views 0.238 -> 0.222 ms; 7x7 window, 6 views 1.116 ->
+// 1.092 ms), and their kernels fit into 40 registers without spills where the view count is a constant
+// (reproj_regs).
 template <int REGS>
 constexpr bool SQUARED_ERRORS = !FAST_MATH && REGS != REPROJ_REGS_MANY_VIEWS;
 

@@ -16,24 +16,6 @@
 
 namespace isti
 {
-// Launches a kernel after what was enqueued before it; `early`: as a programmatic dependent launch
-// (the kernel waits by itself), otherwise in full order (around timing events).
-template <class... P, class... A>
-cudaError_t launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A &...args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = early ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // Enqueues the timewarp of one batch (src/renderer.cu:615-629): mean z of the forward
 // keyframe (two kernels), then one kernel over the output pixels.
 cudaError_t launch_timewarp(isti::FrameParams &p, char *base, cudaStream_t stream, cudaEvent_t after_mean, cudaEvent_t after_nothing)

@@ -13,8 +13,7 @@
 #include "isti_metrics.h"
 #include "host/isti_error.hpp"
 #include "isti_device.cuh"
-#include "isti_tc.cuh"
-#include "isti_unet_ops.h"
+#include "isti_pdl.cuh"
 
 #include <cuda_runtime.h>
 
@@ -60,8 +59,8 @@ __global__ void __launch_bounds__(Q_THREADS) quality_tile_kernel(const uint32_t 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
 
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait();
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites();
     uint32_t pa[PER], pb[PER]; // this thread's staged pixels, read once for the three channels
     uint32_t sq = 0;
 #pragma unroll
@@ -198,8 +197,8 @@ __global__ void __launch_bounds__(THREADS) quality_final_kernel(const double *pa
 {
     __shared__ double ss[THREADS], sq[THREADS];
     double s = 0.0, q = 0.0;
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait();
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites();
     for (size_t i = threadIdx.x; i < n_blocks; i += THREADS) // fixed assignment and order: deterministic
     {
         s += partials[2 * i];
@@ -463,8 +462,8 @@ __global__ void __launch_bounds__(THREADS, 3) flip_tile_kernel(const uint32_t *t
     clear_tail(h1);
     if (tid < FlipTile::ROW_SLACK)
         plane[t.plane() + tid] = zero;
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait();
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites();
     const int step_y = THREADS / t.pitch, step_x = THREADS - step_y * t.pitch;
     for (int i = tid, yy = tid / t.pitch, xx = tid - yy * t.pitch; i < t.plane(); i += THREADS)
     {
@@ -562,8 +561,8 @@ __global__ void __launch_bounds__(THREADS) flip_final_kernel(const double *parti
 {
     __shared__ double ss[THREADS];
     double s = 0.0;
-    isti_tc::griddep_launch_dependents();
-    isti_tc::griddep_wait();
+    isti::dependents_may_launch();
+    isti::wait_for_prerequisites();
     for (size_t i = threadIdx.x; i < n_blocks; i += THREADS)
         s += partials[i];
     ss[threadIdx.x] = s;
@@ -701,10 +700,10 @@ isti_status isti_quality_rgba8(const void *a, const void *b, int32_t width, int3
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid((width + TW - 1) / TW, (height + TH - 1) / TH);
     // (every launch a programmatic dependent of what was before it)
-    cudaError_t e = isti_unet::launch_kernel(quality_tile_kernel, grid, Q_THREADS, 0, s, true, static_cast<const uint32_t *>(a),
+    cudaError_t e = isti::launch_after(true, quality_tile_kernel, grid, Q_THREADS, 0, s, static_cast<const uint32_t *>(a),
                                              static_cast<const uint32_t *>(b), width, height, static_cast<double *>(scratch), gw);
     if (e == cudaSuccess)
-        e = isti_unet::launch_kernel(quality_final_kernel, 1, THREADS, 0, s, true, static_cast<const double *>(scratch),
+        e = isti::launch_after(true, quality_final_kernel, 1, THREADS, 0, s, static_cast<const double *>(scratch),
                                      n_tiles(width, height), 3.0 * (double)width * (double)height, out);
     if (e != cudaSuccess)
         return isti::set_error(ISTI_ERR_CUDA, std::string("isti_quality_rgba8: ") + cudaGetErrorString(e));
@@ -740,10 +739,10 @@ isti_status isti_flip_rgba8(const void *test, const void *reference, int32_t wid
         return isti::set_error(ISTI_ERR_CUDA, std::string("isti_flip_rgba8: ") + cudaGetErrorString(attr_err));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid((width + FTW - 1) / FTW, (height + FTH - 1) / FTH);
-    cudaError_t e = isti_unet::launch_kernel(flip_tile_kernel, grid, THREADS, smem, s, true, static_cast<const uint32_t *>(test),
+    cudaError_t e = isti::launch_after(true, flip_tile_kernel, grid, THREADS, smem, s, static_cast<const uint32_t *>(test),
                                              static_cast<const uint32_t *>(reference), width, height, f, static_cast<double *>(scratch), out_map);
     if (e == cudaSuccess)
-        e = isti_unet::launch_kernel(flip_final_kernel, 1, THREADS, 0, s, true, static_cast<const double *>(scratch),
+        e = isti::launch_after(true, flip_final_kernel, 1, THREADS, 0, s, static_cast<const double *>(scratch),
                                      flip_tiles(width, height), (double)width * (double)height, out_mean);
     if (e != cudaSuccess)
         return isti::set_error(ISTI_ERR_CUDA, std::string("isti_flip_rgba8: ") + cudaGetErrorString(e));

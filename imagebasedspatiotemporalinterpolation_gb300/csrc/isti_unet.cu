@@ -229,7 +229,7 @@ isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, c
             const int grid = std::min(units, sm_count() * per_sm);
             cudaError_t e = smem_limit(row_conv_kernel<0>, smem);
             if (e == cudaSuccess)
-                e = launch_kernel(row_conv_kernel<0>, dim3((unsigned)grid), dim3(PCONV_THREADS), smem, stream, pdl, p, xmap);
+                e = isti::launch_after(pdl, row_conv_kernel<0>, dim3((unsigned)grid), dim3(PCONV_THREADS), smem, stream, p, xmap);
             if (e == cudaSuccess && head && head_fused)
                 *head_fused = true;
             return e == cudaSuccess ? ISTI_OK : cuda_fail(e, "isti_unet_conv launch");
@@ -253,13 +253,13 @@ isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, c
     {
         e = smem_limit(conv_kernel<9>, smem);
         if (e == cudaSuccess)
-            e = launch_kernel(conv_kernel<9>, dim3((unsigned)grid), dim3(PCONV_THREADS), smem, stream, pdl, p, xmap);
+            e = isti::launch_after(pdl, conv_kernel<9>, dim3((unsigned)grid), dim3(PCONV_THREADS), smem, stream, p, xmap);
     }
     else
     {
         e = smem_limit(conv_kernel<1>, smem);
         if (e == cudaSuccess)
-            e = launch_kernel(conv_kernel<1>, dim3((unsigned)grid), dim3(PCONV_THREADS), smem, stream, pdl, p, xmap);
+            e = isti::launch_after(pdl, conv_kernel<1>, dim3((unsigned)grid), dim3(PCONV_THREADS), smem, stream, p, xmap);
     }
     if (e == cudaSuccess)
         e = cudaGetLastError();
@@ -318,10 +318,10 @@ isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, 
     cudaError_t e = smem_limit(kernel, c.smem);
     if (e == cudaSuccess)
     {
-        e = launch_kernel(kernel, grid, dim3(WGRAD_THREADS), c.smem, stream, pdl, p, dymap, xmap);
+        e = isti::launch_after(pdl, kernel, grid, dim3(WGRAD_THREADS), c.smem, stream, p, dymap, xmap);
         const int nw = cout * taps * cin;
         if (e == cudaSuccess)
-            e = launch_kernel(wgrad_reduce_kernel, dim3((unsigned)((nw + (db ? cout : 0) + 31) / 32)), dim3(32, WREDUCE_PARTS), 0, stream, pdl,
+            e = isti::launch_after(pdl, wgrad_reduce_kernel, dim3((unsigned)((nw + (db ? cout : 0) + 31) / 32)), dim3(32, WREDUCE_PARTS), 0, stream,
                               (const float *)p.partial, (const float *)p.bpartial, c.splits, nw, cout, dw, db, accumulate);
     }
     if (e == cudaSuccess)

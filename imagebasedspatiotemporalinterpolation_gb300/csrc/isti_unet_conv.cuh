@@ -8,19 +8,21 @@
 // f32 masters [cout][tap][cin] (tap = 3 * (dy + 1) + (dx + 1) for 3x3, 0 for 1x1) and
 // packed to bf16 operand images by pack_kernel.
 //
-// conv_kernel (forward, and the data gradient with packed transposed weights): one CTA of
-// 128 threads computes a tile of 16 x 8 output pixels (M = 128) x all output channels
-// (N = cout <= 256) into TMEM.  The K loop runs over (tap, chunk of ck input channels)
-// stages through a ring in shared memory:
-//   warp 0, one thread: per stage, ck / 8 TMA boxes {8 channels, 16 x, 8 y} of the input at
-//     the tap's offset (zero fill outside the image = the convolution's zero padding) and
-//     one bulk copy of the stage's packed weights, completion on full[s];
-//   warp 1, one thread: waits full[s], issues ck / 16 tcgen05.mma (K = 16 each) and commits
-//     to empty[s], which frees the stage for the producer; after the last stage, commits
-//     to `done`;
-//   all four warps (epilogue): wait `done`, read their 32 TMEM lanes (= tile rows) with
-//     tcgen05.ld, add the bias, apply ReLU and/or the gradient mask (x > 0 of a saved
-//     activation), convert to bf16 and store the pixel's channels.
+// conv_kernel (forward, and the data gradient with packed transposed weights): persistent CTAs of
+// 192 threads, each computing tiles of 128 output pixels (16 x 8; 128 x 1 in 1x1 layers between
+// planes; M = 128) x all output channels (N = cout <= 256) into TMEM.  The K loop runs over (tap,
+// chunk of ck input channels) stages through a ring in shared memory; producer and MMA issuer are
+// whole warps in step, one elected lane executing the copies and MMAs (isti_tc.cuh):
+//   warp 0: per stage, one TMA box of ck channels x the tile's pixels of the input at the tap's
+//     offset (zero fill outside the image = the convolution's zero padding; NHWC without 5-D
+//     maps: ck / 8 boxes) and one bulk copy of the stage's packed weights, completion on full[s];
+//   warp 1: waits full[s], issues ck / 16 tcgen05.mma (K = 16 each) and commits to empty[s], which
+//     frees the stage for the producer; after a tile's last stage, commits to acc_full of its
+//     accumulator, one of two;
+//   warps 2-5 (epilogue): wait acc_full, read their 32 TMEM lanes (= tile rows) with tcgen05.ld,
+//     add the bias, apply ReLU and/or the gradient mask (x > 0 of a saved activation), convert to
+//     bf16, store the pixel's channels and free the accumulator, while the next tile goes into the
+//     other one.
 // Every mbarrier wait is bounded; on timeout the status word is set, the loops stop, the
 // producer waits (bounded) for the copies it issued, and TMEM is freed before returning.
 //
@@ -30,6 +32,7 @@
 // kernel adds the partials in a fixed order (deterministic).
 #pragma once
 
+#include "isti_pdl.cuh"
 #include "isti_tc.cuh"
 
 #include <cuda_bf16.h>
@@ -41,6 +44,8 @@
 namespace isti_unet
 {
 using namespace isti_tc;
+using isti::dependents_may_launch;
+using isti::wait_for_prerequisites;
 
 constexpr size_t SMEM_BUDGET = 200 * 1024; // shared memory of a CTA that has the SM to itself
 constexpr int TILE_W = 16, TILE_H = 8, TILE_M = TILE_W * TILE_H;
@@ -58,8 +63,8 @@ struct ConvParams
 {
     const __nv_bfloat16 *wpack; // packed weights: per stage ck x cout, K-major core matrices [ck/8][cout/8][8][8]
     const float *bias;          // cout, or null
-    const __nv_bfloat16 *mask;  // NHWC, cout channels: output *= (mask > 0); or null
-    __nv_bfloat16 *out;         // NHWC, cout channels
+    const __nv_bfloat16 *mask;  // cout channels: output *= (mask > 0); or null
+    __nv_bfloat16 *out;         // cout channels
     int32_t *status;
     int w, h, b;
     int cin, cout, ck;          // ck: input channels per stage (16 or 32)
@@ -292,12 +297,12 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     const uint32_t tmem = *tmem_slot;
     const int chunks = p.cin / p.ck;
     if (threadIdx.x == 0)
-        griddep_launch_dependents(); // the next layer may set up while this one runs
+        dependents_may_launch(); // the next layer may set up while this one runs
 
     if (warp == 0)
     {
         const uint32_t leader = elect_one();
-        griddep_wait(); // the previous layer's output is complete (every load below is later)
+        wait_for_prerequisites(); // the previous layer's output is complete (every load below is later)
         fence_proxy_async_global();
         uint32_t g = 0; // stages filled
         RingPos ring;
@@ -374,7 +379,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) conv_kernel(const __grid_con
     }
     else if (warp >= 2)
     {
-        griddep_wait(); // the mask is complete
+        wait_for_prerequisites(); // the mask is complete
         const int q = warp % 4; // the TMEM lane quadrant this warp may read
         const int m = q * 32 + lane, mx = m & ((1 << p.tile_shift) - 1), my = m >> p.tile_shift;
         UnitPos at(blockIdx.x, gridDim.x, p.tiles_x, p.tiles_y);
@@ -475,14 +480,14 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     const uint32_t tmem = *tmem_slot;
 
     if (threadIdx.x == 0)
-        griddep_launch_dependents(); // the next layer may set up while this one runs
+        dependents_may_launch(); // the next layer may set up while this one runs
     if (warp == 0)
     {
         const uint32_t leader = elect_one();
         mbar_expect_tx_if(leader, wbar, w_bytes);
         for (uint32_t o = 0; o < w_bytes; o += 32768u) // pieces of at most 32 KiB (the weights are complete, forward in isti_flownet.cu)
             bulk_load(leader, smem_u32(wsm) + o, reinterpret_cast<const uint8_t *>(p.wpack) + o, min(32768u, w_bytes - o), wbar);
-        griddep_wait(); // the previous layer's output is complete (every activation load below is later)
+        wait_for_prerequisites(); // the previous layer's output is complete (every activation load below is later)
         fence_proxy_async_global();
         uint32_t g = 0;
         RingPos pos;
@@ -553,7 +558,7 @@ __global__ void __launch_bounds__(PCONV_THREADS, 1) row_conv_kernel(const __grid
     }
     else if (warp >= 2)
     {
-        griddep_wait(); // the mask is complete
+        wait_for_prerequisites(); // the mask is complete
         const int q = warp % 4;
         const int m = q * 32 + lane;
         UnitPos at(blockIdx.x, gridDim.x, segs, p.h);
@@ -731,11 +736,11 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     const uint32_t tmem = *tmem_slot;
 
     if (threadIdx.x == 0)
-        griddep_launch_dependents();
+        dependents_may_launch();
     if (warp == 0)
     {
         const uint32_t leader = elect_one();
-        griddep_wait(); // dY and X are complete (every load below is later)
+        wait_for_prerequisites(); // dY and X are complete (every load below is later)
         fence_proxy_async_global();
         const uint32_t tx_bytes = (uint32_t)(boxes * p.box_chunks) * px_bytes + (uint32_t)(p.cin / 8) * b_rows_bytes;
         const int shift0 = mb0 * 16 / co_chunks, group0 = mb0 * 16 % co_chunks; // of the first box
@@ -818,7 +823,7 @@ __global__ void __launch_bounds__(WGRAD_THREADS) wgrad_kernel(const __grid_const
     // The scratch is one for all layers, and the kernels between let this one start before they
     // waited themselves: the reduction of the layer before may still read it.  (Warp 0's wait
     // orders a CTA's stores by way of its copies and products only where it has units.)
-    griddep_wait();
+    wait_for_prerequisites();
     const bool ok = mbar_wait(done, 0, p.status);
     tc_fence_after();
     if (ok)
@@ -865,8 +870,8 @@ __global__ void __launch_bounds__(32 * WREDUCE_PARTS) wgrad_reduce_kernel(const 
                                                                           float *dw, float *db, int accumulate)
 {
     __shared__ float part[WREDUCE_PARTS][32];
-    griddep_launch_dependents();
-    griddep_wait();
+    dependents_may_launch();
+    wait_for_prerequisites();
     const int i = blockIdx.x * 32 + threadIdx.x;
     const bool weight = i < n, used = weight || (db && i < n + nb);
     float s = 0.0f;

@@ -8,7 +8,6 @@
 
 #include <cstddef>
 #include <cstdint>
-#include <utility>
 
 namespace isti_unet
 {
@@ -26,32 +25,15 @@ struct ConvHead
 // (out and mask; dy of the weight gradient).
 constexpr int IN_PLANES = 1, OUT_PLANES = 2;
 
-// pdl: launch as a programmatic dependent of the previous kernel in `stream` (it prepares
-// while that kernel finishes; see griddep_wait in isti_tc.cuh).  It then reads wpack, bias and the
-// head before it waits: only behind a kernel that was itself launched after they were complete.  head: fuse that head into
+// pdl: launch as a programmatic dependent of the previous kernel in `stream` (it prepares while
+// that kernel finishes, isti_pdl.cuh).  It then reads wpack, bias and the head before it waits: only
+// behind a kernel that was itself launched after they were complete.  head: fuse that head into
 // the epilogue where the row-tile kernel runs the layer (then `out` is not written and
 // *head_fused is set); otherwise the layer runs as usual and *head_fused is cleared.
 isti_status conv_launch(int taps, const void *x, int n, int h, int w, int cin, const void *wpack, const float *bias, const void *mask, int relu,
                         void *out, int cout, int32_t *status, cudaStream_t stream, int planes = 0, bool pdl = false,
                         const ConvHead *head = nullptr, bool *head_fused = nullptr);
 
-// <<<grid, block, smem, stream>>> with, when `pdl`, the programmatic-dependent-launch
-// attribute; the kernel must call griddep_wait before it touches the previous kernel's data
-template <typename... K, typename... A>
-cudaError_t launch_kernel(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, A &&...args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = pdl ? attr : nullptr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-}
 // db (may be null): the bias gradient, the column sums of dy
 isti_status wgrad_launch(int taps, const void *dy, const void *x, int n, int h, int w, int cin, int cout, float *dw, float *db, int accumulate,
                          void *scratch, size_t scratch_bytes, int32_t *status, cudaStream_t stream, int planes = 0, bool pdl = false);

@@ -202,7 +202,8 @@ class Renderer:
 
     def render_pairs(self, jobs, chain: bool = False, stream=None) -> None:
         """isti_render_pairs: jobs = [(render_buffers, infos, frame_data), ...], the frames of
-        several keyframe pairs in one persistent launch; each job's result equals
+        several keyframe pairs in one call (many small pairs in one persistent launch, others as
+        batches one after the other); each job's result equals
         render_batch(render_buffers, infos, frame_data, chain)."""
         if not 1 <= len(jobs) <= native.MAX_PAIRS:
             raise ValueError(f"need 1..{native.MAX_PAIRS} keyframe pairs")

@@ -16,7 +16,7 @@ from imagebasedspatiotemporalinterpolation_gb300.scene import Sequence
 @pytest.mark.parametrize("source", ["isti_kernels.cuh", "isti_learned.cuh", "isti_batch.cuh", "isti_metrics.cu"])
 def test_no_read_only_loads(source):
     """Every image, table and intermediate of these kernels may have been written by a kernel that still ran
-    when they started (the rule beside griddepcontrol in isti_kernels.cuh)."""
+    when they started (the rule in isti_pdl.cuh)."""
     with open(os.path.join(_build.CSRC, source)) as f:
         code = re.sub(r"//[^\n]*", "", f.read())
     assert not re.findall(r"__ldg|__restrict__|ld\.global\.nc|__ldca", code)
