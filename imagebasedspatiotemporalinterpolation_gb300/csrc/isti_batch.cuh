@@ -101,7 +101,8 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
         ctrl[5] = 0u;
     }
     __syncthreads();
-    int round = 0;        // TMA rounds of this warp's barrier (its phase carries across units; -1: out of use)
+    int round = 0;        // TMA rounds of this warp's barrier (its phase carries across units)
+    bool marked = false;  // ctrl[5] as of the last reprojection unit (block-uniform)
     uint32_t slot = 0;    // ctrl word holding the current ticket
     // the segment of the current ticket; a block's tickets only grow, so the search resumes
     // where the previous unit's ended
@@ -126,8 +127,8 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
         }
         // once a wait has given up (status word set) the remaining units only count themselves
         // done: the call's outputs are void.  The word was read while the unit before this one ran, so
-        // the unit after one that gave up still runs here: reproj_block announces nothing on a barrier
-        // that is out of step (`round`) and leaves again (ctrl[5])
+        // the block in which a wait gave up would go on to one more reprojection unit and announce its
+        // tiles on barriers whose phase did not complete, which overruns their count: `marked` skips it
         const bool failed = ctrl[2 + slot] != 0;
         const uint32_t old_pair = seg_pair;
         while (t >= seg_end)
@@ -194,10 +195,12 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
                 for (uint32_t yy = threadIdx.y; yy < bp.splat_rows; yy += blockDim.y)
                     splat_pixel(p, view, x, y0 + yy);
             }
-            else
+            else if (!marked)
             {
                 const uint32_t bx = u % bpair.reproj_gx, by = u / bpair.reproj_gx;
                 reproj_block<SW, SI, MAV, REGS, 0, HOOK>(p, bpair.maps, bx, by, u, region, bars, round, *reinterpret_cast<volatile uint32_t *>(ctrl + 5));
+                // written before the barrier inside, and by no warp again before the one that ends this unit
+                marked = *reinterpret_cast<volatile uint32_t *>(ctrl + 5) != 0u;
             }
         }
         if (helper)

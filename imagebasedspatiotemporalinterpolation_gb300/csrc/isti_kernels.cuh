@@ -515,8 +515,7 @@ struct DirRes
 // Squared errors save the square root, but under the cap of 40 registers, which is for many views,
 // the freer schedule spills and the roots are faster (1080p, 3 frames, 6 views: 0.537 ms roots, 0.548
 // squared); under the other caps squares are (2 views 0.238 -> 0.222 ms; 7x7 window, 6 views 1.116 ->
-// 1.092 ms), and their kernels fit into 40 registers without spills where the view count is a constant
-// (reproj_regs).
+// 1.092 ms), also where a constant view count lets their kernels be built at 40 registers (reproj_regs).
 template <int REGS>
 constexpr bool SQUARED_ERRORS = !FAST_MATH && REGS != REPROJ_REGS_MANY_VIEWS;
 
@@ -835,10 +834,9 @@ __host__ __device__ __forceinline__ void window_keys(const unsigned long long *t
 // threads: the body of reproj_kernel, also run as a work unit of batch_kernel.  `maps`: the
 // views' key-tile tensor maps; `bars`: the warps' TMA completion barriers, initialised once per
 // thread block; `round`: TMA rounds this warp's barrier has completed so far (its phase carries
-// over from unit to unit, also across units whose tiles came by plain loads), or -1 once a wait of
-// this warp gave up: the barrier's phase did not complete then, and another arrival would overrun
-// its count, so the warp announces nothing more, in this unit or a later one; `aborted`: a
-// shared word, 0 when the block starts, that a warp whose wait for a key tile gave up sets to 1;
+// over from unit to unit, also across units whose tiles came by plain loads); `aborted`: a
+// shared word, 0 when the block starts, that a warp whose wait for a key tile gave up sets to 1
+// (the block's barriers are out of step then: it must not come here again);
 // `block_id`: the index the test hook `withhold_block` refers to, compiled in only where HOOK is
 // set.  Every thread returns together (early exits are block-uniform or come after the last
 // barrier).
@@ -884,7 +882,7 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
             const uint32_t y0 = yb + (uint32_t)rp * ROWS;
             tma_load_3d(tg, &maps[vw], xs, (int)(v.sy == 1 ? y0 : y0 / v.sy) - SW, k, bar);
         };
-        if (p.use_tma && round >= 0 && lane == 0)
+        if (p.use_tma && lane == 0)
             fetch(0, g0);
         // pixel2CS of the output pixels in the main view (the search target) and in this view (the error)
         const DevView &v0 = p.v[0];
@@ -913,14 +911,14 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
                 const int k = g0 + j, u = j * np + rp;
                 if (p.use_tma)
                 {
-                    // A warp whose copy did not arrive reads nothing more, starts no further copy (see
-                    // `round`) and marks the block, which then leaves after the barrier that ends phase 1,
-                    // writing nothing of this group (the mark is written before that barrier and read
-                    // after it, by every thread).
-                    arrived = round >= 0 && __all_sync(0xffffffffu, mbar_wait_bounded(bar, (uint32_t)(round & 1), p.status, p.wait_limit));
+                    // A warp whose copy did not arrive reads nothing more, starts no further copy (an
+                    // arrival on a barrier whose phase did not complete would overrun its count) and
+                    // marks the block, which then leaves after the barrier that ends phase 1, writing
+                    // nothing of this group (the mark is written before that barrier and read after it,
+                    // by every thread).
+                    arrived = __all_sync(0xffffffffu, mbar_wait_bounded(bar, (uint32_t)(round & 1), p.status, p.wait_limit));
                     if (!arrived)
                     {
-                        round = -1;
                         aborted = 1u;
                         break;
                     }
@@ -1073,9 +1071,9 @@ __device__ __forceinline__ void reproj_block(const FrameParams &p, const CUtenso
 }
 
 // Registers that reproj_kernel is built with under a cap, for a constant view count (nv; 0: known
-// at run time only).  With the view count a constant, the two-view kernel of the 3x3 window and
-// those of the 7x7 window fit into 40 registers without spills, and more resident warps make them
-// faster: 6 frames at 2064x2208, 2 views 0.728 -> 0.685 ms (32 registers: 0.728, spills); 3 frames
+// at run time only).  With the view count a constant, the two-view kernel of the 3x3 window fits
+// into 40 registers without spills and those of the 7x7 window with 22 spilled words, and more resident
+// warps make them faster: 6 frames at 2064x2208, 2 views 0.728 -> 0.685 ms (32 registers: 0.728, spills); 3 frames
 // at 1366x768, 4 views, 7x7 0.367 (56) -> 0.357 (48) -> 0.354 ms.
 constexpr int reproj_regs(int sw, int cap, int nv) { return nv != 0 && (sw == 3 || nv == 2) ? REPROJ_REGS_MANY_VIEWS : cap; }
 
