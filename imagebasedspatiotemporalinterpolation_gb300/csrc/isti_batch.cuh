@@ -102,7 +102,6 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
     }
     __syncthreads();
     int round = 0;        // TMA rounds of this warp's barrier (its phase carries across units)
-    bool marked = false;  // ctrl[5] as of the last reprojection unit (block-uniform)
     uint32_t slot = 0;    // ctrl word holding the current ticket
     // the segment of the current ticket; a block's tickets only grow, so the search resumes
     // where the previous unit's ended
@@ -126,9 +125,7 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
             status_seen = *(volatile int32_t *)bp.status;
         }
         // once a wait has given up (status word set) the remaining units only count themselves
-        // done: the call's outputs are void.  The word was read while the unit before this one ran, so
-        // the block in which a wait gave up would go on to one more reprojection unit and announce its
-        // tiles on barriers whose phase did not complete, which overruns their count: `marked` skips it
+        // done: the call's outputs are void
         const bool failed = ctrl[2 + slot] != 0;
         const uint32_t old_pair = seg_pair;
         while (t >= seg_end)
@@ -195,18 +192,20 @@ __global__ void __maxnreg__(REGS) batch_kernel(const __grid_constant__ BatchPara
                 for (uint32_t yy = threadIdx.y; yy < bp.splat_rows; yy += blockDim.y)
                     splat_pixel(p, view, x, y0 + yy);
             }
-            else if (!marked)
+            else
             {
                 const uint32_t bx = u % bpair.reproj_gx, by = u / bpair.reproj_gx;
                 reproj_block<SW, SI, MAV, REGS, 0, HOOK>(p, bpair.maps, bx, by, u, region, bars, round, *reinterpret_cast<volatile uint32_t *>(ctrl + 5));
-                // written before the barrier inside, and by no warp again before the one that ends this unit
-                marked = *reinterpret_cast<volatile uint32_t *>(ctrl + 5) != 0u;
             }
         }
         if (helper)
         {
             ctrl[slot ^ 1u] = next_t; // every thread read both entries before the previous barrier
-            ctrl[2 + (slot ^ 1u)] = (uint32_t)status_seen;
+            // The status was read when this unit started: where a wait of this very unit gave up, the
+            // block's own mark says so (set, if at all, before the barrier inside reproj_block).  The
+            // block would otherwise go on to another reprojection unit and announce its tiles on barriers
+            // whose phase did not complete, which overruns their count.
+            ctrl[2 + (slot ^ 1u)] = (uint32_t)status_seen | *reinterpret_cast<volatile uint32_t *>(ctrl + 5);
         }
         __syncthreads();
         // the unit's writes (every thread's, ordered by the barrier) are published by one
