@@ -784,9 +784,9 @@ cudaError_t launch_pairs_mode(int mode, int regs, const isti::BatchParams &bp, s
 // Whether isti_render_pairs renders its pairs as batches, one after the other, rather than in the
 // persistent launch.  A batch's kernels run at their own block shapes and registers (the persistent
 // kernel splats with the reprojection's) but cost a pair 12 us of launches; so the persistent launch
-// is left to many small pairs.  Per pair, persistent / batches: 32 pairs of 160x96 7.9 / 12.5 us (one
-// frame), 12.5 / 17.7 (three); of 320x180 25 / 15 and 40 / 28; 8 pairs of 96x64 8.5 / 14, 2 pairs
-// 24 / 19; 6 pairs of 1280x720 to 2064x2208, three frames, 508 / 329.
+// is left to many small pairs.  Per pair, persistent / batches: 32 pairs of 160x96 7.1 / 12.5 us (one
+// frame), 11.1 / 17.7 (three); of 320x180 25 / 15 and 40 / 28; 8 pairs of 96x64 8.5 / 14, 2 pairs
+// 24 / 19; 6 pairs of 1280x720 to 2064x2208, three frames, 500 / 328.
 bool pairs_as_batches(size_t source_pixels, int n_pairs)
 {
     return n_pairs <= 2 || source_pixels >= (size_t)50000 * n_pairs;
